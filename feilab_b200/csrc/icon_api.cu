@@ -207,8 +207,8 @@ struct NodeTables {
     int taps = 0;    // x taps with entries per node (14, or 8 for Kaiser-Bessel)
     float *phix = nullptr, *phiy = nullptr, *w = nullptr;
     int *ix0 = nullptr, *iy0 = nullptr, *row_off = nullptr, *ent_jt = nullptr, *ent_iy0 = nullptr;
-    unsigned short *ent_lb = nullptr;
-    float *ent_phiy = nullptr, *ent_pxy = nullptr;
+    unsigned short *ent_blk = nullptr, *ent_split = nullptr;
+    float *ent_phiy = nullptr, *ent_win = nullptr;
 };
 
 }  // namespace
@@ -289,6 +289,7 @@ struct icon_plan {
     float2 *fline = nullptr;
     size_t smem_x = 0, smem_y = 0, smem_ya = 0;
     int thr_x = 0, thr_y = 0, ex = 16, ey = 16;   // threads and values per thread of x- and y-pass FFTs
+    int thr_ya = 0;                               // threads of the adjoint y-pass
     // tracing: events around every launch while enabled
     bool trace = false;
     long long launches = 0;
@@ -332,7 +333,7 @@ struct icon_plan {
         }
         g.phix = t.phix; g.phiy = t.phiy; g.ix0 = t.ix0; g.iy0 = t.iy0;
         g.cx = cx; g.cy = cy; g.rcx = rcx; g.rcy = rcy; g.row_off = t.row_off; g.ent_jt = t.ent_jt; g.ent_iy0 = t.ent_iy0;
-        g.ent_lb = t.ent_lb; g.ent_phiy = t.ent_phiy; g.ent_pxy = t.ent_pxy;
+        g.ent_blk = t.ent_blk; g.ent_split = t.ent_split; g.ent_phiy = t.ent_phiy; g.ent_win = t.ent_win;
         g.tw0 = tw0; g.tw0h = tw0h; g.tw1 = tw1;
         g.Kt = Kt;
         g.kstride = kt_groups > 1 ? (size_t)n0 * n1t : 0;
@@ -546,17 +547,27 @@ icon_status build_tables(icon_plan *p, const float *xy, const float *w, int M, N
             ky2[a + i] = ky[order[i]];
         }
     }
-    // Per row, the entries whose first rotated y tap r0 = iy0 + n1/2 + 8 is
-    // below v (v = 0..n1+16), relative to the row's first entry.
-    const int ldl = icon::lb_ld(p->n1), r0ofs = p->n1 / 2 + icon::kHalo;
-    std::vector<unsigned short> lb((size_t)n0 * ldl);
+    // Per row, for the adjoint gather: the entries whose first non-zero tap's
+    // buffer row iy0 + tlo + n1/2 + 8 lies below each block of ph rows,
+    // relative to the row's first entry, and the block ranges of the
+    // gather's warps, cut at equal shares of entries + blocks (a block's
+    // store and bounds cost about as much as an entry).
+    const int ph = icon::ywin_ph(p->B), nblk = icon::ywin_blocks(p->n1, p->B), warps = p->thr_ya / 32;
+    const int r0ofs = p->n1 / 2 + icon::kHalo;
+    std::vector<unsigned short> eblk((size_t)n0 * (nblk + 1)), split((size_t)n0 * (warps + 1));
     for (int x = 0; x < n0; ++x) {
         int a = cnt[x], c = cnt[x + 1];
         if (c - a > 65535) return fail(ICON_ERR_INVALID, "more than 65535 window entries on one grid row");
         int e = a;
-        for (int v = 0; v < ldl; ++v) {
-            while (e < c && ky2[e] + r0ofs < v) ++e;
-            lb[(size_t)x * ldl + v] = (unsigned short)(e - a);
+        unsigned short *off = &eblk[(size_t)x * (nblk + 1)], *cut = &split[(size_t)x * (warps + 1)];
+        for (int v = 0; v <= nblk; ++v) {
+            while (e < c && ky2[e] + r0ofs + tlo < v * ph) ++e;
+            off[v] = (unsigned short)(e - a);
+        }
+        const long long total = (long long)(c - a) + nblk;
+        for (int w = 0, v = 0; w <= warps; ++w) {
+            while (v < nblk && (long long)(off[v] + v) * warps < total * w) ++v;
+            cut[w] = (unsigned short)(w == warps ? nblk : v);
         }
         if (c > a && (ky2[a] + r0ofs < 0 || ky2[c - 1] + r0ofs + kTaps > p->n1 + 2 * icon::kHalo))
             return fail(ICON_ERR_INVALID, "window taps outside the rotated y buffer");
@@ -569,10 +580,12 @@ icon_status build_tables(icon_plan *p, const float *xy, const float *w, int M, N
     ICON_TRY(p->arena.upload(&t.row_off, cnt.data(), (size_t)n0 + 1));
     ICON_TRY(p->arena.upload(&t.ent_jt, jt2.data(), E));
     ICON_TRY(p->arena.upload(&t.ent_iy0, ky2.data(), E));
-    ICON_TRY(p->arena.upload(&t.ent_lb, lb.data(), lb.size()));
+    ICON_TRY(p->arena.upload(&t.ent_blk, eblk.data(), eblk.size()));
+    ICON_TRY(p->arena.upload(&t.ent_split, split.data(), split.size()));
     ICON_TRY(p->arena.alloc(&t.ent_phiy, E * icon::kLdPhiy));
-    ICON_TRY(p->arena.alloc(&t.ent_pxy, E * icon::kLdPhiy));
-    icon::k_entry_tables<<<(unsigned)((E + 255) / 256), 256>>>(t.ent_jt, (int)E, t.phiy, t.phix, t.ent_phiy, t.ent_pxy);
+    ICON_TRY(p->arena.alloc(&t.ent_win, (E + icon::kAdjChunk) * icon::ywin_lp(p->B)));   // staged in whole chunks
+    icon::k_entry_tables<<<(unsigned)((E + 255) / 256), 256>>>(t.ent_jt, t.ent_iy0, (int)E, t.phiy, t.phix, tlo, thi, r0ofs,
+                                                               p->B, t.ent_phiy, t.ent_win);
     ICON_CUDA(cudaGetLastError());
     ICON_TRY(p->arena.upload(&t.w, w, (size_t)M));
     return ICON_OK;
@@ -653,7 +666,7 @@ icon_status launch_adjoint(icon_plan *p, const float2 *f_int, int G, int mode, f
     xa.N0 = p->N0; xa.N1 = p->N1; xa.n0 = p->n0; xa.tw0 = p->tw0; xa.G1 = p->G1; xa.rhat = out_int;
     xa.Ahwb = p->Ahwb; xa.part_rtr = p->part_rtr; xa.rcx = p->rcx; xa.rcy = p->rcy; xa.resid = mode == 0 ? 0 : 1;
     WITH_B(p->B,
-        LAUNCH_B(p, K_YA, st, sb.ya * slots, L::ypass_adj(p->ey, gy, p->thr_y, p->smem_ya, st, g, f_int, p->G1));
+        LAUNCH_B(p, K_YA, st, sb.ya * slots, L::ypass_adj(p->ey, gy, p->thr_ya, p->smem_ya, st, g, f_int, p->G1));
         if (p->xt_ok) {
             LAUNCH_B(p, K_XA, st, (mode == 0 ? sb.xa_plain : sb.xa_resid) * slots, L::xtoep(2, st, G, xa));
         } else {
@@ -1052,7 +1065,6 @@ static icon_status plan_create_impl(const icon_geometry *geo, int group, icon_pl
     p->w.resize(p->M);
     px2d(nx, nz, p->th_neg.data(), p->xy.data());
     weights(nx, nz, p->th_neg.data(), p->w.data());
-    ICON_TRY(build_tables(p.get(), p->xy.data(), p->w.data(), p->M, p->nodes));
     std::vector<float> cx = deapod(p->N0, p->n0, p->b0, p->kb0), cy = deapod(p->N1, p->n1, p->b1, p->kb1);
     ICON_TRY(p->arena.upload(&p->cx, cx.data(), cx.size()));
     ICON_TRY(p->arena.upload(&p->cy, cy.data(), cy.size()));
@@ -1096,7 +1108,9 @@ static icon_status plan_create_impl(const icon_geometry *geo, int group, icon_pl
     p->thr_y = p->n1 * B / p->ey;
     p->smem_x = (size_t)p->n0 * B * sizeof(float2);
     p->smem_y = icon::ypass_fwd_smem(p->n1, B);
-    p->smem_ya = icon::ypass_adj_smem(p->n1, B);
+    p->thr_ya = icon::yadj_threads(icon::yadj4_fits(p->n1) ? p->n1 / 32 * B : p->thr_y);
+    p->smem_ya = icon::ypass_adj_smem(p->n1, B, p->thr_ya);
+    ICON_TRY(build_tables(p.get(), p->xy.data(), p->w.data(), p->M, p->nodes));
     // Toeplitz y-length: a circular convolution of the N1 rows with a kernel
     // of support 2 N1 - 1 needs 2 N1 - 1 points; the four-step kernel takes
     // 32 R for R in {4, 6, 8, 10, 12, 16, 20, 24, 32}.  ICON_TOEP_POW2=1 keeps

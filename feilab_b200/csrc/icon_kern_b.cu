@@ -164,12 +164,16 @@ template <int B>
 void Launch<B>::ypass_adj(int E, dim3 grid, int threads, size_t smem, cudaStream_t st, const Geo &g, const float2 *f,
                           float2 *G1)
 {
-    // The band loop needs a full warp; tiny FFTs have fewer threads than that.
-    bool guard = threads < 32;
-    if (guard) threads = 32;
-    if (E == 32) k_ypass_adj<B, 32, false><<<grid, threads, smem, st>>>(g, f, G1);
-    else if (!guard) k_ypass_adj<B, 16, false><<<grid, threads, smem, st>>>(g, f, G1);
-    else k_ypass_adj<B, 16, true><<<grid, threads, smem, st>>>(g, f, G1);
+    switch (yadj4_fits(g.n1) ? g.n1 / 32 : 0) {
+    case 4: k_yadj4<B, 4><<<grid, threads, smem, st>>>(g, f, G1); break;
+    case 8: k_yadj4<B, 8><<<grid, threads, smem, st>>>(g, f, G1); break;
+    case 16: k_yadj4<B, 16><<<grid, threads, smem, st>>>(g, f, G1); break;
+    case 32: k_yadj4<B, 32><<<grid, threads, smem, st>>>(g, f, G1); break;
+    default:
+        if (E == 32) k_ypass_adj<B, 32, false><<<grid, threads, smem, st>>>(g, f, G1);
+        else if (threads == g.n1 * B / 16) k_ypass_adj<B, 16, false><<<grid, threads, smem, st>>>(g, f, G1);
+        else k_ypass_adj<B, 16, true><<<grid, threads, smem, st>>>(g, f, G1);
+    }
 }
 
 template <int B>
@@ -268,6 +272,10 @@ cudaError_t Launch<B>::set_smem(int ex, int ey, size_t, size_t, size_t, size_t, 
     set((const void *)k_ypass_fwd<B, 16, true>);
     set((const void *)k_ypass_adj<B, 16, false>);
     set((const void *)k_ypass_adj<B, 16, true>);
+    set((const void *)k_yadj4<B, 4>);
+    set((const void *)k_yadj4<B, 8>);
+    set((const void *)k_yadj4<B, 16>);
+    set((const void *)k_yadj4<B, 32>);
     set((const void *)k_ypass_toep<B, 16>);
     set((const void *)k_ypass_toep_quad<B, 16>);
     set((const void *)k_ytoep4<B, 4, 0>);

@@ -55,9 +55,10 @@ struct Geo {
     const int *row_off;    // [n0+1] entry range of every grid row x
     const int *ent_jt;     // [M*14] entry: node*16 + x tap, sorted by (row, iy0, node)
     const int *ent_iy0;    // [M*14] iy0 of the entry's node (sort key within a row)
-    const unsigned short *ent_lb;   // [n0][n1+17] per-row lower bounds of r0 (k_ypass_adj)
+    const unsigned short *ent_blk;  // [n0][ywin_blocks+1] entries of a row below each block of buffer rows (adjoint gather)
+    const unsigned short *ent_split; // [n0][ywin_warps+1] block range of each warp of the adjoint gather
     const float *ent_phiy; // [M*14][16] phiy of the entry's node, in entry order
-    const float *ent_pxy;  // [M*14][16] phix[j][t0] * phiy[j][t1], in entry order
+    const float *ent_win;  // [M*14][YWin::LP] phix[j][t0] * phiy[j][t1] laid out on the entry's blocks (YWin)
     const float2 *tw0;     // [n0] exp(-2 pi i q / n0)
     const float2 *tw0h;    // [n0/2] exp(-2 pi i q / (n0/2))
     const float2 *tw1;     // [n1] exp(-2 pi i q / n1)
@@ -72,6 +73,16 @@ struct Geo1 {
     const float *phi1;     // [nx][14]
     const int *i10;        // [nx] first tap, unwrapped, nondecreasing in k
 };
+
+// Layout of the adjoint gather (yadj_gather) for groups of B slices: a warp's
+// lanes are ywin_ph(B) neighbouring buffer rows times B slices (two slices a
+// lane for B = 8), and an entry's window, starting anywhere within a block of
+// ph rows, covers at most nr blocks.
+__host__ __device__ constexpr int ywin_ph(int B) { return B >= 4 ? 8 : B == 2 ? 16 : 32; }
+__host__ __device__ constexpr int ywin_nr(int B) { return B >= 4 ? 3 : 2; }
+__host__ __device__ constexpr int ywin_lp(int B) { return ywin_ph(B) * ywin_nr(B); }
+__host__ __device__ constexpr int ywin_pos(int ph, int p, int k) { return k < 2 ? 2 * p + k : 2 * ph + p; }
+__host__ __device__ constexpr int ywin_blocks(int n1, int B) { return (n1 + 2 * kHalo + ywin_ph(B) - 1) / ywin_ph(B); }
 
 #ifndef ICON_KERNELS_TEMPLATES_ONLY
 // ------------------------------------------------------------- tables ----
@@ -107,21 +118,28 @@ __global__ void k_window(const float *__restrict__ x, int stride, int M, int n, 
 
 // Window values copied into entry order (entry e = node j, x tap t0), so the
 // y-passes read them as contiguous streams: ephiy[e] = phiy[j] (16 floats)
-// and epxy[e][t1] = phix[j][t0] * phiy[j][t1], the product the reference's
-// adjoint CSR stores per grid point and node (NU:44-218).
-__global__ void k_entry_tables(const int *__restrict__ jt, int E, const float *__restrict__ phiy,
-                               const float *__restrict__ phix, float *__restrict__ ephiy, float *__restrict__ epxy)
+// and ewin[e], the products phix[j][t0] * phiy[j][t1] that the reference's
+// adjoint CSR stores per grid point and node (NU:44-218), placed on the
+// blocks of ph buffer rows that the entry's window covers (YWin): the value
+// of row blk*ph + p + ph*k, zero where no tap falls.
+__global__ void k_entry_tables(const int *__restrict__ jt, const int *__restrict__ iy0, int E,
+                               const float *__restrict__ phiy, const float *__restrict__ phix, int tlo, int thi,
+                               int r0ofs, int B, float *__restrict__ ephiy, float *__restrict__ ewin)
 {
     int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= E) return;
     int v = jt[e], j = v >> 4, t0 = v & 15;
     const float px = phix[(size_t)j * kTaps + t0];
 #pragma unroll
-    for (int t = 0; t < kLdPhiy; ++t) {
-        float py = phiy[(size_t)j * kLdPhiy + t];
-        ephiy[(size_t)e * kLdPhiy + t] = py;
-        epxy[(size_t)e * kLdPhiy + t] = px * py;
-    }
+    for (int t = 0; t < kLdPhiy; ++t) ephiy[(size_t)e * kLdPhiy + t] = phiy[(size_t)j * kLdPhiy + t];
+    const int ph = ywin_ph(B), nr = ywin_nr(B), lp = ywin_lp(B);
+    const int o = (iy0[e] + r0ofs + tlo) & (ph - 1);
+    for (int p = 0; p < ph; ++p)
+        for (int k = 0; k < nr; ++k) {
+            const int t = tlo + p + ph * k - o;
+            ewin[(size_t)e * lp + ywin_pos(ph, p, k)] =
+                (t >= tlo && t <= thi) ? px * phiy[(size_t)j * kLdPhiy + t] : 0.f;
+        }
 }
 
 #endif  // ICON_KERNELS_TEMPLATES_ONLY
@@ -534,193 +552,226 @@ __device__ __forceinline__ int lower_bound_s(const int *key, int lo, int hi, int
     return lo;
 }
 
-// Entries of a row staged at a time by the adjoint gather, and the padded
-// stride of a staged phiy window (so that neighbouring windows fall in
-// different shared-memory banks).
-constexpr int kChunk = 304;
-constexpr int kLdPs = 20;
-
-// Entries of grid row x whose first y tap r0 (in the rotated buffer with a
-// halo of kHalo rows on each side, r0 = iy0 + n1/2 + kHalo) is below v, for
-// v = 0..n1+16: [x][lb_ld] counts relative to the row's first entry, rows
-// padded to 16 bytes.
-__host__ __device__ inline int lb_ld(int n1) { return (n1 + 2 * kHalo + 1 + 7) & ~7; }
-
-// Shared-memory layout of k_ypass_adj.  Two chunk buffers of staged entries
-// (f values, phix*phiy window, iy0) and the row's lower-bound table are live
-// while the rows are gathered into registers; the rotated row (padded
-// stride) is written after the last chunk and shares the same bytes.
-__host__ __device__ inline size_t ypass_adj_chunk_bytes(int B)
-{
-    size_t sb = (B == 8) ? 10 : (B == 4) ? 6 : B;
-    return (size_t)kChunk * (sb * sizeof(float2) + kLdPs * sizeof(float) + sizeof(int));
-}
-__host__ __device__ inline size_t ypass_adj_region(int n1, int B)
-{
-    size_t sb = (B == 8) ? 10 : (B == 4) ? 6 : B;
-    size_t row = (size_t)n1 * sb * sizeof(float2);
-    size_t gather = 2 * ypass_adj_chunk_bytes(B) + (((size_t)lb_ld(n1) * sizeof(unsigned short) + 15) & ~(size_t)15);
-    return row > gather ? row : gather;
-}
-// The region above plus the FFT's twiddle table behind it.
-__host__ __device__ inline size_t ypass_adj_smem(int n1, int B)
-{
-    return ypass_adj_region(n1, B) + ypass_tw_bytes(n1);
-}
-
-// Adds the staged entries covering buffer rows i0 .. i0+R-1 (r0 in
-// [i0 - 13, i0 + R - 1]) to acc[k] of row i0 + k: entry e puts
-// (phix * phiy)_e[i0 + k - r0_e] * f_e on row i0 + k when that tap is in
-// 0..13.  Rs holds iy0 (r0 = iy0 + r0ofs); lb is the row's lower-bound
-// table (last index lbmax) and off the index of the chunk's first entry.
-template <int B, int SB, int R>
-__device__ __forceinline__ void gather_rows(int i0, int r0ofs, const unsigned short *lb, int lbmax, int off, int cn,
-                                            const float2 *Qs, const float *Ps, const int *Rs, float2 (&acc)[R][B],
-                                            int tlo, int thi)
-{
-    // lb[lbmax] counts every entry of the row, so clamping an index past it
-    // (alias ranges of wide thread strips) is exact.  Only taps tlo..thi of a
-    // window can be non-zero, so the entries with r0 in [i0 - thi, i0 + R - 1 - tlo]
-    // are the ones that reach these rows.
-    int lo = min(max((int)lb[min(max(i0 - thi, 0), lbmax)] - off, 0), cn);
-    int hi = min(max((int)lb[min(max(i0 + R - tlo, 0), lbmax)] - off, 0), cn);
-    const int iu = i0 - r0ofs;
-    for (int e = lo; e < hi; ++e) {
-        const int t0 = iu - Rs[e];        // tap of row i0; row i0 + k uses t0 + k
-        const float *pe = Ps + e * kLdPs;
-        float p[R];
-#pragma unroll
-        for (int k = 0; k < R; ++k) p[k] = ((unsigned)(t0 + k) < (unsigned)kTaps) ? pe[t0 + k] : 0.f;
-        float2 q[B];
-        load_b<B>(Qs + e * SB, q);
-#pragma unroll
-        for (int k = 0; k < R; ++k) {
-            const float2 pp = make_float2(p[k], p[k]);
-#pragma unroll
-            for (int b = 0; b < B; ++b) acc[k][b] = fma2(q[b], pp, acc[k][b]);
-        }
-    }
-}
-
-
 // -------------------------------------------------------------- K2T ----
 // Adjoint y-pass.  Entry e (node j, x tap t0) of row x adds
 // phiy[j][t1] * phix[j][t0] * f_j to the rotated buffer row r0_e + t1,
-// t1 = 0..13; the reference sums the same terms per grid point through its
-// host-built CSR (NU:1078-1102).  Here a thread owns whole buffer rows and
-// gathers: entries are sorted by r0, so those covering row i are the
-// contiguous range r0 in [i - 13, i], read from the precomputed lower-bound
-// table.  The 8 halo rows on each side alias rows n-8..n-1 and 0..7, so
-// those rows also gather the range of their alias.  Entries are copied in
-// chunks with cp.async (f_j, the phix*phiy window, iy0), the next chunk in
-// flight while the current one is gathered; a thread keeps its rows' sums in
-// registers across chunks, so every row gets its terms in a fixed order, with
-// no atomics.  The sums then go to the rotated row buffer and the inverse FFT
-// along y (NU:1203) reads the rotated row, and its last pass writes the rows
-// Y < N1 of the crop (NU:1104-1121: y = (Y + n1 - N1/2) % n1) straight to
-// G1[x][Y][b].  blockDim.x is max(32, n1*B/E); GUARD when that is more than
-// the FFT's n1*B/E threads.
+// r0 = iy0 + n1/2 + kHalo, t1 = 0..13; the reference sums the same terms per
+// grid point through its host-built CSR (NU:1078-1102).
+//
+// The gather (yadj_gather) has 14 x 14 products per node and slice and is
+// bound by latency and issue.  The row's entries are sorted by r0.  A warp
+// owns a range of blocks of PH buffer rows and walks the entries that reach
+// them once, in order, keeping the NR blocks that the current entry can cover
+// in registers (lane = row of the block x slice): per entry one load of f, NR
+// window values and NR multiply-adds per slice, no test of the window's bounds
+// (ent_win holds zeros there), no atomics, and a block is stored once, when no
+// later entry can reach it.  Ranges are cut at plan creation so that warps get
+// equal shares of entries (rows near x = 0 hold all their entries in a few
+// buffer rows).  Each warp stages its own entries by cp.async, a few chunks
+// deep, so the gather has no block barrier.  Every row gets its terms in the
+// order of the entries.
+// Measured, against chunks staged and gathered by the whole block in two-row
+// strips with a shared-memory FFT behind them: 256 x 128, 61 tilts, 32 slices
+// 167 -> 74 us; 2048 x 400, Kaiser-Bessel, 16 slices 827 -> 441 us; 1024 x
+// 300, 61 tilts, 128 slices 1.84 -> 1.65 ms.  Slower: values loaded straight
+// into registers eight entries ahead (1.8x), one flat loop over the entries
+// with a test for a new block at each (1.2x).
+
+// Grid row of the i-th CTA along blockIdx.y: 0, n0 - 1, 1, n0 - 2, ... .  The
+// rows near x = 0, whose few buffer rows keep few warps busy, start first and
+// do not end the launch.
+__device__ __forceinline__ int yadj_row(int i, int n0) { return (i & 1) ? n0 - ((i + 1) >> 1) : i >> 1; }
+
+template <int B>
+struct YWin {
+    static constexpr int SPL = B == 8 ? 2 : 1;        // slices per lane
+    static constexpr int LPS = B / SPL;               // lanes per row
+    static constexpr int PH = ywin_ph(B), NR = ywin_nr(B), LP = ywin_lp(B);
+    static_assert(LPS * PH == 32, "a warp covers one block");
+};
+
+// Threads of the adjoint y-pass for rows of n1: the FFT's, at least two warps.
+__host__ __device__ constexpr int yadj_threads(int fft_threads) { return fft_threads < 64 ? 64 : fft_threads; }
+// Entries per staged chunk, and chunks in flight per warp: two CTAs per SM for
+// the 1024-point rows of 8-slice groups, and within a block's shared memory
+// for the longest rows.
+constexpr int kAdjChunk = 8;
+__host__ __device__ constexpr int yadj_stages(int threads) { return threads <= 256 ? 3 : 2; }
+__host__ __device__ constexpr int yadj_chunk_bytes(int B)
+{
+    return kAdjChunk * (ywin_lp(B) * (int)sizeof(float) + B * (int)sizeof(float2));
+}
+__host__ __device__ constexpr size_t yadj_rows_bytes(int n1, int B)
+{
+    return (size_t)ywin_blocks(n1, B) * ywin_ph(B) * B * sizeof(float2);
+}
+// Rows, twiddle table, the warps' staged chunks.
+__host__ __device__ inline size_t ypass_adj_smem(int n1, int B, int threads)
+{
+    return yadj_rows_bytes(n1, B) + ypass_tw_bytes(n1) +
+           (size_t)(threads / 32) * yadj_stages(threads) * yadj_chunk_bytes(B);
+}
+
+// Gathers row x's entries into rows[ywin_blocks * PH][B] (every row written)
+// and adds the halo rows to the rows they alias.  All threads of the block
+// take part; ends with a block barrier.
+template <int B, int ST>
+__device__ __forceinline__ void yadj_gather(const Geo &g, int x, const float2 *fg, float2 *rows, char *stage)
+{
+    using Y = YWin<B>;
+    constexpr int PH = Y::PH, NR = Y::NR, LP = Y::LP, SPL = Y::SPL, CH = kAdjChunk, CB = yadj_chunk_bytes(B);
+    constexpr int C = B >= 2 ? B / 2 : 1;            // pieces of f_j
+    const int T = blockDim.x, W = T >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n = g.n1, nblk = ywin_blocks(n, B);
+    const int sl = lane % Y::LPS, ph = lane / Y::LPS;
+    const unsigned short *boff = g.ent_blk + (size_t)x * (nblk + 1);
+    const int b0 = g.ent_split[x * (W + 1) + warp], b1 = g.ent_split[x * (W + 1) + warp + 1];
+    const int e0 = g.row_off[x];
+    const int bs = max(b0 - (NR - 1), 0);            // windows of earlier blocks reach into the first ones
+    const int es = boff[bs], ee = b1 > b0 ? boff[b1] : es;
+    char *const buf = stage + warp * ST * CB;
+    // Node of this lane's piece of f in the chunk from entry c0 on (entries
+    // past ee repeat the last node).
+    const int *jt = g.ent_jt + e0 + lane / C;
+    auto node_of = [&](int c0) { return __ldg(jt + min(c0, max(ee - 1 - lane / C, 0))) >> 4; };
+    // Entries c0 .. c0+7 into buffer s, j their nodes; the windows read on past
+    // ee (the table is padded by a chunk).
+    const float *win = g.ent_win + (size_t)(e0 + es) * LP + 4 * lane;   // of the next chunk to issue
+    auto issue = [&](bool on, int s, int j) {
+        if (on) {
+            float *P = reinterpret_cast<float *>(buf + s * CB);
+            float2 *Q = reinterpret_cast<float2 *>(P + CH * LP);
+#pragma unroll
+            for (int i = 0; i < CH * LP / 4; i += 32)
+                if (CH * LP / 4 - i >= 32 || lane < CH * LP / 4 - i) cp_async<16>(P + 4 * (i + lane), win + 4 * i);
+            if (CH * C == 32 || lane < CH * C) {
+                if constexpr (B >= 2) cp_async<16>(Q + 2 * lane, fg + (size_t)j * B + 2 * (lane % C));
+                else cp_async<8>(Q + lane, fg + j);
+            }
+        }
+        win += CH * LP;
+        cp_async_commit();
+    };
+    int jn;                                          // nodes of the next chunk to issue, loaded a chunk ahead
+    {
+        int js[ST];
+#pragma unroll
+        for (int s = 0; s < ST; ++s) js[s] = node_of(es + s * CH);
+        jn = node_of(es + ST * CH);
+#pragma unroll
+        for (int s = 0; s < ST; ++s) issue(es + s * CH < ee, s, js[s]);
+    }
+    cp_async_wait<ST - 1>();
+    __syncwarp();
+    float2 acc[NR][SPL];
+#pragma unroll
+    for (int k = 0; k < NR; ++k)
+#pragma unroll
+        for (int q = 0; q < SPL; ++q) acc[k][q] = make_float2(0.f, 0.f);
+    int cb = es, cur = 0, left = CH;                 // staged chunk: first entry, buffer, entries not yet summed
+    int done = es;                                   // entries summed when the block's are
+    const float *pe = reinterpret_cast<const float *>(buf) + 2 * ph;    // next entry's window values and f
+    const float2 *qe = reinterpret_cast<const float2 *>(buf + CH * LP * 4) + sl * SPL;
+    int hv = 0;                                      // this lane's block end of the current 32 blocks
+    // One block, its rows in acc[S], the next blocks' in acc[S+1..].
+    auto step = [&](auto Sc, int blk) {
+        constexpr int S = decltype(Sc)::value;
+        auto add = [&](auto Nc) {                    // the next N entries
+            constexpr int N = decltype(Nc)::value;
+            float2 p[N], q[N][SPL];
+            float p2[N];
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+                p[i] = *reinterpret_cast<const float2 *>(pe + i * LP);
+                p2[i] = NR == 3 ? pe[i * LP + 2 * PH - ph] : 0.f;
+                load_b<SPL>(qe + i * B, q[i]);
+            }
+#pragma unroll
+            for (int i = 0; i < N; ++i)
+#pragma unroll
+                for (int v = 0; v < SPL; ++v) {
+                    float2 &a0 = acc[S % NR][v], &a1 = acc[(S + 1) % NR][v], &a2 = acc[(S + NR - 1) % NR][v];
+                    a0 = make_float2(fmaf(q[i][v].x, p[i].x, a0.x), fmaf(q[i][v].y, p[i].x, a0.y));
+                    a1 = make_float2(fmaf(q[i][v].x, p[i].y, a1.x), fmaf(q[i][v].y, p[i].y, a1.y));
+                    if (NR == 3) a2 = make_float2(fmaf(q[i][v].x, p2[i], a2.x), fmaf(q[i][v].y, p2[i], a2.y));
+                }
+            pe += N * LP;
+            qe += N * B;
+        };
+        const int rel = (blk - bs) & 31;
+        if (rel == 0) hv = boff[min(blk + lane + 1, nblk)];
+        const int hi = __shfl_sync(0xffffffffu, hv, rel);
+        int m = hi - done;
+        done = hi;
+        while (m > 0) {
+            if (left == 0) {                         // next chunk: refill this buffer, wait for the next one
+                __syncwarp();
+                issue(cb + ST * CH < ee, cur, jn);
+                jn = node_of(cb + (ST + 1) * CH);
+                cp_async_wait<ST - 1>();
+                __syncwarp();
+                cb += CH;
+                cur = cur + 1 == ST ? 0 : cur + 1;
+                left = CH;
+                pe = reinterpret_cast<const float *>(buf + cur * CB) + 2 * ph;
+                qe = reinterpret_cast<const float2 *>(buf + cur * CB + CH * LP * 4) + sl * SPL;
+            }
+            int k = min(m, left);
+            m -= k;
+            left -= k;
+#pragma unroll 1
+            for (; k >= 4; k -= 4) add(std::integral_constant<int, 4>{});
+            if (k & 2) add(std::integral_constant<int, 2>{});
+            if (k & 1) add(std::integral_constant<int, 1>{});
+        }
+        if (blk >= b0) store_b<SPL>(rows + (size_t)(blk * PH + ph) * B + sl * SPL, acc[S % NR]);
+#pragma unroll
+        for (int v = 0; v < SPL; ++v) acc[S % NR][v] = make_float2(0.f, 0.f);
+    };
+    for (int blk = bs; blk < b1; blk += NR) {
+        step(std::integral_constant<int, 0>{}, blk);
+        if (blk + 1 < b1) step(std::integral_constant<int, 1>{}, blk + 1);
+        if (NR == 3 && blk + 2 < b1) step(std::integral_constant<int, 2>{}, blk + 2);
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    // Halo rows 0..7 and n+8..n+15 alias rows n..n+7 and 8..15.
+    for (int i = threadIdx.x; i < 2 * kHalo * B; i += T) {
+        const int r = i / B, b = i - r * B;
+        float2 *to = rows + (size_t)(r < kHalo ? n + r : r) * B + b;
+        const float2 v = rows[(size_t)(r < kHalo ? r : n + r) * B + b];
+        *to = make_float2(to->x + v.x, to->y + v.y);
+    }
+    __syncthreads();
+}
+
+// Gather, then the inverse FFT along y (NU:1203) of the rotated rows by the
+// shared-memory FFT; its last pass writes the rows Y < N1 of the crop
+// (NU:1104-1121: y = (Y + n1 - N1/2) % n1) straight to G1[x][Y][b].  For the
+// lengths that k_yadj4 does not take; GUARD when the block has more than the
+// FFT's n1*B/E threads (the short ones).
 template <int B, int E, bool GUARD>
 __global__ void FFT_BOUNDS(E) k_ypass_adj(Geo g, const float2 *__restrict__ f, float2 *__restrict__ G1)
 {
     extern __shared__ float2 s[];
-    constexpr int SB = RowStride<B>::v;
-    constexpr int R = E / B;               // rows per thread: thread t owns rows t + k*T, k < R
-    const int grp = blockIdx.x, x = blockIdx.y, n = g.n1, N1 = g.N1;
-    char *const base = reinterpret_cast<char *>(s);
-    const size_t cbytes = ypass_adj_chunk_bytes(B);
-    unsigned short *lb = reinterpret_cast<unsigned short *>(base + 2 * cbytes);
-    const int e0 = g.row_off[x], cnt = g.row_off[x + 1] - e0;
-    const float2 *fg = f + (size_t)grp * g.M * B;
-    const int T = blockDim.x, ldl = lb_ld(n);
-    const int r0ofs = n / 2 + kHalo;
-    const int nch = (cnt + kChunk - 1) / kChunk;
-    // Chunk c lives in buffer c & 1: Qs [kChunk][SB], Ps [kChunk][kLdPs], Rs [kChunk].
-    auto bufQ = [&](int c) { return reinterpret_cast<float2 *>(base + (c & 1) * cbytes); };
-    auto bufP = [&](int c) { return reinterpret_cast<float *>(bufQ(c) + kChunk * SB); };
-    auto bufR = [&](int c) { return reinterpret_cast<int *>(bufP(c) + kChunk * kLdPs); };
-    auto issue = [&](int c) {
-        const int c0 = e0 + c * kChunk, cn = min(kChunk, e0 + cnt - c0);
-        float2 *Qs = bufQ(c);
-        float *Ps = bufP(c);
-        int *Rs = bufR(c);
-        for (int i = threadIdx.x; i < cn; i += T) {
-            const int j = __ldg(&g.ent_jt[c0 + i]) >> 4;
-            const float2 *src = fg + (size_t)j * B;
-            if constexpr (B >= 2) {
-#pragma unroll
-                for (int q = 0; q < B / 2; ++q) cp_async<16>(Qs + i * SB + 2 * q, src + 2 * q);
-            } else {
-                cp_async<8>(Qs + i * SB, src);
-            }
-            const float *pxy = g.ent_pxy + (size_t)(c0 + i) * kLdPhiy;
-#pragma unroll
-            for (int q = 0; q < kLdPhiy / 4; ++q) cp_async<16>(Ps + i * kLdPs + 4 * q, pxy + 4 * q);
-            cp_async<4>(Rs + i, g.ent_iy0 + c0 + i);
-        }
-        cp_async_commit();
-    };
-    // Thread t owns NS strips of RS consecutive rows, strip t + k*T starting
-    // at row RS*(t + k*T); one gather of a strip loads each covering entry
-    // once for its RS rows.
-    constexpr int RS = (B == 8 && R % 2 == 0) ? 2 : 1;
-    constexpr int NS = R / RS;
-    float2 acc[NS][RS][B];
-#pragma unroll
-    for (int k = 0; k < NS; ++k)
-#pragma unroll
-        for (int j = 0; j < RS; ++j)
-#pragma unroll
-            for (int b = 0; b < B; ++b) acc[k][j][b] = make_float2(0.f, 0.f);
-    float2 *tw_s = reinterpret_cast<float2 *>(base + ypass_adj_region(n, B));   // [n] twiddles
+    constexpr bool kSwz = (B == 8);
+    const int grp = blockIdx.x, x = yadj_row(blockIdx.y, g.n0), n = g.n1, N1 = g.N1;
+    float2 *tw_s = reinterpret_cast<float2 *>(reinterpret_cast<char *>(s) + yadj_rows_bytes(n, B));   // [n] twiddles
     const float2 *tws = ypass_tw_shared(n) ? tw_s : g.tw1;
     if (ypass_tw_shared(n)) copy_async(tw_s, g.tw1, (size_t)n * sizeof(float2));
     cp_async_commit();
-    if (nch > 0) {
-        copy_async(lb, g.ent_lb + (size_t)x * ldl, (size_t)ldl * sizeof(unsigned short));
-        issue(0);
-    }
-    for (int c = 0; c < nch; ++c) {
-        cp_async_wait<0>();
-        __syncthreads();                  // chunk c landed; chunk c-1's buffer is free
-        if (c + 1 < nch) issue(c + 1);
-        const int off = c * kChunk, cn = min(kChunk, cnt - off);
-        const float2 *Qs = bufQ(c);
-        const float *Ps = bufP(c);
-        const int *Rs = bufR(c);
-#pragma unroll
-        for (int k = 0; k < NS; ++k) {
-            const int r = RS * (threadIdx.x + k * T);
-            if (r < n) {
-                gather_rows<B, SB, RS>(r + kHalo, r0ofs, lb, ldl - 1, off, cn, Qs, Ps, Rs, acc[k], g.tlo, g.thi);
-                // Rows 0..7 and n-8..n-1 also take the halo rows that alias
-                // them (kHalo is a multiple of RS, so no strip straddles).
-                if (r < kHalo)
-                    gather_rows<B, SB, RS>(r + kHalo + n, r0ofs, lb, ldl - 1, off, cn, Qs, Ps, Rs, acc[k], g.tlo, g.thi);
-                if (r >= n - kHalo)
-                    gather_rows<B, SB, RS>(r + kHalo - n, r0ofs, lb, ldl - 1, off, cn, Qs, Ps, Rs, acc[k], g.tlo, g.thi);
-            }
-        }
-    }
-    cp_async_wait<0>();                   // the twiddles (rows without entries wait here)
-    __syncthreads();                      // the row buffer reuses the chunk buffers
-#pragma unroll
-    for (int k = 0; k < NS; ++k) {
-        const int r = RS * (threadIdx.x + k * T);
-        if (r < n) {
-#pragma unroll
-            for (int j = 0; j < RS; ++j) store_b<B>(s + (size_t)(r + j) * SB, acc[k][j]);
-        }
-    }
-    __syncthreads();
-    float2 *row = s;
+    // stages as yadj_stages(blockDim.x)
+    char *stage = reinterpret_cast<char *>(tw_s) + ypass_tw_bytes(n);
+    if (blockDim.x <= 256) yadj_gather<B, 3>(g, x, f + (size_t)grp * g.M * B, s, stage);
+    else yadj_gather<B, 2>(g, x, f + (size_t)grp * g.M * B, s, stage);
+    float2 *row = s + kHalo * B;
     float2 *out = G1 + ((size_t)grp * g.n0 + x) * N1 * B;
-    auto ld = [=](int q, int b) -> float2 { return row[q * SB + b]; };
+    auto ld = [=](int q, int b) -> float2 { return row[q * B + b]; };
     auto st = [=](int kq, int b, float2 v) {
         int Y = (kq + N1 / 2) & (n - 1);
         if (Y < N1) out[(size_t)Y * B + b] = (kq & 1) ? make_float2(-v.x, -v.y) : v;   // undoes the rotation
     };
-    fft_fused<B, SB, E, GUARD, false, true>(row, n, g.lg1, tws, +1.f, ld, st);
+    fft_fused<B, B, E, GUARD, kSwz, true>(row, n, g.lg1, tws, +1.f, ld, st);
 }
 
 // -------------------------------------------------------------- K1T ----
@@ -1446,6 +1497,65 @@ __global__ void __launch_bounds__(R * B, (R == 20 && B == 8) ? 4 : (512 / (R * B
 __host__ __device__ inline size_t ytoep4_smem(int n1, int B) { return (size_t)n1 * (B + 1) * sizeof(float2); }
 // n1 sizes k_ytoep4 takes (n1 = 32 R, R in ytoep4_radix_ok).
 __host__ __device__ inline bool ytoep4_fits(int n1) { return n1 % 32 == 0 && ytoep4_radix_ok(n1 / 32); }
+
+// ------------------------------------------- adjoint y-pass, 4-step ----
+// The adjoint y-pass (k_ypass_adj) for n1 = 32 R, R = 4, 8, 16 or 32, with
+// the four-step register FFT of k_ytoep4 in its inverse direction: the
+// gathered rows are read once into registers, one transpose through the same
+// shared memory, the outputs Y < N1 stored from registers.
+__host__ __device__ constexpr bool yadj4_fits(int n1) { return n1 == 128 || n1 == 256 || n1 == 512 || n1 == 1024; }
+
+template <int B, int R>
+__global__ void __launch_bounds__(yadj_threads(R * B), 512 / yadj_threads(R * B))
+    k_yadj4(Geo g, const float2 *__restrict__ f, float2 *__restrict__ G1)
+{
+    constexpr int LB = Log2B<B>::v, n = 32 * R;
+    constexpr int NI = (32 + R - 1) / R;
+    extern __shared__ float2 s[];
+    const int grp = blockIdx.x, x = yadj_row(blockIdx.y, g.n0), N1 = g.N1;
+    const int t = threadIdx.x, b = t & (B - 1), u = t >> LB;
+    const bool act = yadj_threads(R * B) == R * B || t < R * B;
+    float2 *tws = reinterpret_cast<float2 *>(reinterpret_cast<char *>(s) + yadj_rows_bytes(n, B));
+    copy_async(tws, g.tw1, (size_t)n * sizeof(float2));
+    cp_async_commit();
+    yadj_gather<B, yadj_stages(yadj_threads(R * B))>(g, x, f + (size_t)grp * g.M * B, s, reinterpret_cast<char *>(tws + n));
+    // 32-point inverse DFT over k2 of rows k = u + R k2, twiddles, transpose.
+    float2 w[32];
+    if (act) {
+#pragma unroll
+        for (int k2 = 0; k2 < 32; ++k2) w[k2] = s[(kHalo + u + R * k2) * B + b];
+    }
+    __syncthreads();   // every row is read before the buffer is rewritten
+    if (act) {
+        dft_dif_inplace<32>(w, +1.f);
+#pragma unroll
+        for (int c = 0; c < 32; ++c) {
+            float2 tw = tws[c * u];
+            tw.y = -tw.y;
+            s[ytoep4_sidx<B, R>(c, u, b)] = c ? cmul(w[brev5(c)], tw) : w[0];
+        }
+    }
+    __syncthreads();
+    if (!act) return;
+    // R-point inverse DFTs over k1 of columns c = u + R i: y = 32 a + c, whose
+    // crop row is (y + N1/2) mod n1; odd y undo the rotation's sign.
+    float2 *out = G1 + ((size_t)grp * g.n0 + x) * N1 * B + b;
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+        const int c = u + R * i;
+        if (c >= 32) break;
+        float2 v[R];
+#pragma unroll
+        for (int k1 = 0; k1 < R; ++k1) v[k1] = s[ytoep4_sidx<B, R>(c, k1, b)];
+        dft_nat<R>(v, +1.f);
+        const float sg = (c & 1) ? -1.f : 1.f;
+#pragma unroll
+        for (int a = 0; a < R; ++a) {
+            const int Y = (32 * a + c + N1 / 2) & (n - 1);
+            if (Y < N1) out[(size_t)Y * B] = make_float2(sg * v[a].x, sg * v[a].y);
+        }
+    }
+}
 
 }  // namespace icon
 
