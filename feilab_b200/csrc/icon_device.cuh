@@ -272,6 +272,46 @@ struct Lg {
     static constexpr int v = R >= 32 ? 5 : R >= 16 ? 4 : R >= 8 ? 3 : R >= 4 ? 2 : R >= 2 ? 1 : 0;
 };
 
+// Radix-2 butterfly a, o <- a + w o, a - w o with w = exp(dir 2 pi i k / 32),
+// k < 16 known at compile time.  The FP32 pipe bounds the y-passes (a packed
+// f32x2 instruction takes it as long as its two scalar ones: 120 lanes per
+// clock and SM for either), so what counts is the number of multiply-adds:
+// w = 1 and w = +-i take additions only, every other w six fused ones in
+// place of a product and two additions (eight), by factoring the larger of
+// cos and sin out: w o = c ((x - r y) + i (y + r x)), r = sin / cos.  A
+// 32-point DFT takes 388 instead of 576 (the 640-point convolution y-pass of 128
+// slices: 490 -> 466 us).
+__device__ __forceinline__ void butterfly(float2 &a, float2 &o, int k, float dir)
+{
+    // tan of 2 pi k / 32 for k <= 4; the other k by symmetry
+    constexpr float T[5] = {0.0f, 0.19891236737965800f, 0.41421356237309505f, 0.66817863791929892f, 1.0f};
+    if (k == 0) {
+        const float2 t = o;
+        o = sub2(a, t);
+        a = add2(a, t);
+    } else if (k == 8) {
+        const float2 t = make_float2(-dir * o.y, dir * o.x);
+        o = make_float2(a.x - t.x, a.y - t.y);
+        a = make_float2(a.x + t.x, a.y + t.y);
+    } else {
+        const float2 w = w32(k, dir);
+        float c, u, v;
+        if (k <= 4 || k >= 12) {
+            const float r = dir * (k <= 4 ? T[k & 7] : -T[(16 - k) & 7]);
+            c = w.x;
+            u = fmaf(-r, o.y, o.x);
+            v = fmaf(r, o.x, o.y);
+        } else {
+            const float r = dir * (k < 8 ? T[(8 - k) & 7] : -T[(k - 8) & 7]);
+            c = w.y;
+            u = fmaf(r, o.x, -o.y);
+            v = fmaf(r, o.y, o.x);
+        }
+        o = make_float2(fmaf(-c, u, a.x), fmaf(-c, v, a.y));
+        a = make_float2(fmaf(c, u, a.x), fmaf(c, v, a.y));
+    }
+}
+
 // One radix-2 stage (butterfly span LEN) of the in-place DIT DFT below, then
 // the next stage; template recursion keeps every index a compile-time constant.
 template <int R, int LEN>
@@ -280,12 +320,7 @@ __device__ __forceinline__ void dft_stage(float2 (&a)[R], float dir)
 #pragma unroll
     for (int i = 0; i < R; i += LEN) {
 #pragma unroll
-        for (int k = 0; k < LEN / 2; ++k) {
-            float2 o = a[i + k + LEN / 2];
-            float2 t = (k == 0) ? o : cmul(w32((k * (32 / LEN)) & 31, dir), o);
-            a[i + k + LEN / 2] = sub2(a[i + k], t);
-            a[i + k] = add2(a[i + k], t);
-        }
+        for (int k = 0; k < LEN / 2; ++k) butterfly(a[i + k], a[i + k + LEN / 2], k * (32 / LEN), dir);
     }
     if constexpr (LEN < R) dft_stage<R, 2 * LEN>(a, dir);
 }
@@ -329,19 +364,6 @@ __host__ __device__ constexpr double ct_cos(double x)
     return sum;
 }
 
-// v * exp(dir * 2 pi i m / n), the factor a compile-time constant.
-template <int N, int M>
-__device__ __forceinline__ float2 tw_mul(float2 v, float dir)
-{
-    if constexpr (M % N == 0) {
-        return v;
-    } else {
-        constexpr float c = (float)ct_cos(ct_angle(M, N)), s = (float)ct_sin(ct_angle(M, N));
-        const float sd = dir * s;
-        return make_float2(fmaf(v.x, c, -sd * v.y), fmaf(v.x, sd, v.y * c));
-    }
-}
-
 // 3- and 5-point DFTs in place (natural order), sign dir.  With
 // w = exp(dir 2 pi i / P): X_k = sum_r x_r w^(r k), written as sums and
 // differences of the symmetric pairs x_r +- x_(P-r).
@@ -351,28 +373,30 @@ __device__ __forceinline__ void dft3(float2 (&a)[3], float dir)
     const float2 s = add2(a[1], a[2]), d = sub2(a[1], a[2]);
     const float2 m = make_float2(fmaf(-0.5f, s.x, a[0].x), fmaf(-0.5f, s.y, a[0].y));
     const float hd = dir * h;
-    const float2 id = make_float2(-hd * d.y, hd * d.x);   // i dir h (x1 - x2)
     a[0] = add2(a[0], s);
-    a[1] = add2(m, id);
-    a[2] = sub2(m, id);
+    a[1] = make_float2(fmaf(-hd, d.y, m.x), fmaf(hd, d.x, m.y));   // m + i dir h (x1 - x2)
+    a[2] = make_float2(fmaf(hd, d.y, m.x), fmaf(-hd, d.x, m.y));
 }
 
 __device__ __forceinline__ void dft5(float2 (&a)[5], float dir)
 {
     constexpr float c1 = (float)ct_cos(ct_angle(1, 5)), c2 = (float)ct_cos(ct_angle(2, 5));
-    constexpr float s1 = (float)ct_sin(ct_angle(1, 5)), s2 = (float)ct_sin(ct_angle(2, 5));
+    constexpr float s1 = (float)ct_sin(ct_angle(1, 5));
+    constexpr float r = (float)(ct_sin(ct_angle(2, 5)) / ct_sin(ct_angle(1, 5)));
     const float2 t1 = add2(a[1], a[4]), t2 = add2(a[2], a[3]), t3 = sub2(a[1], a[4]), t4 = sub2(a[2], a[3]);
     const float2 x0 = a[0];
     const float2 p1 = make_float2(fmaf(c2, t2.x, fmaf(c1, t1.x, x0.x)), fmaf(c2, t2.y, fmaf(c1, t1.y, x0.y)));
     const float2 p2 = make_float2(fmaf(c1, t2.x, fmaf(c2, t1.x, x0.x)), fmaf(c1, t2.y, fmaf(c2, t1.y, x0.y)));
-    // q1 = dir (s1 t3 + s2 t4), q2 = dir (s2 t3 - s1 t4); X1,4 = p1 +- i q1, X2,3 = p2 +- i q2
-    const float2 q1 = make_float2(dir * fmaf(s1, t3.x, s2 * t4.x), dir * fmaf(s1, t3.y, s2 * t4.y));
-    const float2 q2 = make_float2(dir * fmaf(s2, t3.x, -s1 * t4.x), dir * fmaf(s2, t3.y, -s1 * t4.y));
+    // q1 = s1 t3 + s2 t4 = s1 u1, q2 = s2 t3 - s1 t4 = s1 u2;
+    // X1,4 = p1 +- i dir q1, X2,3 = p2 +- i dir q2
+    const float2 u1 = make_float2(fmaf(r, t4.x, t3.x), fmaf(r, t4.y, t3.y));
+    const float2 u2 = make_float2(fmaf(r, t3.x, -t4.x), fmaf(r, t3.y, -t4.y));
+    const float sd = dir * s1;
     a[0] = add2(x0, add2(t1, t2));
-    a[1] = make_float2(p1.x - q1.y, p1.y + q1.x);
-    a[4] = make_float2(p1.x + q1.y, p1.y - q1.x);
-    a[2] = make_float2(p2.x - q2.y, p2.y + q2.x);
-    a[3] = make_float2(p2.x + q2.y, p2.y - q2.x);
+    a[1] = make_float2(fmaf(-sd, u1.y, p1.x), fmaf(sd, u1.x, p1.y));
+    a[4] = make_float2(fmaf(sd, u1.y, p1.x), fmaf(-sd, u1.x, p1.y));
+    a[2] = make_float2(fmaf(-sd, u2.y, p2.x), fmaf(sd, u2.x, p2.y));
+    a[3] = make_float2(fmaf(sd, u2.y, p2.x), fmaf(-sd, u2.x, p2.y));
 }
 
 template <int P>
@@ -383,25 +407,23 @@ __device__ __forceinline__ void dft_small(float2 (&a)[P], float dir)
     else dft5(a, dir);
 }
 
-// Twiddles y[q][k1] *= exp(dir 2 pi i q k1 / R) of the mixed-radix step,
-// each factor a compile-time constant (index sequences unroll q and k1).
-template <int R, int P, int Q, int q, int... K1>
-__device__ __forceinline__ void tw_row(float2 (&yq)[P], float dir, std::integer_sequence<int, K1...>)
+// The k < P Q with k mod P = k1 and k mod Q = k2 (P and Q coprime).
+__host__ __device__ constexpr int crt_index(int P, int Q, int k1, int k2)
 {
-    ((yq[K1] = tw_mul<R, q * K1>(yq[K1], dir)), ...);
-}
-template <int R, int P, int Q, int... Qs>
-__device__ __forceinline__ void tw_all(float2 (&y)[Q][P], float dir, std::integer_sequence<int, Qs...>)
-{
-    (tw_row<R, P, Q, Qs>(y[Qs], dir, std::make_integer_sequence<int, P>{}), ...);
+    int k = k2;
+    while (k % P != k1) k += Q;
+    return k;
 }
 
 // DFT of R values in registers, natural order in and out:
 // a[k] <- sum_r a[r] exp(dir 2 pi i r k / R).  R a power of two (radix-2
 // DIT above, after a bit-reversal that only renames registers) or R = P Q with
-// P = 3 or 5 and Q a power of two (Cooley-Tukey: P-point DFTs over
-// r = Q p + q, twiddles exp(dir 2 pi i q k1 / R), Q-point DFTs over q, k =
-// k1 + P k2).
+// P = 3 or 5 and Q a power of two.  P and Q are coprime, so the prime-factor
+// form (Good 1958) needs no twiddles: with r = (Q p + P q) mod R, the factor
+// of X[k] is exp(dir 2 pi i p k / P) exp(dir 2 pi i q k / Q): P-point DFTs over
+// p, Q-point DFTs over q, and the outputs k by k mod P and k mod Q; all index
+// maps only rename registers (20 points: 208 multiply-adds, 256 with the
+// twiddles of the Cooley-Tukey form).
 template <int R>
 __device__ __forceinline__ void dft_nat(float2 (&a)[R], float dir)
 {
@@ -421,10 +443,9 @@ __device__ __forceinline__ void dft_nat(float2 (&a)[R], float dir)
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
 #pragma unroll
-            for (int p = 0; p < P; ++p) y[q][p] = a[Q * p + q];
+            for (int p = 0; p < P; ++p) y[q][p] = a[(Q * p + P * q) % R];
             dft_small<P>(y[q], dir);
         }
-        tw_all<R, P, Q>(y, dir, std::make_integer_sequence<int, Q>{});
 #pragma unroll
         for (int k1 = 0; k1 < P; ++k1) {
             float2 u[Q];
@@ -432,37 +453,27 @@ __device__ __forceinline__ void dft_nat(float2 (&a)[R], float dir)
             for (int q = 0; q < Q; ++q) u[LQ ? (brev5(q) >> (5 - LQ)) : 0] = y[q][k1];
             dft_inplace<Q>(u, dir);
 #pragma unroll
-            for (int k2 = 0; k2 < Q; ++k2) a[k1 + P * k2] = u[k2];
+            for (int k2 = 0; k2 < Q; ++k2) a[crt_index(P, Q, k1, k2)] = u[k2];
         }
     }
 }
 
-// One radix-2 decimation-in-frequency stage (butterfly span LEN), then the
-// next, shorter one.
-template <int R, int LEN>
-__device__ __forceinline__ void dif_stage(float2 (&a)[R], float dir)
-{
-#pragma unroll
-    for (int i = 0; i < R; i += LEN) {
-#pragma unroll
-        for (int k = 0; k < LEN / 2; ++k) {
-            const float2 p = a[i + k], q = a[i + k + LEN / 2];
-            a[i + k] = add2(p, q);
-            const float2 d = sub2(p, q);
-            a[i + k + LEN / 2] = (k == 0) ? d : cmul(w32((k * (32 / LEN)) & 31, dir), d);
-        }
-    }
-    if constexpr (LEN > 2) dif_stage<R, LEN / 2>(a, dir);
-}
-
-// In-place radix-2 DIF DFT of R values held in registers, a[] given in
-// natural order; on return a[brev(q)] = sum_r x[r] exp(dir*2*pi*i*r*q/R)
-// (brev over log2 R bits).  The mirror of dft_inplace: the two compose
-// without a register permutation in between.
+// DFT of R values held in registers, a[] given in natural order; on return
+// a[brev(q)] = sum_r x[r] exp(dir*2*pi*i*r*q/R) (brev over log2 R bits): the
+// DIT DFT between two bit reversals that only rename registers, so it
+// composes with dft_inplace without a permutation in between.
 template <int R>
 __device__ __forceinline__ void dft_dif_inplace(float2 (&a)[R], float dir)
 {
-    if constexpr (R >= 2) dif_stage<R, R>(a, dir);
+    if constexpr (R >= 2) {
+        constexpr int L = Lg<R>::v;
+        float2 t[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) t[brev5(r) >> (5 - L)] = a[r];
+        dft_inplace<R>(t, dir);
+#pragma unroll
+        for (int r = 0; r < R; ++r) a[brev5(r) >> (5 - L)] = t[r];
+    }
 }
 
 // Position of point p in the intermediate buffer s.  With SWZ, points p and

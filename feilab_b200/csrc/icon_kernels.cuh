@@ -1385,12 +1385,13 @@ __host__ __device__ constexpr bool ytoep4_radix_ok(int R)
 // Toeplitz y-pass of A^H W A m).  MODE 1: part[G][n0][B] <- per slice
 // sum_k K[x][k] |F(pad row)[k]|^2 in FP64 (the step length's denominator).
 // g.n1 = 32 R and g.tw1 its twiddles (the Toeplitz view of the plan).
-// Launch bounds: blocks of R B threads, at least 512 threads per SM; the
+// Launch bounds: blocks of R B threads, 16 warps per SM (128 registers, the
+// transform's 64 among them); the
 // 640-point transform of 8-slice groups (the 1024x300 workload) asks for four
 // blocks per SM (96 registers, a few spilled bytes), which measured 8% faster
 // for MODE 1 and the same for MODE 0 than three blocks at 128 registers.
 template <int B, int R, int MODE>
-__global__ void __launch_bounds__(R * B, (R == 20 && B == 8) ? 4 : (512 / (R * B) < 32 ? 512 / (R * B) : 32))
+__global__ void __launch_bounds__(R * B, (R == 20 && B == 8) ? 4 : 16 / ((R * B + 31) / 32))
     k_ytoep4(Geo g, float2 *__restrict__ G1, double *__restrict__ part)
 {
     constexpr int LB = Log2B<B>::v;
