@@ -2,9 +2,12 @@
 // in its companion tools, on the GPU: stack pre-processing (ICONPreProcess)
 // and, in mask.cu, volume assembly with the cross-validation mask
 // (ICONMask3).  C ABI in include/icon_tools.h.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
+#include <cstdint>
 #include <string>
 #include <vector>
 
@@ -30,105 +33,222 @@ struct PreFactors {
     double f[kPreMaxProjections];
 };
 
-// Fixed-order block reduction of one double per thread (blockDim = 1024).
-__device__ double block_sum(double v, double *red)
-{
-    red[threadIdx.x] = v;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-        __syncthreads();
-    }
-    const double r = red[0];
-    __syncthreads();
-    return r;
-}
-
-// One block per projection k of in[nz][ny][nx] (ICONPreProcess.c:29-85):
+// One cluster of kPreCluster CTAs per projection k of in[nz][ny][nx]
+// (ICONPreProcess.c:29-85):
 //   mode  = bin of the most pixels (first on ties) of a 256-bin histogram of
 //           the central region (10 % margins), bin index
 //           floor((v - min) / step), step = (max - min) / 256 in double; the
 //           largest pixel falls in bin 256, which is not counted
 //   v    -= mode                                (float result)
-//   with factor[k] > 0: mean = sum (v / size in float), var = sum (v - mean)^2 / size
+//   with factor[k] > 0: mean = sum v / size, var = sum (v - mean)^2 / size
 //           (double), v = v / sqrt(var) * sqrt(factor[k])
 // out may equal in.
-__global__ void __launch_bounds__(kPreThreads) k_preprocess(const float *in, float *out, int nx, int ny,
-                                                            int normalize, const __grid_constant__ PreFactors factor)
+//
+// The four passes over a projection (extrema, histogram, moments, result) are
+// bound by memory: 78 us for 61 projections of 1024 x 1024 read and written
+// once.  A CTA takes a band of whole rows and keeps the first of them in
+// shared memory (its only pass over DRAM fills them); the rest of the passes
+// read L2, which holds the bands of the clusters in flight because a CTA's
+// shared memory lets one run per SM.  Extrema, bin counts and moments are
+// combined over the cluster through distributed shared memory in rank order.
+// 61 x 1024 x 1024: 398 us; with one CTA per projection, six passes and
+// divisions in double for every pixel 2374 us.  What is left is issue (about 60
+// instructions a pixel) and the last wave of clusters.
+constexpr int kPreCluster = 8;
+constexpr int kPreCache = 184 * 1024;   // shared memory for rows
+
+// Sum over the block of one double per thread (fixed order), to every thread.
+__device__ double block_sum(double v, double *red)
 {
-    __shared__ double red[kPreThreads];
-    __shared__ int hist[256];
-    __shared__ float smin[kPreThreads], smax[kPreThreads];
-    const size_t size = (size_t)nx * ny;
-    const float *p = in + (size_t)blockIdx.x * size;
-    float *q = out + (size_t)blockIdx.x * size;
-    const int xe = (int)(nx * 0.1), ye = (int)(ny * 0.1);
-    const int cw = nx - 2 * xe, ch = ny - 2 * ye;
-    const int ncore = cw * ch;
-    float lo = p[(size_t)ye * nx + xe], hi = lo;
-    for (int i = threadIdx.x; i < ncore; i += blockDim.x) {
-        const float v = p[(size_t)(ye + i / cw) * nx + xe + i % cw];
-        lo = fminf(lo, v);
-        hi = fmaxf(hi, v);
-    }
-    smin[threadIdx.x] = lo;
-    smax[threadIdx.x] = hi;
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) hist[i] = 0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    __syncthreads();                       // red free
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
     __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) {
-            smin[threadIdx.x] = fminf(smin[threadIdx.x], smin[threadIdx.x + o]);
-            smax[threadIdx.x] = fmaxf(smax[threadIdx.x], smax[threadIdx.x + o]);
+    double r = 0.0;
+    for (int i = 0; i < (int)blockDim.x / 32; ++i) r += red[i];
+    return r;
+}
+
+// VEC: rows are read and written as float4 (nx a multiple of 4, both stacks
+// on 16-byte boundaries).
+template <bool VEC>
+__global__ void __launch_bounds__(kPreThreads, 1) __cluster_dims__(kPreCluster, 1, 1)
+    k_preprocess(const float *in, float *out, int nx, int ny, int normalize, int cache_rows,
+                 const __grid_constant__ PreFactors factor)
+{
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    extern __shared__ __align__(16) float cache[];   // [cache_rows][nx]
+    __shared__ double red[kPreThreads / 32];
+    __shared__ float ext[2];                         // this CTA's extrema, read by the cluster
+    __shared__ int hist[8][256];                     // warps w share copy w % 8
+    __shared__ int bins[256];                        // this CTA's counts, read by the cluster
+    __shared__ double mom[2], mode_s;                // this CTA's moments
+    const int k = blockIdx.x / kPreCluster, rank = (int)cl.block_rank();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, W = blockDim.x >> 5;
+    const size_t size = (size_t)nx * ny;
+    const float *p = in + (size_t)k * size;
+    float *q = out + (size_t)k * size;
+    const int y0 = (int)((long long)ny * rank / kPreCluster), y1 = (int)((long long)ny * (rank + 1) / kPreCluster);
+    const int xe = (int)(nx * 0.1), ye = (int)(ny * 0.1);
+    const int xr = nx - xe, yr = ny - ye;            // core: xe <= x < xr, ye <= y < yr
+    // Calls f(x, v) for the pixels x of row y that this lane takes.
+    auto row = [&](const float *r, auto f) {
+        if constexpr (VEC) {
+            for (int x = 4 * lane; x < nx; x += 128) {
+                const float4 v = *reinterpret_cast<const float4 *>(r + x);
+                f(x, v.x);
+                f(x + 1, v.y);
+                f(x + 2, v.z);
+                f(x + 3, v.w);
+            }
+        } else {
+            for (int x = lane; x < nx; x += 32) f(x, r[x]);
         }
-        __syncthreads();
+    };
+    // Row y from the cache when it is there.
+    auto source = [&](int y) { return y - y0 < cache_rows ? cache + (size_t)(y - y0) * nx : p + (size_t)y * nx; };
+
+    // Extrema of the core; fills the cache.
+    float lo = p[(size_t)ye * nx + xe], hi = lo;
+    for (int y = y0 + warp; y < y1; y += W) {
+        const bool core = y >= ye && y < yr, keep = y - y0 < cache_rows;
+        float *c = cache + (size_t)(y - y0) * nx;
+        row(p + (size_t)y * nx, [&](int x, float v) {
+            if (keep) c[x] = v;
+            if (core && x >= xe && x < xr) {
+                lo = fminf(lo, v);
+                hi = fmaxf(hi, v);
+            }
+        });
     }
-    const double mn = smin[0], mx = smax[0];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    float *red_f = reinterpret_cast<float *>(&hist[0][0]);   // [2][32], before the counts
+    if (lane == 0) {
+        red_f[warp] = lo;
+        red_f[32 + warp] = hi;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int i = 1; i < W; ++i) {
+            lo = fminf(lo, red_f[i]);
+            hi = fmaxf(hi, red_f[32 + i]);
+        }
+        ext[0] = lo;
+        ext[1] = hi;
+    }
+    cl.sync();
+    lo = cl.map_shared_rank(ext, 0)[0];
+    hi = cl.map_shared_rank(ext, 0)[1];
+    for (int r = 1; r < kPreCluster; ++r) {
+        lo = fminf(lo, cl.map_shared_rank(ext, r)[0]);
+        hi = fmaxf(hi, cl.map_shared_rank(ext, r)[1]);
+    }
+    const double mn = lo, mx = hi;
     const double step = (mx - mn) / 256.0;
     double mode = mn;   // a constant core has no spread (the reference divides by zero there)
     if (step > 0.0) {
-        for (int i = threadIdx.x; i < ncore; i += blockDim.x) {
-            const float v = p[(size_t)(ye + i / cw) * nx + xe + i % cw];
-            const int b = (int)floor(((double)v - mn) / step);
-            if (b >= 0 && b < 256) atomicAdd(&hist[b], 1);
+        for (int i = threadIdx.x; i < 8 * 256; i += blockDim.x) (&hist[0][0])[i] = 0;
+        __syncthreads();
+        const double inv = 1.0 / step;
+        int *h = hist[warp & 7];
+        for (int y = max(y0, ye) + warp; y < min(y1, yr); y += W)
+            row(source(y), [&](int x, float v) {
+                if (x < xe || x >= xr) return;
+                // The quotient's floor by a product (its nearest whole number
+                // read from the low bits of t + 1.5 2^52, all in the FP64 pipe),
+                // and by the division itself where the product is near a
+                // whole number (or not finite).
+                const double t = ((double)v - mn) * inv, big = t + 6755399441055744.0, d = t - (big - 6755399441055744.0);
+                int b = __double2loint(big) - (d < 0.0);
+                if (!(fabs(d) > 1e-6)) b = (int)floor(((double)v - mn) / step);
+                if (b >= 0 && b < 256) atomicAdd(&h[b], 1);
+            });
+        __syncthreads();
+        if (threadIdx.x < 256) {
+            int c = 0;
+            for (int i = 0; i < 8; ++i) c += hist[i][threadIdx.x];
+            bins[threadIdx.x] = c;
+        }
+        cl.sync();
+        // First bin with the largest count, over the cluster.
+        if (threadIdx.x < 256) {
+            int c = 0;
+            for (int r = 0; r < kPreCluster; ++r) c += cl.map_shared_rank(bins, r)[threadIdx.x];
+            hist[0][threadIdx.x] = c;
         }
         __syncthreads();
-        // First bin with the largest count.
-        if (threadIdx.x == 0) {
+        if (threadIdx.x < 32) {
             int best = -1, bi = 0;
-            for (int i = 0; i < 256; ++i)
-                if (best < hist[i]) {
-                    best = hist[i];
+            for (int i = lane; i < 256; i += 32)
+                if (best < hist[0][i]) {
+                    best = hist[0][i];
                     bi = i;
                 }
-            red[0] = bi * step + mn;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const int ob = __shfl_xor_sync(0xffffffffu, best, o), oi = __shfl_xor_sync(0xffffffffu, bi, o);
+                if (ob > best || (ob == best && oi < bi)) {
+                    best = ob;
+                    bi = oi;
+                }
+            }
+            if (lane == 0) mode_s = bi * step + mn;
         }
         __syncthreads();
-        mode = red[0];
-        __syncthreads();
+        mode = mode_s;
     }
-    const double f = normalize ? factor.f[blockIdx.x] : 0.0;
-    if (!(f > 0.0)) {
-        for (size_t i = threadIdx.x; i < size; i += blockDim.x) q[i] = (float)((double)p[i] - mode);
-        return;
+    const double f = normalize ? factor.f[k] : 0.0;
+    double scale = 1.0;
+    if (f > 0.0) {
+        // var = (sum v^2 - (sum v)^2 / size) / size in double.  (The mean of
+        // float quotients v / size that the reference subtracts is within
+        // 2^-24 of the mean, and moves the variance by the square of that.)
+        double s1 = 0.0, s2 = 0.0;
+        for (int y = y0 + warp; y < y1; y += W)
+            row(source(y), [&](int, float v0) {
+                const double v = (double)(float)((double)v0 - mode);
+                s1 += v;
+                s2 += v * v;
+            });
+        s1 = block_sum(s1, red);
+        s2 = block_sum(s2, red);
+        if (threadIdx.x == 0) {
+            mom[0] = s1;
+            mom[1] = s2;
+        }
+        cl.sync();
+        s1 = s2 = 0.0;
+        for (int r = 0; r < kPreCluster; ++r) {
+            const double *m = cl.map_shared_rank(mom, r);
+            s1 += m[0];
+            s2 += m[1];
+        }
+        const double var = (s2 - s1 * s1 / (double)size) / (double)size;
+        scale = sqrt(f) / sqrt(var < 0.0 ? 0.0 : var);   // rounding of the sums for a constant stack
     }
-    const float fsize = (float)size;
-    double s = 0.0;
-    for (size_t i = threadIdx.x; i < size; i += blockDim.x) {
-        const float v = (float)((double)p[i] - mode);
-        s += (double)(v / fsize);
+    for (int y = y0 + warp; y < y1; y += W) {
+        const float *r = source(y);
+        float *o = q + (size_t)y * nx;
+        auto result = [&](float v0) {
+            const float v = (float)((double)v0 - mode);
+            return f > 0.0 ? (float)((double)v * scale) : v;
+        };
+        if constexpr (VEC) {
+            for (int x = 4 * lane; x < nx; x += 128) {
+                const float4 v = *reinterpret_cast<const float4 *>(r + x);
+                *reinterpret_cast<float4 *>(o + x) = make_float4(result(v.x), result(v.y), result(v.z), result(v.w));
+            }
+        } else {
+            for (int x = lane; x < nx; x += 32) o[x] = result(r[x]);
+        }
     }
-    const double mean = block_sum(s, red);
-    double s2 = 0.0;
-    for (size_t i = threadIdx.x; i < size; i += blockDim.x) {
-        const double d = (double)(float)((double)p[i] - mode) - mean;
-        s2 += d * d / (double)size;
-    }
-    const double var = block_sum(s2, red);
-    const double sv = sqrt(var), sf = sqrt(f);
-    for (size_t i = threadIdx.x; i < size; i += blockDim.x) {
-        const float v = (float)((double)p[i] - mode);
-        q[i] = (float)((double)v / sv * sf);
-    }
+    cl.sync();   // no CTA leaves while another reads its shared memory
 }
 
 }  // namespace
@@ -153,8 +273,14 @@ icon_status icon_preprocess(const float *d_in, float *d_out, int nx, int ny, int
             if (!(f.f[k] > 0.0)) return tools_fail(ICON_ERR_INVALID, "icon_preprocess: tilt angle gives a non-positive variance");
         }
     }
-    k_preprocess<<<nz, kPreThreads, 0, st>>>(d_in, d_out, nx, ny, norm ? 1 : 0, f);
-    cudaError_t e = cudaGetLastError();
+    const int cache_rows = (int)std::min<size_t>(kPreCache / (sizeof(float) * (size_t)nx), (size_t)ny);
+    const bool vec = nx % 4 == 0 && ((uintptr_t)d_in & 15) == 0 && ((uintptr_t)d_out & 15) == 0;
+    const auto kern = vec ? k_preprocess<true> : k_preprocess<false>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPreCache);
+    if (e == cudaSuccess) {
+        kern<<<nz * kPreCluster, kPreThreads, kPreCache, st>>>(d_in, d_out, nx, ny, norm ? 1 : 0, cache_rows, f);
+        e = cudaGetLastError();
+    }
     if (e != cudaSuccess) return tools_fail(ICON_ERR_CUDA, std::string("icon_preprocess: ") + cudaGetErrorString(e));
     return ICON_OK;
 }
