@@ -17,24 +17,40 @@ __device__ __forceinline__ __nv_bfloat16 tobf(float v) { return __float2bfloat16
 // reference's images (X*N1 + Y).  The network image of slice s is
 // [Hp][Wp] with h = Y, w = X (Hp, Wp: N1, N0 rounded up to multiples of 8).
 
-// Per-slice sums of squares of Re(Ahwb); block s writes ss[s].
-__global__ void k_slice_sumsq(const float2 *__restrict__ Ahwb, int N0, int N1, double *__restrict__ ss)
+// Per-slice sums of squares of Re(Ahwb), in two steps of fixed order: block
+// (c, s) of kSumSqChunks per slice writes part[s][c], then k_slice_sumsq_fin
+// (one warp per slice) ss[s].  One block per slice took 559 us for 8 slices of
+// 1024 x 300 (one SM each); this takes 10 us.
+constexpr int kSumSqChunks = 64;
+
+__global__ void __launch_bounds__(256) k_slice_sumsq(const float2 *__restrict__ Ahwb, int N0, int N1, double *__restrict__ part)
 {
     __shared__ double red[256];
-    const int s = blockIdx.x;
-    const float2 *base = Ahwb + (size_t)s * N0 * N1;
+    const int c = blockIdx.x, s = blockIdx.y, n = N0 * N1;
+    const float2 *base = Ahwb + (size_t)s * n;
+    const int i0 = (int)((long long)n * c / kSumSqChunks), i1 = (int)((long long)n * (c + 1) / kSumSqChunks);
     double acc = 0.0;
-    for (int i = threadIdx.x; i < N0 * N1; i += blockDim.x) {
+#pragma unroll 4
+    for (int i = i0 + threadIdx.x; i < i1; i += 256) {
         double v = base[i].x;
         acc += v * v;
     }
     red[threadIdx.x] = acc;
     __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
+    for (int o = 128; o > 0; o >>= 1) {
         if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
         __syncthreads();
     }
-    if (threadIdx.x == 0) ss[s] = red[0];
+    if (threadIdx.x == 0) part[s * kSumSqChunks + c] = red[0];
+}
+
+__global__ void k_slice_sumsq_fin(const double *__restrict__ part, double *__restrict__ ss)
+{
+    double v = 0.0;
+    for (int c = threadIdx.x; c < kSumSqChunks; c += 32) v += part[blockIdx.x * kSumSqChunks + c];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (threadIdx.x == 0) ss[blockIdx.x] = v;
 }
 
 // Network input x[s][h][w] = Re(Ahwb[s][w][h]) / scale_s for h < N1, w < N0,
@@ -106,28 +122,67 @@ __global__ void k_conv_in(const float *__restrict__ x, const float *__restrict__
     d[1] = reinterpret_cast<uint4 *>(o)[1];
 }
 
-// Weight and bias gradients of the first layer: block = 160 threads, one per
-// output (tap*16 + c, or 144 + c for the bias); each block sums over its
-// strip of per_block pixels into part[blk][160].
-__global__ void k_conv_in_wgrad(const float *__restrict__ x, const __nv_bfloat16 *__restrict__ gz, int n, int H,
-                                int W, int per_block, float *__restrict__ part)
+// Weight and bias gradients of the first layer.  A block takes kInRows image
+// rows, kInCols pixels wide, at a time (tile = blockIdx.x + k*gridDim.x), its
+// input with the border and its output gradients in shared memory.  Thread =
+// (row group, dy, channel): it walks its rows' pixels with the three dx inputs
+// in registers, two shared loads and three multiply-adds a pixel; the dy = 1
+// threads also sum the bias.  part[blk][160] = dw[9][16], db[16], the row
+// groups' sums added in order.  16 x 512 x 256 pixels: 61 us; one thread
+// per weight walking 2048 pixels of global memory took 1669.
+constexpr int kInRows = 8, kInCols = 64, kInGroups = 4;
+
+__global__ void __launch_bounds__(48 * kInGroups) k_conv_in_wgrad(const float *__restrict__ x,
+                                                                  const __nv_bfloat16 *__restrict__ gz, int n, int H,
+                                                                  int W, float *__restrict__ part)
 {
-    const int o = threadIdx.x, c = o % 16, t = o / 16;
-    const size_t p0 = (size_t)blockIdx.x * per_block, total = (size_t)n * H * W;
-    float acc = 0.f;
-    for (int k = 0; k < per_block; ++k) {
-        const size_t p = p0 + k;
-        if (p >= total) break;
-        const float g = bf(gz[p * 16 + c]);
-        if (t == 9) {
-            acc += g;
-        } else {
-            const int xw = (int)(p % W), xh = (int)((p / W) % H), im = (int)(p / ((size_t)W * H));
-            const int hh = xh + t / 3 - 1, ww = xw + t % 3 - 1;
-            if (hh >= 0 && hh < H && ww >= 0 && ww < W) acc = fmaf(g, x[((size_t)im * H + hh) * W + ww], acc);
+    constexpr int T = 48 * kInGroups;
+    __shared__ float sx[kInRows + 2][kInCols + 2];
+    __shared__ float sg[kInRows][kInCols][17];
+    __shared__ float red[kInGroups][160];
+    const int t = threadIdx.x, c = t & 15, dy = (t >> 4) % 3, grp = t / 48;
+    const int tw = (W + kInCols - 1) / kInCols, th = (H + kInRows - 1) / kInRows;
+    const long long tiles = (long long)n * tw * th;
+    float acc[3] = {0.f, 0.f, 0.f}, bacc = 0.f;
+    for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int w0 = (int)(tile % tw) * kInCols, h0 = (int)((tile / tw) % th) * kInRows, im = (int)(tile / ((long long)tw * th));
+        __syncthreads();
+        for (int i = t; i < (kInRows + 2) * (kInCols + 2); i += T) {
+            const int px = i % (kInCols + 2), r = i / (kInCols + 2), hh = h0 + r - 1, ww = w0 + px - 1;
+            sx[r][px] = (hh >= 0 && hh < H && ww >= 0 && ww < W) ? x[((size_t)im * H + hh) * W + ww] : 0.f;
+        }
+        for (int i = t; i < kInRows * kInCols * 2; i += T) {     // 8 channels a piece
+            const int q = i & 1, px = (i >> 1) % kInCols, r = (i >> 1) / kInCols, hh = h0 + r, ww = w0 + px;
+            uint4 v = make_uint4(0, 0, 0, 0);
+            if (hh < H && ww < W) v = *reinterpret_cast<const uint4 *>(gz + (((size_t)im * H + hh) * W + ww) * 16 + 8 * q);
+            const __nv_bfloat16 *e = reinterpret_cast<const __nv_bfloat16 *>(&v);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) sg[r][px][8 * q + k] = bf(e[k]);
+        }
+        __syncthreads();
+        for (int r = grp; r < kInRows; r += kInGroups) {
+            float x0 = sx[r + dy][0], x1 = sx[r + dy][1];
+#pragma unroll 8
+            for (int px = 0; px < kInCols; ++px) {
+                const float g = sg[r][px][c], x2 = sx[r + dy][px + 2];
+                acc[0] = fmaf(g, x0, acc[0]);
+                acc[1] = fmaf(g, x1, acc[1]);
+                acc[2] = fmaf(g, x2, acc[2]);
+                bacc += g;
+                x0 = x1;
+                x1 = x2;
+            }
         }
     }
-    part[(size_t)blockIdx.x * 160 + o] = acc;
+#pragma unroll
+    for (int dx = 0; dx < 3; ++dx) red[grp][(3 * dy + dx) * 16 + c] = acc[dx];
+    if (dy == 1) red[grp][144 + c] = bacc;
+    __syncthreads();
+    if (t < 160) {
+        float a = red[0][t];
+        for (int k = 1; k < kInGroups; ++k) a += red[k][t];
+        part[(size_t)blockIdx.x * 160 + t] = a;
+    }
 }
 
 // ------------------------------------------------------------ pool / upsample
@@ -238,67 +293,209 @@ __global__ void k_relu_bwd(__nv_bfloat16 *__restrict__ g, const __nv_bfloat16 *_
 // ------------------------------------------------------------ weight gradients
 // dW[tap][co][ci] = sum over pixels of gz[p][co] * X[p shifted by tap][ci] for
 // a 3x3 convolution whose input is X0 (c0 channels) concatenated with X1 (c1
-// channels), and db[co] = sum gz[p][co].  Block = 16 x 16 threads over one
-// (16 co, 16 ci) tile; it walks the 64-pixel row segments item = split +
-// k*nsplit and writes its sums to part[split][tap][co][ci] (bias sums to
-// bpart[split][co] from the ci-tile 0 blocks).
-constexpr int kWgSeg = 64;
+// channels), and db[co] = sum gz[p][co]: nine matrix products with the pixels
+// as the inner dimension, 16 to 128 rows and 16 to 192 columns, on the tensor
+// cores by warp-level mma (m16n8k16, BF16 products, FP32 sums).  (The tiles are
+// too small for tcgen05: of its 64 rows at least 48 would be padding at 16
+// channels, and its operands could not share one staged row between the three
+// dx, which here are the same shared-memory rows read one pixel on.)
+//
+// A CTA of four warps takes an output tile of 16 WCO MC x 16 MI channels and a
+// contiguous share of the image rows, cut into 64 pixels wide strips.  It
+// walks down a strip with a ring of rows in shared memory (cp.async, two rows
+// ahead; five of X, so that each row of X is loaded once for its three dy, and
+// three of gz) whose 16-byte pieces are XOR-swizzled by the pixel, so that
+// every ldmatrix is free of bank conflicts at any dx.  A warp's tile is
+// 16 WCO x 16; the KW warps of one tile take the strip's 16-pixel steps in
+// turn.  Per step and warp: WCO + 9 ldmatrix and 18 WCO mma.  Every warp writes
+// its own partial sums, part[split KW + k][tap][co][ci], added in order by
+// k_sum_parts.  16 x 512 x 256 pixels, all 13 layers: 0.89 ms; one multiply-add a thread from
+// shared memory took 11.8 ms.
+constexpr int kWgStrip = 64, kWgXRows = 5, kWgGRows = 3;
 
-__global__ void __launch_bounds__(256) k_wgrad3x3(const __nv_bfloat16 *__restrict__ X0, int c0,
-                                                   const __nv_bfloat16 *__restrict__ X1, int c1,
-                                                   const __nv_bfloat16 *__restrict__ gz, int N, int n, int H, int W,
-                                                   int nsplit, float *__restrict__ part, float *__restrict__ bpart)
+__device__ __forceinline__ void ldsm_t(uint32_t (&r)[4], uint32_t addr)
 {
-    __shared__ float sg[kWgSeg][17];
-    __shared__ float sx[3][kWgSeg + 2][17];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;   // ci, co within the tile
-    const int co0 = blockIdx.y * 16, ci0 = blockIdx.z * 16;
-    const int Cin = c0 + c1;
-    const bool second = ci0 >= c0;
-    const __nv_bfloat16 *X = second ? X1 : X0;
-    const int CX = second ? c1 : c0, cx0 = second ? ci0 - c0 : ci0;
-    const int segs = (W + kWgSeg - 1) / kWgSeg;
-    const long long items = (long long)n * H * segs;
-    float acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    float bacc = 0.f;
-    for (long long it = blockIdx.x; it < items; it += nsplit) {
-        const int seg = (int)(it % segs);
-        const long long r = it / segs;
-        const int h = (int)(r % H), im = (int)(r / H), w0 = seg * kWgSeg;
-        __syncthreads();
-        for (int i = threadIdx.x; i < kWgSeg * 16; i += 256) {
-            const int px = i / 16, c = i % 16, w = w0 + px;
-            sg[px][c] = (w < W) ? bf(gz[(((size_t)im * H + h) * W + w) * N + co0 + c]) : 0.f;
-        }
-        for (int i = threadIdx.x; i < 3 * (kWgSeg + 2) * 16; i += 256) {
-            const int c = i % 16, px = (i / 16) % (kWgSeg + 2), dy = i / (16 * (kWgSeg + 2));
-            const int hh = h + dy - 1, ww = w0 + px - 1;
-            sx[dy][px][c] = (hh >= 0 && hh < H && ww >= 0 && ww < W)
-                                ? bf(X[(((size_t)im * H + hh) * W + ww) * CX + cx0 + c])
-                                : 0.f;
-        }
-        __syncthreads();
-        for (int px = 0; px < kWgSeg; ++px) {
-            const float g = sg[px][ty];
-            bacc += g;
-#pragma unroll
-            for (int t = 0; t < 9; ++t) acc[t] = fmaf(g, sx[t / 3][px + t % 3][tx], acc[t]);
-        }
-    }
-    const size_t base = (size_t)blockIdx.x * 9 * N * Cin;
-#pragma unroll
-    for (int t = 0; t < 9; ++t) part[base + ((size_t)t * N + co0 + ty) * Cin + ci0 + tx] = acc[t];
-    if (blockIdx.z == 0 && tx == 0) bpart[(size_t)blockIdx.x * N + co0 + ty] = bacc;
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr));
+}
+__device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
+{
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// 16-byte copy, or 16 zero bytes where !on.
+__device__ __forceinline__ void cp16_or_zero(uint32_t dst, const void *src, bool on)
+{
+    const int n = on ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
 }
 
-// out[i] = sum over s < nsplit of part[s][i], in order of s.
-__global__ void k_sum_parts(const float *__restrict__ part, int nsplit, size_t len, float *__restrict__ out)
+// Byte offset of 16-byte piece `ch` of pixel px in a row of PC pieces per pixel.
+template <int PC>
+__device__ __forceinline__ uint32_t wg_off(int px, int ch)
 {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= len) return;
+    const int sw = PC == 2 ? (px >> 2) & 1 : PC == 4 ? (px >> 1) & 3 : px & 7;
+    return (uint32_t)((px * PC + (ch ^ sw)) * 16);
+}
+
+template <int WCO, int MC, int MI, int KW>
+struct WgShape {
+    static_assert(MC * MI * KW == 4, "four warps");
+    static constexpr int CO = 16 * WCO * MC, CI = 16 * MI, GC = CO / 8, XC = CI / 8;
+    static constexpr int XB = (kWgStrip + 2) * XC * 16, GB = kWgStrip * GC * 16;   // bytes of a staged row
+    static constexpr int SMEM = kWgXRows * XB + kWgGRows * GB;
+};
+
+template <int WCO, int MC, int MI, int KW>
+__global__ void __launch_bounds__(128) k_wgrad3x3(const __nv_bfloat16 *__restrict__ X0, int c0,
+                                                   const __nv_bfloat16 *__restrict__ X1, int c1,
+                                                   const __nv_bfloat16 *__restrict__ gz, int N, int n, int H, int W,
+                                                   float *__restrict__ part, float *__restrict__ bpart)
+{
+    using S = WgShape<WCO, MC, MI, KW>;
+    extern __shared__ __align__(128) unsigned char wg_smem[];
+    const uint32_t sx = (uint32_t)__cvta_generic_to_shared(wg_smem), sg = sx + kWgXRows * S::XB;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int kw = warp % KW, mi = (warp / KW) % MI, mc = warp / (KW * MI);
+    const int co0 = blockIdx.y * S::CO, ci0 = blockIdx.z * S::CI, Cin = c0 + c1;
+    const bool second = ci0 >= c0;                       // tiles do not straddle the inputs
+    const __nv_bfloat16 *X = second ? X1 + (ci0 - c0) : X0 + ci0;
+    const int CX = second ? c1 : c0;
+    const bool bias = blockIdx.z == 0 && mi == 0;
+    // ldmatrix addresses within a row: gz pieces (pixel, co), X pieces (pixel + dx, ci).
+    const int lr = lane & 7, lm = lane >> 3;
+    uint32_t aoff[WCO], xoff[3];
+#pragma unroll
+    for (int v = 0; v < WCO; ++v) aoff[v] = wg_off<S::GC>(lr + 8 * (lm >> 1), 2 * (mc * WCO + v) + (lm & 1));
+#pragma unroll
+    for (int dx = 0; dx < 3; ++dx) xoff[dx] = wg_off<S::XC>(lr + 8 * (lm & 1) + dx, 2 * mi + (lm >> 1));
+    float acc[WCO][9][2][4], bacc[WCO][4];
+#pragma unroll
+    for (int v = 0; v < WCO; ++v) {
+#pragma unroll
+        for (int t = 0; t < 9; ++t)
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) acc[v][t][j][q] = 0.f;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) bacc[v][q] = 0.f;
+    }
+    const int strips = (W + kWgStrip - 1) / kWgStrip;
+    const long long rows = (long long)n * strips * H;    // (image, strip, row), row fastest
+    long long r = rows * blockIdx.x / gridDim.x;
+    const long long r_end = rows * (blockIdx.x + 1) / gridDim.x;
+    while (r < r_end) {
+        const int h0 = (int)(r % H), w0 = (int)((r / H) % strips) * kWgStrip, im = (int)(r / ((long long)H * strips));
+        const int cnt = (int)min((long long)(H - h0), r_end - r);
+        auto load_x = [&](int j) {                       // row h0 + j (j >= -1) into slot (j + 1) % kWgXRows
+            const int hh = h0 + j;
+            const uint32_t dst = sx + ((j + 1) % kWgXRows) * S::XB;
+            const bool in = hh >= 0 && hh < H;
+            const __nv_bfloat16 *src = X + ((size_t)im * H + (in ? hh : 0)) * W * CX;
+            for (int i = tid; i < (kWgStrip + 2) * S::XC; i += 128) {
+                const int px = i / S::XC, ch = i % S::XC, ww = w0 + px - 1;
+                const bool on = in && ww >= 0 && ww < W;
+                cp16_or_zero(dst + wg_off<S::XC>(px, ch), src + (on ? (size_t)ww * CX + 8 * ch : 0), on);
+            }
+        };
+        auto load_g = [&](int j) {
+            const uint32_t dst = sg + (j % kWgGRows) * S::GB;
+            const __nv_bfloat16 *src = gz + ((size_t)im * H + h0 + j) * W * N + co0;
+            for (int i = tid; i < kWgStrip * S::GC; i += 128) {
+                const int px = i / S::GC, ch = i % S::GC, ww = w0 + px;
+                const bool on = ww < W;
+                cp16_or_zero(dst + wg_off<S::GC>(px, ch), src + (on ? (size_t)ww * N + 8 * ch : 0), on);
+            }
+        };
+        auto issue = [&](int j) {                        // what step j needs beyond step j - 1
+            if (j < cnt) {
+                load_x(j + 1);
+                load_g(j);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        __syncthreads();                                 // the last strip's rows are consumed
+        load_x(-1);
+        load_x(0);
+        issue(0);
+        issue(1);
+        for (int j = 0; j < cnt; ++j) {
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncthreads();                             // step j has landed, step j - 1 is consumed
+            issue(j + 2);
+            const uint32_t grow = sg + (j % kWgGRows) * S::GB;
+#pragma unroll
+            for (int k = 0; k < kWgStrip / 16 / KW; ++k) {
+                const int ks = k * KW + kw;
+                uint32_t a[WCO][4];
+#pragma unroll
+                for (int v = 0; v < WCO; ++v) ldsm_t(a[v], grow + aoff[v] + ks * 16 * S::GC * 16);
+                if (bias) {
+#pragma unroll
+                    for (int v = 0; v < WCO; ++v) mma_16816(bacc[v], a[v], 0x3f803f80u, 0x3f803f80u);   // times one
+                }
+#pragma unroll
+                for (int dy = 0; dy < 3; ++dy) {
+                    const uint32_t xrow = sx + ((j + dy) % kWgXRows) * S::XB + ks * 16 * S::XC * 16;
+#pragma unroll
+                    for (int dx = 0; dx < 3; ++dx) {
+                        uint32_t b[4];
+                        ldsm_t(b, xrow + xoff[dx]);
+#pragma unroll
+                        for (int v = 0; v < WCO; ++v) {
+                            mma_16816(acc[v][3 * dy + dx][0], a[v], b[0], b[1]);
+                            mma_16816(acc[v][3 * dy + dx][1], a[v], b[2], b[3]);
+                        }
+                    }
+                }
+            }
+        }
+        r += cnt;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    // Accumulator (g, t): rows co = g, g + 8, columns ci = 2t, 2t + 1 of each half.
+    const size_t ps = (size_t)blockIdx.x * KW + kw;
+    const int g = lane >> 2, t2 = 2 * (lane & 3);
+#pragma unroll
+    for (int v = 0; v < WCO; ++v) {
+        const int co = co0 + (mc * WCO + v) * 16 + g, ci = ci0 + mi * 16 + t2;
+#pragma unroll
+        for (int t = 0; t < 9; ++t)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                float *o = part + ((ps * 9 + t) * N + co) * Cin + ci + 8 * j;
+                *reinterpret_cast<float2 *>(o) = make_float2(acc[v][t][j][0], acc[v][t][j][1]);
+                *reinterpret_cast<float2 *>(o + (size_t)8 * Cin) = make_float2(acc[v][t][j][2], acc[v][t][j][3]);
+            }
+        if (bias && t2 == 0) {
+            bpart[ps * N + co] = bacc[v][0];
+            bpart[ps * N + co + 8] = bacc[v][2];
+        }
+    }
+}
+
+// out[i] = sum over s < nsplit of part[s][i]: 32 outputs a block, warp w takes
+// the parts s = w, w + 8, ... in order, and the eight sums are added in order.
+__global__ void __launch_bounds__(256) k_sum_parts(const float *__restrict__ part, int nsplit, size_t len, float *__restrict__ out)
+{
+    __shared__ float red[8][32];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const size_t i = (size_t)blockIdx.x * 32 + lane;
     float a = 0.f;
-    for (int s = 0; s < nsplit; ++s) a += part[(size_t)s * len + i];
-    out[i] = a;
+    if (i < len) {
+#pragma unroll 8
+        for (int s = w; s < nsplit; s += 8) a += part[(size_t)s * len + i];
+    }
+    red[w][lane] = a;
+    __syncthreads();
+    if (w == 0 && i < len) {
+#pragma unroll
+        for (int k = 1; k < 8; ++k) a += red[k][lane];
+        out[i] = a;
+    }
 }
 
 // ------------------------------------------------------------ output layer

@@ -95,8 +95,48 @@ size_t layout_params(std::vector<TcLayer> *layers, size_t *out_w)
     return off;
 }
 
-// Scratch sizes of the weight-gradient reduction (splits per layer).
-int wgrad_splits(int N, int Cin) { return std::max(1, std::min(256, 1184 / ((N / 16) * (Cin / 16)))); }
+// Launch of k_wgrad3x3 for one layer: its tile and the shares of the rows, for
+// about three CTAs of four warps per SM over all tiles, each share at least
+// four rows long.  The tile is the widest that divides the layer's channels
+// (and, for a concatenated input, both inputs).
+struct WgPlan {
+    int kind, co, ci, kw;    // template instance, tile, partial sums per CTA
+    int splits(int N, int Cin, long long rows) const
+    {
+        const int tiles = (N / co) * (Cin / ci);
+        return (int)std::max<long long>(1, std::min<long long>((444 + tiles - 1) / tiles, rows / 4));
+    }
+};
+WgPlan wgrad_plan(int N, int cin0, int cin1)
+{
+    const bool ci32 = cin0 % 32 == 0 && cin1 % 32 == 0;
+    if (N % 64 == 0 && ci32) return {3, 64, 32, 1};
+    if (N % 32 == 0 && ci32) return {2, 32, 32, 2};
+    if (N % 32 == 0) return {1, 32, 16, 4};
+    return {0, 16, 16, 4};
+}
+long long wgrad_rows(int S, int H, int W) { return (long long)S * H * ((W + ws::kWgStrip - 1) / ws::kWgStrip); }
+
+template <int WCO, int MC, int MI, int KW>
+cudaError_t wgrad_go(dim3 grid, cudaStream_t st, const __nv_bfloat16 *X0, int c0, const __nv_bfloat16 *X1, int c1,
+                     const __nv_bfloat16 *gz, int N, int n, int H, int W, float *part, float *bpart)
+{
+    constexpr int smem = ws::WgShape<WCO, MC, MI, KW>::SMEM;
+    const auto k = ws::k_wgrad3x3<WCO, MC, MI, KW>;
+    if (smem > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return e;
+    }
+    k<<<grid, 128, smem, st>>>(X0, c0, X1, c1, gz, N, n, H, W, part, bpart);
+    return cudaGetLastError();
+}
+
+// Blocks of the first layer's weight gradient.
+unsigned in_wgrad_blocks(int n, int H, int W)
+{
+    const long long tiles = (long long)n * ((W + ws::kInCols - 1) / ws::kInCols) * ((H + ws::kInRows - 1) / ws::kInRows);
+    return (unsigned)std::min<long long>(tiles, 592);
+}
 
 struct Img {
     bf16 *p = nullptr;
@@ -152,7 +192,7 @@ struct icon_ws {
     size_t nparam = 0, out_off = 0;
     float *params = nullptr, *grads = nullptr, *am = nullptr, *av = nullptr;
     float *x = nullptr, *t = nullptr, *y = nullptr, *dy = nullptr, *in_scale = nullptr;
-    double *ss = nullptr, *lpart = nullptr;
+    double *ss = nullptr, *sspart = nullptr, *lpart = nullptr;
     float *part = nullptr, *bpart = nullptr;
     size_t part_len = 0, bpart_len = 0;
     // activations and their gradients
@@ -199,7 +239,8 @@ struct icon_ws {
 
     icon_status forward(const float2 *Ahwb, int S, cudaStream_t st)
     {
-        ws::k_slice_sumsq<<<S, 256, 0, st>>>(Ahwb, N0, N1, ss);
+        ws::k_slice_sumsq<<<dim3(ws::kSumSqChunks, S), 256, 0, st>>>(Ahwb, N0, N1, sspart);
+        ws::k_slice_sumsq_fin<<<S, 32, 0, st>>>(sspart, ss);
         const size_t npix = (size_t)S * Hp * Wp;
         ws::k_net_input<<<grid1(npix, 256), 256, 0, st>>>(Ahwb, ss, N0, N1, Hp, Wp, S, x, in_scale);
         ws::k_conv_in<<<grid1(npix, 128), 128, 0, st>>>(x, params + kInW, params + kInB, S, Hp, Wp, e0a.p);
@@ -238,18 +279,23 @@ struct icon_ws {
         const size_t cnt8 = (size_t)S * out.H * out.W * out.C / 8;
         ws::k_relu_bwd<<<grid1(cnt8, 256), 256, 0, st>>>(gout.p, out.p, cnt8);
         const int Cin = L.cin0 + L.cin1;
-        const int segs = (out.W + ws::kWgSeg - 1) / ws::kWgSeg;
-        const long long items = (long long)S * out.H * segs;
-        int nsplit = wgrad_splits(L.N, Cin);
-        if (nsplit > items) nsplit = (int)items;
+        const WgPlan wp = wgrad_plan(L.N, L.cin0, L.cin1);
+        const int nsplit = wp.splits(L.N, Cin, wgrad_rows(S, out.H, out.W)), nparts = nsplit * wp.kw;
         const size_t wlen = (size_t)9 * L.N * Cin;
-        if ((size_t)nsplit * wlen > part_len || (size_t)nsplit * L.N > bpart_len)
+        if ((size_t)nparts * wlen > part_len || (size_t)nparts * L.N > bpart_len)
             return net_fail(ICON_ERR_INVALID, "warm start: weight-gradient scratch too small");
-        dim3 g(nsplit, L.N / 16, Cin / 16);
-        ws::k_wgrad3x3<<<g, 256, 0, st>>>(in0.p, L.cin0, in1 ? in1->p : nullptr, L.cin1, gout.p, L.N, S, out.H,
-                                           out.W, nsplit, part, bpart);
-        ws::k_sum_parts<<<grid1(wlen, 256), 256, 0, st>>>(part, nsplit, wlen, grads + L.w_off);
-        ws::k_sum_parts<<<grid1(L.N, 256), 256, 0, st>>>(bpart, nsplit, L.N, grads + L.b_off);
+        const dim3 g(nsplit, L.N / wp.co, Cin / wp.ci);
+        const bf16 *x1 = in1 ? in1->p : nullptr;
+        cudaError_t e = cudaSuccess;
+        switch (wp.kind) {
+        case 0: e = wgrad_go<1, 1, 1, 4>(g, st, in0.p, L.cin0, x1, L.cin1, gout.p, L.N, S, out.H, out.W, part, bpart); break;
+        case 1: e = wgrad_go<2, 1, 1, 4>(g, st, in0.p, L.cin0, x1, L.cin1, gout.p, L.N, S, out.H, out.W, part, bpart); break;
+        case 2: e = wgrad_go<2, 1, 2, 2>(g, st, in0.p, L.cin0, x1, L.cin1, gout.p, L.N, S, out.H, out.W, part, bpart); break;
+        default: e = wgrad_go<2, 2, 2, 1>(g, st, in0.p, L.cin0, x1, L.cin1, gout.p, L.N, S, out.H, out.W, part, bpart); break;
+        }
+        NET_CUDA(e);
+        ws::k_sum_parts<<<grid1(wlen, 32), 256, 0, st>>>(part, nparts, wlen, grads + L.w_off);
+        ws::k_sum_parts<<<grid1(L.N, 32), 256, 0, st>>>(bpart, nparts, L.N, grads + L.b_off);
         NET_CUDA(cudaGetLastError());
         if (gin0)
             NET_TRY(ws_conv3x3_launch(gout.p, L.N, nullptr, 0, S, out.H, out.W, L.wt, nullptr, Cin, 0, gin0->p,
@@ -276,7 +322,7 @@ struct icon_ws {
             const unsigned nb = grid1(npix, 256);
             if ((size_t)nb * 17 > part_len) return net_fail(ICON_ERR_INVALID, "warm start: output scratch too small");
             ws::k_conv_out_bwd<<<nb, 256, 0, st>>>(d0.p, dy, params + out_off, npix, g_d0.p, part);
-            ws::k_sum_parts<<<1, 32, 0, st>>>(part, (int)nb, 17, grads + out_off);
+            ws::k_sum_parts<<<1, 256, 0, st>>>(part, (int)nb, 17, grads + out_off);
         }
         NET_TRY(layer_bwd(D0B, g_d0, d0, d0a, nullptr, &g_d0a, 0, nullptr, S, st));
         NET_TRY(layer_bwd(D0A, g_d0a, d0a, u0, &e0, &g_u0, 0, &g_e0, S, st));
@@ -300,12 +346,11 @@ struct icon_ws {
         {
             const size_t cnt8 = (size_t)S * Hp * Wp * 16 / 8;
             ws::k_relu_bwd<<<grid1(cnt8, 256), 256, 0, st>>>(g_e0a.p, e0a.p, cnt8);
-            const int per = 2048;
-            const unsigned nb = grid1(npix, per);
+            const unsigned nb = in_wgrad_blocks(S, Hp, Wp);
             if ((size_t)nb * 160 > part_len)
                 return net_fail(ICON_ERR_INVALID, "warm start: input-layer scratch too small");
-            ws::k_conv_in_wgrad<<<nb, 160, 0, st>>>(x, g_e0a.p, S, Hp, Wp, per, part);
-            ws::k_sum_parts<<<1, 160, 0, st>>>(part, (int)nb, 160, grads + kInW);
+            ws::k_conv_in_wgrad<<<nb, 48 * ws::kInGroups, 0, st>>>(x, g_e0a.p, S, Hp, Wp, part);
+            ws::k_sum_parts<<<grid1(160, 32), 256, 0, st>>>(part, (int)nb, 160, grads + kInW);
         }
         NET_CUDA(cudaGetLastError());
         return ICON_OK;
@@ -377,12 +422,15 @@ icon_status icon_ws_create(icon_plan *plan, int capacity, icon_ws **out)
     NET_TRY(M.alloc(&w->dy, npix));
     NET_TRY(M.alloc(&w->in_scale, capacity));
     NET_TRY(M.alloc(&w->ss, capacity));
+    NET_TRY(M.alloc(&w->sspart, (size_t)capacity * ws::kSumSqChunks));
     NET_TRY(M.alloc(&w->lpart, grid1(npix, 256)));
-    size_t need = std::max<size_t>((size_t)grid1(npix, 256) * 17, (size_t)grid1(npix, 2048) * 160), bneed = 0;
-    for (auto &L : w->layers) {
-        const int Cin = L.cin0 + L.cin1, ns = wgrad_splits(L.N, Cin);
-        need = std::max(need, (size_t)ns * 9 * L.N * Cin);
-        bneed = std::max(bneed, (size_t)ns * L.N);
+    size_t need = std::max<size_t>((size_t)grid1(npix, 256) * 17, (size_t)592 * 160), bneed = 0;
+    for (auto &L : w->layers) {   // the most partial sums any batch makes
+        const int Cin = L.cin0 + L.cin1;
+        const WgPlan wp = wgrad_plan(L.N, L.cin0, L.cin1);
+        const size_t np = (size_t)wp.splits(L.N, Cin, 1LL << 40) * wp.kw;
+        need = std::max(need, np * 9 * L.N * Cin);
+        bneed = std::max(bneed, np * L.N);
     }
     w->part_len = need;
     w->bpart_len = bneed;
