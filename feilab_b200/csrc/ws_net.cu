@@ -119,7 +119,7 @@ long long wgrad_rows(int S, int H, int W) { return (long long)S * H * ((W + ws::
 
 template <int WCO, int MC, int MI, int KW>
 cudaError_t wgrad_go(dim3 grid, cudaStream_t st, const __nv_bfloat16 *X0, int c0, const __nv_bfloat16 *X1, int c1,
-                     const __nv_bfloat16 *gz, int N, int n, int H, int W, float *part, float *bpart)
+                     const __nv_bfloat16 *gz, int N, int n, int H, int W, float *part)
 {
     constexpr int smem = ws::WgShape<WCO, MC, MI, KW>::SMEM;
     const auto k = ws::k_wgrad3x3<WCO, MC, MI, KW>;
@@ -127,7 +127,7 @@ cudaError_t wgrad_go(dim3 grid, cudaStream_t st, const __nv_bfloat16 *X0, int c0
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return e;
     }
-    k<<<grid, 128, smem, st>>>(X0, c0, X1, c1, gz, N, n, H, W, part, bpart);
+    k<<<grid, 128, smem, st>>>(X0, c0, X1, c1, gz, N, n, H, W, part);
     return cudaGetLastError();
 }
 
@@ -193,8 +193,8 @@ struct icon_ws {
     float *params = nullptr, *grads = nullptr, *am = nullptr, *av = nullptr;
     float *x = nullptr, *t = nullptr, *y = nullptr, *dy = nullptr, *in_scale = nullptr;
     double *ss = nullptr, *sspart = nullptr, *lpart = nullptr;
-    float *part = nullptr, *bpart = nullptr;
-    size_t part_len = 0, bpart_len = 0;
+    float *part = nullptr;
+    size_t part_len = 0;
     // activations and their gradients
     Img e0a, e0, u0, d0a, d0, p0, e1a, e1, u1, d1a, d1, p1, e2a, e2, u2, d2a, d2, p2, ba, b;
     Img g_e0a, g_e0, g_u0, g_d0a, g_d0, g_p0, g_e1a, g_e1, g_u1, g_d1a, g_d1, g_p1, g_e2a, g_e2, g_u2, g_d2a, g_d2,
@@ -269,6 +269,11 @@ struct icon_ws {
         return ICON_OK;
     }
 
+    void sum_parts(int n, size_t len, float *out, cudaStream_t st)
+    {
+        ws::k_sum_parts<<<grid1(len, 32), 32 * ws::kSumWarps, 0, st>>>(part, n, len, out);
+    }
+
     // Gradients of one 3x3 layer: ReLU backward of gout in place, weight and
     // bias gradients, and (when gin0) the input gradient split over gin0 /
     // gin1 (acc0: add to gin0).
@@ -282,20 +287,19 @@ struct icon_ws {
         const WgPlan wp = wgrad_plan(L.N, L.cin0, L.cin1);
         const int nsplit = wp.splits(L.N, Cin, wgrad_rows(S, out.H, out.W)), nparts = nsplit * wp.kw;
         const size_t wlen = (size_t)9 * L.N * Cin;
-        if ((size_t)nparts * wlen > part_len || (size_t)nparts * L.N > bpart_len)
+        if ((size_t)nparts * (wlen + L.N) > part_len)
             return net_fail(ICON_ERR_INVALID, "warm start: weight-gradient scratch too small");
         const dim3 g(nsplit, L.N / wp.co, Cin / wp.ci);
         const bf16 *x1 = in1 ? in1->p : nullptr;
         cudaError_t e = cudaSuccess;
         switch (wp.kind) {
-        case 0: e = wgrad_go<1, 1, 1, 4>(g, st, in0.p, L.cin0, x1, L.cin1, gout.p, L.N, S, out.H, out.W, part, bpart); break;
-        case 1: e = wgrad_go<2, 1, 1, 4>(g, st, in0.p, L.cin0, x1, L.cin1, gout.p, L.N, S, out.H, out.W, part, bpart); break;
-        case 2: e = wgrad_go<2, 1, 2, 2>(g, st, in0.p, L.cin0, x1, L.cin1, gout.p, L.N, S, out.H, out.W, part, bpart); break;
-        default: e = wgrad_go<2, 2, 2, 1>(g, st, in0.p, L.cin0, x1, L.cin1, gout.p, L.N, S, out.H, out.W, part, bpart); break;
+        case 0: e = wgrad_go<1, 1, 1, 4>(g, st, in0.p, L.cin0, x1, L.cin1, gout.p, L.N, S, out.H, out.W, part); break;
+        case 1: e = wgrad_go<2, 1, 1, 4>(g, st, in0.p, L.cin0, x1, L.cin1, gout.p, L.N, S, out.H, out.W, part); break;
+        case 2: e = wgrad_go<2, 1, 2, 2>(g, st, in0.p, L.cin0, x1, L.cin1, gout.p, L.N, S, out.H, out.W, part); break;
+        default: e = wgrad_go<2, 2, 2, 1>(g, st, in0.p, L.cin0, x1, L.cin1, gout.p, L.N, S, out.H, out.W, part); break;
         }
         NET_CUDA(e);
-        ws::k_sum_parts<<<grid1(wlen, 32), 256, 0, st>>>(part, nparts, wlen, grads + L.w_off);
-        ws::k_sum_parts<<<grid1(L.N, 32), 256, 0, st>>>(bpart, nparts, L.N, grads + L.b_off);
+        sum_parts(nparts, wlen + L.N, grads + L.w_off, st);   // the bias follows the weights in both
         NET_CUDA(cudaGetLastError());
         if (gin0)
             NET_TRY(ws_conv3x3_launch(gout.p, L.N, nullptr, 0, S, out.H, out.W, L.wt, nullptr, Cin, 0, gin0->p,
@@ -319,10 +323,10 @@ struct icon_ws {
     {
         const size_t npix = (size_t)S * Hp * Wp;
         {
-            const unsigned nb = grid1(npix, 256);
+            const unsigned nb = std::min<unsigned>(grid1(npix, 256), ws::kOutBlocks);
             if ((size_t)nb * 17 > part_len) return net_fail(ICON_ERR_INVALID, "warm start: output scratch too small");
             ws::k_conv_out_bwd<<<nb, 256, 0, st>>>(d0.p, dy, params + out_off, npix, g_d0.p, part);
-            ws::k_sum_parts<<<1, 256, 0, st>>>(part, (int)nb, 17, grads + out_off);
+            sum_parts((int)nb, 17, grads + out_off, st);
         }
         NET_TRY(layer_bwd(D0B, g_d0, d0, d0a, nullptr, &g_d0a, 0, nullptr, S, st));
         NET_TRY(layer_bwd(D0A, g_d0a, d0a, u0, &e0, &g_u0, 0, &g_e0, S, st));
@@ -350,7 +354,7 @@ struct icon_ws {
             if ((size_t)nb * 160 > part_len)
                 return net_fail(ICON_ERR_INVALID, "warm start: input-layer scratch too small");
             ws::k_conv_in_wgrad<<<nb, 48 * ws::kInGroups, 0, st>>>(x, g_e0a.p, S, Hp, Wp, part);
-            ws::k_sum_parts<<<grid1(160, 32), 256, 0, st>>>(part, (int)nb, 160, grads + kInW);
+            sum_parts((int)nb, 160, grads + kInW, st);
         }
         NET_CUDA(cudaGetLastError());
         return ICON_OK;
@@ -424,18 +428,15 @@ icon_status icon_ws_create(icon_plan *plan, int capacity, icon_ws **out)
     NET_TRY(M.alloc(&w->ss, capacity));
     NET_TRY(M.alloc(&w->sspart, (size_t)capacity * ws::kSumSqChunks));
     NET_TRY(M.alloc(&w->lpart, grid1(npix, 256)));
-    size_t need = std::max<size_t>((size_t)grid1(npix, 256) * 17, (size_t)592 * 160), bneed = 0;
+    size_t need = (size_t)ws::kOutBlocks * 160;
     for (auto &L : w->layers) {   // the most partial sums any batch makes
         const int Cin = L.cin0 + L.cin1;
         const WgPlan wp = wgrad_plan(L.N, L.cin0, L.cin1);
         const size_t np = (size_t)wp.splits(L.N, Cin, 1LL << 40) * wp.kw;
-        need = std::max(need, np * 9 * L.N * Cin);
-        bneed = std::max(bneed, np * L.N);
+        need = std::max(need, np * (9 * Cin + 1) * L.N);
     }
     w->part_len = need;
-    w->bpart_len = bneed;
     NET_TRY(M.alloc(&w->part, need));
-    NET_TRY(M.alloc(&w->bpart, bneed));
     struct A {
         Img *m, *g;
         int level, C;
