@@ -3,6 +3,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -112,7 +113,7 @@ int *device_err_flag()
 icon_status ws_conv3x3_launch(const void *in0, int cin0, const void *in1, int cin1, int nimg, int H, int W,
                               const void *w, const float *bias, int N, int relu, void *out0, int nsplit, int acc0,
                               void *out1, int acc1, cudaStream_t st, unsigned long long wait_ns = ws::kWaitNs,
-                              int hold = 0)
+                              int hold = 0, int up0 = 0)
 {
     if (!in0 || !w || !out0 || nimg < 1 || H < 1 || W < 1) return ws_fail(ICON_ERR_INVALID, "conv3x3: bad argument");
     if (N < 16 || N > 256 || N % 16) return ws_fail(ICON_ERR_INVALID, "conv3x3: N must be a multiple of 16 in 16..256");
@@ -124,11 +125,6 @@ icon_status ws_conv3x3_launch(const void *in0, int cin0, const void *in1, int ci
         return ws_fail(ICON_ERR_INVALID, "conv3x3: bad output split");
     int *err = device_err_flag();
     if (!err) return ws_fail(ICON_ERR_CUDA, "conv3x3: error flag allocation failed");
-    CUtensorMap m0, m1, mw;
-    icon_status s;
-    if ((s = act_map(&m0, in0, nimg, H, W, cin0, cc)) != ICON_OK) return s;
-    if ((s = act_map(&m1, in1 ? in1 : in0, nimg, H, W, in1 ? cin1 : cin0, cc)) != ICON_OK) return s;
-    if ((s = weight_map(&mw, w, N, cin0 + cin1, cc)) != ICON_OK) return s;
     ws::ConvArgs a;
     a.nin = in1 ? 2 : 1;
     a.cin0 = cin0;
@@ -147,6 +143,34 @@ icon_status ws_conv3x3_launch(const void *in0, int cin0, const void *in1, int ci
     a.err = err;
     a.wait_ns = wait_ns;
     a.hold = hold;
+    if (!hold) {
+        const int cin = cin0 + cin1, th = ws::conv_halo_rows(N, cin);
+        const auto lg = [](int c) { return c == 16 ? 1 : c == 32 ? 2 : c == 64 ? 3 : c == 128 ? 4 : -1; };
+        if (th && lg(cin0) > 0 && (!cin1 || lg(cin1) > 0)) {
+            ws::HaloArgs h{a, (const __nv_bfloat16 *)in0, (const __nv_bfloat16 *)in1, (const __nv_bfloat16 *)w, lg(cin0),
+                           cin1 ? lg(cin1) : 0, up0, nimg};
+            size_t smem = ws::conv_halo_smem(N, cin, th);
+            const long long tiles = (long long)nimg * ((H + th - 1) / th) * ((W + ws::kTileM - 1) / ws::kTileM);
+            // CTAs per SM: shared memory and TMEM (512 columns)
+            uint32_t cols = 32;
+            while ((int)cols < th * N) cols <<= 1;
+            const int per_sm = (int)std::min<size_t>(std::min<size_t>(226 * 1024 / (smem + 1024), 512 / cols), 8);
+            const unsigned grid = (unsigned)std::min<long long>(tiles, 148LL * per_sm);
+            // No more of them on an SM than its TMEM holds at once.
+            smem = std::max<size_t>(smem, 227 * 1024 / (per_sm + 1) - 896);
+            const auto kern = th == 4 ? ws::k_conv3x3_halo<4> : ws::k_conv3x3_halo<2>;
+            WS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024));
+            kern<<<grid, ws::kConvThreads, smem, st>>>(h);
+            WS_CUDA(cudaGetLastError());
+            return ICON_OK;
+        }
+    }
+    if (up0) return ws_fail(ICON_ERR_INVALID, "conv3x3: no kernel for an upsampled input of this size");
+    CUtensorMap m0, m1, mw;
+    icon_status s;
+    if ((s = act_map(&m0, in0, nimg, H, W, cin0, cc)) != ICON_OK) return s;
+    if ((s = act_map(&m1, in1 ? in1 : in0, nimg, H, W, in1 ? cin1 : cin0, cc)) != ICON_OK) return s;
+    if ((s = weight_map(&mw, w, N, cin0 + cin1, cc)) != ICON_OK) return s;
     const size_t smem = ws::conv_smem_bytes(N, cc);
     {
         // The shared-memory limit is a per-device attribute of the kernel.

@@ -91,35 +91,61 @@ __global__ void k_net_output(const float *__restrict__ y, const float *__restric
 }
 
 // ------------------------------------------------------------ first layer
-// 3x3 convolution of the one-channel input to 16 channels, bias, ReLU.
-// w: [9][16] FP32, tap = 3*dy + dx.
-__global__ void k_conv_in(const float *__restrict__ x, const float *__restrict__ w, const float *__restrict__ bias,
-                          int n, int H, int W, __nv_bfloat16 *__restrict__ y)
+// 3x3 convolution of the one-channel input to 16 channels, bias, ReLU; two
+// neighbouring pixels (W is even) a thread, so that a shared-memory load of four
+// weights feeds eight multiply-adds.  w: [9][16] FP32, tap = 3*dy + dx.
+// 8 x 304 x 1024 pixels: 38 us; one pixel a thread and a load per weight took 50.
+__global__ void __launch_bounds__(128) k_conv_in(const float *__restrict__ x, const float *__restrict__ w,
+                                                 const float *__restrict__ bias, int n, int H, int W,
+                                                 __nv_bfloat16 *__restrict__ y)
 {
-    __shared__ float sw[9 * 16 + 16];
+    __shared__ __align__(16) float sw[9 * 16 + 16];
     for (int i = threadIdx.x; i < 9 * 16; i += blockDim.x) sw[i] = w[i];
     for (int i = threadIdx.x; i < 16; i += blockDim.x) sw[144 + i] = bias[i];
     __syncthreads();
-    const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= (size_t)n * H * W) return;
-    const int xw = (int)(p % W), xh = (int)((p / W) % H), im = (int)(p / ((size_t)W * H));
-    float in[9];
+    const size_t p2 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (2 * p2 >= (size_t)n * H * W) return;
+    const int xw = 2 * (int)(p2 % (W / 2)), xh = (int)((p2 / (W / 2)) % H), im = (int)(p2 / ((size_t)(W / 2) * H));
+    float in[3][4];
 #pragma unroll
-    for (int t = 0; t < 9; ++t) {
-        const int hh = xh + t / 3 - 1, ww = xw + t % 3 - 1;
-        in[t] = (hh >= 0 && hh < H && ww >= 0 && ww < W) ? x[((size_t)im * H + hh) * W + ww] : 0.f;
+    for (int r = 0; r < 3; ++r) {
+        const int hh = xh + r - 1;
+        const float *row = x + ((size_t)im * H + hh) * W + xw;
+        const bool on = hh >= 0 && hh < H;
+        const float2 mid = on ? *reinterpret_cast<const float2 *>(row) : make_float2(0.f, 0.f);
+        in[r][0] = on && xw > 0 ? row[-1] : 0.f;
+        in[r][1] = mid.x;
+        in[r][2] = mid.y;
+        in[r][3] = on && xw + 2 < W ? row[2] : 0.f;
     }
-    __align__(16) __nv_bfloat16 o[16];
+    __align__(16) __nv_bfloat16 o[2][16];
 #pragma unroll
-    for (int c = 0; c < 16; ++c) {
-        float a = sw[144 + c];
+    for (int c = 0; c < 16; c += 4) {
+        const float4 b4 = *reinterpret_cast<const float4 *>(sw + 144 + c);
+        float a[2][4] = {{b4.x, b4.y, b4.z, b4.w}, {b4.x, b4.y, b4.z, b4.w}};
 #pragma unroll
-        for (int t = 0; t < 9; ++t) a = fmaf(sw[t * 16 + c], in[t], a);
-        o[c] = tobf(fmaxf(a, 0.f));
+        for (int t = 0; t < 9; ++t) {
+            const float4 w4 = *reinterpret_cast<const float4 *>(sw + t * 16 + c);
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const float v = in[t / 3][t % 3 + q];
+                a[q][0] = fmaf(w4.x, v, a[q][0]);
+                a[q][1] = fmaf(w4.y, v, a[q][1]);
+                a[q][2] = fmaf(w4.z, v, a[q][2]);
+                a[q][3] = fmaf(w4.w, v, a[q][3]);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) o[q][c + k] = tobf(fmaxf(a[q][k], 0.f));
     }
-    uint4 *d = reinterpret_cast<uint4 *>(y + p * 16);
-    d[0] = reinterpret_cast<uint4 *>(o)[0];
-    d[1] = reinterpret_cast<uint4 *>(o)[1];
+    uint4 *d = reinterpret_cast<uint4 *>(y + 2 * p2 * 16);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        d[2 * q] = reinterpret_cast<uint4 *>(o[q])[0];
+        d[2 * q + 1] = reinterpret_cast<uint4 *>(o[q])[1];
+    }
 }
 
 // Weight and bias gradients of the first layer.  A block takes kInRows image
@@ -349,7 +375,7 @@ struct WgShape {
 };
 
 template <int WCO, int MC, int MI, int KW>
-__global__ void __launch_bounds__(128) k_wgrad3x3(const __nv_bfloat16 *__restrict__ X0, int c0,
+__global__ void __launch_bounds__(128) k_wgrad3x3(const __nv_bfloat16 *__restrict__ X0, int c0, int up0,
                                                    const __nv_bfloat16 *__restrict__ X1, int c1,
                                                    const __nv_bfloat16 *__restrict__ gz, int N, int n, int H, int W,
                                                    float *__restrict__ part)
@@ -362,7 +388,7 @@ __global__ void __launch_bounds__(128) k_wgrad3x3(const __nv_bfloat16 *__restric
     const int co0 = blockIdx.y * S::CO, ci0 = blockIdx.z * S::CI, Cin = c0 + c1;
     const bool second = ci0 >= c0;                       // tiles do not straddle the inputs
     const __nv_bfloat16 *X = second ? X1 + (ci0 - c0) : X0 + ci0;
-    const int CX = second ? c1 : c0;
+    const int CX = second ? c1 : c0, up = second ? 0 : up0;   // up0: X0 is read as its 2x nearest upsampling
     const bool bias = blockIdx.z == 0 && mi == 0;
     // ldmatrix addresses within a row: gz pieces (pixel, co), X pieces (pixel + dx, ci).
     const int lr = lane & 7, lm = lane >> 3;
@@ -394,11 +420,11 @@ __global__ void __launch_bounds__(128) k_wgrad3x3(const __nv_bfloat16 *__restric
             const int hh = h0 + j;
             const uint32_t dst = sx + ((j + 1) % kWgXRows) * S::XB;
             const bool in = hh >= 0 && hh < H;
-            const __nv_bfloat16 *src = X + ((size_t)im * H + (in ? hh : 0)) * W * CX;
+            const __nv_bfloat16 *src = X + ((size_t)im * (H >> up) + (in ? hh >> up : 0)) * (W >> up) * CX;
             for (int i = tid; i < (kWgStrip + 2) * S::XC; i += 128) {
                 const int px = i / S::XC, ch = i % S::XC, ww = w0 + px - 1;
                 const bool on = in && ww >= 0 && ww < W;
-                cp16_or_zero(dst + wg_off<S::XC>(px, ch), src + (on ? (size_t)ww * CX + 8 * ch : 0), on);
+                cp16_or_zero(dst + wg_off<S::XC>(px, ch), src + (on ? (ww >> up) * CX + 8 * ch : 0), on);
             }
         };
         auto load_g = [&](int j) {

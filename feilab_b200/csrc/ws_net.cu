@@ -35,7 +35,7 @@ extern "C" void icon_internal_set_error(const char *msg);
 icon_status ws_conv3x3_launch(const void *in0, int cin0, const void *in1, int cin1, int nimg, int H, int W,
                               const void *w, const float *bias, int N, int relu, void *out0, int nsplit, int acc0,
                               void *out1, int acc1, cudaStream_t st, unsigned long long wait_ns = 2000000000ull,
-                              int hold = 0);
+                              int hold = 0, int up0 = 0);
 
 namespace {
 
@@ -118,7 +118,7 @@ WgPlan wgrad_plan(int N, int cin0, int cin1)
 long long wgrad_rows(int S, int H, int W) { return (long long)S * H * ((W + ws::kWgStrip - 1) / ws::kWgStrip); }
 
 template <int WCO, int MC, int MI, int KW>
-cudaError_t wgrad_go(dim3 grid, cudaStream_t st, const __nv_bfloat16 *X0, int c0, const __nv_bfloat16 *X1, int c1,
+cudaError_t wgrad_go(dim3 grid, cudaStream_t st, const __nv_bfloat16 *X0, int c0, int up0, const __nv_bfloat16 *X1, int c1,
                      const __nv_bfloat16 *gz, int N, int n, int H, int W, float *part)
 {
     constexpr int smem = ws::WgShape<WCO, MC, MI, KW>::SMEM;
@@ -127,7 +127,7 @@ cudaError_t wgrad_go(dim3 grid, cudaStream_t st, const __nv_bfloat16 *X0, int c0
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return e;
     }
-    k<<<grid, 128, smem, st>>>(X0, c0, X1, c1, gz, N, n, H, W, part);
+    k<<<grid, 128, smem, st>>>(X0, c0, up0, X1, c1, gz, N, n, H, W, part);
     return cudaGetLastError();
 }
 
@@ -196,7 +196,7 @@ struct icon_ws {
     float *part = nullptr;
     size_t part_len = 0;
     // activations and their gradients
-    Img e0a, e0, u0, d0a, d0, p0, e1a, e1, u1, d1a, d1, p1, e2a, e2, u2, d2a, d2, p2, ba, b;
+    Img e0a, e0, d0a, d0, p0, e1a, e1, u1, d1a, d1, p1, e2a, e2, u2, d2a, d2, p2, ba, b;
     Img g_e0a, g_e0, g_u0, g_d0a, g_d0, g_p0, g_e1a, g_e1, g_u1, g_d1a, g_d1, g_p1, g_e2a, g_e2, g_u2, g_d2a, g_d2,
         g_p2, g_ba, g_b;
 
@@ -218,11 +218,12 @@ struct icon_ws {
         return ICON_OK;
     }
 
-    icon_status conv(int li, const Img &in0, const Img *in1, Img &out, int S, cudaStream_t st)
+    // up0: in0 is the half-size image whose upsampling the layer reads.
+    icon_status conv(int li, const Img &in0, const Img *in1, Img &out, int S, cudaStream_t st, int up0 = 0)
     {
         const TcLayer &L = layers[li];
         return ws_conv3x3_launch(in0.p, in0.C, in1 ? in1->p : nullptr, in1 ? in1->C : 0, S, out.H, out.W, L.wb,
-                                 params + L.b_off, L.N, 1, out.p, L.N, 0, nullptr, 0, st);
+                                 params + L.b_off, L.N, 1, out.p, L.N, 0, nullptr, 0, st, 2000000000ull, 0, up0);
     }
 
     void pool(const Img &in, Img &out, int S, cudaStream_t st)
@@ -243,7 +244,7 @@ struct icon_ws {
         ws::k_slice_sumsq_fin<<<S, 32, 0, st>>>(sspart, ss);
         const size_t npix = (size_t)S * Hp * Wp;
         ws::k_net_input<<<grid1(npix, 256), 256, 0, st>>>(Ahwb, ss, N0, N1, Hp, Wp, S, x, in_scale);
-        ws::k_conv_in<<<grid1(npix, 128), 128, 0, st>>>(x, params + kInW, params + kInB, S, Hp, Wp, e0a.p);
+        ws::k_conv_in<<<grid1(npix / 2, 128), 128, 0, st>>>(x, params + kInW, params + kInB, S, Hp, Wp, e0a.p);
         NET_CUDA(cudaGetLastError());
         NET_TRY(conv(C0B, e0a, nullptr, e0, S, st));
         pool(e0, p0, S, st);
@@ -261,8 +262,7 @@ struct icon_ws {
         up(d2, u1, S, st);
         NET_TRY(conv(D1A, u1, &e1, d1a, S, st));
         NET_TRY(conv(D1B, d1a, nullptr, d1, S, st));
-        up(d1, u0, S, st);
-        NET_TRY(conv(D0A, u0, &e0, d0a, S, st));
+        NET_TRY(conv(D0A, d1, &e0, d0a, S, st, 1));   // d1 upsampled as it is read
         NET_TRY(conv(D0B, d0a, nullptr, d0, S, st));
         ws::k_conv_out<<<grid1(npix, 256), 256, 0, st>>>(d0.p, params + out_off, params + out_off + 16, npix, y);
         NET_CUDA(cudaGetLastError());
@@ -278,7 +278,7 @@ struct icon_ws {
     // bias gradients, and (when gin0) the input gradient split over gin0 /
     // gin1 (acc0: add to gin0).
     icon_status layer_bwd(int li, Img &gout, const Img &out, const Img &in0, const Img *in1, Img *gin0, int acc0,
-                          Img *gin1, int S, cudaStream_t st)
+                          Img *gin1, int S, cudaStream_t st, int up0 = 0)
     {
         const TcLayer &L = layers[li];
         const size_t cnt8 = (size_t)S * out.H * out.W * out.C / 8;
@@ -293,10 +293,10 @@ struct icon_ws {
         const bf16 *x1 = in1 ? in1->p : nullptr;
         cudaError_t e = cudaSuccess;
         switch (wp.kind) {
-        case 0: e = wgrad_go<1, 1, 1, 4>(g, st, in0.p, L.cin0, x1, L.cin1, gout.p, L.N, S, out.H, out.W, part); break;
-        case 1: e = wgrad_go<2, 1, 1, 4>(g, st, in0.p, L.cin0, x1, L.cin1, gout.p, L.N, S, out.H, out.W, part); break;
-        case 2: e = wgrad_go<2, 1, 2, 2>(g, st, in0.p, L.cin0, x1, L.cin1, gout.p, L.N, S, out.H, out.W, part); break;
-        default: e = wgrad_go<2, 2, 2, 1>(g, st, in0.p, L.cin0, x1, L.cin1, gout.p, L.N, S, out.H, out.W, part); break;
+        case 0: e = wgrad_go<1, 1, 1, 4>(g, st, in0.p, L.cin0, up0, x1, L.cin1, gout.p, L.N, S, out.H, out.W, part); break;
+        case 1: e = wgrad_go<2, 1, 1, 4>(g, st, in0.p, L.cin0, up0, x1, L.cin1, gout.p, L.N, S, out.H, out.W, part); break;
+        case 2: e = wgrad_go<2, 1, 2, 2>(g, st, in0.p, L.cin0, up0, x1, L.cin1, gout.p, L.N, S, out.H, out.W, part); break;
+        default: e = wgrad_go<2, 2, 2, 1>(g, st, in0.p, L.cin0, up0, x1, L.cin1, gout.p, L.N, S, out.H, out.W, part); break;
         }
         NET_CUDA(e);
         sum_parts(nparts, wlen + L.N, grads + L.w_off, st);   // the bias follows the weights in both
@@ -329,7 +329,7 @@ struct icon_ws {
             sum_parts((int)nb, 17, grads + out_off, st);
         }
         NET_TRY(layer_bwd(D0B, g_d0, d0, d0a, nullptr, &g_d0a, 0, nullptr, S, st));
-        NET_TRY(layer_bwd(D0A, g_d0a, d0a, u0, &e0, &g_u0, 0, &g_e0, S, st));
+        NET_TRY(layer_bwd(D0A, g_d0a, d0a, d1, &e0, &g_u0, 0, &g_e0, S, st, 1));
         up_bwd(g_u0, g_d1, S, st);
         NET_TRY(layer_bwd(D1B, g_d1, d1, d1a, nullptr, &g_d1a, 0, nullptr, S, st));
         NET_TRY(layer_bwd(D1A, g_d1a, d1a, u1, &e1, &g_u1, 0, &g_e1, S, st));
@@ -440,7 +440,7 @@ icon_status icon_ws_create(icon_plan *plan, int capacity, icon_ws **out)
     struct A {
         Img *m, *g;
         int level, C;
-    } acts[] = {{&w->e0a, &w->g_e0a, 0, 16}, {&w->e0, &w->g_e0, 0, 16},  {&w->u0, &w->g_u0, 0, 32},
+    } acts[] = {{&w->e0a, &w->g_e0a, 0, 16}, {&w->e0, &w->g_e0, 0, 16},  {nullptr, &w->g_u0, 0, 32},
                 {&w->d0a, &w->g_d0a, 0, 16}, {&w->d0, &w->g_d0, 0, 16},  {&w->p0, &w->g_p0, 1, 16},
                 {&w->e1a, &w->g_e1a, 1, 32}, {&w->e1, &w->g_e1, 1, 32},  {&w->u1, &w->g_u1, 1, 64},
                 {&w->d1a, &w->g_d1a, 1, 32}, {&w->d1, &w->g_d1, 1, 32},  {&w->p1, &w->g_p1, 2, 32},
@@ -448,7 +448,7 @@ icon_status icon_ws_create(icon_plan *plan, int capacity, icon_ws **out)
                 {&w->d2a, &w->g_d2a, 2, 64}, {&w->d2, &w->g_d2, 2, 64},  {&w->p2, &w->g_p2, 3, 64},
                 {&w->ba, &w->g_ba, 3, 128},  {&w->b, &w->g_b, 3, 128}};
     for (auto &a : acts) {
-        NET_TRY(w->img(*a.m, a.level, a.C));
+        if (a.m) NET_TRY(w->img(*a.m, a.level, a.C));
         NET_TRY(w->img(*a.g, a.level, a.C));
     }
     *out = w.release();

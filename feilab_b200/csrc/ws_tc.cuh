@@ -150,6 +150,20 @@ __device__ __forceinline__ uint64_t smem_desc_kmajor(uint32_t saddr, int sw)
     return d;
 }
 
+// Shared-memory matrix descriptor of an unswizzled K-major tile: core matrices
+// of 8 rows x 16 bytes stored as 128 consecutive bytes, `lbo` bytes from one
+// to the next along K and 128 bytes along the rows.  Rows are 16 bytes apart
+// throughout, so a tile may start at any row.
+__device__ __forceinline__ uint64_t smem_desc_planar(uint32_t saddr, uint32_t lbo)
+{
+    uint64_t d = 0;
+    d |= (uint64_t)((saddr >> 4) & 0x3FFF);
+    d |= (uint64_t)((lbo >> 4) & 0x3FFF) << 16;               // leading byte offset
+    d |= (uint64_t)(128u >> 4) << 32;                         // stride byte offset
+    d |= (uint64_t)1 << 46;                                   // descriptor version
+    return d;
+}
+
 // Instruction descriptor: kind::f16 with BF16 A and B (both K-major), FP32
 // accumulator, M x N.
 __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N)
