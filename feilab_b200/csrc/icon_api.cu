@@ -601,12 +601,6 @@ icon_status check_plan(const icon_plan *p, int S)
 
 inline int groups(const icon_plan *p, int S) { return (S + p->B - 1) / p->B; }
 
-inline int grid1d(size_t total)
-{
-    size_t b = (total + 255) / 256;
-    return (int)std::min<size_t>(std::max<size_t>(b, 1), 148 * 16);
-}
-
 // ------------------------------------------------------------- stages ----
 // Algorithmic bytes per slot (one slice of a group) of each stage: the data a
 // stage must read and write at least once; per-group tables are divided by B.
@@ -923,7 +917,7 @@ icon_status solve_from_rows_warm(icon_plan *p, const icon_solve_cfg *cfg, int G,
     ICON_TRY(ensure_toeplitz(p, st));
     ICON_TRY(launch_adjoint(p, p->f, G, 0, p->Ahwb, st));
     const size_t NN = (size_t)p->N0 * p->N1;
-    LAUNCH(p, K_LAYOUT, st, icon::k_img_out<float2><<<grid1d((size_t)Sc * NN), 256, 0, st>>>(p->Ahwb, p->ws_A, Sc, p->N0, p->N1, p->B));
+    WITH_B(p->B, LAUNCH(p, K_LAYOUT, st, L::img_out(st, groups(p, Sc), p->Ahwb, p->ws_A, Sc, p->N0, p->N1)))
     ICON_CUDA(cudaGetLastError());
     const int wcap = iconx::ws_capacity(p->ws);
     for (int s0 = 0; s0 < Sc; s0 += wcap)
@@ -932,8 +926,7 @@ icon_status solve_from_rows_warm(icon_plan *p, const icon_solve_cfg *cfg, int G,
     int iters = 0;
     ICON_TRY(icon_solve_warm(p, cfg, p->ws_A, p->ws_m, Sc, &p->wcfg, why.data(), &iters, st));
     for (int s = 0; s < Sc; ++s) (why[s] == ICON_WARM_ACCEPTED ? p->warm_accepted : p->warm_redone)++;
-    const size_t tot = (size_t)G * p->N1 * p->N0 * p->B;
-    LAUNCH(p, K_LAYOUT, st, icon::k_img_in<float><<<grid1d(tot), 256, 0, st>>>(p->ws_m, p->m, Sc, p->N0, p->N1, p->B, tot));
+    WITH_B(p->B, LAUNCH(p, K_LAYOUT, st, L::img_in(st, G, p->ws_m, p->m, Sc, p->N0, p->N1)))
     ICON_CUDA(cudaGetLastError());
     return ICON_OK;
 }
@@ -1311,10 +1304,9 @@ icon_status icon_nufft_forward(icon_plan *p, const float *d_img, void *d_nodes, 
     DeviceGuard guard(p->dev);
     cudaStream_t st = (cudaStream_t)stream;
     int G = groups(p, S);
-    size_t tot = (size_t)G * p->N1 * p->N0 * p->B;
-    LAUNCH(p, K_LAYOUT, st, icon::k_img_in<float><<<grid1d(tot), 256, 0, st>>>(d_img, p->m, S, p->N0, p->N1, p->B, tot));
+    WITH_B(p->B, LAUNCH(p, K_LAYOUT, st, L::img_in(st, G, d_img, p->m, S, p->N0, p->N1)))
     ICON_TRY(launch_forward(p, p->nodes, p->m, true, G, 0, p->f, st));
-    LAUNCH(p, K_LAYOUT, st, icon::k_nodes_out<<<grid1d((size_t)S * p->M), 256, 0, st>>>(p->f, (float2 *)d_nodes, S, p->M, p->B));
+    WITH_B(p->B, LAUNCH(p, K_LAYOUT, st, L::nodes_out(st, G, p->f, (float2 *)d_nodes, S, p->M)))
     ICON_CUDA(cudaGetLastError());
     return ICON_OK;
 }
@@ -1326,10 +1318,9 @@ icon_status icon_nufft_forward_complex(icon_plan *p, const void *d_img, void *d_
     DeviceGuard guard(p->dev);
     cudaStream_t st = (cudaStream_t)stream;
     int G = groups(p, S);
-    size_t tot = (size_t)G * p->N1 * p->N0 * p->B;
-    LAUNCH(p, K_LAYOUT, st, icon::k_img_in<float2><<<grid1d(tot), 256, 0, st>>>((const float2 *)d_img, p->imgc, S, p->N0, p->N1, p->B, tot));
+    WITH_B(p->B, LAUNCH(p, K_LAYOUT, st, L::img_in(st, G, (const float2 *)d_img, p->imgc, S, p->N0, p->N1)))
     ICON_TRY(launch_forward(p, p->nodes, p->imgc, false, G, 0, p->f, st));
-    LAUNCH(p, K_LAYOUT, st, icon::k_nodes_out<<<grid1d((size_t)S * p->M), 256, 0, st>>>(p->f, (float2 *)d_nodes, S, p->M, p->B));
+    WITH_B(p->B, LAUNCH(p, K_LAYOUT, st, L::nodes_out(st, G, p->f, (float2 *)d_nodes, S, p->M)))
     ICON_CUDA(cudaGetLastError());
     return ICON_OK;
 }
@@ -1341,10 +1332,9 @@ icon_status icon_nufft_adjoint(icon_plan *p, const void *d_nodes, void *d_img, i
     DeviceGuard guard(p->dev);
     cudaStream_t st = (cudaStream_t)stream;
     int G = groups(p, S);
-    size_t tot = (size_t)G * p->M * p->B;
-    LAUNCH(p, K_LAYOUT, st, icon::k_nodes_in<<<grid1d(tot), 256, 0, st>>>((const float2 *)d_nodes, p->f, S, p->M, p->B, tot));
+    WITH_B(p->B, LAUNCH(p, K_LAYOUT, st, L::nodes_in(st, G, (const float2 *)d_nodes, p->f, S, p->M)))
     ICON_TRY(launch_adjoint(p, p->f, G, 0, p->imgc, st));
-    LAUNCH(p, K_LAYOUT, st, icon::k_img_out<float2><<<grid1d((size_t)S * p->N0 * p->N1), 256, 0, st>>>(p->imgc, (float2 *)d_img, S, p->N0, p->N1, p->B));
+    WITH_B(p->B, LAUNCH(p, K_LAYOUT, st, L::img_out(st, groups(p, S), p->imgc, (float2 *)d_img, S, p->N0, p->N1)))
     ICON_CUDA(cudaGetLastError());
     return ICON_OK;
 }
@@ -1357,7 +1347,7 @@ icon_status icon_rows_forward(icon_plan *p, const float *d_rows, void *d_b, int 
     cudaStream_t st = (cudaStream_t)stream;
     int G = groups(p, S);
     ICON_TRY(launch_rows(p, d_rows, S, G, p->P, st));   // unweighted b into scratch
-    LAUNCH(p, K_LAYOUT, st, icon::k_nodes_out<<<grid1d((size_t)S * p->M), 256, 0, st>>>(p->P, (float2 *)d_b, S, p->M, p->B));
+    WITH_B(p->B, LAUNCH(p, K_LAYOUT, st, L::nodes_out(st, G, p->P, (float2 *)d_b, S, p->M)))
     ICON_CUDA(cudaGetLastError());
     return ICON_OK;
 }
@@ -1371,7 +1361,7 @@ icon_status icon_prepare_rhs(icon_plan *p, const float *d_rows, void *d_Ahwb, in
     int G = groups(p, S);
     ICON_TRY(launch_rows(p, d_rows, S, G, nullptr, st));
     ICON_TRY(launch_adjoint(p, p->f, G, 0, p->imgc, st));
-    LAUNCH(p, K_LAYOUT, st, icon::k_img_out<float2><<<grid1d((size_t)S * p->N0 * p->N1), 256, 0, st>>>(p->imgc, (float2 *)d_Ahwb, S, p->N0, p->N1, p->B));
+    WITH_B(p->B, LAUNCH(p, K_LAYOUT, st, L::img_out(st, groups(p, S), p->imgc, (float2 *)d_Ahwb, S, p->N0, p->N1)))
     ICON_CUDA(cudaGetLastError());
     return ICON_OK;
 }
@@ -1402,7 +1392,7 @@ icon_status icon_prepare_rhs_stack(icon_plan *p, const float *d_stack, int ny, i
     ICON_TRY(launch_rows_at(p, d_stack + (size_t)y0 * nx, nx, (size_t)ny * nx, skip_section < 0 ? INT_MAX : skip_section,
                             S, G, nullptr, st));
     ICON_TRY(launch_adjoint(p, p->f, G, 0, p->imgc, st));
-    LAUNCH(p, K_LAYOUT, st, icon::k_img_out<float2><<<grid1d((size_t)S * p->N0 * p->N1), 256, 0, st>>>(p->imgc, (float2 *)d_Ahwb, S, p->N0, p->N1, p->B));
+    WITH_B(p->B, LAUNCH(p, K_LAYOUT, st, L::img_out(st, groups(p, S), p->imgc, (float2 *)d_Ahwb, S, p->N0, p->N1)))
     ICON_CUDA(cudaGetLastError());
     return ICON_OK;
 }
@@ -1553,8 +1543,8 @@ icon_status icon_solve(icon_plan *p, const icon_solve_cfg *cfg, const void *d_Ah
     int G = groups(p, S);
     size_t tot = (size_t)G * p->N1 * p->N0 * p->B;
     ICON_TRY(ensure_toeplitz(p, st));
-    LAUNCH(p, K_LAYOUT, st, icon::k_img_in<float2><<<grid1d(tot), 256, 0, st>>>((const float2 *)d_Ahwb, p->Ahwb, S, p->N0, p->N1, p->B, tot));
-    if (warm_start) LAUNCH(p, K_LAYOUT, st, icon::k_img_in<float><<<grid1d(tot), 256, 0, st>>>(d_m, p->m, S, p->N0, p->N1, p->B, tot));
+    WITH_B(p->B, LAUNCH(p, K_LAYOUT, st, L::img_in(st, G, (const float2 *)d_Ahwb, p->Ahwb, S, p->N0, p->N1)))
+    if (warm_start) WITH_B(p->B, LAUNCH(p, K_LAYOUT, st, L::img_in(st, G, d_m, p->m, S, p->N0, p->N1)))
     else ICON_CUDA(cudaMemsetAsync(p->m, 0, tot * sizeof(float), st));
     double *hist = nullptr;
     size_t slots = (size_t)G * p->B;
@@ -1571,7 +1561,7 @@ icon_status icon_solve(icon_plan *p, const icon_solve_cfg *cfg, const void *d_Ah
     if (rc == ICON_OK) rc = flush_update(p, st);
     p->upd_pending = false;
     if (rc == ICON_OK) {
-        LAUNCH(p, K_LAYOUT, st, icon::k_img_out<float><<<grid1d((size_t)S * p->N0 * p->N1), 256, 0, st>>>(p->m, d_m, S, p->N0, p->N1, p->B));
+        WITH_B(p->B, LAUNCH(p, K_LAYOUT, st, L::img_out(st, groups(p, S), p->m, d_m, S, p->N0, p->N1)))
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) rc = fail(ICON_ERR_CUDA, cudaGetErrorString(e));
     }
@@ -1604,13 +1594,13 @@ icon_status icon_solve_until(icon_plan *p, const icon_solve_cfg *cfg, const void
     const int G = groups(p, S);
     const size_t tot = (size_t)G * p->N1 * p->N0 * p->B;
     ICON_TRY(ensure_toeplitz(p, st));
-    LAUNCH(p, K_LAYOUT, st, icon::k_img_in<float2><<<grid1d(tot), 256, 0, st>>>((const float2 *)d_Ahwb, p->Ahwb, S, p->N0, p->N1, p->B, tot));
-    if (warm_start) LAUNCH(p, K_LAYOUT, st, icon::k_img_in<float><<<grid1d(tot), 256, 0, st>>>(d_m, p->m, S, p->N0, p->N1, p->B, tot));
+    WITH_B(p->B, LAUNCH(p, K_LAYOUT, st, L::img_in(st, G, (const float2 *)d_Ahwb, p->Ahwb, S, p->N0, p->N1)))
+    if (warm_start) WITH_B(p->B, LAUNCH(p, K_LAYOUT, st, L::img_in(st, G, d_m, p->m, S, p->N0, p->N1)))
     else ICON_CUDA(cudaMemsetAsync(p->m, 0, tot * sizeof(float), st));
     int done = 0;
     icon_status rc = run_schedule_tol(p, cfg, G, S, tol, check_every, &done, h_step, st);
     if (rc == ICON_OK) {
-        LAUNCH(p, K_LAYOUT, st, icon::k_img_out<float><<<grid1d((size_t)S * p->N0 * p->N1), 256, 0, st>>>(p->m, d_m, S, p->N0, p->N1, p->B));
+        WITH_B(p->B, LAUNCH(p, K_LAYOUT, st, L::img_out(st, groups(p, S), p->m, d_m, S, p->N0, p->N1)))
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) rc = fail(ICON_ERR_CUDA, cudaGetErrorString(e));
     }
@@ -1643,8 +1633,7 @@ icon_status icon_reproject(icon_plan *p, const float *d_m, float tilt_deg, float
     DeviceGuard guard(p->dev);
     cudaStream_t st = (cudaStream_t)stream;
     int G = groups(p, S);
-    size_t tot = (size_t)G * p->N1 * p->N0 * p->B;
-    LAUNCH(p, K_LAYOUT, st, icon::k_img_in<float><<<grid1d(tot), 256, 0, st>>>(d_m, p->m, S, p->N0, p->N1, p->B, tot));
+    WITH_B(p->B, LAUNCH(p, K_LAYOUT, st, L::img_in(st, G, d_m, p->m, S, p->N0, p->N1)))
     ICON_CUDA(cudaGetLastError());
     return reproject_internal(p, p->m, tilt_deg, d_out, S, st);
 }
@@ -1669,7 +1658,7 @@ icon_status icon_reconstruct_host(icon_plan *p, const icon_solve_cfg *cfg, const
         if (e != cudaSuccess) { rc = fail(ICON_ERR_CUDA, cudaGetErrorString(e)); break; }
         if ((rc = launch_rows(p, p->rows, Sc, G, nullptr, st)) != ICON_OK) break;
         if ((rc = solve_from_rows(p, cfg, G, Sc, st)) != ICON_OK) break;
-        LAUNCH(p, K_LAYOUT, st, icon::k_img_out<float><<<grid1d((size_t)Sc * NN), 256, 0, st>>>(p->m, d_mo, Sc, p->N0, p->N1, p->B));
+        WITH_B(p->B, LAUNCH(p, K_LAYOUT, st, L::img_out(st, groups(p, Sc), p->m, d_mo, Sc, p->N0, p->N1)))
         if (h_reproj && (rc = reproject_internal(p, p->m, p->reproj_deg, p->outrp, Sc, st)) != ICON_OK) break;
         if ((e = cudaMemcpyAsync(h_m + (size_t)s0 * NN, d_mo, sizeof(float) * NN * Sc, cudaMemcpyDeviceToHost, st)) != cudaSuccess) {
             rc = fail(ICON_ERR_CUDA, cudaGetErrorString(e));
@@ -1788,7 +1777,7 @@ icon_status plan_stage_out(icon_plan *p, int S, const icon_solve_cfg *cfg, float
         p->upd_G = groups(p, S);
         ICON_TRY(flush_update(p, st));
     }
-    LAUNCH(p, K_LAYOUT, st, icon::k_img_out<float><<<grid1d((size_t)S * p->N0 * p->N1), 256, 0, st>>>(p->m, d_out, S, p->N0, p->N1, p->B));
+    WITH_B(p->B, LAUNCH(p, K_LAYOUT, st, L::img_out(st, groups(p, S), p->m, d_out, S, p->N0, p->N1)))
     ICON_CUDA(cudaGetLastError());
     return ICON_OK;
 }

@@ -198,6 +198,44 @@ void Launch<B>::rows_fwd(int E, dim3 grid, int threads, size_t smem, cudaStream_
     else k_rows_fwd<B, 16><<<grid, threads, smem, st>>>(g, g1, rows, sstride, istride, skip, S, f, bout);
 }
 
+template <int B, typename T, bool IN>
+static void img_move(cudaStream_t st, int G, const T *src, T *dst, int S, int N0, int N1)
+{
+    using I = ImgTile<T, B>;
+    const dim3 grid((N1 + I::TY - 1) / I::TY, (N0 + I::TX - 1) / I::TX, G);
+    k_img_move<T, B, IN><<<grid, 256, 0, st>>>(src, dst, S, N0, N1);
+}
+template <int B>
+void Launch<B>::img_in(cudaStream_t st, int G, const float *src, float *dst, int S, int N0, int N1)
+{
+    img_move<B, float, true>(st, G, src, dst, S, N0, N1);
+}
+template <int B>
+void Launch<B>::img_in(cudaStream_t st, int G, const float2 *src, float2 *dst, int S, int N0, int N1)
+{
+    img_move<B, float2, true>(st, G, src, dst, S, N0, N1);
+}
+template <int B>
+void Launch<B>::img_out(cudaStream_t st, int G, const float *src, float *dst, int S, int N0, int N1)
+{
+    img_move<B, float, false>(st, G, src, dst, S, N0, N1);
+}
+template <int B>
+void Launch<B>::img_out(cudaStream_t st, int G, const float2 *src, float2 *dst, int S, int N0, int N1)
+{
+    img_move<B, float2, false>(st, G, src, dst, S, N0, N1);
+}
+template <int B>
+void Launch<B>::nodes_in(cudaStream_t st, int G, const float2 *src, float2 *dst, int S, int M)
+{
+    k_nodes_in<B><<<dim3((M + 127) / 128, G), 128, 0, st>>>(src, dst, S, M);
+}
+template <int B>
+void Launch<B>::nodes_out(cudaStream_t st, int G, const float2 *src, float2 *dst, int S, int M)
+{
+    k_nodes_out<B><<<dim3((M + 127) / 128, G), 128, 0, st>>>(src, dst, S, M);
+}
+
 template <int B>
 void Launch<B>::img_out_file(dim3 grid, cudaStream_t st, const float *m, float *out, int S, int N0, int N1)
 {

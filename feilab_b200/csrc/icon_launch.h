@@ -33,6 +33,14 @@ struct Launch {
     static void rows_fwd(int E, dim3 grid, int threads, size_t smem, cudaStream_t st, const Geo &g, const Geo1 &g1,
                          const float *rows, size_t sstride, size_t istride, int skip, int S, float2 *f,
                          float2 *bout);
+    // Caller layout <-> batched layout of G groups: images [S][N0][N1] (complex
+    // or real) and nodes [S][M].
+    static void img_in(cudaStream_t st, int G, const float *src, float *dst, int S, int N0, int N1);
+    static void img_in(cudaStream_t st, int G, const float2 *src, float2 *dst, int S, int N0, int N1);
+    static void img_out(cudaStream_t st, int G, const float *src, float *dst, int S, int N0, int N1);
+    static void img_out(cudaStream_t st, int G, const float2 *src, float2 *dst, int S, int N0, int N1);
+    static void nodes_in(cudaStream_t st, int G, const float2 *src, float2 *dst, int S, int M);
+    static void nodes_out(cudaStream_t st, int G, const float2 *src, float2 *dst, int S, int M);
     static void img_out_file(dim3 grid, cudaStream_t st, const float *m, float *out, int S, int N0, int N1);
     static void row_adj(int E, dim3 grid, int threads, size_t smem, cudaStream_t st, const Geo &g, const Geo1 &g1,
                         const float2 *f, float *out, int S);
