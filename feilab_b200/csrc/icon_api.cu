@@ -703,7 +703,7 @@ icon_status launch_iteration(icon_plan *p, int G, bool clamp, int data_type, flo
     ICON_TRY(launch_adjoint(p, p->f, G, 1, p->rhat, st));                       // rhat = A^H f - Ahwb, ||rhat||^2
     ICON_TRY(launch_forward(p, p->nodes, p->rhat, false, G, 2, nullptr, st));   // r = A rhat, sum w|r|^2
     int kb = (p->M * p->B + 255) / 256;
-    LAUNCH(p, K_ALPHA, st, icon::k_alpha<<<G, 32 * p->B, 0, st>>>(p->part_rtr, p->N1, p->part_rtar, kb, p->B, p->alpha, hist_a, hist_r));
+    WITH_B(p->B, LAUNCH(p, K_ALPHA, st, L::alpha(st, G, p->part_rtr, p->N1, p->part_rtar, kb, p->alpha, hist_a, hist_r)))
     int per_group = p->N1 * p->N0 * p->B;
     dim3 gu((unsigned)std::min<size_t>(((size_t)per_group + 255) / 256, 512), G);
     WITH_B(p->B, LAUNCH_B(p, K_UPD, st, stage_bytes(p, p->nodes).upd * G * p->B,
@@ -790,7 +790,7 @@ icon_status launch_iteration_xt_raw(icon_plan *p, int G, bool upd, bool clamp_pr
         LAUNCH_B(p, K_XTM, st, (2 * G1b + NN * 12) * slots, L::xtoep(1, st, G, xa));
         LAUNCH_B(p, K_YQ, st, G1b * slots + Kb * G,
                  L::ypass_toep_quad(p->ey, gy, p->thr_y, p->smem_yt, st, g, p->G1, p->part_rtar)))
-    LAUNCH(p, K_ALPHA, st, icon::k_alpha<<<G, 32 * p->B, 0, st>>>(p->part_rtr, p->N1, p->part_rtar, p->n0, p->B, p->alpha, hist_a, hist_r));
+    WITH_B(p->B, LAUNCH(p, K_ALPHA, st, L::alpha(st, G, p->part_rtr, p->N1, p->part_rtar, p->n0, p->alpha, hist_a, hist_r)))
     ICON_CUDA(cudaGetLastError());
     return ICON_OK;
 }
@@ -830,7 +830,7 @@ icon_status launch_iteration_toep(icon_plan *p, int G, bool clamp, int data_type
         LAUNCH_B(p, K_XF, st, (NN * 8 + G1b) * slots, L::xpass_fwd(false, p->ex, gx, p->thr_x, p->smem_x, st, g, p->rhat, p->G1));
         LAUNCH_B(p, K_YQ, st, G1b * slots + Kb * G,
                  L::ypass_toep_quad(p->ey, gy, p->thr_y, p->smem_yt, st, g, p->G1, p->part_rtar)))
-    LAUNCH(p, K_ALPHA, st, icon::k_alpha<<<G, 32 * p->B, 0, st>>>(p->part_rtr, p->N1, p->part_rtar, p->n0, p->B, p->alpha, hist_a, hist_r));
+    WITH_B(p->B, LAUNCH(p, K_ALPHA, st, L::alpha(st, G, p->part_rtr, p->N1, p->part_rtar, p->n0, p->alpha, hist_a, hist_r)))
     int per_group = p->N1 * p->N0 * p->B;
     dim3 gu((unsigned)std::min<size_t>(((size_t)per_group + 255) / 256, 512), G);
     WITH_B(p->B, LAUNCH_B(p, K_UPD, st, stage_bytes(p, p->nodes).upd * G * p->B,

@@ -198,6 +198,13 @@ void Launch<B>::rows_fwd(int E, dim3 grid, int threads, size_t smem, cudaStream_
     else k_rows_fwd<B, 16><<<grid, threads, smem, st>>>(g, g1, rows, sstride, istride, skip, S, f, bout);
 }
 
+template <int B>
+void Launch<B>::alpha(cudaStream_t st, int G, const double *rtr, int nr, const double *rtar, int na, double *alpha,
+                      double *hist_alpha, double *hist_rtr)
+{
+    k_alpha<B><<<G, kAlphaThreads, 0, st>>>(rtr, nr, rtar, na, alpha, hist_alpha, hist_rtr);
+}
+
 template <int B, typename T, bool IN>
 static void img_move(cudaStream_t st, int G, const T *src, T *dst, int S, int N0, int N1)
 {

@@ -33,6 +33,9 @@ struct Launch {
     static void rows_fwd(int E, dim3 grid, int threads, size_t smem, cudaStream_t st, const Geo &g, const Geo1 &g1,
                          const float *rows, size_t sstride, size_t istride, int skip, int S, float2 *f,
                          float2 *bout);
+    // Step length of G groups from nr and na partial sums per slice.
+    static void alpha(cudaStream_t st, int G, const double *rtr, int nr, const double *rtar, int na, double *alpha,
+                      double *hist_alpha, double *hist_rtr);
     // Caller layout <-> batched layout of G groups: images [S][N0][N1] (complex
     // or real) and nodes [S][M].
     static void img_in(cudaStream_t st, int G, const float *src, float *dst, int S, int N0, int N1);
