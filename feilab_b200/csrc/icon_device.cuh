@@ -458,6 +458,30 @@ __device__ __forceinline__ void dft_nat(float2 (&a)[R], float dir)
     }
 }
 
+// dft_nat of values whose upper half a[R/2..] is zero (and is not read).  For a
+// power of two the first stage only copies; for P = 3 or 5 times one the
+// P-point DFTs take the zeros as literals.
+template <int R>
+__device__ __forceinline__ void dft_half_nat(float2 (&a)[R], float dir)
+{
+    if constexpr ((R & (R - 1)) == 0) {
+        constexpr int L = Lg<R>::v;
+        float2 t[R];
+#pragma unroll
+        for (int r = 0; r < R / 2; ++r) {
+            t[brev5(r) >> (5 - L)] = a[r];
+            t[(brev5(r) >> (5 - L)) + 1] = a[r];
+        }
+        if constexpr (R >= 4) dft_stage<R, 4>(t, dir);
+#pragma unroll
+        for (int r = 0; r < R; ++r) a[r] = t[r];
+    } else {
+#pragma unroll
+        for (int r = R / 2; r < R; ++r) a[r] = make_float2(0.f, 0.f);
+        dft_nat<R>(a, dir);
+    }
+}
+
 // DFT of R values held in registers, a[] given in natural order; on return
 // a[brev(q)] = sum_r x[r] exp(dir*2*pi*i*r*q/R) (brev over log2 R bits): the
 // DIT DFT between two bit reversals that only rename registers, so it

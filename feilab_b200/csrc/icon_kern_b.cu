@@ -139,10 +139,26 @@ cudaError_t Launch<B>::xtoep_prepare(int n0)
     }
 }
 
+template <int B, int R>
+static void yfwd4_go(bool herm, dim3 grid, cudaStream_t st, const Geo &g, const float2 *G1, float2 *P)
+{
+    const int threads = yfwd_threads(R * B, B);
+    const size_t smem = yfwd4_smem(32 * R, B);
+    if (herm) k_yfwd4<B, R, true><<<grid, threads, smem, st>>>(g, G1, P);
+    else k_yfwd4<B, R, false><<<grid, threads, smem, st>>>(g, G1, P);
+}
+
 template <int B>
 void Launch<B>::ypass_fwd(int E, bool herm, dim3 grid, int threads, size_t smem, cudaStream_t st, const Geo &g,
                           const float2 *G1, float2 *P)
 {
+    switch (yadj4_fits(g.n1) ? g.n1 / 32 : 0) {
+    case 4: yfwd4_go<B, 4>(herm, grid, st, g, G1, P); return;
+    case 8: yfwd4_go<B, 8>(herm, grid, st, g, G1, P); return;
+    case 16: yfwd4_go<B, 16>(herm, grid, st, g, G1, P); return;
+    case 32: yfwd4_go<B, 32>(herm, grid, st, g, G1, P); return;
+    default: break;
+    }
     if (E == 32) {
         if (herm) k_ypass_fwd<B, 32, true><<<grid, threads, smem, st>>>(g, G1, P);
         else k_ypass_fwd<B, 32, false><<<grid, threads, smem, st>>>(g, G1, P);
@@ -317,6 +333,14 @@ cudaError_t Launch<B>::set_smem(int ex, int ey, size_t, size_t, size_t, size_t, 
     set((const void *)k_ypass_fwd<B, 16, true>);
     set((const void *)k_ypass_adj<B, 16, false>);
     set((const void *)k_ypass_adj<B, 16, true>);
+    set((const void *)k_yfwd4<B, 4, false>);
+    set((const void *)k_yfwd4<B, 4, true>);
+    set((const void *)k_yfwd4<B, 8, false>);
+    set((const void *)k_yfwd4<B, 8, true>);
+    set((const void *)k_yfwd4<B, 16, false>);
+    set((const void *)k_yfwd4<B, 16, true>);
+    set((const void *)k_yfwd4<B, 32, false>);
+    set((const void *)k_yfwd4<B, 32, true>);
     set((const void *)k_yadj4<B, 4>);
     set((const void *)k_yadj4<B, 8>);
     set((const void *)k_yadj4<B, 16>);

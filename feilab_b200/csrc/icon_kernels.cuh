@@ -314,75 +314,54 @@ __host__ __device__ inline size_t ypass_fwd_smem(int n1, int B)
     return (size_t)(n1 + 2 * kHalo) * sb * sizeof(float2) + ypass_fwd_pre_bytes() + ypass_tw_bytes(n1);
 }
 
-// Forward y-pass fused with the y-direction interpolation.  Row x of G1 holds
-// the N1 nonzero columns; column Y sits at y with (y + N1/2) % n1 == Y.
-// P[G][M][14][B]: P[j][t0] = sum_t1 phiy[j][t1] * G[x][(iy0_j + t1) mod n1],
-// x = (ix0_j + t0) mod n0.  (NU:669-727 sum the same 196 products per node.)
-// The row is copied to shared memory and the tables of the row's first
-// entries are copied behind it; the FFT waits only for the row.  One thread
-// per entry then computes all B slices of it from the rotated row; entries
-// past the copied ones are loaded one round ahead.
-//
-// HERM (the forward transform of a real image, cunfft_trafo_2d_R2C2,
-// NU:984-1076, whose cuFFT R2C keeps half the spectrum): G1 row n0 - x is the
-// conjugate of row x, so its FFT along y is the conjugate mirror of row x's,
-// buf'[q] = conj(buf[-q mod n1]).  The grid then covers rows x = 0..n0/2
-// only; each CTA also interpolates the entries of row n0 - x, reading the 14
-// taps of an entry from the mirrored window in reverse order and storing the
-// conjugate of the sum.  The x-pass writes only rows 0..n0/2 of G1.
-template <int B, int E, bool HERM>
-__global__ void FFT_BOUNDS(E) k_ypass_fwd(Geo g, const float2 *__restrict__ G1, float2 *__restrict__ P)
-{
-    extern __shared__ float2 s[];
-    constexpr int SB = YfStride<B>::v;
-    constexpr bool kPairs = (B == 8);   // 64-byte rows read as 128-byte row pairs
-    const int grp = blockIdx.x, x = blockIdx.y, n = g.n1, N1 = g.N1;
-    const int xp = (g.n0 - x) & (g.n0 - 1);   // the mirror row (HERM)
-    const int T = blockDim.x;
-    const float2 *rowin = G1 + ((size_t)grp * g.n0 + x) * N1 * B;
-    float2 *row = s + kHalo * SB;
-    float *pre_phi = reinterpret_cast<float *>(s + (size_t)(n + 2 * kHalo) * SB);   // [kPreEntries][16]
-    int *pre_jt = reinterpret_cast<int *>(pre_phi + kPreEntries * kLdPhiy);           // [kPreEntries]
-    int *pre_iy = pre_jt + kPreEntries;                                                 // [kPreEntries]
-    float2 *tw_s = reinterpret_cast<float2 *>(pre_iy + kPreEntries);                    // [n] twiddles
-    const float2 *tws = ypass_tw_shared(n) ? tw_s : g.tw1;
-    // Entries: row x's (ca of them), then with HERM and xp != x the mirror
-    // row's (cb); i-th entry of the combined list at global index ent(i).
-    const int ea = g.row_off[x], ca = g.row_off[x + 1] - ea;
-    const int eb = (HERM && xp != x) ? g.row_off[xp] : 0;
-    const int cb = (HERM && xp != x) ? g.row_off[xp + 1] - eb : 0;
-    const int cnt = ca + cb;
-    auto ent = [=](int i) { return i < ca ? ea + i : eb + (i - ca); };
-    const int staged = min(cnt, min(T, kPreEntries));
-    // Group 1: the N1 nonzero values of the row (contiguous in G1) and the
-    // FFT's twiddle table.
-    copy_async(row, rowin, (size_t)N1 * B * sizeof(float2));
-    if (ypass_tw_shared(n)) copy_async(tw_s, g.tw1, (size_t)n * sizeof(float2));
-    cp_async_commit();
-    // Group 2: tables of the first entries.
-    if ((int)threadIdx.x < staged) {
-        const int e = ent(threadIdx.x);
-        const float *src = g.ent_phiy + (size_t)e * kLdPhiy;
-        float *dst = pre_phi + threadIdx.x * kLdPhiy;
-#pragma unroll
-        for (int q = 0; q < kLdPhiy / 4; ++q) cp_async<16>(dst + 4 * q, src + 4 * q);
-        cp_async<4>(pre_jt + threadIdx.x, g.ent_jt + e);
-        cp_async<4>(pre_iy + threadIdx.x, g.ent_iy0 + e);
+// The entries of a CTA of the forward y-pass: row x's (ca of them from ea on),
+// then with HERM and a mirror row of its own that row's (from eb on), cnt in
+// all.  The tables of the first `staged` are in shared memory (copied while
+// the FFT runs): phi windows [.][16], node*16 + x tap, iy0.
+struct YfEntries {
+    int ea, ca, eb, cnt, staged;
+    float *phi;
+    int *jt, *iy;
+    __device__ __forceinline__ int at(int i) const { return i < ca ? ea + i : eb + (i - ca); }
+    __device__ __forceinline__ YfEntries(const Geo &g, int x, bool herm, float *pre, int T)
+    {
+        const int xp = (g.n0 - x) & (g.n0 - 1);   // the mirror row (HERM)
+        const bool two = herm && xp != x;
+        ea = g.row_off[x];
+        ca = g.row_off[x + 1] - ea;
+        eb = two ? g.row_off[xp] : 0;
+        cnt = ca + (two ? g.row_off[xp + 1] - eb : 0);
+        staged = min(cnt, min(T, kPreEntries));
+        phi = pre;
+        jt = reinterpret_cast<int *>(phi + kPreEntries * kLdPhiy);
+        iy = jt + kPreEntries;
     }
-    cp_async_commit();
-    cp_async_wait<1>();
-    __syncthreads();
-    auto ld = [=](int y, int b) -> float2 {
-        int Y = (y + N1 / 2) & (n - 1);
-        float2 v = (Y < N1) ? row[Y * B + b] : make_float2(0.f, 0.f);
-        return (y & 1) ? make_float2(-v.x, -v.y) : v;      // rotates the output by n/2
-    };
-    auto st = [=](int q, int b, float2 v) { row[q * SB + b] = v; };
-    fft_fused<B, SB, E, false, kPairs, true>(row, n, g.lg1, tws, -1.f, ld, st);
-    cp_async_wait<0>();
-    __syncthreads();
-    fill_halo<B, SB>(s, n);
-    __syncthreads();
+    __device__ __forceinline__ void stage(const Geo &g) const
+    {
+        if ((int)threadIdx.x < staged) {
+            const int e = at(threadIdx.x);
+            const float *src = g.ent_phiy + (size_t)e * kLdPhiy;
+            float *dst = phi + threadIdx.x * kLdPhiy;
+#pragma unroll
+            for (int q = 0; q < kLdPhiy / 4; ++q) cp_async<16>(dst + 4 * q, src + 4 * q);
+            cp_async<4>(jt + threadIdx.x, g.ent_jt + e);
+            cp_async<4>(iy + threadIdx.x, g.ent_iy0 + e);
+        }
+        cp_async_commit();
+    }
+};
+
+// The interpolation of a CTA's entries from the rotated rows s[n1 + 16][SB]:
+// one thread per entry, entries past the staged ones loaded one round ahead.
+template <int B, int SB, bool HERM>
+__device__ __forceinline__ void yfwd_interp(const Geo &g, const float2 *s, int grp, const YfEntries &en,
+                                            float2 *__restrict__ P)
+{
+    constexpr bool kPairs = (B == 8);   // 64-byte rows read as 128-byte row pairs
+    const int n = g.n1, T = blockDim.x, ca = en.ca, cnt = en.cnt, staged = en.staged;
+    const float *pre_phi = en.phi;
+    const int *pre_jt = en.jt, *pre_iy = en.iy;
+    auto ent = [&](int i) { return en.at(i); };
     const size_t pbase = (size_t)grp * g.M * kTaps * B;
     const int rofs = n / 2 + kHalo;
     struct Ent {
@@ -486,6 +465,56 @@ __global__ void FFT_BOUNDS(E) k_ypass_fwd(Geo g, const float2 *__restrict__ G1, 
         cur = nxt;
         i = i2;
     }
+}
+
+// Forward y-pass fused with the y-direction interpolation.  Row x of G1 holds
+// the N1 nonzero columns; column Y sits at y with (y + N1/2) % n1 == Y.
+// P[G][M][14][B]: P[j][t0] = sum_t1 phiy[j][t1] * G[x][(iy0_j + t1) mod n1],
+// x = (ix0_j + t0) mod n0.  (NU:669-727 sum the same 196 products per node.)
+// The row is copied to shared memory and the tables of the row's first
+// entries are copied behind it; the FFT waits only for the row.  One thread
+// per entry then computes all B slices of it from the rotated row; entries
+// past the copied ones are loaded one round ahead.
+//
+// HERM (the forward transform of a real image, cunfft_trafo_2d_R2C2,
+// NU:984-1076, whose cuFFT R2C keeps half the spectrum): G1 row n0 - x is the
+// conjugate of row x, so its FFT along y is the conjugate mirror of row x's,
+// buf'[q] = conj(buf[-q mod n1]).  The grid then covers rows x = 0..n0/2
+// only; each CTA also interpolates the entries of row n0 - x, reading the 14
+// taps of an entry from the mirrored window in reverse order and storing the
+// conjugate of the sum.  The x-pass writes only rows 0..n0/2 of G1.
+template <int B, int E, bool HERM>
+__global__ void FFT_BOUNDS(E) k_ypass_fwd(Geo g, const float2 *__restrict__ G1, float2 *__restrict__ P)
+{
+    extern __shared__ float2 s[];
+    constexpr int SB = YfStride<B>::v;
+    constexpr bool kPairs = (B == 8);   // 64-byte rows read as 128-byte row pairs
+    const int grp = blockIdx.x, x = blockIdx.y, n = g.n1, N1 = g.N1;
+    const float2 *rowin = G1 + ((size_t)grp * g.n0 + x) * N1 * B;
+    float2 *row = s + kHalo * SB;
+    const YfEntries en(g, x, HERM, reinterpret_cast<float *>(s + (size_t)(n + 2 * kHalo) * SB), blockDim.x);
+    float2 *tw_s = reinterpret_cast<float2 *>(en.iy + kPreEntries);                     // [n] twiddles
+    const float2 *tws = ypass_tw_shared(n) ? tw_s : g.tw1;
+    // Group 1: the N1 nonzero values of the row (contiguous in G1) and the
+    // FFT's twiddle table.  Group 2: tables of the first entries.
+    copy_async(row, rowin, (size_t)N1 * B * sizeof(float2));
+    if (ypass_tw_shared(n)) copy_async(tw_s, g.tw1, (size_t)n * sizeof(float2));
+    cp_async_commit();
+    en.stage(g);
+    cp_async_wait<1>();
+    __syncthreads();
+    auto ld = [=](int y, int b) -> float2 {
+        int Y = (y + N1 / 2) & (n - 1);
+        float2 v = (Y < N1) ? row[Y * B + b] : make_float2(0.f, 0.f);
+        return (y & 1) ? make_float2(-v.x, -v.y) : v;      // rotates the output by n/2
+    };
+    auto st = [=](int q, int b, float2 v) { row[q * SB + b] = v; };
+    fft_fused<B, SB, E, false, kPairs, true>(row, n, g.lg1, tws, -1.f, ld, st);
+    cp_async_wait<0>();
+    __syncthreads();
+    fill_halo<B, SB>(s, n);
+    __syncthreads();
+    yfwd_interp<B, SB, HERM>(g, s, grp, en, P);
 }
 
 // --------------------------------------------------------------- K3 ----
@@ -1412,7 +1441,8 @@ __global__ void FFT_BOUNDS(E) k_ypass_toep_quad(Geo g, const float2 *__restrict_
 // no reordering pass.  The N1 inputs of a row are loaded from global memory
 // straight into registers (the B slices of a point are B consecutive float2,
 // so a warp reads 256 contiguous bytes) and the N1 outputs stored from
-// registers; the zero padding is never loaded.  Shared memory holds only the
+// registers; the zero padding, which the rows a >= R/2 are (N1 <= 16 R), is
+// neither loaded nor transformed.  Shared memory holds only the
 // transposed [32][R][B] values, with k1 XOR-swizzled by the low bits of c so
 // that the column-wise writes and row-wise reads of a warp spread over the
 // banks (for a power-of-two R two wavefronts per 32 x 8 bytes).  Each
@@ -1471,7 +1501,7 @@ __global__ void __launch_bounds__(R * B, (R == 20 && B == 8) ? 4 : 16 / ((R * B 
             const float2 *rb = row + (c * B + b);   // point y = 32 a + c at rb[32 B a]
             const int na = (N1 - c + 31) >> 5;      // points y < N1
 #pragma unroll
-            for (int a = 0; a < R; ++a) v[i][a] = a < na ? rb[32 * B * a] : make_float2(0.f, 0.f);
+            for (int a = 0; a < R / 2; ++a) v[i][a] = a < na ? rb[32 * B * a] : make_float2(0.f, 0.f);
         }
         cp_async_wait<0>();
         __syncthreads();   // the twiddle table is in shared memory
@@ -1479,7 +1509,7 @@ __global__ void __launch_bounds__(R * B, (R == 20 && B == 8) ? 4 : 16 / ((R * B 
         for (int i = 0; i < NI; ++i) {
             const int c = u + R * i;
             if (c >= 32) break;
-            dft_nat<R>(v[i], -1.f);
+            dft_half_nat<R>(v[i], -1.f);
 #pragma unroll
             for (int k1 = 1; k1 < R; ++k1) v[i][k1] = cmul(v[i][k1], tws[c * k1]);
 #pragma unroll
@@ -1543,7 +1573,7 @@ __global__ void __launch_bounds__(R * B, (R == 20 && B == 8) ? 4 : 16 / ((R * B 
             float2 *rb = row + (c * B + b);
             const int na = (N1 - c + 31) >> 5;
 #pragma unroll
-            for (int a = 0; a < R; ++a)
+            for (int a = 0; a < R / 2; ++a)
                 if (a < na) rb[32 * B * a] = v[a];
         }
     }
@@ -1553,12 +1583,89 @@ __host__ __device__ inline size_t ytoep4_smem(int n1, int B) { return (size_t)n1
 // n1 sizes k_ytoep4 takes (n1 = 32 R, R in ytoep4_radix_ok).
 __host__ __device__ inline bool ytoep4_fits(int n1) { return n1 % 32 == 0 && ytoep4_radix_ok(n1 / 32); }
 
-// ------------------------------------------- adjoint y-pass, 4-step ----
-// The adjoint y-pass (k_ypass_adj) for n1 = 32 R, R = 4, 8, 16 or 32, with
-// the four-step register FFT of k_ytoep4 in its inverse direction: the
-// gathered rows are read once into registers, one transpose through the same
-// shared memory, the outputs Y < N1 stored from registers.
+// -------------------------------------------- NUFFT y-passes, 4-step ----
+// The y-passes of the NUFFT (k_ypass_fwd, k_ypass_adj) for n1 = 32 R, R = 4, 8,
+// 16 or 32, with the four-step register FFT of k_ytoep4: no staging copy of the
+// row, one transpose instead of two or three, inputs loaded and outputs stored
+// straight from registers.  The image row sits at Y - h, h = N1/2, and the
+// buffer is rotated by n1/2; both shifts cost nothing here.  With Y = 32 a + c
+// and d = c - h the sums are those of k_ytoep4 with c replaced by d: twiddles
+// wn^(d k1), and 32-point DFTs over d mod 32, so column c goes to position
+// d mod 32 of the transposed buffer; and frequency u + R k2 belongs in row
+// u + R ((k2 + 16) mod 32), which only renames registers.  N1 <= n1/2, so the
+// rows a >= R/2 are zero going in and not needed coming out.
 __host__ __device__ constexpr bool yadj4_fits(int n1) { return n1 == 128 || n1 == 256 || n1 == 512 || n1 == 1024; }
+
+// Threads of the forward y-pass: the FFT's, at least four warps (entries are
+// spread over all; eight for the one- and two-slice groups of small calls).
+__host__ __device__ constexpr int yfwd_threads(int fft_threads, int B)
+{
+    const int least = B >= 4 ? 64 : 256;
+    return fft_threads < least ? least : fft_threads;
+}
+__host__ __device__ constexpr size_t yfwd4_smem(int n1, int B)
+{
+    return (size_t)(n1 + 2 * kHalo) * ((B == 8) ? 8 : (B == 4) ? 6 : B) * sizeof(float2) +
+           (size_t)kPreEntries * kPreRecord + (size_t)n1 * sizeof(float2);
+}
+
+template <int B, int R, bool HERM>
+__global__ void __launch_bounds__(yfwd_threads(R * B, B), 512 / yfwd_threads(R * B, B))
+    k_yfwd4(Geo g, const float2 *__restrict__ G1, float2 *__restrict__ P)
+{
+    constexpr int LB = Log2B<B>::v, n = 32 * R, SB = YfStride<B>::v;
+    constexpr int NI = (32 + R - 1) / R;
+    extern __shared__ float2 s[];
+    const int grp = blockIdx.x, x = blockIdx.y, N1 = g.N1, h = N1 / 2;
+    const int t = threadIdx.x, b = t & (B - 1), u = t >> LB;
+    const bool act = yfwd_threads(R * B, B) == R * B || t < R * B;
+    const float2 *row = G1 + ((size_t)grp * g.n0 + x) * N1 * B;
+    float2 *tws = s + (size_t)(n + 2 * kHalo) * SB;
+    copy_async(tws, g.tw1, (size_t)n * sizeof(float2));
+    cp_async_commit();
+    const YfEntries en(g, x, HERM, reinterpret_cast<float *>(tws + n), blockDim.x);
+    en.stage(g);
+    float2 v[NI][R];
+    if (act) {
+#pragma unroll
+        for (int i = 0; i < NI; ++i) {
+            const int c = u + R * i, na = (N1 - c + 31) >> 5;
+            const float2 *rb = row + (c * B + b);
+#pragma unroll
+            for (int a = 0; a < R / 2; ++a) v[i][a] = c < 32 && a < na ? rb[32 * B * a] : make_float2(0.f, 0.f);
+        }
+    }
+    cp_async_wait<1>();
+    __syncthreads();                                     // the twiddle table is in shared memory
+    if (act) {
+#pragma unroll
+        for (int i = 0; i < NI; ++i) {
+            const int c = u + R * i, d = c - h;
+            if (c >= 32) break;
+            dft_half_nat<R>(v[i], -1.f);
+#pragma unroll
+            for (int k1 = 0; k1 < R; ++k1)
+                s[ytoep4_sidx<B, R>(d & 31, k1, b)] = k1 ? cmul(v[i][k1], tws[(d * k1) & (n - 1)]) : v[i][0];
+        }
+    }
+    __syncthreads();
+    float2 w[32];
+    if (act) {
+#pragma unroll
+        for (int c = 0; c < 32; ++c) w[brev5(c)] = s[ytoep4_sidx<B, R>(c, u, b)];
+    }
+    __syncthreads();                                     // the buffer is read before the rows are written
+    if (act) {
+        dft_inplace<32>(w, -1.f);
+#pragma unroll
+        for (int k2 = 0; k2 < 32; ++k2) s[(size_t)(kHalo + u + R * ((k2 + 16) & 31)) * SB + b] = w[k2];
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    fill_halo<B, SB>(s, n);
+    __syncthreads();
+    yfwd_interp<B, SB, HERM>(g, s, grp, en, P);
+}
 
 template <int B, int R>
 __global__ void __launch_bounds__(yadj_threads(R * B), 512 / yadj_threads(R * B))
@@ -1578,37 +1685,36 @@ __global__ void __launch_bounds__(yadj_threads(R * B), 512 / yadj_threads(R * B)
     float2 w[32];
     if (act) {
 #pragma unroll
-        for (int k2 = 0; k2 < 32; ++k2) w[k2] = s[(kHalo + u + R * k2) * B + b];
+        for (int k2 = 0; k2 < 32; ++k2) w[k2] = s[(kHalo + u + R * ((k2 + 16) & 31)) * B + b];
     }
     __syncthreads();   // every row is read before the buffer is rewritten
+    const int h = N1 / 2;
     if (act) {
-        dft_dif_inplace<32>(w, +1.f);
+        dft_dif_inplace<32>(w, +1.f);                    // position d mod 32 at w[brev5(.)]
 #pragma unroll
-        for (int c = 0; c < 32; ++c) {
-            float2 tw = tws[c * u];
+        for (int dm = 0; dm < 32; ++dm) {
+            const int c = (dm + h) & 31;
+            float2 tw = tws[((c - h) * u) & (n - 1)];
             tw.y = -tw.y;
-            s[ytoep4_sidx<B, R>(c, u, b)] = c ? cmul(w[brev5(c)], tw) : w[0];
+            s[ytoep4_sidx<B, R>(c, u, b)] = cmul(w[brev5(dm)], tw);
         }
     }
     __syncthreads();
     if (!act) return;
-    // R-point inverse DFTs over k1 of columns c = u + R i: y = 32 a + c, whose
-    // crop row is (y + N1/2) mod n1; odd y undo the rotation's sign.
+    // R-point inverse DFTs over k1 of columns c = u + R i: rows Y = 32 a + c < N1.
     float2 *out = G1 + ((size_t)grp * g.n0 + x) * N1 * B + b;
 #pragma unroll
     for (int i = 0; i < NI; ++i) {
-        const int c = u + R * i;
+        const int c = u + R * i, na = (N1 - c + 31) >> 5;
         if (c >= 32) break;
         float2 v[R];
 #pragma unroll
         for (int k1 = 0; k1 < R; ++k1) v[k1] = s[ytoep4_sidx<B, R>(c, k1, b)];
         dft_nat<R>(v, +1.f);
-        const float sg = (c & 1) ? -1.f : 1.f;
+        float2 *rb = out + c * B;
 #pragma unroll
-        for (int a = 0; a < R; ++a) {
-            const int Y = (32 * a + c + N1 / 2) & (n - 1);
-            if (Y < N1) out[(size_t)Y * B] = make_float2(sg * v[a].x, sg * v[a].y);
-        }
+        for (int a = 0; a < R / 2; ++a)
+            if (a < na) rb[32 * B * a] = v[a];
     }
 }
 
