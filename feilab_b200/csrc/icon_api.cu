@@ -264,8 +264,8 @@ struct icon_plan {
     // iteration's update m -= alpha Re r-hat into the next iteration's forward
     // x-pass; flush_update applies a pending one where the loop ends.
     bool xt_ok = false;         // k_xtoep has a variant for n0
-    // TMA staging of the x-kernels' columns: tensor maps over G1, Ahwb, r-hat
-    // and m (xt_tma), boxes of xt_bh slices; device error flag of their
+    // TMA staging of the x-kernels' columns: tensor maps over G1 and Ahwb
+    // (xt_tma), boxes of xt_bh slices; device error flag of their
     // bounded waits.
     // Warm start of the reconstruct calls (icon_plan_set_warm_start): the
     // network, the acceptance test, caller-layout buffers of A^H W b and m,
@@ -275,9 +275,9 @@ struct icon_plan {
     float2 *ws_A = nullptr;
     float *ws_m = nullptr;
     long long warm_accepted = 0, warm_redone = 0;
-    bool xt_tma = false, xt_tma_m = false;
+    bool xt_tma = false;
     int xt_bh = 1, xt_box_g1 = 0, xt_box_img = 0;
-    CUtensorMap tm_g1, tm_ahwb, tm_rre, tm_m;
+    CUtensorMap tm_g1, tm_ahwb;
     float *rre = nullptr;       // [Gcap][N1][N0][B] Re r-hat of the Toeplitz x-kernels (the deferred update's input)
     int *dev_err = nullptr;
     bool upd_pending = false, upd_clamp = false;
@@ -355,15 +355,12 @@ struct icon_plan {
     void fill_xt(icon::XtArgs &xa) const
     {
         xa.use_tma = xt_tma ? 1 : 0;
-        xa.tma_m = xt_tma_m ? 1 : 0;
         xa.box_g1 = xt_box_g1;
         xa.box_img = xt_box_img;
         xa.err = dev_err;
         if (xt_tma) {
             xa.tm_g1 = tm_g1;
             xa.tm_ahwb = tm_ahwb;
-            xa.tm_rre = tm_rre;
-            xa.tm_m = tm_m;
         }
     }
     Geo1 geo1() const
@@ -459,7 +456,7 @@ bool make_map(CUtensorMap *m, void *base, int rank, const cuuint64_t *dims, cons
 
 // Tensor maps for the x-kernels' TMA staging (k_xtoep): possible when a CTA
 // takes at least 2 slices (boxes of 16 bytes or more, every coordinate and
-// stride a multiple of 16 bytes); m needs 4.  ICON_XT_TMA=0 keeps the
+// stride a multiple of 16 bytes).  ICON_XT_TMA=0 keeps the
 // per-thread cp.async staging.
 void setup_xt_tma(icon_plan *p)
 {
@@ -485,15 +482,7 @@ void setup_xt_tma(icon_plan *p)
         ok = ok && make_map(&p->tm_ahwb, p->Ahwb, 3, dims, str, box);
 
     }
-    bool ok_m = BH >= 4;
-    if (ok_m) {   // m [Gcap N1][N0][B] floats
-        const cuuint64_t dims[3] = {Bz, N0, G * N1};
-        const cuuint64_t str[2] = {Bz * 4, N0 * Bz * 4};
-        const cuuint32_t box[3] = {(cuuint32_t)BH, (cuuint32_t)p->xt_box_img, 1};
-        ok_m = make_map(&p->tm_m, p->m, 3, dims, str, box) && make_map(&p->tm_rre, p->rre, 3, dims, str, box);
-    }
     p->xt_tma = ok;
-    p->xt_tma_m = ok && ok_m;
 }
 
 // Builds window tables and the per-row entry lists of M nodes at xy.
@@ -634,9 +623,21 @@ icon_status launch_forward(icon_plan *p, const NodeTables &t, const void *img_in
     // A real image's spectrum is Hermitian: the y-pass takes grid rows
     // 0..n0/2 and interpolates the mirror rows' entries from them.
     dim3 gx(p->N1, G), gy(G, real_in ? p->n0 / 2 + 1 : p->n0);
+    icon::XtArgs xa{};
+    if (p->xt_ok) {
+        xa.N0 = p->N0; xa.N1 = p->N1; xa.n0 = p->n0; xa.tw0 = p->tw0; xa.tw0h = p->tw0h; xa.G1 = p->G1;
+        xa.rcx = p->rcx; xa.rcy = p->rcy;
+        if (real_in) {
+            xa.m = (float *)img_int; xa.Gh = p->G1; xa.gh_rows = p->n0; xa.deapod = 1;   // read only: upd is 0
+        } else {
+            xa.img = (const float2 *)img_int;
+        }
+    }
     WITH_B(p->B,
         LAUNCH_B(p, K_XF, st, (real_in ? sb.xf_real : sb.xf_cplx) * slots,
-                 L::xpass_fwd(real_in, p->ex, gx, p->thr_x, p->smem_x, st, g, img_int, p->G1));
+                 if (!p->xt_ok) L::xpass_fwd(real_in, p->ex, gx, p->thr_x, p->smem_x, st, g, img_int, p->G1);
+                 else if (real_in) L::xtoep_real(st, G, xa);
+                 else L::xtoep(0, st, G, xa));
         LAUNCH_B(p, K_YF, st, (real_in ? sb.yf_real : sb.yf) * slots,
                  L::ypass_fwd(p->ey, real_in, gy, p->thr_y, p->smem_y, st, g, p->G1, p->P)))
     int kb = (t.M * p->B + 255) / 256;
@@ -779,14 +780,19 @@ icon_status launch_iteration_xt_raw(icon_plan *p, int G, bool upd, bool clamp_pr
     const double NN = (double)p->N0 * p->N1, G1b = (double)p->n0 * p->N1 * 8, Kb = (double)p->n0 * p->n1t * 4;
     icon::XtArgs xa{};
     p->fill_xt(xa);
-    xa.N0 = p->N0; xa.N1 = p->N1; xa.n0 = p->n0; xa.tw0 = p->tw0; xa.G1 = p->G1; xa.m = p->m;
+    // The rows of m's spectrum past n0/2 are the conjugates of the others: only
+    // the half is stored, in the NUFFT's scratch.
+    xa.N0 = p->N0; xa.N1 = p->N1; xa.n0 = p->n0; xa.tw0 = p->tw0; xa.tw0h = p->tw0h; xa.G1 = p->G1; xa.m = p->m;
+    xa.Gh = p->P; xa.gh_rows = p->n0 / 2 + 1;
     xa.rre_in = p->rre; xa.alpha = p->alpha; xa.upd = upd ? 1 : 0; xa.clamp = clamp_prev ? 1 : 0;
     xa.data_type = data_type; xa.thr = thr; xa.rre = p->rre; xa.Ahwb = p->Ahwb; xa.part_rtr = p->part_rtr;
-    const double xf_bytes = (xa.upd ? NN * 12 : NN * 4) + G1b;   // m (read, written), Re r-hat; G1 written
+    const double Gh = (double)(p->n0 / 2 + 1) * p->N1 * 8;
+    const double xf_bytes = (xa.upd ? NN * 12 : NN * 4) + Gh;   // m (read, written), Re r-hat; half spectrum written
     dim3 gy(G, p->n0);
     WITH_B(p->B,
-        LAUNCH_B(p, K_XTF, st, xf_bytes * slots, L::xtoep(0, st, G, xa));
-        LAUNCH_B(p, K_YT, st, (2 * G1b) * slots + Kb * G, L::ypass_toep(p->ey, gy, p->thr_y, p->smem_yt, st, g, p->G1));
+        LAUNCH_B(p, K_XTF, st, xf_bytes * slots, L::xtoep_real(st, G, xa));
+        LAUNCH_B(p, K_YT, st, (Gh + G1b) * slots + Kb * G,
+                 L::ypass_toep(p->ey, gy, p->thr_y, p->smem_yt, st, g, p->G1, p->P));
         LAUNCH_B(p, K_XTM, st, (2 * G1b + NN * 12) * slots, L::xtoep(1, st, G, xa));
         LAUNCH_B(p, K_YQ, st, G1b * slots + Kb * G,
                  L::ypass_toep_quad(p->ey, gy, p->thr_y, p->smem_yt, st, g, p->G1, p->part_rtar)))
@@ -823,7 +829,7 @@ icon_status launch_iteration_toep(icon_plan *p, int G, bool clamp, int data_type
     dim3 gx(p->N1, G), gy(G, p->n0);
     WITH_B(p->B,
         LAUNCH_B(p, K_XF, st, (NN * 4 + G1b) * slots, L::xpass_fwd_full(p->ex, gx, p->thr_x, p->smem_x, st, g, p->m, p->G1));
-        LAUNCH_B(p, K_YT, st, (2 * G1b) * slots + Kb * G, L::ypass_toep(p->ey, gy, p->thr_y, p->smem_yt, st, g, p->G1));
+        LAUNCH_B(p, K_YT, st, (2 * G1b) * slots + Kb * G, L::ypass_toep(p->ey, gy, p->thr_y, p->smem_yt, st, g, p->G1, nullptr));
         LAUNCH_B(p, K_XA, st, (G1b + NN * 16) * slots,
                  L::xpass_adj(1, p->ex, gx, p->thr_x, p->smem_x + sizeof(double) * p->thr_x, st, g, p->G1, p->rhat,
                               p->Ahwb, p->part_rtr));
@@ -1139,7 +1145,8 @@ static icon_status plan_create_impl(const icon_geometry *geo, int group, icon_pl
     // Scratch for Gcap groups.
     size_t G = p->Gcap, Bz = B;
     ICON_TRY(p->arena.alloc(&p->G1, G * p->n0 * p->N1 * Bz));
-    ICON_TRY(p->arena.alloc(&p->P, G * p->M * kTaps * Bz));
+    // NUFFT partials, or the half spectrum of the Toeplitz iteration's image
+    ICON_TRY(p->arena.alloc(&p->P, G * std::max((size_t)p->M * kTaps, (size_t)(p->n0 / 2 + 1) * p->N1) * Bz));
     ICON_TRY(p->arena.alloc(&p->f, G * p->M * Bz));
     ICON_TRY(p->arena.alloc(&p->fline, G * p->nx * Bz));
     size_t NN = (size_t)p->N0 * p->N1;

@@ -45,36 +45,37 @@ void Launch<B>::xpass_fwd_full(int E, dim3 grid, int threads, size_t smem, cudaS
 // {4, 6, 8, 10, 12, 16, 20, 24, 32}; blockDim = n1*B/32, shared memory
 // n1*B float2.
 template <int B, int MODE>
-static void launch_ytoep4(dim3 grid, cudaStream_t st, const Geo &g, float2 *G1, double *part)
+static void launch_ytoep4(dim3 grid, cudaStream_t st, const Geo &g, float2 *G1, const float2 *Gh, double *part)
 {
     const int threads = g.n1 * B / 32;
     const size_t smem = ytoep4_smem(g.n1, B);
     switch (g.n1 / 32) {
-    case 4: k_ytoep4<B, 4, MODE><<<grid, threads, smem, st>>>(g, G1, part); break;
-    case 6: k_ytoep4<B, 6, MODE><<<grid, threads, smem, st>>>(g, G1, part); break;
-    case 8: k_ytoep4<B, 8, MODE><<<grid, threads, smem, st>>>(g, G1, part); break;
-    case 10: k_ytoep4<B, 10, MODE><<<grid, threads, smem, st>>>(g, G1, part); break;
-    case 12: k_ytoep4<B, 12, MODE><<<grid, threads, smem, st>>>(g, G1, part); break;
-    case 16: k_ytoep4<B, 16, MODE><<<grid, threads, smem, st>>>(g, G1, part); break;
-    case 20: k_ytoep4<B, 20, MODE><<<grid, threads, smem, st>>>(g, G1, part); break;
-    case 24: k_ytoep4<B, 24, MODE><<<grid, threads, smem, st>>>(g, G1, part); break;
-    default: k_ytoep4<B, 32, MODE><<<grid, threads, smem, st>>>(g, G1, part); break;
+    case 4: k_ytoep4<B, 4, MODE><<<grid, threads, smem, st>>>(g, G1, Gh, part); break;
+    case 6: k_ytoep4<B, 6, MODE><<<grid, threads, smem, st>>>(g, G1, Gh, part); break;
+    case 8: k_ytoep4<B, 8, MODE><<<grid, threads, smem, st>>>(g, G1, Gh, part); break;
+    case 10: k_ytoep4<B, 10, MODE><<<grid, threads, smem, st>>>(g, G1, Gh, part); break;
+    case 12: k_ytoep4<B, 12, MODE><<<grid, threads, smem, st>>>(g, G1, Gh, part); break;
+    case 16: k_ytoep4<B, 16, MODE><<<grid, threads, smem, st>>>(g, G1, Gh, part); break;
+    case 20: k_ytoep4<B, 20, MODE><<<grid, threads, smem, st>>>(g, G1, Gh, part); break;
+    case 24: k_ytoep4<B, 24, MODE><<<grid, threads, smem, st>>>(g, G1, Gh, part); break;
+    default: k_ytoep4<B, 32, MODE><<<grid, threads, smem, st>>>(g, G1, Gh, part); break;
     }
 }
 
 template <int B>
-void Launch<B>::ypass_toep(int E, dim3 grid, int threads, size_t smem, cudaStream_t st, const Geo &g, float2 *G1)
+void Launch<B>::ypass_toep(int E, dim3 grid, int threads, size_t smem, cudaStream_t st, const Geo &g, float2 *G1,
+                           const float2 *Gh)
 {
-    if (ytoep4_fits(g.n1)) launch_ytoep4<B, 0>(grid, st, g, G1, nullptr);
-    else if (E == 32) k_ypass_toep<B, 32><<<grid, threads, smem, st>>>(g, G1);
-    else k_ypass_toep<B, 16><<<grid, threads, smem, st>>>(g, G1);
+    if (ytoep4_fits(g.n1)) launch_ytoep4<B, 0>(grid, st, g, G1, Gh, nullptr);
+    else if (E == 32) k_ypass_toep<B, 32><<<grid, threads, smem, st>>>(g, G1, Gh);
+    else k_ypass_toep<B, 16><<<grid, threads, smem, st>>>(g, G1, Gh);
 }
 
 template <int B>
 void Launch<B>::ypass_toep_quad(int E, dim3 grid, int threads, size_t smem, cudaStream_t st, const Geo &g,
                                 const float2 *G1, double *part)
 {
-    if (ytoep4_fits(g.n1)) launch_ytoep4<B, 1>(grid, st, g, const_cast<float2 *>(G1), part);
+    if (ytoep4_fits(g.n1)) launch_ytoep4<B, 1>(grid, st, g, const_cast<float2 *>(G1), nullptr, part);
     else if (E == 32) k_ypass_toep_quad<B, 32><<<grid, threads, smem, st>>>(g, G1, part);
     else k_ypass_toep_quad<B, 16><<<grid, threads, smem, st>>>(g, G1, part);
 }
@@ -115,6 +116,42 @@ static cudaError_t xt_attr()
     X(4096, (B < 2 ? B : 2), 4, 3)                    \
     X(8192, 1, 4, 4)
 
+// k_xtoep_real for n0, by its half length: all B slices up to 1024, then at
+// most 8192 / N.
+#define ICON_XTR_SHAPES(X)                           \
+    X(128, B, 1, 0)                                   \
+    X(256, B, 2, 0)                                   \
+    X(512, B, 3, 0)                                   \
+    X(1024, B, 4, 0)                                  \
+    X(2048, B, 5, 0)                                  \
+    X(4096, (B < 4 ? B : 4), 3, 3)                    \
+    X(8192, (B < 2 ? B : 2), 4, 3)
+
+template <int B, int BH, int LA, int LNB>
+static void xtr_go(cudaStream_t st, int G, const XtArgs &a)
+{
+    using S = XtShape<BH, LA, LNB>;
+    k_xtoep_real<B, BH, LA, LNB><<<dim3((unsigned)(a.N1 * (B / BH)), (unsigned)G), S::T, sizeof(float2) * S::N * BH, st>>>(a);
+}
+template <int B, int BH, int LA, int LNB>
+static cudaError_t xtr_attr()
+{
+    return cudaFuncSetAttribute((const void *)k_xtoep_real<B, BH, LA, LNB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)sizeof(float2) * XtShape<BH, LA, LNB>::N * BH);
+}
+
+template <int B>
+void Launch<B>::xtoep_real(cudaStream_t st, int G, const XtArgs &a)
+{
+    switch (a.n0) {
+#define X(N, BH, LA, LNB) \
+    case N: xtr_go<B, BH, LA, LNB>(st, G, a); break;
+        ICON_XTR_SHAPES(X)
+#undef X
+    default: break;
+    }
+}
+
 template <int B>
 bool Launch<B>::xtoep(int mode, cudaStream_t st, int G, const XtArgs &a)
 {
@@ -130,10 +167,19 @@ bool Launch<B>::xtoep(int mode, cudaStream_t st, int G, const XtArgs &a)
 template <int B>
 cudaError_t Launch<B>::xtoep_prepare(int n0)
 {
+    cudaError_t e = cudaSuccess;
     switch (n0) {
 #define X(N, BH, LA, LNB) \
-    case N: return xt_attr<B, BH, LA, LNB>();
+    case N: e = xt_attr<B, BH, LA, LNB>(); break;
         ICON_XT_SHAPES(X)
+#undef X
+    default: break;
+    }
+    if (e != cudaSuccess) return e;
+    switch (n0) {
+#define X(N, BH, LA, LNB) \
+    case N: return xtr_attr<B, BH, LA, LNB>();
+        ICON_XTR_SHAPES(X)
 #undef X
     default: return cudaSuccess;
     }

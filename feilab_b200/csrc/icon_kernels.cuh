@@ -1343,32 +1343,47 @@ __host__ __device__ inline size_t ypass_toep_smem(int n1, int B)
     return (size_t)n1 * sb * sizeof(float2) + (size_t)n1 * sizeof(float) + ypass_tw_bytes(n1);
 }
 
+// Row of the i-th CTA along blockIdx.y: 0, n0/2, 1, n0 - 1, 2, n0 - 2, ... .
+__device__ __forceinline__ int half_row(int i, int n0)
+{
+    const int p = i >> 1;
+    return (i & 1) ? (p ? n0 - p : n0 / 2) : p;
+}
+
 // Toeplitz y-pass: per (group, grid row x) the row of the x-transformed
 // padded image (the N1 values of G1 row x, placed at y = Y), FFT along y,
 // times K[x][.], inverse FFT along y, the N1 values y = Y < N1 written back to
-// row x of G1 (in place: a CTA reads its row whole before it writes).  One of
+// row x of G1 (in place: a CTA reads its row whole before it writes; with Gh
+// from the half spectrum of a real image, as k_ytoep4).  One of
 // the two y-passes of A^H W A m; the x-passes are k_xpass_fwd_r2c<FULL> and
-// k_xpass_adj with unit deapodisation.
+// k_xpass_adj with unit deapodisation, or k_xtoep_real and k_xtoep.
 template <int B, int E>
-__global__ void FFT_BOUNDS(E) k_ypass_toep(Geo g, float2 *__restrict__ G1)
+__global__ void FFT_BOUNDS(E) k_ypass_toep(Geo g, float2 *__restrict__ G1, const float2 *__restrict__ Gh)
 {
     extern __shared__ float2 s[];
     constexpr int SB = YfStride<B>::v;
     constexpr bool kSwz = (B == 8);
-    const int grp = blockIdx.x, x = blockIdx.y, n = g.n1, N1 = g.N1;
+    const int grp = blockIdx.x, n = g.n1, N1 = g.N1;
+    const int x = Gh ? half_row(blockIdx.y, g.n0) : blockIdx.y;
+    const bool mir = Gh && 2 * x > g.n0;
     float2 *buf = s;
     float *krow = reinterpret_cast<float *>(s + (size_t)n * SB);
     float2 *tw_s = reinterpret_cast<float2 *>(krow + n);
     const float2 *tws = ypass_tw_shared(n) ? tw_s : g.tw1;
     float2 *row = G1 + ((size_t)grp * g.n0 + x) * N1 * B;
-    copy_async(buf, row, (size_t)N1 * B * sizeof(float2));        // [N1][B], contiguous
+    const float2 *rin = Gh ? Gh + ((size_t)grp * (g.n0 / 2 + 1) + (mir ? g.n0 - x : x)) * N1 * B : row;
+    copy_async(buf, rin, (size_t)N1 * B * sizeof(float2));        // [N1][B], contiguous
     copy_async(krow, g.Kt + toep_kernel_index(g, grp) * g.kstride + (size_t)x * n, (size_t)n * sizeof(float));
     if (ypass_tw_shared(n)) copy_async(tw_s, g.tw1, (size_t)n * sizeof(float2));
     cp_async_commit();
     cp_async_wait<0>();
     __syncthreads();
     const float2 *in = buf;
-    auto ld = [=](int y, int b) -> float2 { return y < N1 ? in[y * B + b] : make_float2(0.f, 0.f); };
+    const float sg = mir ? -1.f : 1.f;
+    auto ld = [=](int y, int b) -> float2 {
+        const float2 v = y < N1 ? in[y * B + b] : make_float2(0.f, 0.f);
+        return make_float2(v.x, sg * v.y);
+    };
     auto st2 = [=](int q, int b, float2 v) {
         if (q < N1) row[(size_t)q * B + b] = v;
     };
@@ -1465,8 +1480,10 @@ __host__ __device__ constexpr bool ytoep4_radix_ok(int R)
     return R == 4 || R == 6 || R == 8 || R == 10 || R == 12 || R == 16 || R == 20 || R == 24 || R == 32;
 }
 
-// MODE 0: row x of G1 <- crop F^-1(K[x][.] . F(pad row)), in place (the
-// Toeplitz y-pass of A^H W A m).  MODE 1: part[G][n0][B] <- per slice
+// MODE 0: row x of G1 <- crop F^-1(K[x][.] . F(pad row)) (the Toeplitz y-pass
+// of A^H W A m), in place, or with Gh from the half spectrum of a real image
+// (k_xtoep_real; row n0 - x is the conjugate of row x), which is read twice
+// within L2 instead of written and read whole.  MODE 1: part[G][n0][B] <- per slice
 // sum_k K[x][k] |F(pad row)[k]|^2 in FP64 (the step length's denominator).
 // g.n1 = 32 R and g.tw1 its twiddles (the Toeplitz view of the plan).
 // Launch bounds: blocks of R B threads, 16 warps per SM (128 registers, the
@@ -1476,14 +1493,18 @@ __host__ __device__ constexpr bool ytoep4_radix_ok(int R)
 // for MODE 1 and the same for MODE 0 than three blocks at 128 registers.
 template <int B, int R, int MODE>
 __global__ void __launch_bounds__(R * B, (R == 20 && B == 8) ? 4 : 16 / ((R * B + 31) / 32))
-    k_ytoep4(Geo g, float2 *__restrict__ G1, double *__restrict__ part)
+    k_ytoep4(Geo g, float2 *__restrict__ G1, const float2 *__restrict__ Gh, double *__restrict__ part)
 {
     constexpr int LB = Log2B<B>::v;
     constexpr int NI = (32 + R - 1) / R;     // columns per thread in the first step (the last may be short)
     extern __shared__ float2 s[];
-    const int grp = blockIdx.x, x = blockIdx.y, N1 = g.N1;
+    const int grp = blockIdx.x, N1 = g.N1;
+    // With Gh rows x and n0 - x run together (0, n0/2, 1, n0 - 1, 2, ..).
+    const int x = Gh ? half_row(blockIdx.y, g.n0) : blockIdx.y;
     const int t = threadIdx.x, b = t & (B - 1), u = t >> LB;
     float2 *row = G1 + ((size_t)grp * g.n0 + x) * N1 * B;
+    const bool mir = MODE == 0 && Gh && 2 * x > g.n0;
+    const float2 *rin = MODE == 0 && Gh ? Gh + ((size_t)grp * (g.n0 / 2 + 1) + (mir ? g.n0 - x : x)) * N1 * B : row;
     const float *krow = g.Kt + toep_kernel_index(g, grp) * g.kstride + (size_t)x * (32 * R);
     // The twiddle table wn^q, q < 32 R, copied behind the transposed values;
     // every twiddle of the two steps is read from it.
@@ -1498,10 +1519,14 @@ __global__ void __launch_bounds__(R * B, (R == 20 && B == 8) ? 4 : 16 / ((R * B 
         for (int i = 0; i < NI; ++i) {
             const int c = u + R * i;
             if (c >= 32) break;
-            const float2 *rb = row + (c * B + b);   // point y = 32 a + c at rb[32 B a]
+            const float2 *rb = rin + (c * B + b);   // point y = 32 a + c at rb[32 B a]
             const int na = (N1 - c + 31) >> 5;      // points y < N1
 #pragma unroll
             for (int a = 0; a < R / 2; ++a) v[i][a] = a < na ? rb[32 * B * a] : make_float2(0.f, 0.f);
+            if (mir) {
+#pragma unroll
+                for (int a = 0; a < R / 2; ++a) v[i][a].y = -v[i][a].y;
+            }
         }
         cp_async_wait<0>();
         __syncthreads();   // the twiddle table is in shared memory
@@ -1751,8 +1776,12 @@ namespace icon {
 struct XtArgs {
     int N0, N1, n0;
     const float2 *tw0;       // [n0] exp(-2 pi i q / n0)
+    const float2 *tw0h;      // [n0/2] exp(-2 pi i q / (n0/2))
     float2 *G1;              // [G][n0][N1][B]
-    float *m;                // [G][N1][N0][B] real image (forward input; updated in place when upd)
+    float *m;                // real forward: [G][N1][N0][B] image (updated in place when upd)
+    float2 *Gh;              // real forward: rows x = 0..n0/2 out, [G][gh_rows][N1][B]
+    int gh_rows, deapod;     // gh_rows >= n0/2 + 1; deapod: the image times rcx[X] rcy[Y]
+    const float2 *img;       // complex forward: [G][N1][N0][B], deapodised
     const float *rre_in;     // update: Re r-hat of the iteration being finished, [G][N1][N0][B]
     const double *alpha;     // update: [G*B] step lengths
     int upd, clamp, data_type;
@@ -1761,15 +1790,14 @@ struct XtArgs {
     float *rre;              // mid: Re r-hat out, [G][N1][N0][B] (the update needs only the real part)
     const float2 *Ahwb;      // mid / adjoint with resid: [G][N1][N0][B]
     double *part_rtr;        // mid / adjoint with resid: [G][N1][B] partial |r-hat|^2 per column
-    const float *rcx, *rcy;  // adjoint: deapodisation reciprocals 1/cx [N0], 1/cy [N1]
+    const float *rcx, *rcy;  // deapodisation reciprocals 1/cx [N0], 1/cy [N1]
     int resid;               // adjoint: subtract Ahwb and sum |.|^2 (else the plain adjoint)
     // TMA staging of the columns (use_tma; BH >= 2): the plan's G1 as 2-D
-    // [Gcap n0 rows][N1 B 2 floats], its Ahwb and r-hat as 3-D
-    // [Gcap N1][N0][B 2 floats], and (tma_m; BH >= 4) its m and Re r-hat
-    // as [Gcap N1][N0][B floats]; boxes of BH slices by box_g1 / box_img rows.
+    // [Gcap n0 rows][N1 B 2 floats], its Ahwb as 3-D [Gcap N1][N0][B 2 floats];
+    // boxes of BH slices by box_g1 / box_img rows.
     // Every wait on the loads is bounded and reports through err.
-    CUtensorMap tm_g1, tm_ahwb, tm_rre, tm_m;
-    int use_tma, tma_m, box_g1, box_img;
+    CUtensorMap tm_g1, tm_ahwb;
+    int use_tma, box_g1, box_img;
     int *err;
 };
 
@@ -1824,11 +1852,10 @@ __device__ __forceinline__ void xt_twiddle(float2 (&v)[R], const float2 *__restr
 }
 
 // Forward transform from the step-1 registers v[i][a] (input at
-// x = 32 NB a + u + U i) to G1 rows u + U kc of column `col` (pointer to
-// row 0 of the column for this thread's slice; rows N1*B float2 apart).
+// x = 32 NB a + u + U i) to w[kc], frequency u + U kc.
 template <int BH, int LA, int LNB>
 __device__ __forceinline__ void xt_forward(float2 (&v)[32 >> LA][1 << LA], float2 *s, int u, int sl,
-                                           const float2 *__restrict__ tw, float2 *col, size_t rstride)
+                                           const float2 *__restrict__ tw, float2 (&w)[32])
 {
     using S = XtShape<BH, LA, LNB>;
     constexpr int NA = S::NA, NB = S::NB, U = S::U;
@@ -1863,15 +1890,24 @@ __device__ __forceinline__ void xt_forward(float2 (&v)[32 >> LA][1 << LA], float
         }
         __syncthreads();
     }
-    float2 w[32];
     {
         const int ka = u % NA, kb = u / NA;
 #pragma unroll
         for (int c = 0; c < 32; ++c) w[brev5(c)] = (NB > 1) ? s[S::e2(ka, kb, c, sl)] : s[S::e1(ka, c, sl)];
     }
     dft_inplace<32>(w, -1.f);
+}
+
+// The same, the frequencies stored to G1 rows u + U kc of column `col` (pointer
+// to row 0 of the column for this thread's slice; rows N1*B float2 apart).
+template <int BH, int LA, int LNB>
+__device__ __forceinline__ void xt_forward_rows(float2 (&v)[32 >> LA][1 << LA], float2 *s, int u, int sl,
+                                                const float2 *__restrict__ tw, float2 *col, size_t rstride)
+{
+    float2 w[32];
+    xt_forward<BH, LA, LNB>(v, s, u, sl, tw, w);
     float2 *p = col + (size_t)u * rstride;
-    const size_t step = (size_t)U * rstride;
+    const size_t step = (size_t)XtShape<BH, LA, LNB>::U * rstride;
 #pragma unroll
     for (int kc = 0; kc < 32; ++kc, p += step) *p = w[kc];
 }
@@ -1942,13 +1978,13 @@ __device__ __forceinline__ void xt_inverse(float2 (&v)[32 >> LA][1 << LA], float
     }
 }
 
-// MODE 0: G1 <- F_x(pad m) for every row, m first updated (upd: m <- m -
-// alpha Re r-hat_in, clamped on ICON steps, as k_update).  MODE 1: r-hat =
-// crop F_x^-1(G1) - Ahwb (stored, |r-hat|^2 partial sums per column), then
+// MODE 0: G1 <- F_x(pad (img / (cx cy))) of a complex image (k_xpass_fwd's
+// work).  MODE 1: r-hat = crop F_x^-1(G1) - Ahwb (its real part stored,
+// |r-hat|^2 partial sums per column), then
 // G1 <- F_x(pad r-hat) in place.  MODE 2: the last x-pass of the NUFFT
 // adjoint (k_xpass_adj's work): out = crop F_x^-1(G1) / (cx cy), with resid
 // minus Ahwb and the |.|^2 partial sums.  Grid: (N1 * B/BH, G), half-group
-// fastest.
+// fastest.  The forward transform of a real image is k_xtoep_real.
 template <int B, int BH, int LA, int LNB, int MODE>
 __global__ void __launch_bounds__(XtShape<BH, LA, LNB>::T, (XtShape<BH, LA, LNB>::T >= 256) ? 2 : 4)
     k_xtoep(const __grid_constant__ XtArgs g)
@@ -1956,9 +1992,9 @@ __global__ void __launch_bounds__(XtShape<BH, LA, LNB>::T, (XtShape<BH, LA, LNB>
     using S = XtShape<BH, LA, LNB>;
     constexpr int NA = S::NA, NB = S::NB, U = S::U, H = B / BH;
     extern __shared__ __align__(128) float2 s[];
-    __shared__ __align__(8) uint64_t bar[2];   // TMA: [0] the G1 or m column, [1] the Ahwb or r-hat column
+    __shared__ __align__(8) uint64_t bar[2];   // TMA: [0] the G1 column, [1] the Ahwb column
     constexpr bool kTma = BH >= 2;
-    const bool tma = kTma && g.use_tma;
+    const bool tma = kTma && MODE >= 1 && g.use_tma;
     double *red = reinterpret_cast<double *>(s + S::N * BH);
     const int Y = blockIdx.x / H, h = blockIdx.x % H, grp = blockIdx.y;
     const int t = threadIdx.x, sl = t % BH, u = t / BH, bsl = h * BH + sl;   // bsl: slice within the group
@@ -2023,85 +2059,37 @@ __global__ void __launch_bounds__(XtShape<BH, LA, LNB>::T, (XtShape<BH, LA, LNB>
         cp_async_commit();
     }
     if constexpr (MODE == 0) {
-        // The m column (N0 x BH floats) into s and, for the update, the r-hat
-        // column into As, by cp.async; then into registers.
-        float *Ms = reinterpret_cast<float *>(s);
-        float *Rs = reinterpret_cast<float *>(As);   // Re r-hat column, [N0][BH] floats
-        if (tma && g.tma_m) {
-            // m and (for the update) the Re r-hat column by TMA, boxes of
-            // box_img points: m as [X][BH] floats into s, Re r-hat into Rs.
-            const int nbox = (N0 + g.box_img - 1) / g.box_img;
-            if (t == 0) {
-                ws::mbar_expect_tx(&bar[0], (uint32_t)(nbox * g.box_img * BH * sizeof(float)));
-                for (int k = 0; k < nbox; ++k)
-                    ws::tma_load_3d(Ms + k * g.box_img * BH, &g.tm_m, h * BH, k * g.box_img, grp * N1 + Y, &bar[0]);
-                if (g.upd) {
-                    ws::mbar_expect_tx(&bar[1], (uint32_t)(nbox * g.box_img * BH * sizeof(float)));
-                    for (int k = 0; k < nbox; ++k)
-                        ws::tma_load_3d(Rs + k * g.box_img * BH, &g.tm_rre, h * BH, k * g.box_img, grp * N1 + Y,
-                                        &bar[1]);
-                }
+        // The image column into As, then deapodised into registers.
+        const float2 *src = g.img + ibase - sl;
+        if constexpr (BH >= 2) {
+            constexpr int P = BH / 2;
+            for (int idx = t; idx < N0 * P; idx += S::T) {
+                const int X = idx / P, c = idx - X * P;
+                cp_async<16>(As + X * BH + 2 * c, src + (size_t)X * B + 2 * c);
             }
-            if (!xt_tma_wait(&bar[0], g.err)) return;
-            if (g.upd && !xt_tma_wait(&bar[1], g.err)) return;
         } else {
-            const float *msrc = g.m + ibase - sl;           // point X of this CTA's slices at msrc + X*B
-            const float *rsrc = g.rre_in + ibase - sl;
-            for (int X = t; X < N0; X += S::T) {
-                if constexpr (BH == 4) cp_async<16>(Ms + X * 4, msrc + (size_t)X * B);
-                else if constexpr (BH == 2) cp_async<8>(Ms + X * 2, msrc + (size_t)X * B);
-                else if constexpr (BH == 1) cp_async<4>(Ms + X, msrc + (size_t)X * B);
-                else {
-                    cp_async<16>(Ms + X * BH, msrc + (size_t)X * B);
-                    cp_async<16>(Ms + X * BH + 4, msrc + (size_t)X * B + 4);
-                }
-            }
-            if (g.upd) {
-                for (int X = t; X < N0; X += S::T) {
-                    if constexpr (BH == 4) cp_async<16>(Rs + X * 4, rsrc + (size_t)X * B);
-                    else if constexpr (BH == 2) cp_async<8>(Rs + X * 2, rsrc + (size_t)X * B);
-                    else if constexpr (BH == 1) cp_async<4>(Rs + X, rsrc + (size_t)X * B);
-                    else {
-                        cp_async<16>(Rs + X * BH, rsrc + (size_t)X * B);
-                        cp_async<16>(Rs + X * BH + 4, rsrc + (size_t)X * B + 4);
-                    }
-                }
-            }
-            cp_async_commit();
-            cp_async_wait<0>();
-            __syncthreads();
+            for (int X = t; X < N0; X += S::T) cp_async<8>(As + X, src + (size_t)X * B);
         }
-        if (g.upd) {
-            // m <- m - alpha Re r-hat (k_update's arithmetic), clamped on ICON
-            // steps, over the staged column by all threads (coalesced stores).
-            float *mdst = g.m + ibase - sl;
-            for (int idx = t; idx < N0 * BH; idx += S::T) {
-                const int X = idx / BH, q = idx - X * BH;
-                const double al = g.alpha[grp * B + h * BH + q];
-                float nv = (float)((double)Ms[idx] - al * (double)Rs[idx]);
-                if (g.clamp) {
-                    if (g.data_type == 1) {
-                        if (nv > g.thr) nv = g.thr;
-                    } else {
-                        if (nv < g.thr) nv = g.thr;
-                    }
-                }
-                Ms[idx] = nv;
-                mdst[(size_t)X * B + q] = nv;
-            }
-            __syncthreads();
-        }
+        cp_async_commit();
+        cp_async_wait<0>();
+        __syncthreads();
+        const float rcyY = g.rcy[Y];
 #pragma unroll
         for (int i = 0; i < S::NI1; ++i) {
             const int tau = u + U * i;
 #pragma unroll
             for (int a = 0; a < NA; ++a) {
                 const int X = (32 * NB * a + tau + half) & (n - 1);
-                v[i][a] = make_float2(X < N0 ? Ms[X * BH + sl] : 0.f, 0.f);
+                float2 q = make_float2(0.f, 0.f);
+                if (X < N0) {
+                    const float r = __ldg(&g.rcx[X]) * rcyY;
+                    q = As[X * BH + sl];
+                    q = make_float2(q.x * r, q.y * r);
+                }
+                v[i][a] = q;
             }
         }
-        __syncthreads();   // the staged m is read before step 1 rewrites s
-        xt_forward<BH, LA, LNB>(v, s, u, sl, g.tw0, col, rstride);
+        xt_forward_rows<BH, LA, LNB>(v, s, u, sl, g.tw0, col, rstride);
     } else if constexpr (MODE == 2) {
         if (tma) {
             if (!xt_tma_wait(&bar[0], g.err)) return;
@@ -2180,7 +2168,7 @@ __global__ void __launch_bounds__(XtShape<BH, LA, LNB>::T, (XtShape<BH, LA, LNB>
                 v[i][a] = r;
             }
         }
-        xt_forward<BH, LA, LNB>(v, s, u, sl, g.tw0, col, rstride);
+        xt_forward_rows<BH, LA, LNB>(v, s, u, sl, g.tw0, col, rstride);
         // per-slice FP64 sum in a fixed order (thread t holds slice t % BH)
         red[t] = acc;
         __syncthreads();
@@ -2189,6 +2177,97 @@ __global__ void __launch_bounds__(XtShape<BH, LA, LNB>::T, (XtShape<BH, LA, LNB>
             __syncthreads();
         }
         if (t < BH) g.part_rtr[((size_t)grp * N1 + Y) * B + h * BH + t] = red[t];
+    }
+}
+
+// Forward x-transform of a real image, with half-length FFTs: the n0 values
+// x(t) of a slice's padded column are packed as z(q) = x(2q) + i x(2q+1), one
+// FFT of length N = n0/2 (the three steps of xt_forward), and with Z = FFT(z),
+// W = exp(-2 pi i / n0):
+//   X(k) = (Z(k) + conj Z(N-k)) / 2 - i W^k (Z(k) - conj Z(N-k)) / 2,  k = 0..N;
+// rows past n0/2 are the conjugates of these and are not stored (the y-passes
+// read them as such).  Toeplitz iteration: m is first updated (upd: m <- m -
+// alpha Re r-hat_in, clamped on ICON steps, as k_update); NUFFT: deapodised.
+// Each slice stays its own transform.  Grid (N1 * B/BH, G).
+// Bound by memory and latency: 128 slices of 1024 x 300 with the update,
+// 366 us with full-length transforms and every row stored, 234 us so.
+template <int B, int BH, int LA, int LNB>
+__global__ void __launch_bounds__(XtShape<BH, LA, LNB>::T, (XtShape<BH, LA, LNB>::T >= 256) ? 2 : 4)
+    k_xtoep_real(const __grid_constant__ XtArgs g)
+{
+    using S = XtShape<BH, LA, LNB>;
+    constexpr int NA = S::NA, NB = S::NB, U = S::U, H = B / BH, N = S::N;
+    extern __shared__ __align__(128) float2 s[];
+    const int Y = blockIdx.x / H, h = blockIdx.x % H, grp = blockIdx.y;
+    const int t = threadIdx.x, sl = t % BH, u = t / BH;
+    const int N0 = g.N0, N1 = g.N1, half = N0 / 2;
+    const size_t ibase = (((size_t)grp * N1 + Y) * N0) * B + h * BH;       // image point X at ibase + X*B
+    // The m column [N0][BH] and, for the update, the Re r-hat column: N0 <= N,
+    // so both fit in the N*BH*8 bytes of s.
+    float *Ms = reinterpret_cast<float *>(s), *Rs = Ms + N * BH;
+    auto stage = [&](float *dst, const float *src) {
+        if constexpr (BH == B && B >= 4) {
+            for (int i = t; i < N0 * (BH / 4); i += S::T) cp_async<16>(dst + 4 * i, src + 4 * i);
+        } else if constexpr (BH >= 4) {
+            for (int i = t; i < N0 * (BH / 4); i += S::T) {
+                const int X = i / (BH / 4), c = i % (BH / 4);
+                cp_async<16>(dst + 4 * i, src + (size_t)X * B + 4 * c);
+            }
+        } else {
+            for (int X = t; X < N0; X += S::T) cp_async<4 * BH>(dst + X * BH, src + (size_t)X * B);
+        }
+    };
+    stage(Ms, g.m + ibase);
+    if (g.upd) stage(Rs, g.rre_in + ibase);
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+    if (g.upd) {
+        // m <- m - alpha Re r-hat (k_update's arithmetic), clamped on ICON steps.
+        float *mdst = g.m + ibase;
+        const double al = g.alpha[grp * B + h * BH + sl];                    // S::T is a multiple of BH
+        for (int idx = t; idx < N0 * BH; idx += S::T) {
+            float nv = (float)((double)Ms[idx] - al * (double)Rs[idx]);
+            if (g.clamp) {
+                if (g.data_type == 1) {
+                    if (nv > g.thr) nv = g.thr;
+                } else {
+                    if (nv < g.thr) nv = g.thr;
+                }
+            }
+            Ms[idx] = nv;
+            mdst[(size_t)(idx / BH) * B + sl] = nv;
+        }
+        __syncthreads();
+    }
+    const float rcyY = g.deapod ? g.rcy[Y] : 1.f;
+    auto xval = [&](int q) -> float {
+        const int X = (q + half) & (2 * N - 1);
+        if (X >= N0) return 0.f;
+        const float v = Ms[X * BH + sl];
+        return g.deapod ? v * (__ldg(&g.rcx[X]) * rcyY) : v;
+    };
+    float2 v[S::NI1][NA];
+#pragma unroll
+    for (int i = 0; i < S::NI1; ++i)
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+            const int q = 2 * (32 * NB * a + u + U * i);
+            v[i][a] = make_float2(xval(q), xval(q + 1));
+        }
+    __syncthreads();   // the staged columns are read before step 1 rewrites s
+    float2 w[32];
+    xt_forward<BH, LA, LNB>(v, s, u, sl, g.tw0h, w);
+    __syncthreads();   // every read of s by the transform is done
+#pragma unroll
+    for (int kc = 0; kc < 32; ++kc) s[(u + U * kc) * BH + sl] = w[kc];
+    __syncthreads();
+    float2 *out = g.Gh + ((size_t)grp * g.gh_rows * N1 + Y) * B + h * BH + sl;
+    for (int k = u; k <= N; k += U) {
+        const float2 zk = s[(k & (N - 1)) * BH + sl], zm = s[((N - k) & (N - 1)) * BH + sl];
+        const float2 fe = make_float2(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y));
+        const float2 fo = make_float2(0.5f * (zk.y + zm.y), -0.5f * (zk.x - zm.x));
+        out[(size_t)k * N1 * B] = cadd(fe, cmul(__ldg(&g.tw0[k]), fo));
     }
 }
 

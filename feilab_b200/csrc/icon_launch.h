@@ -20,7 +20,9 @@ struct Launch {
                                const float *in, float2 *G1);
     // Toeplitz y-passes: A^H W A on the rows of G1 in place, and the step
     // length's quadratic form into part[G][n0][B].
-    static void ypass_toep(int E, dim3 grid, int threads, size_t smem, cudaStream_t st, const Geo &g, float2 *G1);
+    // (with Gh, from the half spectrum of a real image).
+    static void ypass_toep(int E, dim3 grid, int threads, size_t smem, cudaStream_t st, const Geo &g, float2 *G1,
+                           const float2 *Gh);
     static void ypass_toep_quad(int E, dim3 grid, int threads, size_t smem, cudaStream_t st, const Geo &g,
                                 const float2 *G1, double *part);
     static void ypass_fwd(int E, bool herm, dim3 grid, int threads, size_t smem, cudaStream_t st, const Geo &g, const float2 *G1,
@@ -52,12 +54,14 @@ struct Launch {
     // The same from the real part of r-hat alone (the Toeplitz x-kernels' output).
     static void update_re(dim3 grid, cudaStream_t st, float *m, const float *rre, const double *alpha, int per_group,
                           int clamp, int data_type, float thr);
-    // Three-step x-passes (k_xtoep) over G groups: mode 0 the Toeplitz forward
-    // of the real image (with the fused update when a.upd), mode 1 the
+    // Three-step x-passes (k_xtoep) over G groups: mode 0 the forward of a
+    // complex image, mode 1 the
     // Toeplitz inverse, r-hat and forward of r-hat, mode 2 the NUFFT adjoint's
     // x-pass (deapodised, optionally minus Ahwb with |.|^2 sums).  Returns
     // false when n0 has no variant (the caller then uses the Stockham kernels).
     static bool xtoep(int mode, cudaStream_t st, int G, const XtArgs &a);
+    // The forward of a real image (k_xtoep_real; n0 as xtoep).
+    static void xtoep_real(cudaStream_t st, int G, const XtArgs &a);
     // Raises the shared-memory limit of the k_xtoep variants for n0.
     static cudaError_t xtoep_prepare(int n0);
     // Raises the dynamic shared-memory limit of every kernel variant a plan uses.
