@@ -738,9 +738,28 @@ icon_status ensure_toeplitz(icon_plan *p, cudaStream_t st)
     const float *w = p->wgroups > 0 ? p->wuniq : p->nodes.w;
     dim3 grid((p->n1t + icon::kToepTile - 1) / icon::kToepTile, (p->n0 + icon::kToepTile - 1) / icon::kToepTile,
               groups_needed);
-    icon::k_toep_kernel<<<grid, 256, 0, st>>>(xy_d, w, p->wgroups > 0 ? (size_t)p->M : 0, p->M, p->N0, p->N1, p->n0,
-                                              p->n1t, icon::ytoep4_fits(p->n1t) ? p->n1t / 32 : 0, p->Kt);
+    // Node ranges: enough CTAs for the SMs, as far as G1, which no one reads
+    // before the next transform writes it, holds their sums.
+    const size_t plane = (size_t)p->n0 * p->n1t;
+    const size_t ctas = (size_t)grid.x * grid.y * grid.z;
+    // The nodes' sines and cosines go before them.
+    const size_t trig = (size_t)p->M * icon::kToepTrig, have = (size_t)p->Gcap * p->n0 * p->N1 * p->B;   // doubles
+    const size_t room = have > trig ? (have - trig) / (plane * groups_needed) : 0;
+    const int split = (int)std::max<size_t>(1, std::min({(size_t)16, (296 + ctas - 1) / ctas, room}));
+    double *tr = (double *)p->G1, *part = tr + trig;
+    if (have < trig) ICON_CUDA(cudaMalloc(&tr, sizeof(double) * trig));   // more tilts than image rows
+    icon::k_toep_trig<<<(p->M + 127) / 128, 128, 0, st>>>(xy_d, p->M, p->N0, p->N1, tr);
+    grid.z = groups_needed * split;
+    icon::k_toep_kernel<<<grid, 256, 0, st>>>(tr, w, p->wgroups > 0 ? (size_t)p->M : 0, p->M, p->N0, p->N1, p->n0,
+                                              p->n1t, icon::ytoep4_fits(p->n1t) ? p->n1t / 32 : 0, split, part, p->Kt);
+    if (split > 1)
+        icon::k_toep_sum<<<dim3((unsigned)((plane + 255) / 256), groups_needed), 256, 0, st>>>(
+            part, split, plane, 1.0 / ((double)p->n0 * (double)p->n1t), p->Kt);
     ICON_CUDA(cudaGetLastError());
+    if (have < trig) {
+        ICON_CUDA(cudaStreamSynchronize(st));
+        ICON_CUDA(cudaFree(tr));
+    }
     p->kt_groups = groups_needed;
     p->kt_stale = false;
     return ICON_OK;
@@ -1136,7 +1155,7 @@ static icon_status plan_create_impl(const icon_geometry *geo, int group, icon_pl
         return fail(ICON_ERR_INVALID, "FFT buffer exceeds shared memory");
     {
         cudaError_t e = cudaSuccess;
-        WITH_B(B, e = L::set_smem(p->ex, p->ey, p->smem_x, need_x, p->smem_y, p->smem_ya, p->smem_yt))
+        WITH_B(B, e = L::set_smem(p->ex, p->ey, p->n1, p->n1t))
         if (e != cudaSuccess) return fail(ICON_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
         WITH_B(B, e = L::xtoep_prepare(p->n0))
         if (e != cudaSuccess) return fail(ICON_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));

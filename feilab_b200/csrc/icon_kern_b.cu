@@ -131,7 +131,8 @@ template <int B, int BH, int LA, int LNB>
 static void xtr_go(cudaStream_t st, int G, const XtArgs &a)
 {
     using S = XtShape<BH, LA, LNB>;
-    k_xtoep_real<B, BH, LA, LNB><<<dim3((unsigned)(a.N1 * (B / BH)), (unsigned)G), S::T, sizeof(float2) * S::N * BH, st>>>(a);
+    k_xtoep_real<B, BH, LA, LNB><<<dim3((unsigned)(a.N1 * (B / BH)), (unsigned)G), xtr_threads(S::T),
+                                     sizeof(float2) * S::N * BH, st>>>(a);
 }
 template <int B, int BH, int LA, int LNB>
 static cudaError_t xtr_attr()
@@ -338,9 +339,10 @@ void Launch<B>::update_re(dim3 grid, cudaStream_t st, float *m, const float *rre
 // of a plan: plans of different sizes share the variants of one B, so every
 // variant gets the device's opt-in maximum (what a launch actually asks for
 // still sets the occupancy).  Lowering it to one plan's size would make a
-// larger plan's next launch fail.
+// larger plan's next launch fail.  Only the variants that a plan of these
+// sizes launches are set: all of a B's take 0.3 ms of the small plans' 1.4.
 template <int B>
-cudaError_t Launch<B>::set_smem(int ex, int ey, size_t, size_t, size_t, size_t, size_t)
+cudaError_t Launch<B>::set_smem(int ex, int ey, int n1, int n1t)
 {
     int dev = 0, optin = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -350,67 +352,65 @@ cudaError_t Launch<B>::set_smem(int ex, int ey, size_t, size_t, size_t, size_t, 
         cudaError_t r = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
         if (r != cudaSuccess && e == cudaSuccess) e = r;
     };
-    (void)ex;
-    (void)ey;
-    set((const void *)k_xpass_fwd<true, B, 32>);
-    set((const void *)k_xpass_fwd<false, B, 32>);
-    set((const void *)k_xpass_fwd_r2c<B, 32>);
-    set((const void *)k_xpass_fwd_r2c<B, 32, true>);
-    set((const void *)k_xpass_fwd<true, B, 32, true>);
-    set((const void *)k_xpass_adj<0, B, 32>);
-    set((const void *)k_xpass_adj<1, B, 32>);
-    set((const void *)k_rows_fwd<B, 32>);
-    set((const void *)k_row_adj<B, 32>);
-    set((const void *)k_xpass_fwd<true, B, 16>);
-    set((const void *)k_xpass_fwd<false, B, 16>);
-    set((const void *)k_xpass_fwd_r2c<B, 16>);
-    set((const void *)k_xpass_fwd_r2c<B, 16, true>);
-    set((const void *)k_xpass_fwd<true, B, 16, true>);
-    set((const void *)k_xpass_adj<0, B, 16>);
-    set((const void *)k_xpass_adj<1, B, 16>);
-    set((const void *)k_rows_fwd<B, 16>);
-    set((const void *)k_row_adj<B, 16>);
-    set((const void *)k_ypass_fwd<B, 32, false>);
-    set((const void *)k_ypass_fwd<B, 32, true>);
-    set((const void *)k_ypass_adj<B, 32, false>);
-    set((const void *)k_ypass_toep<B, 32>);
-    set((const void *)k_ypass_toep_quad<B, 32>);
-    set((const void *)k_ypass_fwd<B, 16, false>);
-    set((const void *)k_ypass_fwd<B, 16, true>);
-    set((const void *)k_ypass_adj<B, 16, false>);
-    set((const void *)k_ypass_adj<B, 16, true>);
-    set((const void *)k_yfwd4<B, 4, false>);
-    set((const void *)k_yfwd4<B, 4, true>);
-    set((const void *)k_yfwd4<B, 8, false>);
-    set((const void *)k_yfwd4<B, 8, true>);
-    set((const void *)k_yfwd4<B, 16, false>);
-    set((const void *)k_yfwd4<B, 16, true>);
-    set((const void *)k_yfwd4<B, 32, false>);
-    set((const void *)k_yfwd4<B, 32, true>);
-    set((const void *)k_yadj4<B, 4>);
-    set((const void *)k_yadj4<B, 8>);
-    set((const void *)k_yadj4<B, 16>);
-    set((const void *)k_yadj4<B, 32>);
-    set((const void *)k_ypass_toep<B, 16>);
-    set((const void *)k_ypass_toep_quad<B, 16>);
-    set((const void *)k_ytoep4<B, 4, 0>);
-    set((const void *)k_ytoep4<B, 6, 0>);
-    set((const void *)k_ytoep4<B, 8, 0>);
-    set((const void *)k_ytoep4<B, 10, 0>);
-    set((const void *)k_ytoep4<B, 12, 0>);
-    set((const void *)k_ytoep4<B, 16, 0>);
-    set((const void *)k_ytoep4<B, 20, 0>);
-    set((const void *)k_ytoep4<B, 24, 0>);
-    set((const void *)k_ytoep4<B, 32, 0>);
-    set((const void *)k_ytoep4<B, 4, 1>);
-    set((const void *)k_ytoep4<B, 6, 1>);
-    set((const void *)k_ytoep4<B, 8, 1>);
-    set((const void *)k_ytoep4<B, 10, 1>);
-    set((const void *)k_ytoep4<B, 12, 1>);
-    set((const void *)k_ytoep4<B, 16, 1>);
-    set((const void *)k_ytoep4<B, 20, 1>);
-    set((const void *)k_ytoep4<B, 24, 1>);
-    set((const void *)k_ytoep4<B, 32, 1>);
+    if (ex == 32) {
+        set((const void *)k_xpass_fwd<true, B, 32>);
+        set((const void *)k_xpass_fwd<false, B, 32>);
+        set((const void *)k_xpass_fwd_r2c<B, 32>);
+        set((const void *)k_xpass_fwd_r2c<B, 32, true>);
+        set((const void *)k_xpass_fwd<true, B, 32, true>);
+        set((const void *)k_xpass_adj<0, B, 32>);
+        set((const void *)k_xpass_adj<1, B, 32>);
+        set((const void *)k_rows_fwd<B, 32>);
+        set((const void *)k_row_adj<B, 32>);
+    } else {
+        set((const void *)k_xpass_fwd<true, B, 16>);
+        set((const void *)k_xpass_fwd<false, B, 16>);
+        set((const void *)k_xpass_fwd_r2c<B, 16>);
+        set((const void *)k_xpass_fwd_r2c<B, 16, true>);
+        set((const void *)k_xpass_fwd<true, B, 16, true>);
+        set((const void *)k_xpass_adj<0, B, 16>);
+        set((const void *)k_xpass_adj<1, B, 16>);
+        set((const void *)k_rows_fwd<B, 16>);
+        set((const void *)k_row_adj<B, 16>);
+    }
+    switch (yadj4_fits(n1) ? n1 / 32 : 0) {
+#define X(R) \
+    case R: \
+        set((const void *)k_yfwd4<B, R, false>); \
+        set((const void *)k_yfwd4<B, R, true>); \
+        set((const void *)k_yadj4<B, R>); \
+        break;
+        X(4) X(8) X(16) X(32)
+#undef X
+    default:
+        if (ey == 32) {
+            set((const void *)k_ypass_fwd<B, 32, false>);
+            set((const void *)k_ypass_fwd<B, 32, true>);
+            set((const void *)k_ypass_adj<B, 32, false>);
+        } else {
+            set((const void *)k_ypass_fwd<B, 16, false>);
+            set((const void *)k_ypass_fwd<B, 16, true>);
+            set((const void *)k_ypass_adj<B, 16, false>);
+            set((const void *)k_ypass_adj<B, 16, true>);
+        }
+    }
+    switch (ytoep4_fits(n1t) ? n1t / 32 : 0) {
+#define X(R) \
+    case R: \
+        set((const void *)k_ytoep4<B, R, 0>); \
+        set((const void *)k_ytoep4<B, R, 1>); \
+        break;
+        X(4) X(6) X(8) X(10) X(12) X(16) X(20) X(24) X(32)
+#undef X
+    default:
+        if (ey == 32) {
+            set((const void *)k_ypass_toep<B, 32>);
+            set((const void *)k_ypass_toep_quad<B, 32>);
+        } else {
+            set((const void *)k_ypass_toep<B, 16>);
+            set((const void *)k_ypass_toep_quad<B, 16>);
+        }
+    }
     return e;
 }
 

@@ -1228,14 +1228,15 @@ __global__ void k_update(float *__restrict__ m, const RT *__restrict__ rhat, con
 // approximation (they differ by the window error, ~1e-6 relative).
 //
 // K is a sum over the M nodes of rank-one products, computed in double as a
-// matrix product: a CTA owns a 64 x 64 tile of K (thread: 4 x 4 entries),
-// takes the nodes 32 at a time, evaluates their Dirichlet factors for the
-// tile's 64 k0 and 64 k1 into shared memory, and accumulates.  sin(pi u) and
+// matrix product: a CTA owns a 128 x 128 tile of K (thread: 8 x 8 entries, in
+// pairs 32 apart so that shared loads are conflict-free),
+// takes the nodes 16 at a time, evaluates their Dirichlet factors for the
+// tile's 128 k0 and 128 k1 into shared memory, and accumulates.  sin(pi u) and
 // sin(pi u (2N-1)) at u = x - k/n are formed from per-node and per-k sines
 // and cosines by the angle-difference formula; every argument is exact in
 // double (x is a float, k/n a dyadic fraction).
-constexpr int kToepTile = 64;
-constexpr int kToepNodes = 32;
+constexpr int kToepTile = 128;
+constexpr int kToepNodes = 16;
 
 // u = x - k/n is exact in double; at an integer u the angle-difference
 // formula leaves rounding noise in both sines, so integers are caught first.
@@ -1250,24 +1251,47 @@ __device__ __forceinline__ double dirichlet(double x, double kn, double sa, doub
 }
 
 #ifndef ICON_KERNELS_TEMPLATES_ONLY
-// xy: [M][2] node coordinates, w: [M] weights (group g's at w + g*wstride for
-// blockIdx.z = g); K: [G][n0][n1] float.  With perm_r > 0 each row is stored
+// Per node: sin, cos of pi x0, pi (2N0-1) x0, the same for x1; x0, x1.
+constexpr int kToepTrig = 10;
+__global__ void k_toep_trig(const float *__restrict__ xy, int M, int N0, int N1, double *__restrict__ trig)
+{
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= M) return;
+    const double x0 = (double)xy[2 * (size_t)j], x1 = (double)xy[2 * (size_t)j + 1];
+    double *t = trig + (size_t)j * kToepTrig;
+    sincospi(x0, &t[0], &t[1]);
+    sincospi((2.0 * N0 - 1.0) * x0, &t[2], &t[3]);
+    sincospi(x1, &t[4], &t[5]);
+    sincospi((2.0 * N1 - 1.0) * x1, &t[6], &t[7]);
+    t[8] = x0;
+    t[9] = x1;
+}
+
+// trig: [M][10] (k_toep_trig), w: [M] weights (set g's at w + g*wstride, g =
+// blockIdx.z / split); K: [G][n0][n1] float.  With perm_r > 0 each row is stored
 // in the order k_ytoep4 reads it: frequency k1 of row k0 at
-// (k1 mod R) * 32 + k1 / R, R = perm_r = n1 / 32.
-__global__ void __launch_bounds__(256) k_toep_kernel(const float *__restrict__ xy, const float *__restrict__ w,
+// (k1 mod R) * 32 + k1 / R, R = perm_r = n1 / 32.  split > 1: the nodes are cut
+// into `split` ranges, one per blockIdx.z mod split, whose sums go to
+// part[G][split][n0][n1] in double (k_toep_sum adds them in order): a kernel of
+// 1024 x 512 has 32 tiles for 148 SMs; its 31,232 nodes take 3.4 ms, and took 6.4
+// ms in one range by 64 x 64 tiles that evaluated the nodes' sines each.
+__global__ void __launch_bounds__(256, 1) k_toep_kernel(const double *__restrict__ trig, const float *__restrict__ w,
                                                      size_t wstride, int M, int N0, int N1, int n0, int n1,
-                                                     int perm_r, float *__restrict__ K)
+                                                     int perm_r, int split, double *__restrict__ part,
+                                                     float *__restrict__ K)
 {
     __shared__ __align__(16) double F0[kToepNodes][kToepTile];   // w_j D_N0(x_j0 - k0/n0)
     __shared__ __align__(16) double F1[kToepNodes][kToepTile];   // D_N1(x_j1 - k1/n1)
-    __shared__ double nd[kToepNodes][10];            // per node: sin, cos of pi x0, pi (2N0-1) x0, same for x1; x0, x1
+    __shared__ double nd[kToepNodes][kToepTrig];     // the chunk's nodes
     const int t = threadIdx.x;
-    const int k1b = blockIdx.x * kToepTile, k0b = blockIdx.y * kToepTile, grp = blockIdx.z;
+    const int k1b = blockIdx.x * kToepTile, k0b = blockIdx.y * kToepTile, grp = blockIdx.z / split;
+    const int rng = blockIdx.z - grp * split;
+    const int j_lo = (int)((long long)M * rng / split), j_hi = (int)((long long)M * (rng + 1) / split);
     const float *wg = w + (size_t)grp * wstride;
     const double a0 = 2.0 * N0 - 1.0, a1 = 2.0 * N1 - 1.0;
-    // This thread's k for the factor tables: column c = t % 64 of both tiles,
-    // nodes t / 64 + 4 i.
-    const int c = t & (kToepTile - 1), r0 = t >> 6;
+    // This thread's k for the factor tables: column c = t % 128 of both tiles,
+    // nodes t / 128 + 2 i.
+    const int c = t & (kToepTile - 1), r0 = t >> 7;
     double sk0, ck0, skb0, ckb0, sk1, ck1, skb1, ckb1;
     const double u0 = (double)(k0b + c) / n0, u1 = (double)(k1b + c) / n1;
     {
@@ -1276,62 +1300,67 @@ __global__ void __launch_bounds__(256) k_toep_kernel(const float *__restrict__ x
         sincospi(u1, &sk1, &ck1);
         sincospi(a1 * u1, &skb1, &ckb1);
     }
-    const int ty = t >> 4, tx = t & 15;              // outputs k0 = 4 ty + i, k1 = 4 tx + j
-    double acc[4][4];
+    const int ty = t >> 4, tx = t & 15;              // outputs k0 = 2 ty + 32 (i / 2) + i % 2, k1 = 2 tx + 32 (j / 2) + j % 2
+    double acc[8][8];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.0;
-    for (int j0 = 0; j0 < M; j0 += kToepNodes) {
+        for (int j = 0; j < 8; ++j) acc[i][j] = 0.0;
+    for (int j0 = j_lo; j0 < j_hi; j0 += kToepNodes) {
         __syncthreads();                             // the previous chunk's tables are consumed
-        if (t < kToepNodes) {
-            const int j = j0 + t;
-            double x0 = 0.0, x1 = 0.0;
-            if (j < M) {
-                x0 = (double)xy[2 * (size_t)j];
-                x1 = (double)xy[2 * (size_t)j + 1];
-            }
-            sincospi(x0, &nd[t][0], &nd[t][1]);
-            sincospi(a0 * x0, &nd[t][2], &nd[t][3]);
-            sincospi(x1, &nd[t][4], &nd[t][5]);
-            sincospi(a1 * x1, &nd[t][6], &nd[t][7]);
-            nd[t][8] = x0;
-            nd[t][9] = x1;
-        }
+        for (int i = t; i < kToepNodes * kToepTrig; i += 256)      // nodes past the range weigh 0
+            (&nd[0][0])[i] = trig[min((size_t)j0 * kToepTrig + i, (size_t)M * kToepTrig - 1)];
         __syncthreads();
 #pragma unroll
-        for (int i = 0; i < kToepNodes / 4; ++i) {
-            const int r = r0 + 4 * i, j = j0 + r;
-            const double wj = j < M ? (double)wg[j] : 0.0;
+        for (int i = 0; i < kToepNodes / 2; ++i) {
+            const int r = r0 + 2 * i, j = j0 + r;
+            const double wj = j < j_hi ? (double)wg[j] : 0.0;
             F0[r][c] = wj * dirichlet(nd[r][8], u0, nd[r][0], nd[r][1], nd[r][2], nd[r][3], sk0, ck0, skb0, ckb0, a0);
             F1[r][c] = dirichlet(nd[r][9], u1, nd[r][4], nd[r][5], nd[r][6], nd[r][7], sk1, ck1, skb1, ckb1, a1);
         }
         __syncthreads();
-#pragma unroll 4
+#pragma unroll 2
         for (int r = 0; r < kToepNodes; ++r) {
-            const double2 p0 = *reinterpret_cast<const double2 *>(&F0[r][4 * ty]);
-            const double2 p1 = *reinterpret_cast<const double2 *>(&F0[r][4 * ty + 2]);
-            const double2 q0 = *reinterpret_cast<const double2 *>(&F1[r][4 * tx]);
-            const double2 q1 = *reinterpret_cast<const double2 *>(&F1[r][4 * tx + 2]);
-            const double a[4] = {p0.x, p0.y, p1.x, p1.y}, b[4] = {q0.x, q0.y, q1.x, q1.y};
+            double a[8], b[8];
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int q = 0; q < 4; ++q) {
+                const double2 p = *reinterpret_cast<const double2 *>(&F0[r][2 * ty + 32 * q]);
+                const double2 v = *reinterpret_cast<const double2 *>(&F1[r][2 * tx + 32 * q]);
+                a[2 * q] = p.x;
+                a[2 * q + 1] = p.y;
+                b[2 * q] = v.x;
+                b[2 * q + 1] = v.y;
+            }
 #pragma unroll
-                for (int jj = 0; jj < 4; ++jj) acc[i][jj] = fma(a[i], b[jj], acc[i][jj]);
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int jj = 0; jj < 8; ++jj) acc[i][jj] = fma(a[i], b[jj], acc[i][jj]);
         }
     }
     const double scale = 1.0 / ((double)n0 * (double)n1);
     float *Kg = K + (size_t)grp * n0 * n1;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int k0 = k0b + 4 * ty + i;
+    for (int i = 0; i < 8; ++i) {
+        const int k0 = k0b + 2 * ty + 32 * (i / 2) + i % 2;
 #pragma unroll
-        for (int jj = 0; jj < 4; ++jj) {
-            const int k1 = k1b + 4 * tx + jj;
+        for (int jj = 0; jj < 8; ++jj) {
+            const int k1 = k1b + 2 * tx + 32 * (jj / 2) + jj % 2;
             const int pos = perm_r > 0 ? (k1 % perm_r) * 32 + k1 / perm_r : k1;
-            if (k0 < n0 && k1 < n1) Kg[(size_t)k0 * n1 + pos] = (float)(acc[i][jj] * scale);
+            if (k0 >= n0 || k1 >= n1) continue;
+            if (split > 1) part[((size_t)blockIdx.z * n0 + k0) * n1 + pos] = acc[i][jj];
+            else Kg[(size_t)k0 * n1 + pos] = (float)(acc[i][jj] * scale);
         }
     }
+}
+
+__global__ void k_toep_sum(const double *__restrict__ part, int split, size_t plane, double scale, float *__restrict__ K)
+{
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= plane) return;
+    part += (size_t)blockIdx.y * split * plane;
+    double a = part[i];
+    for (int r = 1; r < split; ++r) a += part[(size_t)r * plane + i];
+    K[(size_t)blockIdx.y * plane + i] = (float)(a * scale);
 }
 #endif  // ICON_KERNELS_TEMPLATES_ONLY
 
@@ -1852,50 +1881,57 @@ __device__ __forceinline__ void xt_twiddle(float2 (&v)[R], const float2 *__restr
 }
 
 // Forward transform from the step-1 registers v[i][a] (input at
-// x = 32 NB a + u + U i) to w[kc], frequency u + U kc.
+// x = 32 NB a + u + U i) to w[kc], frequency u + U kc.  Threads past the
+// transform's (!act) only take part in the barriers.
 template <int BH, int LA, int LNB>
 __device__ __forceinline__ void xt_forward(float2 (&v)[32 >> LA][1 << LA], float2 *s, int u, int sl,
-                                           const float2 *__restrict__ tw, float2 (&w)[32])
+                                           const float2 *__restrict__ tw, float2 (&w)[32], bool act = true)
 {
     using S = XtShape<BH, LA, LNB>;
     constexpr int NA = S::NA, NB = S::NB, U = S::U;
+    if (act) {
 #pragma unroll
-    for (int i = 0; i < S::NI1; ++i) {
-        const int tau = u + U * i;
-        float2 a[NA];
+        for (int i = 0; i < S::NI1; ++i) {
+            const int tau = u + U * i;
+            float2 a[NA];
 #pragma unroll
-        for (int j = 0; j < NA; ++j) a[brev5(j) >> (5 - LA)] = v[i][j];
-        dft_inplace<NA>(a, -1.f);
-        if (tau) xt_twiddle<NA, false>(a, tw, tau);
+            for (int j = 0; j < NA; ++j) a[brev5(j) >> (5 - LA)] = v[i][j];
+            dft_inplace<NA>(a, -1.f);
+            if (tau) xt_twiddle<NA, false>(a, tw, tau);
 #pragma unroll
-        for (int ka = 0; ka < NA; ++ka) s[S::e1(ka, tau, sl)] = a[ka];
+            for (int ka = 0; ka < NA; ++ka) s[S::e1(ka, tau, sl)] = a[ka];
+        }
     }
     __syncthreads();
     if constexpr (NB > 1) {
         float2 v2[S::NI2][NB];
+        if (act) {
 #pragma unroll
-        for (int i = 0; i < S::NI2; ++i) {
-            const int t2 = u + U * i, c = t2 & 31, ka = t2 >> 5;
+            for (int i = 0; i < S::NI2; ++i) {
+                const int t2 = u + U * i, c = t2 & 31, ka = t2 >> 5;
 #pragma unroll
-            for (int b = 0; b < NB; ++b) v2[i][brev5(b) >> (5 - LNB)] = s[S::e1(ka, 32 * b + c, sl)];
+                for (int b = 0; b < NB; ++b) v2[i][brev5(b) >> (5 - LNB)] = s[S::e1(ka, 32 * b + c, sl)];
+            }
         }
         __syncthreads();
+        if (act) {
 #pragma unroll
-        for (int i = 0; i < S::NI2; ++i) {
-            const int t2 = u + U * i, c = t2 & 31, ka = t2 >> 5;
-            dft_inplace<NB>(v2[i], -1.f);
-            if (c) xt_twiddle<NB, false>(v2[i], tw, NA * c);
+            for (int i = 0; i < S::NI2; ++i) {
+                const int t2 = u + U * i, c = t2 & 31, ka = t2 >> 5;
+                dft_inplace<NB>(v2[i], -1.f);
+                if (c) xt_twiddle<NB, false>(v2[i], tw, NA * c);
 #pragma unroll
-            for (int kb = 0; kb < NB; ++kb) s[S::e2(ka, kb, c, sl)] = v2[i][kb];
+                for (int kb = 0; kb < NB; ++kb) s[S::e2(ka, kb, c, sl)] = v2[i][kb];
+            }
         }
         __syncthreads();
     }
-    {
+    if (act) {
         const int ka = u % NA, kb = u / NA;
 #pragma unroll
         for (int c = 0; c < 32; ++c) w[brev5(c)] = (NB > 1) ? s[S::e2(ka, kb, c, sl)] : s[S::e1(ka, c, sl)];
     }
-    dft_inplace<32>(w, -1.f);
+    if (act) dft_inplace<32>(w, -1.f);
 }
 
 // The same, the frequencies stored to G1 rows u + U kc of column `col` (pointer
@@ -2180,6 +2216,10 @@ __global__ void __launch_bounds__(XtShape<BH, LA, LNB>::T, (XtShape<BH, LA, LNB>
     }
 }
 
+// Threads of k_xtoep_real: the transform's T, at least 64 for the copies and
+// the untangling (a one-slice group of n0 = 128 has T = 2).
+__host__ __device__ constexpr int xtr_threads(int T) { return T < 64 ? 64 : T; }
+
 // Forward x-transform of a real image, with half-length FFTs: the n0 values
 // x(t) of a slice's padded column are packed as z(q) = x(2q) + i x(2q+1), one
 // FFT of length N = n0/2 (the three steps of xt_forward), and with Z = FFT(z),
@@ -2192,14 +2232,15 @@ __global__ void __launch_bounds__(XtShape<BH, LA, LNB>::T, (XtShape<BH, LA, LNB>
 // Bound by memory and latency: 128 slices of 1024 x 300 with the update,
 // 366 us with full-length transforms and every row stored, 234 us so.
 template <int B, int BH, int LA, int LNB>
-__global__ void __launch_bounds__(XtShape<BH, LA, LNB>::T, (XtShape<BH, LA, LNB>::T >= 256) ? 2 : 4)
+__global__ void __launch_bounds__(xtr_threads(XtShape<BH, LA, LNB>::T), (XtShape<BH, LA, LNB>::T >= 256) ? 2 : 4)
     k_xtoep_real(const __grid_constant__ XtArgs g)
 {
     using S = XtShape<BH, LA, LNB>;
-    constexpr int NA = S::NA, NB = S::NB, U = S::U, H = B / BH, N = S::N;
+    constexpr int NA = S::NA, NB = S::NB, U = S::U, H = B / BH, N = S::N, T = xtr_threads(S::T);
     extern __shared__ __align__(128) float2 s[];
     const int Y = blockIdx.x / H, h = blockIdx.x % H, grp = blockIdx.y;
     const int t = threadIdx.x, sl = t % BH, u = t / BH;
+    const bool act = T == S::T || t < S::T;
     const int N0 = g.N0, N1 = g.N1, half = N0 / 2;
     const size_t ibase = (((size_t)grp * N1 + Y) * N0) * B + h * BH;       // image point X at ibase + X*B
     // The m column [N0][BH] and, for the update, the Re r-hat column: N0 <= N,
@@ -2207,14 +2248,14 @@ __global__ void __launch_bounds__(XtShape<BH, LA, LNB>::T, (XtShape<BH, LA, LNB>
     float *Ms = reinterpret_cast<float *>(s), *Rs = Ms + N * BH;
     auto stage = [&](float *dst, const float *src) {
         if constexpr (BH == B && B >= 4) {
-            for (int i = t; i < N0 * (BH / 4); i += S::T) cp_async<16>(dst + 4 * i, src + 4 * i);
+            for (int i = t; i < N0 * (BH / 4); i += T) cp_async<16>(dst + 4 * i, src + 4 * i);
         } else if constexpr (BH >= 4) {
-            for (int i = t; i < N0 * (BH / 4); i += S::T) {
+            for (int i = t; i < N0 * (BH / 4); i += T) {
                 const int X = i / (BH / 4), c = i % (BH / 4);
                 cp_async<16>(dst + 4 * i, src + (size_t)X * B + 4 * c);
             }
         } else {
-            for (int X = t; X < N0; X += S::T) cp_async<4 * BH>(dst + X * BH, src + (size_t)X * B);
+            for (int X = t; X < N0; X += T) cp_async<4 * BH>(dst + X * BH, src + (size_t)X * B);
         }
     };
     stage(Ms, g.m + ibase);
@@ -2225,8 +2266,8 @@ __global__ void __launch_bounds__(XtShape<BH, LA, LNB>::T, (XtShape<BH, LA, LNB>
     if (g.upd) {
         // m <- m - alpha Re r-hat (k_update's arithmetic), clamped on ICON steps.
         float *mdst = g.m + ibase;
-        const double al = g.alpha[grp * B + h * BH + sl];                    // S::T is a multiple of BH
-        for (int idx = t; idx < N0 * BH; idx += S::T) {
+        const double al = g.alpha[grp * B + h * BH + sl];                    // T is a multiple of BH
+        for (int idx = t; idx < N0 * BH; idx += T) {
             float nv = (float)((double)Ms[idx] - al * (double)Rs[idx]);
             if (g.clamp) {
                 if (g.data_type == 1) {
@@ -2248,22 +2289,26 @@ __global__ void __launch_bounds__(XtShape<BH, LA, LNB>::T, (XtShape<BH, LA, LNB>
         return g.deapod ? v * (__ldg(&g.rcx[X]) * rcyY) : v;
     };
     float2 v[S::NI1][NA];
+    if (act) {
 #pragma unroll
-    for (int i = 0; i < S::NI1; ++i)
+        for (int i = 0; i < S::NI1; ++i)
 #pragma unroll
-        for (int a = 0; a < NA; ++a) {
-            const int q = 2 * (32 * NB * a + u + U * i);
-            v[i][a] = make_float2(xval(q), xval(q + 1));
-        }
+            for (int a = 0; a < NA; ++a) {
+                const int q = 2 * (32 * NB * a + u + U * i);
+                v[i][a] = make_float2(xval(q), xval(q + 1));
+            }
+    }
     __syncthreads();   // the staged columns are read before step 1 rewrites s
     float2 w[32];
-    xt_forward<BH, LA, LNB>(v, s, u, sl, g.tw0h, w);
+    xt_forward<BH, LA, LNB>(v, s, u, sl, g.tw0h, w, act);
     __syncthreads();   // every read of s by the transform is done
+    if (act) {
 #pragma unroll
-    for (int kc = 0; kc < 32; ++kc) s[(u + U * kc) * BH + sl] = w[kc];
+        for (int kc = 0; kc < 32; ++kc) s[(u + U * kc) * BH + sl] = w[kc];
+    }
     __syncthreads();
     float2 *out = g.Gh + ((size_t)grp * g.gh_rows * N1 + Y) * B + h * BH + sl;
-    for (int k = u; k <= N; k += U) {
+    for (int k = u; k <= N; k += T / BH) {
         const float2 zk = s[(k & (N - 1)) * BH + sl], zm = s[((N - k) & (N - 1)) * BH + sl];
         const float2 fe = make_float2(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y));
         const float2 fo = make_float2(0.5f * (zk.y + zm.y), -0.5f * (zk.x - zm.x));

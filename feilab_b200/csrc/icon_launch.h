@@ -64,9 +64,10 @@ struct Launch {
     static void xtoep_real(cudaStream_t st, int G, const XtArgs &a);
     // Raises the shared-memory limit of the k_xtoep variants for n0.
     static cudaError_t xtoep_prepare(int n0);
-    // Raises the dynamic shared-memory limit of every kernel variant a plan uses.
-    static cudaError_t set_smem(int ex, int ey, size_t smem_x, size_t need_x, size_t smem_y, size_t smem_ya,
-                                size_t smem_yt);
+    // Raises the dynamic shared-memory limit of every kernel variant a plan uses
+    // (besides xtoep_prepare's): values per FFT thread, y lengths of the NUFFT
+    // and of the Toeplitz operator.
+    static cudaError_t set_smem(int ex, int ey, int n1, int n1t);
 };
 
 }  // namespace icon
