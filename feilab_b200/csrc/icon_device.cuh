@@ -367,44 +367,92 @@ __host__ __device__ constexpr double ct_cos(double x)
 // 3- and 5-point DFTs in place (natural order), sign dir.  With
 // w = exp(dir 2 pi i / P): X_k = sum_r x_r w^(r k), written as sums and
 // differences of the symmetric pairs x_r +- x_(P-r).
+// Z: inputs known to be zero, bit r for x_r (they are not read).
+template <bool ZA, bool ZB>
+__device__ __forceinline__ float2 zadd(float2 a, float2 b)
+{
+    if constexpr (ZA && ZB) return make_float2(0.f, 0.f);
+    else if constexpr (ZA) return b;
+    else if constexpr (ZB) return a;
+    else return add2(a, b);
+}
+template <bool ZA, bool ZB>
+__device__ __forceinline__ float2 zsub(float2 a, float2 b)
+{
+    if constexpr (ZA && ZB) return make_float2(0.f, 0.f);
+    else if constexpr (ZA) return make_float2(-b.x, -b.y);
+    else if constexpr (ZB) return a;
+    else return sub2(a, b);
+}
+// a + c b with a real constant c
+template <bool ZA, bool ZB>
+__device__ __forceinline__ float2 zfma(float c, float2 b, float2 a)
+{
+    if constexpr (ZB) return ZA ? make_float2(0.f, 0.f) : a;
+    else if constexpr (ZA) return make_float2(c * b.x, c * b.y);
+    else return make_float2(fmaf(c, b.x, a.x), fmaf(c, b.y, a.y));
+}
+
+template <unsigned Z>
 __device__ __forceinline__ void dft3(float2 (&a)[3], float dir)
 {
+    constexpr bool z0 = Z & 1, z1 = Z & 2, z2 = Z & 4, zt = z1 && z2;
     constexpr float h = 0.8660254037844386f;   // sin(2 pi / 3)
-    const float2 s = add2(a[1], a[2]), d = sub2(a[1], a[2]);
-    const float2 m = make_float2(fmaf(-0.5f, s.x, a[0].x), fmaf(-0.5f, s.y, a[0].y));
+    const float2 s = zadd<z1, z2>(a[1], a[2]), d = zsub<z1, z2>(a[1], a[2]), x0 = a[0];
+    const float2 m = zfma<z0, zt>(-0.5f, s, x0);
     const float hd = dir * h;
-    a[0] = add2(a[0], s);
+    a[0] = zadd<z0, zt>(x0, s);
     a[1] = make_float2(fmaf(-hd, d.y, m.x), fmaf(hd, d.x, m.y));   // m + i dir h (x1 - x2)
     a[2] = make_float2(fmaf(hd, d.y, m.x), fmaf(-hd, d.x, m.y));
 }
 
+template <unsigned Z>
 __device__ __forceinline__ void dft5(float2 (&a)[5], float dir)
 {
+    constexpr bool z0 = Z & 1, z1 = Z & 2, z2 = Z & 4, z3 = Z & 8, z4 = Z & 16;
+    constexpr bool za = z1 && z4, zb = z2 && z3;     // the pairs' sums and differences
     constexpr float c1 = (float)ct_cos(ct_angle(1, 5)), c2 = (float)ct_cos(ct_angle(2, 5));
     constexpr float s1 = (float)ct_sin(ct_angle(1, 5));
     constexpr float r = (float)(ct_sin(ct_angle(2, 5)) / ct_sin(ct_angle(1, 5)));
-    const float2 t1 = add2(a[1], a[4]), t2 = add2(a[2], a[3]), t3 = sub2(a[1], a[4]), t4 = sub2(a[2], a[3]);
+    const float2 t1 = zadd<z1, z4>(a[1], a[4]), t2 = zadd<z2, z3>(a[2], a[3]);
+    const float2 t3 = zsub<z1, z4>(a[1], a[4]), t4 = zsub<z2, z3>(a[2], a[3]);
     const float2 x0 = a[0];
-    const float2 p1 = make_float2(fmaf(c2, t2.x, fmaf(c1, t1.x, x0.x)), fmaf(c2, t2.y, fmaf(c1, t1.y, x0.y)));
-    const float2 p2 = make_float2(fmaf(c1, t2.x, fmaf(c2, t1.x, x0.x)), fmaf(c1, t2.y, fmaf(c2, t1.y, x0.y)));
+    const float2 p1 = zfma<z0 && za, zb>(c2, t2, zfma<z0, za>(c1, t1, x0));
+    const float2 p2 = zfma<z0 && za, zb>(c1, t2, zfma<z0, za>(c2, t1, x0));
     // q1 = s1 t3 + s2 t4 = s1 u1, q2 = s2 t3 - s1 t4 = s1 u2;
     // X1,4 = p1 +- i dir q1, X2,3 = p2 +- i dir q2
-    const float2 u1 = make_float2(fmaf(r, t4.x, t3.x), fmaf(r, t4.y, t3.y));
-    const float2 u2 = make_float2(fmaf(r, t3.x, -t4.x), fmaf(r, t3.y, -t4.y));
+    const float2 u1 = zfma<za, zb>(r, t4, t3);
+    const float2 u2 = zb ? zfma<true, za>(r, t3, x0) : zfma<false, za>(r, t3, make_float2(-t4.x, -t4.y));
     const float sd = dir * s1;
-    a[0] = add2(x0, add2(t1, t2));
+    a[0] = zadd<z0, za && zb>(x0, zadd<za, zb>(t1, t2));
     a[1] = make_float2(fmaf(-sd, u1.y, p1.x), fmaf(sd, u1.x, p1.y));
     a[4] = make_float2(fmaf(sd, u1.y, p1.x), fmaf(-sd, u1.x, p1.y));
     a[2] = make_float2(fmaf(-sd, u2.y, p2.x), fmaf(sd, u2.x, p2.y));
     a[3] = make_float2(fmaf(sd, u2.y, p2.x), fmaf(-sd, u2.x, p2.y));
 }
 
-template <int P>
+template <int P, unsigned Z>
 __device__ __forceinline__ void dft_small(float2 (&a)[P], float dir)
 {
     static_assert(P == 3 || P == 5, "radix 3 or 5");
-    if constexpr (P == 3) dft3(a, dir);
-    else dft5(a, dir);
+    if constexpr (P == 3) dft3<Z>(a, dir);
+    else dft5<Z>(a, dir);
+}
+
+// Zero inputs of the P-point DFT of q in the prime-factor form of an R-point DFT
+// whose inputs from R/2 on are zero (HALF).
+template <int R, int P, int Q, bool HALF>
+__host__ __device__ constexpr unsigned pfa_zeros(int q)
+{
+    unsigned z = 0;
+    for (int p = 0; p < P; ++p)
+        if (HALF && (Q * p + P * q) % R >= R / 2) z |= 1u << p;
+    return z;
+}
+template <int R, int P, int Q, bool HALF, int... Qs>
+__device__ __forceinline__ void pfa_small(float2 (&y)[Q][P], float dir, std::integer_sequence<int, Qs...>)
+{
+    (dft_small<P, pfa_zeros<R, P, Q, HALF>(Qs)>(y[Qs], dir), ...);
 }
 
 // The k < P Q with k mod P = k1 and k mod Q = k2 (P and Q coprime).
@@ -424,7 +472,8 @@ __host__ __device__ constexpr int crt_index(int P, int Q, int k1, int k2)
 // p, Q-point DFTs over q, and the outputs k by k mod P and k mod Q; all index
 // maps only rename registers (20 points: 208 multiply-adds, 256 with the
 // twiddles of the Cooley-Tukey form).
-template <int R>
+// HALF: the inputs from a[R/2] on are zero (and not read; R = P Q only).
+template <int R, bool HALF = false>
 __device__ __forceinline__ void dft_nat(float2 (&a)[R], float dir)
 {
     if constexpr ((R & (R - 1)) == 0) {
@@ -443,9 +492,10 @@ __device__ __forceinline__ void dft_nat(float2 (&a)[R], float dir)
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
 #pragma unroll
-            for (int p = 0; p < P; ++p) y[q][p] = a[(Q * p + P * q) % R];
-            dft_small<P>(y[q], dir);
+            for (int p = 0; p < P; ++p)
+                if (!HALF || (Q * p + P * q) % R < R / 2) y[q][p] = a[(Q * p + P * q) % R];
         }
+        pfa_small<R, P, Q, HALF>(y, dir, std::make_integer_sequence<int, Q>{});
 #pragma unroll
         for (int k1 = 0; k1 < P; ++k1) {
             float2 u[Q];
@@ -460,7 +510,7 @@ __device__ __forceinline__ void dft_nat(float2 (&a)[R], float dir)
 
 // dft_nat of values whose upper half a[R/2..] is zero (and is not read).  For a
 // power of two the first stage only copies; for P = 3 or 5 times one the
-// P-point DFTs take the zeros as literals.
+// P-point DFTs leave the zeros out.
 template <int R>
 __device__ __forceinline__ void dft_half_nat(float2 (&a)[R], float dir)
 {
@@ -476,9 +526,7 @@ __device__ __forceinline__ void dft_half_nat(float2 (&a)[R], float dir)
 #pragma unroll
         for (int r = 0; r < R; ++r) a[r] = t[r];
     } else {
-#pragma unroll
-        for (int r = R / 2; r < R; ++r) a[r] = make_float2(0.f, 0.f);
-        dft_nat<R>(a, dir);
+        dft_nat<R, true>(a, dir);
     }
 }
 

@@ -1503,6 +1503,8 @@ __device__ __forceinline__ int ytoep4_sidx(int c, int k1, int b)
     return ((c * R + (k1 ^ (c & SWM))) << LB) + b;
 }
 
+constexpr int kLdK = 36;   // stride of a k1's 32 factors of K in shared memory
+
 // Lengths R of the first step k_ytoep4 is built for.
 __host__ __device__ constexpr bool ytoep4_radix_ok(int R)
 {
@@ -1539,6 +1541,11 @@ __global__ void __launch_bounds__(R * B, (R == 20 && B == 8) ? 4 : 16 / ((R * B 
     // every twiddle of the two steps is read from it.
     float2 *tws = s + 32 * R * B;
     for (int q = t; q < 32 * R / 2; q += R * B) cp_async<16>(tws + 2 * q, g.tw1 + 2 * q);
+    // K[x], 32 factors a k1 (a stride of 36 spreads the k1 of a warp's lanes over
+    // the banks), needed only between the two transforms: its own group.
+    cp_async_commit();
+    float *ks = reinterpret_cast<float *>(tws + 32 * R);
+    for (int q = t; q < 8 * R; q += R * B) cp_async<16>(ks + (q >> 3) * kLdK + 4 * (q & 7), krow + 4 * q);
     cp_async_commit();
 
     // Step 1: R-point DFTs over a, twiddles wn^(c k1), transpose.
@@ -1557,7 +1564,7 @@ __global__ void __launch_bounds__(R * B, (R == 20 && B == 8) ? 4 : 16 / ((R * B 
                 for (int a = 0; a < R / 2; ++a) v[i][a].y = -v[i][a].y;
             }
         }
-        cp_async_wait<0>();
+        cp_async_wait<1>();
         __syncthreads();   // the twiddle table is in shared memory
 #pragma unroll
         for (int i = 0; i < NI; ++i) {
@@ -1570,6 +1577,7 @@ __global__ void __launch_bounds__(R * B, (R == 20 && B == 8) ? 4 : 16 / ((R * B 
             for (int k1 = 0; k1 < R; ++k1) s[ytoep4_sidx<B, R>(c, k1, b)] = v[i][k1];
         }
     }
+    cp_async_wait<0>();
     __syncthreads();
     // Step 2: 32-point DFT over c for k1 = u: w[k2] = X[u + R k2].
     float2 w[32];
@@ -1577,12 +1585,12 @@ __global__ void __launch_bounds__(R * B, (R == 20 && B == 8) ? 4 : 16 / ((R * B 
     for (int c = 0; c < 32; ++c) w[brev5(c)] = s[ytoep4_sidx<B, R>(c, u, b)];
     dft_inplace<32>(w, -1.f);
     // K[x][u + R k2] for k2 = 0..31: 32 consecutive floats of the permuted row.
-    const float4 *kq = reinterpret_cast<const float4 *>(krow + 32 * u);
+    const float4 *kq = reinterpret_cast<const float4 *>(ks + kLdK * u);
     if constexpr (MODE == 1) {
         double acc = 0.0;
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-            const float4 k4 = __ldg(&kq[q]);
+            const float4 k4 = kq[q];
             const float kv[4] = {k4.x, k4.y, k4.z, k4.w};
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -1599,7 +1607,7 @@ __global__ void __launch_bounds__(R * B, (R == 20 && B == 8) ? 4 : 16 / ((R * B 
         // In place: w[k2] *= K, then the DIF inverse leaves Z[c] at w[brev5(c)].
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-            const float4 k4 = __ldg(&kq[q]);
+            const float4 k4 = kq[q];
             const float kv[4] = {k4.x, k4.y, k4.z, k4.w};
 #pragma unroll
             for (int j = 0; j < 4; ++j) w[4 * q + j] = make_float2(w[4 * q + j].x * kv[j], w[4 * q + j].y * kv[j]);
@@ -1633,7 +1641,10 @@ __global__ void __launch_bounds__(R * B, (R == 20 && B == 8) ? 4 : 16 / ((R * B 
     }
 }
 
-__host__ __device__ inline size_t ytoep4_smem(int n1, int B) { return (size_t)n1 * (B + 1) * sizeof(float2); }
+__host__ __device__ inline size_t ytoep4_smem(int n1, int B)
+{
+    return (size_t)n1 * (B + 1) * sizeof(float2) + (size_t)(n1 / 32) * kLdK * sizeof(float);
+}
 // n1 sizes k_ytoep4 takes (n1 = 32 R, R in ytoep4_radix_ok).
 __host__ __device__ inline bool ytoep4_fits(int n1) { return n1 % 32 == 0 && ytoep4_radix_ok(n1 / 32); }
 
