@@ -461,7 +461,7 @@ bool make_map(CUtensorMap *m, void *base, int rank, const cuuint64_t *dims, cons
 void setup_xt_tma(icon_plan *p)
 {
     const int n0 = p->n0, B = p->B;
-    p->xt_bh = n0 <= 1024 ? B : n0 == 2048 ? std::min(B, 4) : n0 == 4096 ? std::min(B, 2) : 1;
+    p->xt_bh = n0 < 1024 ? B : n0 <= 2048 ? std::min(B, 4) : n0 == 4096 ? std::min(B, 2) : 1;
     const char *env = std::getenv("ICON_XT_TMA");
     if (!p->xt_ok || p->xt_bh < 2 || (env && env[0] == '0')) return;
     const int BH = p->xt_bh;

@@ -111,7 +111,7 @@ static cudaError_t xt_attr()
     X(128, B, 2, 0)                                   \
     X(256, B, 3, 0)                                   \
     X(512, B, 4, 0)                                   \
-    X(1024, B, 5, 0)                                  \
+    X(1024, (B < 4 ? B : 4), 5, 0)                    \
     X(2048, (B < 4 ? B : 4), 3, 3)                    \
     X(4096, (B < 2 ? B : 2), 4, 3)                    \
     X(8192, 1, 4, 4)
