@@ -194,6 +194,7 @@ __device__ __forceinline__ void store_b(float2 *__restrict__ p, const float2 (&v
 template <bool REAL_IN, int B, int E, bool FULL = false>
 __global__ void FFT_BOUNDS(E) k_xpass_fwd(Geo g, const void *__restrict__ in, float2 *__restrict__ G1)
 {
+    pdl_wait();
     extern __shared__ float2 s[];
     const int Y = blockIdx.x, grp = blockIdx.y, n = g.n0, N0 = g.N0, N1 = g.N1;
     const float rcyY = g.rcy[Y];
@@ -239,6 +240,7 @@ __global__ void FFT_BOUNDS(E) k_xpass_fwd(Geo g, const void *__restrict__ in, fl
 template <int B, int E, bool FULL = false>
 __global__ void FFT_BOUNDS(E) k_xpass_fwd_r2c(Geo g, const float *__restrict__ in, float2 *__restrict__ G1)
 {
+    pdl_wait();
     extern __shared__ float2 s[];
     const int Y = blockIdx.x, grp = blockIdx.y, n = g.n0, N = g.n0 / 2, N0 = g.N0, N1 = g.N1;
     const float rcyY = g.rcy[Y];
@@ -486,6 +488,7 @@ __device__ __forceinline__ void yfwd_interp(const Geo &g, const float2 *s, int g
 template <int B, int E, bool HERM>
 __global__ void FFT_BOUNDS(E) k_ypass_fwd(Geo g, const float2 *__restrict__ G1, float2 *__restrict__ P)
 {
+    pdl_wait();
     extern __shared__ float2 s[];
     constexpr int SB = YfStride<B>::v;
     constexpr bool kPairs = (B == 8);   // 64-byte rows read as 128-byte row pairs
@@ -525,6 +528,7 @@ __global__ void FFT_BOUNDS(E) k_ypass_fwd(Geo g, const float2 *__restrict__ G1, 
 template <int MODE, int B>
 __global__ void k_interp_fin(Geo g, const float2 *__restrict__ P, float2 *__restrict__ f, double *__restrict__ part)
 {
+    pdl_wait();
     __shared__ double red[256];
     constexpr int LB = Log2B<B>::v;
     const int grp = blockIdx.y;
@@ -782,6 +786,7 @@ __device__ __forceinline__ void yadj_gather(const Geo &g, int x, const float2 *f
 template <int B, int E, bool GUARD>
 __global__ void FFT_BOUNDS(E) k_ypass_adj(Geo g, const float2 *__restrict__ f, float2 *__restrict__ G1)
 {
+    pdl_wait();
     extern __shared__ float2 s[];
     constexpr bool kSwz = (B == 8);
     const int grp = blockIdx.x, x = yadj_row(blockIdx.y, g.n0), n = g.n1, N1 = g.N1;
@@ -813,6 +818,7 @@ template <int MODE, int B, int E>
 __global__ void FFT_BOUNDS(E) k_xpass_adj(Geo g, const float2 *__restrict__ G1, float2 *__restrict__ out,
                                           const float2 *__restrict__ Ahwb, double *__restrict__ part)
 {
+    pdl_wait();
     extern __shared__ float2 s[];
     double *red = (double *)(s + (size_t)g.n0 * B);
     const int Y = blockIdx.x, grp = blockIdx.y, n = g.n0, N0 = g.N0, N1 = g.N1;
@@ -882,6 +888,7 @@ __global__ void FFT_BOUNDS(E) k_rows_fwd(Geo g, Geo1 g1, const float *__restrict
                                          size_t istride, int skip, int S, float2 *__restrict__ f,
                                          float2 *__restrict__ bout)
 {
+    pdl_wait();
     extern __shared__ float2 s[];
     constexpr int LB = Log2B<B>::v;
     const int i = blockIdx.x, grp = blockIdx.y, n = g.n0, N = g.nx;
@@ -927,6 +934,7 @@ __global__ void FFT_BOUNDS(E) k_rows_fwd(Geo g, Geo1 g1, const float *__restrict
 template <int B, int E>
 __global__ void FFT_BOUNDS(E) k_row_adj(Geo g, Geo1 g1, const float2 *__restrict__ f, float *__restrict__ out, int S)
 {
+    pdl_wait();
     extern __shared__ float2 s[];
     const int grp = blockIdx.x, n = g.n0, N = g.nx;
     const float2 *fg = f + (size_t)grp * N * B;
@@ -983,6 +991,7 @@ struct ImgTile {
 template <typename T, int B, bool IN>
 __global__ void __launch_bounds__(256) k_img_move(const T *__restrict__ src, T *__restrict__ dst, int S, int N0, int N1)
 {
+    pdl_wait();
     using I = ImgTile<T, B>;
     __shared__ __align__(16) unsigned char raw[I::SMEM];
     T *s = reinterpret_cast<T *>(raw);
@@ -1026,6 +1035,7 @@ __global__ void __launch_bounds__(256) k_img_move(const T *__restrict__ src, T *
 template <int B>
 __global__ void k_img_out_file(const float *__restrict__ src, float *__restrict__ dst, int S, int N0, int N1)
 {
+    pdl_wait();
     const size_t plane = (size_t)N0 * N1;
     const int G = (S + B - 1) / B;
     const size_t total = (size_t)G * plane;
@@ -1059,6 +1069,7 @@ __global__ void k_img_out_file(const float *__restrict__ src, float *__restrict_
 template <int B>
 __global__ void k_nodes_in(const float2 *__restrict__ src, float2 *__restrict__ dst, int S, int M)
 {
+    pdl_wait();
     const int grp = blockIdx.y, j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= M) return;
     float2 v[B];
@@ -1073,6 +1084,7 @@ __global__ void k_nodes_in(const float2 *__restrict__ src, float2 *__restrict__ 
 template <int B>
 __global__ void k_nodes_out(const float2 *__restrict__ src, float2 *__restrict__ dst, int S, int M)
 {
+    pdl_wait();
     const int grp = blockIdx.y, j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= M) return;
     float2 v[B];
@@ -1099,6 +1111,7 @@ __global__ void __launch_bounds__(kAlphaThreads) k_alpha(const double *__restric
                                                          double *__restrict__ alpha, double *__restrict__ hist_alpha,
                                                          double *__restrict__ hist_rtr)
 {
+    pdl_wait();
     __shared__ double red[2][kAlphaThreads / 32][B];
     const int grp = blockIdx.x, t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const double *p1 = part_rtr + (size_t)grp * nr * B, *p2 = part_rtar + (size_t)grp * na * B;
@@ -1166,6 +1179,7 @@ template <int B, bool MEASURE = false, typename RT = float2>
 __global__ void k_update(float *__restrict__ m, const RT *__restrict__ rhat, const double *__restrict__ alpha,
                          int per_group, int clamp, int data_type, float thr, double *__restrict__ step_part = nullptr)
 {
+    pdl_wait();
     const int grp = blockIdx.y;
     float *mg = m + (size_t)grp * per_group;
     const RT *rg = rhat + (size_t)grp * per_group;
@@ -1389,6 +1403,7 @@ __device__ __forceinline__ int half_row(int i, int n0)
 template <int B, int E>
 __global__ void FFT_BOUNDS(E) k_ypass_toep(Geo g, float2 *__restrict__ G1, const float2 *__restrict__ Gh)
 {
+    pdl_wait();
     extern __shared__ float2 s[];
     constexpr int SB = YfStride<B>::v;
     constexpr bool kSwz = (B == 8);
@@ -1433,6 +1448,7 @@ __global__ void FFT_BOUNDS(E) k_ypass_toep(Geo g, float2 *__restrict__ G1, const
 template <int B, int E>
 __global__ void FFT_BOUNDS(E) k_ypass_toep_quad(Geo g, const float2 *__restrict__ G1, double *__restrict__ part)
 {
+    pdl_wait();
     extern __shared__ float2 s[];
     constexpr int SB = YfStride<B>::v;
     constexpr bool kSwz = (B == 8);
@@ -1526,6 +1542,7 @@ template <int B, int R, int MODE>
 __global__ void __launch_bounds__(R * B, (R == 20 && B == 8) ? 4 : 16 / ((R * B + 31) / 32))
     k_ytoep4(Geo g, float2 *__restrict__ G1, const float2 *__restrict__ Gh, double *__restrict__ part)
 {
+    pdl_wait();
     constexpr int LB = Log2B<B>::v;
     constexpr int NI = (32 + R - 1) / R;     // columns per thread in the first step (the last may be short)
     extern __shared__ float2 s[];
@@ -1678,6 +1695,7 @@ template <int B, int R, bool HERM>
 __global__ void __launch_bounds__(yfwd_threads(R * B, B), 512 / yfwd_threads(R * B, B))
     k_yfwd4(Geo g, const float2 *__restrict__ G1, float2 *__restrict__ P)
 {
+    pdl_wait();
     constexpr int LB = Log2B<B>::v, n = 32 * R, SB = YfStride<B>::v;
     constexpr int NI = (32 + R - 1) / R;
     extern __shared__ float2 s[];
@@ -1736,6 +1754,7 @@ template <int B, int R>
 __global__ void __launch_bounds__(yadj_threads(R * B), 512 / yadj_threads(R * B))
     k_yadj4(Geo g, const float2 *__restrict__ f, float2 *__restrict__ G1)
 {
+    pdl_wait();
     constexpr int LB = Log2B<B>::v, n = 32 * R;
     constexpr int NI = (32 + R - 1) / R;
     extern __shared__ float2 s[];
@@ -2036,6 +2055,7 @@ template <int B, int BH, int LA, int LNB, int MODE>
 __global__ void __launch_bounds__(XtShape<BH, LA, LNB>::T, (XtShape<BH, LA, LNB>::T >= 256) ? 2 : 4)
     k_xtoep(const __grid_constant__ XtArgs g)
 {
+    pdl_wait();
     using S = XtShape<BH, LA, LNB>;
     constexpr int NA = S::NA, NB = S::NB, U = S::U, H = B / BH;
     extern __shared__ __align__(128) float2 s[];
@@ -2246,6 +2266,7 @@ template <int B, int BH, int LA, int LNB>
 __global__ void __launch_bounds__(xtr_threads(XtShape<BH, LA, LNB>::T), (XtShape<BH, LA, LNB>::T >= 256) ? 2 : 4)
     k_xtoep_real(const __grid_constant__ XtArgs g)
 {
+    pdl_wait();
     using S = XtShape<BH, LA, LNB>;
     constexpr int NA = S::NA, NB = S::NB, U = S::U, H = B / BH, N = S::N, T = xtr_threads(S::T);
     extern __shared__ __align__(128) float2 s[];
