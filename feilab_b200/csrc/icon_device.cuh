@@ -13,18 +13,9 @@
 
 #include <utility>
 
-namespace icon {
+#include "pdl.cuh"
 
-// First statement of every kernel that is launched with programmatic dependent
-// launch: wait until the stream's previous kernel has completed and its writes
-// are visible, then let the next launch's blocks become resident.  All data is
-// touched after it, so each kernel still sees everything before it in the stream.
-// Without the attribute both are no-ops.
-__device__ __forceinline__ void pdl_wait()
-{
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
+namespace icon {
 
 constexpr int kTaps = 14;   // 2m+2 taps per dimension, m = 6 (nufft_gpu_v8.cuh:5, NU:226)
 constexpr int kHalf = 6;    // window half-width m

@@ -10,28 +10,6 @@
 
 namespace icon {
 
-// Launches with programmatic dependent launch: the kernel's blocks may become
-// resident while the stream's previous kernel drains, and wait (pdl_wait, first
-// thing in every kernel launched here) until that kernel has completed before
-// they touch data.  The launches of an iteration follow one another within
-// microseconds of work at small sizes: one 64 x 40 slice forward 25.6 -> 19.9 us,
-// 32 slices of 256 x 128 with the NUFFT operator 2.63 -> 2.47 ms.
-template <class... P, class... A>
-static void pdl(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A... args)
-{
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t c{};
-    c.gridDim = grid;
-    c.blockDim = dim3((unsigned)threads);
-    c.dynamicSmemBytes = smem;
-    c.stream = st;
-    c.attrs = &at;
-    c.numAttrs = 1;
-    cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
-}
-
 template <int B>
 void Launch<B>::xpass_fwd(bool real_in, int E, dim3 grid, int threads, size_t smem, cudaStream_t st, const Geo &g,
                           const void *in, float2 *G1)

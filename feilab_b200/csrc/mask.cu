@@ -53,6 +53,7 @@ template <int B, int E>
 __global__ void __launch_bounds__(512) k_mask_rows_fwd(const float *__restrict__ slices, float2 *__restrict__ C, int n,
                                                         int lg, const float2 *__restrict__ tw)
 {
+    icon::pdl_wait();
     extern __shared__ float2 s[];
     const int y0 = 2 * B * blockIdx.x, sl = blockIdx.y, P = mask_pitch(n);
     const float *rows = slices + ((size_t)sl * n + y0) * n;
@@ -75,6 +76,7 @@ template <int B, int E>
 __global__ void __launch_bounds__(512) k_mask_cols(float2 *__restrict__ C, const float *__restrict__ M, int n, int lg,
                                                     const float2 *__restrict__ tw, int ystart, int thickness)
 {
+    icon::pdl_wait();
     extern __shared__ float2 s[];
     const int kx0 = B * blockIdx.x, sl = blockIdx.y, P = mask_pitch(n);
     float2 *col = C + (size_t)sl * n * P + kx0;
@@ -100,6 +102,7 @@ __global__ void __launch_bounds__(512) k_mask_rows_inv(const float2 *__restrict_
                                                         int lg, const float2 *__restrict__ tw, int ystart,
                                                         int thickness, float inv_norm)
 {
+    icon::pdl_wait();
     extern __shared__ float2 s[];
     const int r0 = 2 * B * blockIdx.x, sl = blockIdx.y, P = mask_pitch(n);
     const float2 *rows = C + ((size_t)sl * n + ystart) * P;
@@ -135,9 +138,9 @@ void mask_launch(const float *slices, float2 *C, const float *M, float *out, int
                  int ystart, int thickness, cudaStream_t st)
 {
     const size_t row_smem = sizeof(float2) * n * BR, col_smem = sizeof(float2) * n * BC;
-    k_mask_rows_fwd<BR, E><<<dim3(n / (2 * BR), S), n * BR / E, row_smem, st>>>(slices, C, n, lg, tw);
-    k_mask_cols<BC, E><<<dim3((n / 2 + BC) / BC, S), n * BC / E, col_smem, st>>>(C, M, n, lg, tw, ystart, thickness);
-    k_mask_rows_inv<BR, E><<<dim3((thickness + 2 * BR - 1) / (2 * BR), S), n * BR / E, row_smem, st>>>(
+    icon::pdl(k_mask_rows_fwd<BR, E>, dim3(n / (2 * BR), S), n * BR / E, row_smem, st, slices, C, n, lg, tw);
+    icon::pdl(k_mask_cols<BC, E>, dim3((n / 2 + BC) / BC, S), n * BC / E, col_smem, st, C, M, n, lg, tw, ystart, thickness);
+    icon::pdl(k_mask_rows_inv<BR, E>, dim3((thickness + 2 * BR - 1) / (2 * BR), S), n * BR / E, row_smem, st, 
         C, out, n, lg, tw, ystart, thickness, 1.f / ((float)n * (float)n));
 }
 

@@ -1,0 +1,43 @@
+// pdl.cuh -- programmatic dependent launch: the launcher and the wait that belongs
+// to it.
+#pragma once
+#include <cuda_runtime.h>
+
+namespace icon {
+
+// First statement of every kernel that is launched with programmatic dependent
+// launch: wait until the stream's previous kernel has completed and its writes
+// are visible, then let the next launch's blocks become resident.  All data is
+// touched after it, so each kernel still sees everything before it in the stream.
+// Without the attribute both are no-ops.
+__device__ __forceinline__ void pdl_wait()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// Launches with programmatic dependent launch: the kernel's blocks may become
+// resident while the stream's previous kernel drains, and wait (pdl_wait, first
+// thing in every kernel launched here) until that kernel has completed before
+// they touch data.  Taken where launches follow one another within microseconds to
+// tens of microseconds of work: one 64 x 40 slice forward 25.6 -> 19.9 us, 10
+// iterations with the NUFFT operator on 32 slices of 256 x 128 2.63 -> 2.47 ms,
+// warm-start network, 16 slices of 256 x 128: predict 1.005 -> 0.978, gradients 3.47 ->
+// 3.44 ms; mask of 32 slices of 512 x 512 202 -> 186 us.
+template <class... P, class... A>
+inline void pdl(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A... args)
+{
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = dim3((unsigned)threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+
+}  // namespace icon

@@ -160,7 +160,7 @@ icon_status ws_conv3x3_launch(const void *in0, int cin0, const void *in1, int ci
             smem = std::max<size_t>(smem, 227 * 1024 / (per_sm + 1) - 896);
             const auto kern = th == 4 ? ws::k_conv3x3_halo<4> : ws::k_conv3x3_halo<2>;
             WS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024));
-            kern<<<grid, ws::kConvThreads, smem, st>>>(h);
+            icon::pdl(kern, grid, ws::kConvThreads, smem, st, h);
             WS_CUDA(cudaGetLastError());
             return ICON_OK;
         }
@@ -186,7 +186,7 @@ icon_status ws_conv3x3_launch(const void *in0, int cin0, const void *in1, int ci
         }
     }
     dim3 grid((W + ws::kTileM - 1) / ws::kTileM, H, nimg);
-    ws::k_conv3x3_tc<<<grid, ws::kConvThreads, smem, st>>>(m0, m1, mw, a);
+    icon::pdl(ws::k_conv3x3_tc, grid, ws::kConvThreads, smem, st, m0, m1, mw, a);
     WS_CUDA(cudaGetLastError());
     return ICON_OK;
 }

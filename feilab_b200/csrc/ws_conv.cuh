@@ -18,6 +18,7 @@
 // connections), so the concatenation is never stored.  Weights are
 // [tap][N][Cin] BF16 with tap = 3*dy + dx.
 #pragma once
+#include "pdl.cuh"
 #include "ws_tc.cuh"
 
 namespace ws {
@@ -65,6 +66,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
 k_conv3x3_tc(const __grid_constant__ CUtensorMap in0, const __grid_constant__ CUtensorMap in1,
              const __grid_constant__ CUtensorMap wmap, ConvArgs a)
 {
+    icon::pdl_wait();
     extern __shared__ unsigned char smem_raw[];
     unsigned char *base = reinterpret_cast<unsigned char *>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const size_t abytes = conv_stage_a_bytes(a.cc), bbytes = conv_stage_b_bytes(a.N, a.cc);
@@ -260,6 +262,7 @@ struct HaloArgs {
 template <int TH>
 __global__ void __launch_bounds__(kConvThreads) k_conv3x3_halo(const HaloArgs h)
 {
+    icon::pdl_wait();
     extern __shared__ unsigned char smem_raw[];
     const ConvArgs &a = h.c;
     unsigned char *base = reinterpret_cast<unsigned char *>(((uintptr_t)smem_raw + 127) & ~(uintptr_t)127);

@@ -7,6 +7,8 @@
 #include <cuda_bf16.h>
 #include <cstdint>
 
+#include "pdl.cuh"
+
 namespace ws {
 
 __device__ __forceinline__ float bf(const __nv_bfloat16 v) { return __bfloat162float(v); }
@@ -25,6 +27,7 @@ constexpr int kSumSqChunks = 64;
 
 __global__ void __launch_bounds__(256) k_slice_sumsq(const float2 *__restrict__ Ahwb, int N0, int N1, double *__restrict__ part)
 {
+    icon::pdl_wait();
     __shared__ double red[256];
     const int c = blockIdx.x, s = blockIdx.y, n = N0 * N1;
     const float2 *base = Ahwb + (size_t)s * n;
@@ -46,6 +49,7 @@ __global__ void __launch_bounds__(256) k_slice_sumsq(const float2 *__restrict__ 
 
 __global__ void k_slice_sumsq_fin(const double *__restrict__ part, double *__restrict__ ss)
 {
+    icon::pdl_wait();
     double v = 0.0;
     for (int c = threadIdx.x; c < kSumSqChunks; c += 32) v += part[blockIdx.x * kSumSqChunks + c];
 #pragma unroll
@@ -58,6 +62,7 @@ __global__ void k_slice_sumsq_fin(const double *__restrict__ part, double *__res
 __global__ void k_net_input(const float2 *__restrict__ Ahwb, const double *__restrict__ ss, int N0, int N1, int Hp,
                             int Wp, int S, float *__restrict__ x, float *__restrict__ scale)
 {
+    icon::pdl_wait();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t total = (size_t)S * Hp * Wp;
     if (i >= total) return;
@@ -72,6 +77,7 @@ __global__ void k_net_input(const float2 *__restrict__ Ahwb, const double *__res
 __global__ void k_net_target(const float *__restrict__ m, const float *__restrict__ scale, float gain, int N0, int N1,
                              int Hp, int Wp, int S, float *__restrict__ t)
 {
+    icon::pdl_wait();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t total = (size_t)S * Hp * Wp;
     if (i >= total) return;
@@ -83,6 +89,7 @@ __global__ void k_net_target(const float *__restrict__ m, const float *__restric
 __global__ void k_net_output(const float *__restrict__ y, const float *__restrict__ scale, float gain, int N0, int N1,
                              int Hp, int Wp, int S, float *__restrict__ m)
 {
+    icon::pdl_wait();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t total = (size_t)S * N0 * N1;
     if (i >= total) return;
@@ -99,6 +106,7 @@ __global__ void __launch_bounds__(128) k_conv_in(const float *__restrict__ x, co
                                                  const float *__restrict__ bias, int n, int H, int W,
                                                  __nv_bfloat16 *__restrict__ y)
 {
+    icon::pdl_wait();
     __shared__ __align__(16) float sw[9 * 16 + 16];
     for (int i = threadIdx.x; i < 9 * 16; i += blockDim.x) sw[i] = w[i];
     for (int i = threadIdx.x; i < 16; i += blockDim.x) sw[144 + i] = bias[i];
@@ -162,6 +170,7 @@ __global__ void __launch_bounds__(48 * kInGroups) k_conv_in_wgrad(const float *_
                                                                   const __nv_bfloat16 *__restrict__ gz, int n, int H,
                                                                   int W, float *__restrict__ part)
 {
+    icon::pdl_wait();
     constexpr int T = 48 * kInGroups;
     __shared__ float sx[kInRows + 2][kInCols + 2];
     __shared__ float sg[kInRows][kInCols][17];
@@ -215,6 +224,7 @@ __global__ void __launch_bounds__(48 * kInGroups) k_conv_in_wgrad(const float *_
 // 2x2 average pooling; C a multiple of 8 (8 channels per thread).
 __global__ void k_pool2(const __nv_bfloat16 *__restrict__ in, int n, int H, int W, int C, __nv_bfloat16 *__restrict__ out)
 {
+    icon::pdl_wait();
     const int Ho = H / 2, Wo = W / 2, C8 = C / 8;
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (size_t)n * Ho * Wo * C8) return;
@@ -240,6 +250,7 @@ __global__ void k_pool2(const __nv_bfloat16 *__restrict__ in, int n, int H, int 
 __global__ void k_pool2_bwd(const __nv_bfloat16 *__restrict__ gout, int n, int H, int W, int C, int accumulate,
                             __nv_bfloat16 *__restrict__ gin)
 {
+    icon::pdl_wait();
     const int Ho = H / 2, Wo = W / 2, C8 = C / 8;
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (size_t)n * H * W * C8) return;
@@ -265,6 +276,7 @@ __global__ void k_pool2_bwd(const __nv_bfloat16 *__restrict__ gout, int n, int H
 // Nearest 2x upsampling: out[h][w] = in[h/2][w/2] (H, W = output size).
 __global__ void k_up2(const __nv_bfloat16 *__restrict__ in, int n, int H, int W, int C, __nv_bfloat16 *__restrict__ out)
 {
+    icon::pdl_wait();
     const int C8 = C / 8;
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (size_t)n * H * W * C8) return;
@@ -280,6 +292,7 @@ __global__ void k_up2(const __nv_bfloat16 *__restrict__ in, int n, int H, int W,
 __global__ void k_up2_bwd(const __nv_bfloat16 *__restrict__ gout, int n, int H, int W, int C,
                           __nv_bfloat16 *__restrict__ gin)
 {
+    icon::pdl_wait();
     const int C8 = C / 8;
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (size_t)n * H * W * C8) return;
@@ -304,6 +317,7 @@ __global__ void k_up2_bwd(const __nv_bfloat16 *__restrict__ gout, int n, int H, 
 // ReLU gradient in place: g = g where y > 0, else 0 (y is the ReLU output).
 __global__ void k_relu_bwd(__nv_bfloat16 *__restrict__ g, const __nv_bfloat16 *__restrict__ y, size_t count8)
 {
+    icon::pdl_wait();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count8) return;
     uint4 gv = reinterpret_cast<uint4 *>(g)[i];
@@ -380,6 +394,7 @@ __global__ void __launch_bounds__(128) k_wgrad3x3(const __nv_bfloat16 *__restric
                                                    const __nv_bfloat16 *__restrict__ gz, int N, int n, int H, int W,
                                                    float *__restrict__ part)
 {
+    icon::pdl_wait();
     using S = WgShape<WCO, MC, MI, KW>;
     extern __shared__ __align__(128) unsigned char wg_smem[];
     const uint32_t sx = (uint32_t)__cvta_generic_to_shared(wg_smem), sg = sx + kWgXRows * S::XB;
@@ -512,6 +527,7 @@ constexpr int kSumWarps = 32;
 
 __global__ void __launch_bounds__(32 * kSumWarps) k_sum_parts(const float *__restrict__ part, int nsplit, size_t len, float *__restrict__ out)
 {
+    icon::pdl_wait();
     __shared__ float red[kSumWarps][33];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const size_t i = (size_t)blockIdx.x * 32 + lane;
@@ -534,6 +550,7 @@ __global__ void __launch_bounds__(32 * kSumWarps) k_sum_parts(const float *__res
 __global__ void k_conv_out(const __nv_bfloat16 *__restrict__ d, const float *__restrict__ w, const float *__restrict__ b,
                            size_t npix, float *__restrict__ y)
 {
+    icon::pdl_wait();
     const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= npix) return;
     const uint4 *v = reinterpret_cast<const uint4 *>(d + p * 16);
@@ -554,6 +571,7 @@ __global__ void k_conv_out(const __nv_bfloat16 *__restrict__ d, const float *__r
 __global__ void k_mse(const float *__restrict__ y, const float *__restrict__ t, int S, int Hp, int Wp, int Hv, int Wv,
                       float *__restrict__ dy, double *__restrict__ lpart)
 {
+    icon::pdl_wait();
     __shared__ double red[256];
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t total = (size_t)S * Hp * Wp;
@@ -589,6 +607,7 @@ __global__ void __launch_bounds__(256) k_conv_out_bwd(const __nv_bfloat16 *__res
                                                       const float *__restrict__ w, size_t npix,
                                                       __nv_bfloat16 *__restrict__ gd, float *__restrict__ part)
 {
+    icon::pdl_wait();
     __shared__ float red[8][17];
     float loc[17], wv[16];
 #pragma unroll
@@ -633,6 +652,7 @@ __global__ void __launch_bounds__(256) k_conv_out_bwd(const __nv_bfloat16 *__res
 __global__ void k_adam(float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m, float *__restrict__ v,
                        size_t n, float lr, float b1, float b2, float eps, float c1, float c2)
 {
+    icon::pdl_wait();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float gi = g[i];
@@ -649,6 +669,7 @@ __global__ void k_adam(float *__restrict__ p, const float *__restrict__ g, float
 __global__ void k_weights_bf16(const float *__restrict__ w, int N, int Cin, __nv_bfloat16 *__restrict__ wb,
                                __nv_bfloat16 *__restrict__ wt)
 {
+    icon::pdl_wait();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (size_t)9 * N * Cin) return;
     const int ci = (int)(i % Cin), co = (int)((i / Cin) % N), tap = (int)(i / ((size_t)Cin * N));

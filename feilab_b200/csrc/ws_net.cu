@@ -127,7 +127,7 @@ cudaError_t wgrad_go(dim3 grid, cudaStream_t st, const __nv_bfloat16 *X0, int c0
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return e;
     }
-    k<<<grid, 128, smem, st>>>(X0, c0, up0, X1, c1, gz, N, n, H, W, part);
+    icon::pdl(k, grid, 128, smem, st, X0, c0, up0, X1, c1, gz, N, n, H, W, part);
     return cudaGetLastError();
 }
 
@@ -212,7 +212,7 @@ struct icon_ws {
     {
         for (auto &L : layers) {
             const size_t n = (size_t)9 * L.N * (L.cin0 + L.cin1);
-            ws::k_weights_bf16<<<grid1(n, 256), 256, 0, st>>>(params + L.w_off, L.N, L.cin0 + L.cin1, L.wb, L.wt);
+            icon::pdl(ws::k_weights_bf16, grid1(n, 256), 256, 0, st, params + L.w_off, L.N, L.cin0 + L.cin1, L.wb, L.wt);
         }
         NET_CUDA(cudaGetLastError());
         return ICON_OK;
@@ -229,22 +229,22 @@ struct icon_ws {
     void pool(const Img &in, Img &out, int S, cudaStream_t st)
     {
         size_t n = (size_t)S * out.H * out.W * (in.C / 8);
-        ws::k_pool2<<<grid1(n, 256), 256, 0, st>>>(in.p, S, in.H, in.W, in.C, out.p);
+        icon::pdl(ws::k_pool2, grid1(n, 256), 256, 0, st, in.p, S, in.H, in.W, in.C, out.p);
     }
 
     void up(const Img &in, Img &out, int S, cudaStream_t st)
     {
         size_t n = (size_t)S * out.H * out.W * (out.C / 8);
-        ws::k_up2<<<grid1(n, 256), 256, 0, st>>>(in.p, S, out.H, out.W, out.C, out.p);
+        icon::pdl(ws::k_up2, grid1(n, 256), 256, 0, st, in.p, S, out.H, out.W, out.C, out.p);
     }
 
     icon_status forward(const float2 *Ahwb, int S, cudaStream_t st)
     {
-        ws::k_slice_sumsq<<<dim3(ws::kSumSqChunks, S), 256, 0, st>>>(Ahwb, N0, N1, sspart);
-        ws::k_slice_sumsq_fin<<<S, 32, 0, st>>>(sspart, ss);
+        icon::pdl(ws::k_slice_sumsq, dim3(ws::kSumSqChunks, S), 256, 0, st, Ahwb, N0, N1, sspart);
+        icon::pdl(ws::k_slice_sumsq_fin, S, 32, 0, st, sspart, ss);
         const size_t npix = (size_t)S * Hp * Wp;
-        ws::k_net_input<<<grid1(npix, 256), 256, 0, st>>>(Ahwb, ss, N0, N1, Hp, Wp, S, x, in_scale);
-        ws::k_conv_in<<<grid1(npix / 2, 128), 128, 0, st>>>(x, params + kInW, params + kInB, S, Hp, Wp, e0a.p);
+        icon::pdl(ws::k_net_input, grid1(npix, 256), 256, 0, st, Ahwb, ss, N0, N1, Hp, Wp, S, x, in_scale);
+        icon::pdl(ws::k_conv_in, grid1(npix / 2, 128), 128, 0, st, x, params + kInW, params + kInB, S, Hp, Wp, e0a.p);
         NET_CUDA(cudaGetLastError());
         NET_TRY(conv(C0B, e0a, nullptr, e0, S, st));
         pool(e0, p0, S, st);
@@ -264,14 +264,14 @@ struct icon_ws {
         NET_TRY(conv(D1B, d1a, nullptr, d1, S, st));
         NET_TRY(conv(D0A, d1, &e0, d0a, S, st, 1));   // d1 upsampled as it is read
         NET_TRY(conv(D0B, d0a, nullptr, d0, S, st));
-        ws::k_conv_out<<<grid1(npix, 256), 256, 0, st>>>(d0.p, params + out_off, params + out_off + 16, npix, y);
+        icon::pdl(ws::k_conv_out, grid1(npix, 256), 256, 0, st, d0.p, params + out_off, params + out_off + 16, npix, y);
         NET_CUDA(cudaGetLastError());
         return ICON_OK;
     }
 
     void sum_parts(int n, size_t len, float *out, cudaStream_t st)
     {
-        ws::k_sum_parts<<<grid1(len, 32), 32 * ws::kSumWarps, 0, st>>>(part, n, len, out);
+        icon::pdl(ws::k_sum_parts, grid1(len, 32), 32 * ws::kSumWarps, 0, st, part, n, len, out);
     }
 
     // Gradients of one 3x3 layer: ReLU backward of gout in place, weight and
@@ -282,7 +282,7 @@ struct icon_ws {
     {
         const TcLayer &L = layers[li];
         const size_t cnt8 = (size_t)S * out.H * out.W * out.C / 8;
-        ws::k_relu_bwd<<<grid1(cnt8, 256), 256, 0, st>>>(gout.p, out.p, cnt8);
+        icon::pdl(ws::k_relu_bwd, grid1(cnt8, 256), 256, 0, st, gout.p, out.p, cnt8);
         const int Cin = L.cin0 + L.cin1;
         const WgPlan wp = wgrad_plan(L.N, L.cin0, L.cin1);
         const int nsplit = wp.splits(L.N, Cin, wgrad_rows(S, out.H, out.W)), nparts = nsplit * wp.kw;
@@ -310,13 +310,13 @@ struct icon_ws {
     void pool_bwd(const Img &gout, Img &gin, int S, cudaStream_t st)
     {
         size_t n = (size_t)S * gin.H * gin.W * (gin.C / 8);
-        ws::k_pool2_bwd<<<grid1(n, 256), 256, 0, st>>>(gout.p, S, gin.H, gin.W, gin.C, 1, gin.p);
+        icon::pdl(ws::k_pool2_bwd, grid1(n, 256), 256, 0, st, gout.p, S, gin.H, gin.W, gin.C, 1, gin.p);
     }
 
     void up_bwd(const Img &gout, Img &gin, int S, cudaStream_t st)
     {
         size_t n = (size_t)S * gin.H * gin.W * (gin.C / 8);
-        ws::k_up2_bwd<<<grid1(n, 256), 256, 0, st>>>(gout.p, S, gin.H, gin.W, gin.C, gin.p);
+        icon::pdl(ws::k_up2_bwd, grid1(n, 256), 256, 0, st, gout.p, S, gin.H, gin.W, gin.C, gin.p);
     }
 
     icon_status backward(int S, cudaStream_t st)
@@ -325,7 +325,7 @@ struct icon_ws {
         {
             const unsigned nb = std::min<unsigned>(grid1(npix, 256), ws::kOutBlocks);
             if ((size_t)nb * 17 > part_len) return net_fail(ICON_ERR_INVALID, "warm start: output scratch too small");
-            ws::k_conv_out_bwd<<<nb, 256, 0, st>>>(d0.p, dy, params + out_off, npix, g_d0.p, part);
+            icon::pdl(ws::k_conv_out_bwd, nb, 256, 0, st, d0.p, dy, params + out_off, npix, g_d0.p, part);
             sum_parts((int)nb, 17, grads + out_off, st);
         }
         NET_TRY(layer_bwd(D0B, g_d0, d0, d0a, nullptr, &g_d0a, 0, nullptr, S, st));
@@ -349,11 +349,11 @@ struct icon_ws {
         NET_TRY(layer_bwd(C0B, g_e0, e0, e0a, nullptr, &g_e0a, 0, nullptr, S, st));
         {
             const size_t cnt8 = (size_t)S * Hp * Wp * 16 / 8;
-            ws::k_relu_bwd<<<grid1(cnt8, 256), 256, 0, st>>>(g_e0a.p, e0a.p, cnt8);
+            icon::pdl(ws::k_relu_bwd, grid1(cnt8, 256), 256, 0, st, g_e0a.p, e0a.p, cnt8);
             const unsigned nb = in_wgrad_blocks(S, Hp, Wp);
             if ((size_t)nb * 160 > part_len)
                 return net_fail(ICON_ERR_INVALID, "warm start: input-layer scratch too small");
-            ws::k_conv_in_wgrad<<<nb, 48 * ws::kInGroups, 0, st>>>(x, g_e0a.p, S, Hp, Wp, part);
+            icon::pdl(ws::k_conv_in_wgrad, nb, 48 * ws::kInGroups, 0, st, x, g_e0a.p, S, Hp, Wp, part);
             sum_parts((int)nb, 160, grads + kInW, st);
         }
         NET_CUDA(cudaGetLastError());
@@ -549,7 +549,7 @@ icon_status icon_ws_predict(icon_ws *w, const void *d_Ahwb, float *d_m0, int S, 
     cudaStream_t st = (cudaStream_t)stream;
     NET_TRY(w->forward((const float2 *)d_Ahwb, S, st));
     const size_t nout = (size_t)S * w->N1 * w->N0;
-    ws::k_net_output<<<grid1(nout, 256), 256, 0, st>>>(w->y, w->in_scale, w->gain, w->N0, w->N1, w->Hp, w->Wp, S,
+    icon::pdl(ws::k_net_output, grid1(nout, 256), 256, 0, st, w->y, w->in_scale, w->gain, w->N0, w->N1, w->Hp, w->Wp, S,
                                                          d_m0);
     NET_CUDA(cudaGetLastError());
     return ICON_OK;
@@ -564,10 +564,10 @@ icon_status icon_ws_backprop(icon_ws *w, const void *d_Ahwb, const float *d_targ
     cudaStream_t st = (cudaStream_t)stream;
     NET_TRY(w->forward((const float2 *)d_Ahwb, S, st));
     const size_t npix = (size_t)S * w->Hp * w->Wp;
-    ws::k_net_target<<<grid1(npix, 256), 256, 0, st>>>(d_target, w->in_scale, w->gain, w->N0, w->N1, w->Hp, w->Wp, S,
+    icon::pdl(ws::k_net_target, grid1(npix, 256), 256, 0, st, d_target, w->in_scale, w->gain, w->N0, w->N1, w->Hp, w->Wp, S,
                                                          w->t);
     const unsigned nb = grid1(npix, 256);
-    ws::k_mse<<<nb, 256, 0, st>>>(w->y, w->t, S, w->Hp, w->Wp, w->N1, w->N0, w->dy, w->lpart);
+    icon::pdl(ws::k_mse, nb, 256, 0, st, w->y, w->t, S, w->Hp, w->Wp, w->N1, w->N0, w->dy, w->lpart);
     NET_CUDA(cudaGetLastError());
     NET_TRY(w->backward(S, st));
     if (h_loss) {
@@ -590,7 +590,7 @@ icon_status icon_ws_update(icon_ws *w, float lr, void *stream)
     w->step += 1;
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.f - std::pow(b1, (float)w->step), c2 = 1.f - std::pow(b2, (float)w->step);
-    ws::k_adam<<<grid1(w->nparam, 256), 256, 0, st>>>(w->params, w->grads, w->am, w->av, w->nparam, lr, b1, b2, 1e-8f,
+    icon::pdl(ws::k_adam, grid1(w->nparam, 256), 256, 0, st, w->params, w->grads, w->am, w->av, w->nparam, lr, b1, b2, 1e-8f,
                                                       c1, c2);
     NET_CUDA(cudaGetLastError());
     return w->refresh_bf16(st);
