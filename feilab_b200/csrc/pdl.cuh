@@ -22,8 +22,8 @@ __device__ __forceinline__ void pdl_wait()
 // they touch data.  Taken where launches follow one another within microseconds to
 // tens of microseconds of work: one 64 x 40 slice forward 25.6 -> 19.9 us, 10
 // iterations with the NUFFT operator on 32 slices of 256 x 128 2.63 -> 2.47 ms,
-// warm-start network, 16 slices of 256 x 128: predict 1.005 -> 0.978, gradients 3.47 ->
-// 3.44 ms; mask of 32 slices of 512 x 512 202 -> 186 us.
+// warm-start predict of 8 slices of 1024 x 300 1.005 -> 0.978 ms, gradients of 16
+// slices of 512 x 256 3.47 -> 3.44 ms, mask of 16 slices of 1024 x 1024 202 -> 186 us.
 template <class... P, class... A>
 inline void pdl(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A... args)
 {

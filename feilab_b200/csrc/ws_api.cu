@@ -123,6 +123,9 @@ icon_status ws_conv3x3_launch(const void *in0, int cin0, const void *in1, int ci
     if (!cc) return ws_fail(ICON_ERR_INVALID, "conv3x3: input channels must be multiples of 16");
     if (nsplit <= 0 || nsplit > N || nsplit % 16 || (nsplit < N && !out1))
         return ws_fail(ICON_ERR_INVALID, "conv3x3: bad output split");
+    // The loads and stores move 16 bytes (a tensor map refuses such inputs too).
+    if (((uintptr_t)in0 | (uintptr_t)in1 | (uintptr_t)w | (uintptr_t)out0 | (uintptr_t)out1) & 15)
+        return ws_fail(ICON_ERR_CUDA, "conv3x3: images and weights must start at 16-byte boundaries");
     int *err = device_err_flag();
     if (!err) return ws_fail(ICON_ERR_CUDA, "conv3x3: error flag allocation failed");
     ws::ConvArgs a;
