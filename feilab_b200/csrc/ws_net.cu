@@ -271,7 +271,15 @@ struct icon_ws {
 
     void sum_parts(int n, size_t len, float *out, cudaStream_t st)
     {
-        icon::pdl(ws::k_sum_parts, grid1(len, 32), 32 * ws::kSumWarps, 0, st, part, n, len, out);
+        // Four outputs a thread where the parts stay aligned and that leaves a block
+        // per SM; there the warps follow the parts, about eight a warp.
+        if (len % 4 == 0 && len >= 148 * 128) {
+            int W = 4;
+            while (W < ws::kSumWarps && W * 8 < n) W *= 2;
+            icon::pdl(ws::k_sum_parts<4>, grid1(len, 128), 32 * W, 0, st, part, n, len, out);
+        } else {
+            icon::pdl(ws::k_sum_parts<1>, grid1(len, 32), 32 * ws::kSumWarps, 0, st, part, n, len, out);
+        }
     }
 
     // Gradients of one 3x3 layer: ReLU backward of gout in place, weight and
