@@ -113,7 +113,7 @@ int *device_err_flag()
 icon_status ws_conv3x3_launch(const void *in0, int cin0, const void *in1, int cin1, int nimg, int H, int W,
                               const void *w, const float *bias, int N, int relu, void *out0, int nsplit, int acc0,
                               void *out1, int acc1, cudaStream_t st, unsigned long long wait_ns = ws::kWaitNs,
-                              int hold = 0, int up0 = 0)
+                              int hold = 0, int up0 = 0, const void *mask0 = nullptr)
 {
     if (!in0 || !w || !out0 || nimg < 1 || H < 1 || W < 1) return ws_fail(ICON_ERR_INVALID, "conv3x3: bad argument");
     if (N < 16 || N > 256 || N % 16) return ws_fail(ICON_ERR_INVALID, "conv3x3: N must be a multiple of 16 in 16..256");
@@ -141,6 +141,7 @@ icon_status ws_conv3x3_launch(const void *in0, int cin0, const void *in1, int ci
     a.out1 = (__nv_bfloat16 *)out1;
     a.acc0 = acc0;
     a.acc1 = acc1;
+    a.mask0 = (const __nv_bfloat16 *)mask0;
     a.bias = bias;
     a.relu = relu;
     a.err = err;

@@ -36,6 +36,7 @@ struct ConvArgs {
     int nsplit;              // out0 takes channels [0, nsplit), out1 [nsplit, N)
     __nv_bfloat16 *out0, *out1;
     int acc0, acc1;          // 1: add to the output's values
+    const __nv_bfloat16 *mask0;   // out0 is zeroed where this image of its shape is not positive (ReLU gradient), or null
     const float *bias;       // [N] or null
     int relu;
     int *err;                // device error flag
@@ -47,6 +48,19 @@ struct ConvArgs {
     // more than its loads deliver, so the wait for it can only run out.
     int hold;
 };
+
+// v = 0 where y is not positive.
+__device__ __forceinline__ void relu_mask(float (&v)[16], const __nv_bfloat16 *y)
+{
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const uint4 u = reinterpret_cast<const uint4 *>(y)[q];
+        const __nv_bfloat16 *e = reinterpret_cast<const __nv_bfloat16 *>(&u);
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (!(__bfloat162float(e[i]) > 0.f)) v[8 * q + i] = 0.f;
+    }
+}
 
 __host__ __device__ inline size_t conv_stage_a_bytes(int cc) { return (size_t)kTileM * cc * 2; }
 __host__ __device__ inline size_t conv_stage_b_bytes(int N, int cc) { return (((size_t)N * cc * 2) + 1023) & ~(size_t)1023; }
@@ -186,6 +200,7 @@ k_conv3x3_tc(const __grid_constant__ CUtensorMap in0, const __grid_constant__ CU
                     v[2 * i + 1] += o.y;
                 }
             }
+            if (first && a.mask0) relu_mask(v, a.mask0 + pix * C + c);
             uint4 pk[2];
             uint32_t *pw = reinterpret_cast<uint32_t *>(pk);
 #pragma unroll
@@ -378,6 +393,7 @@ __global__ void __launch_bounds__(kConvThreads) k_conv3x3_halo(const HaloArgs h)
                         v[2 * i + 1] += o.y;
                     }
                 }
+                if (f && a.mask0) relu_mask(v, a.mask0 + pix * C + c);
                 uint32_t pk[8];
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {

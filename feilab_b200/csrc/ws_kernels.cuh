@@ -246,9 +246,11 @@ __global__ void k_pool2(const __nv_bfloat16 *__restrict__ in, int n, int H, int 
     *reinterpret_cast<uint4 *>(out + (((size_t)im * Ho + ho) * Wo + wo) * C + 8 * c8) = *reinterpret_cast<uint4 *>(o);
 }
 
-// Gradient of the pooling: gin[2h+dy][2w+dx] (+)= gout[h][w] / 4 (H, W = input size).
-__global__ void k_pool2_bwd(const __nv_bfloat16 *__restrict__ gout, int n, int H, int W, int C, int accumulate,
-                            __nv_bfloat16 *__restrict__ gin)
+// Gradient of the pooling, added to what the skip connection left there, through
+// the ReLU of y, the pooled image: gin[2h+dy][2w+dx] = y > 0 ? gin + gout[h][w] / 4
+// : 0 (H, W = input size).
+__global__ void k_pool2_bwd(const __nv_bfloat16 *__restrict__ gout, int n, int H, int W, int C,
+                            const __nv_bfloat16 *__restrict__ y, __nv_bfloat16 *__restrict__ gin)
 {
     icon::pdl_wait();
     const int Ho = H / 2, Wo = W / 2, C8 = C / 8;
@@ -259,17 +261,14 @@ __global__ void k_pool2_bwd(const __nv_bfloat16 *__restrict__ gout, int n, int H
     const int w = (int)(q % W), h = (int)((q / W) % H), im = (int)(q / ((size_t)W * H));
     const uint4 g = *reinterpret_cast<const uint4 *>(gout + (((size_t)im * Ho + h / 2) * Wo + w / 2) * C + 8 * c8);
     const __nv_bfloat16 *ge = reinterpret_cast<const __nv_bfloat16 *>(&g);
+    const uint4 yv = *reinterpret_cast<const uint4 *>(y + q * C + 8 * c8);
+    const __nv_bfloat16 *ye = reinterpret_cast<const __nv_bfloat16 *>(&yv);
     uint4 *dst = reinterpret_cast<uint4 *>(gin + q * C + 8 * c8);
     __align__(16) __nv_bfloat16 o[8];
-    if (accumulate) {
-        const uint4 old = *dst;
-        const __nv_bfloat16 *oe = reinterpret_cast<const __nv_bfloat16 *>(&old);
+    const uint4 old = *dst;
+    const __nv_bfloat16 *oe = reinterpret_cast<const __nv_bfloat16 *>(&old);
 #pragma unroll
-        for (int k = 0; k < 8; ++k) o[k] = tobf(bf(oe[k]) + 0.25f * bf(ge[k]));
-    } else {
-#pragma unroll
-        for (int k = 0; k < 8; ++k) o[k] = tobf(0.25f * bf(ge[k]));
-    }
+    for (int k = 0; k < 8; ++k) o[k] = bf(ye[k]) > 0.f ? tobf(bf(oe[k]) + 0.25f * bf(ge[k])) : tobf(0.f);
     *dst = *reinterpret_cast<uint4 *>(o);
 }
 
@@ -287,10 +286,10 @@ __global__ void k_up2(const __nv_bfloat16 *__restrict__ in, int n, int H, int W,
         *reinterpret_cast<const uint4 *>(in + (((size_t)im * (H / 2) + h / 2) * (W / 2) + w / 2) * C + 8 * c8);
 }
 
-// Gradient of the upsampling: gin[h][w] = sum of gout over its 2x2 block
-// (H, W = input size).
+// Gradient of the upsampling, through the ReLU of y, the upsampled image: gin[h][w]
+// = y > 0 ? sum of gout over its 2x2 block : 0 (H, W = input size).
 __global__ void k_up2_bwd(const __nv_bfloat16 *__restrict__ gout, int n, int H, int W, int C,
-                          __nv_bfloat16 *__restrict__ gin)
+                          const __nv_bfloat16 *__restrict__ y, __nv_bfloat16 *__restrict__ gin)
 {
     icon::pdl_wait();
     const int C8 = C / 8;
@@ -299,6 +298,8 @@ __global__ void k_up2_bwd(const __nv_bfloat16 *__restrict__ gout, int n, int H, 
     const int c8 = (int)(i % C8);
     const size_t q = i / C8;
     const int w = (int)(q % W), h = (int)((q / W) % H), im = (int)(q / ((size_t)W * H));
+    const uint4 yv = *reinterpret_cast<const uint4 *>(y + q * C + 8 * c8);
+    const __nv_bfloat16 *ye = reinterpret_cast<const __nv_bfloat16 *>(&yv);
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     for (int dy = 0; dy < 2; ++dy)
         for (int dx = 0; dx < 2; ++dx) {
@@ -310,24 +311,8 @@ __global__ void k_up2_bwd(const __nv_bfloat16 *__restrict__ gout, int n, int H, 
         }
     __align__(16) __nv_bfloat16 o[8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) o[k] = tobf(acc[k]);
+    for (int k = 0; k < 8; ++k) o[k] = bf(ye[k]) > 0.f ? tobf(acc[k]) : tobf(0.f);
     *reinterpret_cast<uint4 *>(gin + q * C + 8 * c8) = *reinterpret_cast<uint4 *>(o);
-}
-
-// ReLU gradient in place: g = g where y > 0, else 0 (y is the ReLU output).
-__global__ void k_relu_bwd(__nv_bfloat16 *__restrict__ g, const __nv_bfloat16 *__restrict__ y, size_t count8)
-{
-    icon::pdl_wait();
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count8) return;
-    uint4 gv = reinterpret_cast<uint4 *>(g)[i];
-    const uint4 yv = reinterpret_cast<const uint4 *>(y)[i];
-    __nv_bfloat16 *ge = reinterpret_cast<__nv_bfloat16 *>(&gv);
-    const __nv_bfloat16 *ye = reinterpret_cast<const __nv_bfloat16 *>(&yv);
-#pragma unroll
-    for (int k = 0; k < 8; ++k)
-        if (!(bf(ye[k]) > 0.f)) ge[k] = tobf(0.f);
-    reinterpret_cast<uint4 *>(g)[i] = gv;
 }
 
 // ------------------------------------------------------------ weight gradients
@@ -613,7 +598,8 @@ __global__ void k_mse(const float *__restrict__ y, const float *__restrict__ t, 
     if (threadIdx.x == 0) lpart[blockIdx.x] = red[0];
 }
 
-// Backward of the output layer: gd[p][c] = dy[p] * w[c] (BF16), and per-block
+// Backward of the output layer and of the ReLU before it: gd[p][c] = d[p][c] > 0 ?
+// dy[p] * w[c] : 0 (BF16), and per-block
 // partial sums of dw[c] = sum dy[p] d[p][c] and db = sum dy[p] (part[blk][17])
 // over the pixels p = thread + k * threads, summed in a thread, then over its
 // warp and the block in fixed order.  (One pixel per thread, a 17-wide tree in
@@ -643,7 +629,7 @@ __global__ void __launch_bounds__(256) k_conv_out_bwd(const __nv_bfloat16 *__res
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
                 loc[8 * q + k] = fmaf(g, bf(e[k]), loc[8 * q + k]);
-                o[8 * q + k] = tobf(g * wv[8 * q + k]);
+                o[8 * q + k] = bf(e[k]) > 0.f ? tobf(g * wv[8 * q + k]) : tobf(0.f);
             }
         }
         loc[16] += g;

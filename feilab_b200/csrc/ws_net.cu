@@ -35,7 +35,7 @@ extern "C" void icon_internal_set_error(const char *msg);
 icon_status ws_conv3x3_launch(const void *in0, int cin0, const void *in1, int cin1, int nimg, int H, int W,
                               const void *w, const float *bias, int N, int relu, void *out0, int nsplit, int acc0,
                               void *out1, int acc1, cudaStream_t st, unsigned long long wait_ns = 2000000000ull,
-                              int hold = 0, int up0 = 0);
+                              int hold = 0, int up0 = 0, const void *mask0 = nullptr);
 
 namespace {
 
@@ -282,15 +282,15 @@ struct icon_ws {
         }
     }
 
-    // Gradients of one 3x3 layer: ReLU backward of gout in place, weight and
-    // bias gradients, and (when gin0) the input gradient split over gin0 /
-    // gin1 (acc0: add to gin0).
+    // Gradients of one 3x3 layer from gout, the gradient before its ReLU (every
+    // kernel that produces one zeroes it where the ReLU's output is not positive; 14
+    // passes of their own took 196 us at 16 x 512 x 256 pixels): weight and bias
+    // gradients, and (when gin0) the input gradient split over gin0 / gin1 (acc0:
+    // add to gin0; relu_in: in0 is a ReLU's output, whose gradient gin0 becomes).
     icon_status layer_bwd(int li, Img &gout, const Img &out, const Img &in0, const Img *in1, Img *gin0, int acc0,
-                          Img *gin1, int S, cudaStream_t st, int up0 = 0)
+                          Img *gin1, int S, cudaStream_t st, int up0 = 0, bool relu_in = false)
     {
         const TcLayer &L = layers[li];
-        const size_t cnt8 = (size_t)S * out.H * out.W * out.C / 8;
-        icon::pdl(ws::k_relu_bwd, grid1(cnt8, 256), 256, 0, st, gout.p, out.p, cnt8);
         const int Cin = L.cin0 + L.cin1;
         const WgPlan wp = wgrad_plan(L.N, L.cin0, L.cin1);
         const int nsplit = wp.splits(L.N, Cin, wgrad_rows(S, out.H, out.W)), nparts = nsplit * wp.kw;
@@ -311,20 +311,21 @@ struct icon_ws {
         NET_CUDA(cudaGetLastError());
         if (gin0)
             NET_TRY(ws_conv3x3_launch(gout.p, L.N, nullptr, 0, S, out.H, out.W, L.wt, nullptr, Cin, 0, gin0->p,
-                                      L.cin0, acc0, gin1 ? gin1->p : nullptr, 0, st));
+                                      L.cin0, acc0, gin1 ? gin1->p : nullptr, 0, st, 2000000000ull, 0, 0,
+                                      relu_in ? in0.p : nullptr));
         return ICON_OK;
     }
 
-    void pool_bwd(const Img &gout, Img &gin, int S, cudaStream_t st)
+    void pool_bwd(const Img &gout, Img &gin, const Img &y, int S, cudaStream_t st)
     {
         size_t n = (size_t)S * gin.H * gin.W * (gin.C / 8);
-        icon::pdl(ws::k_pool2_bwd, grid1(n, 256), 256, 0, st, gout.p, S, gin.H, gin.W, gin.C, 1, gin.p);
+        icon::pdl(ws::k_pool2_bwd, grid1(n, 256), 256, 0, st, gout.p, S, gin.H, gin.W, gin.C, y.p, gin.p);
     }
 
-    void up_bwd(const Img &gout, Img &gin, int S, cudaStream_t st)
+    void up_bwd(const Img &gout, Img &gin, const Img &y, int S, cudaStream_t st)
     {
         size_t n = (size_t)S * gin.H * gin.W * (gin.C / 8);
-        icon::pdl(ws::k_up2_bwd, grid1(n, 256), 256, 0, st, gout.p, S, gin.H, gin.W, gin.C, gin.p);
+        icon::pdl(ws::k_up2_bwd, grid1(n, 256), 256, 0, st, gout.p, S, gin.H, gin.W, gin.C, y.p, gin.p);
     }
 
     icon_status backward(int S, cudaStream_t st)
@@ -336,28 +337,26 @@ struct icon_ws {
             icon::pdl(ws::k_conv_out_bwd, nb, 256, 0, st, d0.p, dy, params + out_off, npix, g_d0.p, part);
             sum_parts((int)nb, 17, grads + out_off, st);
         }
-        NET_TRY(layer_bwd(D0B, g_d0, d0, d0a, nullptr, &g_d0a, 0, nullptr, S, st));
+        NET_TRY(layer_bwd(D0B, g_d0, d0, d0a, nullptr, &g_d0a, 0, nullptr, S, st, 0, true));
         NET_TRY(layer_bwd(D0A, g_d0a, d0a, d1, &e0, &g_u0, 0, &g_e0, S, st, 1));
-        up_bwd(g_u0, g_d1, S, st);
-        NET_TRY(layer_bwd(D1B, g_d1, d1, d1a, nullptr, &g_d1a, 0, nullptr, S, st));
+        up_bwd(g_u0, g_d1, d1, S, st);
+        NET_TRY(layer_bwd(D1B, g_d1, d1, d1a, nullptr, &g_d1a, 0, nullptr, S, st, 0, true));
         NET_TRY(layer_bwd(D1A, g_d1a, d1a, u1, &e1, &g_u1, 0, &g_e1, S, st));
-        up_bwd(g_u1, g_d2, S, st);
-        NET_TRY(layer_bwd(D2B, g_d2, d2, d2a, nullptr, &g_d2a, 0, nullptr, S, st));
+        up_bwd(g_u1, g_d2, d2, S, st);
+        NET_TRY(layer_bwd(D2B, g_d2, d2, d2a, nullptr, &g_d2a, 0, nullptr, S, st, 0, true));
         NET_TRY(layer_bwd(D2A, g_d2a, d2a, u2, &e2, &g_u2, 0, &g_e2, S, st));
-        up_bwd(g_u2, g_b, S, st);
-        NET_TRY(layer_bwd(C3B, g_b, b, ba, nullptr, &g_ba, 0, nullptr, S, st));
+        up_bwd(g_u2, g_b, b, S, st);
+        NET_TRY(layer_bwd(C3B, g_b, b, ba, nullptr, &g_ba, 0, nullptr, S, st, 0, true));
         NET_TRY(layer_bwd(C3A, g_ba, ba, p2, nullptr, &g_p2, 0, nullptr, S, st));
-        pool_bwd(g_p2, g_e2, S, st);
-        NET_TRY(layer_bwd(C2B, g_e2, e2, e2a, nullptr, &g_e2a, 0, nullptr, S, st));
+        pool_bwd(g_p2, g_e2, e2, S, st);
+        NET_TRY(layer_bwd(C2B, g_e2, e2, e2a, nullptr, &g_e2a, 0, nullptr, S, st, 0, true));
         NET_TRY(layer_bwd(C2A, g_e2a, e2a, p1, nullptr, &g_p1, 0, nullptr, S, st));
-        pool_bwd(g_p1, g_e1, S, st);
-        NET_TRY(layer_bwd(C1B, g_e1, e1, e1a, nullptr, &g_e1a, 0, nullptr, S, st));
+        pool_bwd(g_p1, g_e1, e1, S, st);
+        NET_TRY(layer_bwd(C1B, g_e1, e1, e1a, nullptr, &g_e1a, 0, nullptr, S, st, 0, true));
         NET_TRY(layer_bwd(C1A, g_e1a, e1a, p0, nullptr, &g_p0, 0, nullptr, S, st));
-        pool_bwd(g_p0, g_e0, S, st);
-        NET_TRY(layer_bwd(C0B, g_e0, e0, e0a, nullptr, &g_e0a, 0, nullptr, S, st));
+        pool_bwd(g_p0, g_e0, e0, S, st);
+        NET_TRY(layer_bwd(C0B, g_e0, e0, e0a, nullptr, &g_e0a, 0, nullptr, S, st, 0, true));
         {
-            const size_t cnt8 = (size_t)S * Hp * Wp * 16 / 8;
-            icon::pdl(ws::k_relu_bwd, grid1(cnt8, 256), 256, 0, st, g_e0a.p, e0a.p, cnt8);
             const unsigned nb = in_wgrad_blocks(S, Hp, Wp);
             if ((size_t)nb * 160 > part_len)
                 return net_fail(ICON_ERR_INVALID, "warm start: input-layer scratch too small");
