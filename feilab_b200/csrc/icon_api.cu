@@ -226,7 +226,7 @@ struct icon_plan {
     float reproj_deg = 0.f;   // angle of icon_reconstruct_host's reprojection
     Arena arena;
     NodeTables nodes;
-    float *cx = nullptr, *cy = nullptr, *rcx = nullptr, *rcy = nullptr, *phi1 = nullptr;
+    float *rcx = nullptr, *rcy = nullptr, *phi1 = nullptr;
     int *i10 = nullptr;
     float2 *tw0 = nullptr, *tw0h = nullptr, *tw1 = nullptr;
     // Length of the Toeplitz y-transforms: the smallest 32 R >= 2 N1 - 1 that
@@ -332,7 +332,7 @@ struct icon_plan {
             g.wstride = (size_t)M;
         }
         g.phix = t.phix; g.phiy = t.phiy; g.ix0 = t.ix0; g.iy0 = t.iy0;
-        g.cx = cx; g.cy = cy; g.rcx = rcx; g.rcy = rcy; g.row_off = t.row_off; g.ent_jt = t.ent_jt; g.ent_iy0 = t.ent_iy0;
+        g.rcx = rcx; g.rcy = rcy; g.row_off = t.row_off; g.ent_jt = t.ent_jt; g.ent_iy0 = t.ent_iy0;
         g.ent_blk = t.ent_blk; g.ent_split = t.ent_split; g.ent_phiy = t.ent_phiy; g.ent_win = t.ent_win;
         g.tw0 = tw0; g.tw0h = tw0h; g.tw1 = tw1;
         g.Kt = Kt;
@@ -1084,8 +1084,6 @@ static icon_status plan_create_impl(const icon_geometry *geo, int group, icon_pl
     px2d(nx, nz, p->th_neg.data(), p->xy.data());
     weights(nx, nz, p->th_neg.data(), p->w.data());
     std::vector<float> cx = deapod(p->N0, p->n0, p->b0, p->kb0), cy = deapod(p->N1, p->n1, p->b1, p->kb1);
-    ICON_TRY(p->arena.upload(&p->cx, cx.data(), cx.size()));
-    ICON_TRY(p->arena.upload(&p->cy, cy.data(), cy.size()));
     std::vector<float> rcx(cx.size()), rcy(cy.size());
     for (size_t i = 0; i < cx.size(); ++i) rcx[i] = (float)(1.0 / (double)cx[i]);
     for (size_t i = 0; i < cy.size(); ++i) rcy[i] = (float)(1.0 / (double)cy[i]);

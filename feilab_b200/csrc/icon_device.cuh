@@ -160,73 +160,11 @@ __device__ __forceinline__ void fft_smem(float2 *s, int n, int lg, int B, const 
     }
 }
 
-// ---- batched FFT with compile-time batch B and row stride SB (>= B) ----
-// Same Stockham passes as fft_pass/fft_smem over s[n][SB] (values of slice b
-// at s[pos*SB + b]); B and SB are powers of two or padded strides known at
-// compile time, so all index arithmetic is shifts and masks.
+// log2 of the slices per group.
 template <int B>
 struct Log2B {
     static constexpr int v = (B >= 8) ? 3 : (B >= 4) ? 2 : (B >= 2) ? 1 : 0;
 };
-
-template <int R, int B, int SB>
-__device__ __forceinline__ void fft_pass_b(float2 *s, int n, int Ns, const float2 *__restrict__ tw, float dir)
-{
-    constexpr int Q = 16 / R;
-    constexpr int LB = Log2B<B>::v;
-    const int nb = n / R;
-    const int T = blockDim.x;
-    const int step = n / (Ns * R);
-    float2 v[Q][R];
-    int jq[Q], bq[Q];
-#pragma unroll
-    for (int q = 0; q < Q; ++q) {
-        int item = threadIdx.x + q * T;
-        int b = item & (B - 1), j = item >> LB;
-        jq[q] = j;
-        bq[q] = b;
-        int k = j & (Ns - 1);
-        float2 in[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) in[r] = s[(j + r * nb) * SB + b];
-        if (Ns > 1) {
-#pragma unroll
-            for (int r = 1; r < R; ++r) {
-                float2 w = __ldg(&tw[r * k * step]);
-                w.y = -dir * w.y;
-                in[r] = cmul(in[r], w);
-            }
-        }
-        dft<R, 1>(in, v[q], dir);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < Q; ++q) {
-        int j = jq[q], b = bq[q];
-        int k = j & (Ns - 1);
-        int base = (j - k) * R + k;
-#pragma unroll
-        for (int r = 0; r < R; ++r) s[(base + r * Ns) * SB + b] = v[q][r];
-    }
-    __syncthreads();
-}
-
-// blockDim.x == n*B/16; call after a __syncthreads().
-template <int B, int SB>
-__device__ __forceinline__ void fft_batched(float2 *s, int n, int lg, const float2 *__restrict__ tw, float dir)
-{
-    int Ns = 1;
-    switch (lg & 3) {
-    case 1: fft_pass_b<2, B, SB>(s, n, Ns, tw, dir); Ns = 2; break;
-    case 2: fft_pass_b<4, B, SB>(s, n, Ns, tw, dir); Ns = 4; break;
-    case 3: fft_pass_b<8, B, SB>(s, n, Ns, tw, dir); Ns = 8; break;
-    default: break;
-    }
-    while (Ns < n) {
-        fft_pass_b<16, B, SB>(s, n, Ns, tw, dir);
-        Ns *= 16;
-    }
-}
 
 // ---- fused FFT: E values per thread, I/O through functors ---------------
 // exp(dir * 2*pi*i * k / 32) for compile-time k.
@@ -241,25 +179,6 @@ __device__ __forceinline__ float2 w32(int k, float dir)
         -0.19509032201612826f, 0.0f, 0.19509032201612826f, 0.38268343236508977f, 0.55557023301960218f,
         0.70710678118654752f, 0.83146961230254524f, 0.92387953251128674f, 0.98078528040323043f};
     return make_float2(C[k & 31], dir * C[(k + 24) & 31]);
-}
-
-// out[q] = sum_r in[r*IS] exp(dir*2*pi*i*r*q/R), R <= 32, unrolled.
-template <int R, int IS>
-__device__ __forceinline__ void dft32(const float2 *in, float2 *out, float dir)
-{
-    if constexpr (R == 1) {
-        out[0] = in[0];
-    } else {
-        float2 e[R / 2], o[R / 2];
-        dft32<R / 2, 2 * IS>(in, e, dir);
-        dft32<R / 2, 2 * IS>(in + IS, o, dir);
-#pragma unroll
-        for (int k = 0; k < R / 2; ++k) {
-            float2 t = (k == 0) ? o[k] : cmul(w32(k * (32 / R), dir), o[k]);
-            out[k] = cadd(e[k], t);
-            out[k + R / 2] = csub(e[k], t);
-        }
-    }
 }
 
 // Bit reversal of r < 32 over 5 bits, branch- and loop-free so that it folds

@@ -48,10 +48,8 @@ struct Geo {
     const float *phiy;     // [M][16] window values, y taps, 2 zero pads
     const int *ix0;        // [M] first x tap, unwrapped: floor(n0*x0) - 6
     const int *iy0;        // [M] first y tap, unwrapped
-    const float *cx;       // [N0] deapodisation factor along x (NU:22-42)
-    const float *cy;       // [N1] deapodisation factor along y
-    const float *rcx;      // [N0] 1/cx, rounded once from double
-    const float *rcy;      // [N1] 1/cy
+    const float *rcx;      // [N0] 1/cx, the deapodisation factor along x (NU:22-42), rounded once from double
+    const float *rcy;      // [N1] 1/cy, along y
     const int *row_off;    // [n0+1] entry range of every grid row x
     const int *ent_jt;     // [M*14] entry: node*16 + x tap, sorted by (row, iy0, node)
     const int *ent_iy0;    // [M*14] iy0 of the entry's node (sort key within a row)
@@ -65,7 +63,6 @@ struct Geo {
     const float *Kt;       // [n0][n1] Toeplitz kernel of A^H W A, group g's at Kt + kidx[g]*kstride
     size_t kstride;        // 0: one kernel for every group; n0*n1: one per distinct weight set
     const int *kidx;       // [G] kernel of each group (per-group weights), or null
-
 };
 
 // 1-D row-transform tables (cunfft_initPlan_1d, NU:1298-1391).
@@ -569,17 +566,6 @@ __device__ __forceinline__ int lower_bound_i(const int *__restrict__ key, int lo
     while (lo < hi) {
         int mid = (lo + hi) >> 1;
         if (__ldg(&key[mid]) < v) lo = mid + 1;
-        else hi = mid;
-    }
-    return lo;
-}
-
-// Index of the first of the sorted keys key[lo..hi) that is >= v (shared memory).
-__device__ __forceinline__ int lower_bound_s(const int *key, int lo, int hi, int v)
-{
-    while (lo < hi) {
-        int mid = (lo + hi) >> 1;
-        if (key[mid] < v) lo = mid + 1;
         else hi = mid;
     }
     return lo;

@@ -19,8 +19,8 @@ struct Launch {
     static void xpass_fwd_full(int E, dim3 grid, int threads, size_t smem, cudaStream_t st, const Geo &g,
                                const float *in, float2 *G1);
     // Toeplitz y-passes: A^H W A on the rows of G1 in place, and the step
-    // length's quadratic form into part[G][n0][B].
-    // (with Gh, from the half spectrum of a real image).
+    // length's quadratic form into part[G][n0][B].  With Gh the input is the half
+    // spectrum of a real image (k_xtoep_real's output) instead of G1.
     static void ypass_toep(int E, dim3 grid, int threads, size_t smem, cudaStream_t st, const Geo &g, float2 *G1,
                            const float2 *Gh);
     static void ypass_toep_quad(int E, dim3 grid, int threads, size_t smem, cudaStream_t st, const Geo &g,
@@ -55,9 +55,9 @@ struct Launch {
     static void update_re(dim3 grid, cudaStream_t st, float *m, const float *rre, const double *alpha, int per_group,
                           int clamp, int data_type, float thr);
     // Three-step x-passes (k_xtoep) over G groups: mode 0 the forward of a
-    // complex image, mode 1 the
-    // Toeplitz inverse, r-hat and forward of r-hat, mode 2 the NUFFT adjoint's
-    // x-pass (deapodised, optionally minus Ahwb with |.|^2 sums).  Returns
+    // complex image, mode 1 the Toeplitz inverse, r-hat and forward of r-hat,
+    // mode 2 the NUFFT adjoint's x-pass (deapodised, optionally minus Ahwb with
+    // |.|^2 sums).  Returns
     // false when n0 has no variant (the caller then uses the Stockham kernels).
     static bool xtoep(int mode, cudaStream_t st, int G, const XtArgs &a);
     // The forward of a real image (k_xtoep_real; n0 as xtoep).
