@@ -738,15 +738,17 @@ icon_status ensure_toeplitz(icon_plan *p, cudaStream_t st)
     const float *w = p->wgroups > 0 ? p->wuniq : p->nodes.w;
     dim3 grid((p->n1t + icon::kToepTile - 1) / icon::kToepTile, (p->n0 + icon::kToepTile - 1) / icon::kToepTile,
               groups_needed);
-    // Node ranges: enough CTAs for the SMs, as far as G1, which no one reads
-    // before the next transform writes it, holds their sums.
+    // Node ranges: enough CTAs for the SMs, as far as P, which like G1 no one
+    // reads before the next transform writes it, holds their sums (7 slices of 1239
+    // x 52 with 76 tilts: 32 tiles, first solve 11 ms; 34 ms in the three ranges that G1 holds).
     const size_t plane = (size_t)p->n0 * p->n1t;
     const size_t ctas = (size_t)grid.x * grid.y * grid.z;
-    // The nodes' sines and cosines go before them.
-    const size_t trig = (size_t)p->M * icon::kToepTrig, have = (size_t)p->Gcap * p->n0 * p->N1 * p->B;   // doubles
-    const size_t room = have > trig ? (have - trig) / (plane * groups_needed) : 0;
+    const size_t room = (size_t)p->Gcap * p->B * std::max((size_t)p->M * kTaps, (size_t)(p->n0 / 2 + 1) * p->N1) /
+                        (plane * groups_needed);          // float2 as doubles
     const int split = (int)std::max<size_t>(1, std::min({(size_t)16, (296 + ctas - 1) / ctas, room}));
-    double *tr = (double *)p->G1, *part = tr + trig;
+    // The nodes' sines and cosines in G1.
+    const size_t trig = (size_t)p->M * icon::kToepTrig, have = (size_t)p->Gcap * p->n0 * p->N1 * p->B;   // doubles
+    double *tr = (double *)p->G1, *part = (double *)p->P;
     if (have < trig) ICON_CUDA(cudaMalloc(&tr, sizeof(double) * trig));   // more tilts than image rows
     icon::k_toep_trig<<<(p->M + 127) / 128, 128, 0, st>>>(xy_d, p->M, p->N0, p->N1, tr);
     grid.z = groups_needed * split;
