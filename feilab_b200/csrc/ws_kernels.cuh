@@ -1,5 +1,6 @@
-// ws_kernels.cuh -- SIMT kernels of the warm-start U-Net: everything but the
-// 3x3 tensor-core convolutions (ws_conv.cuh).  Activations are NHWC BF16
+// ws_kernels.cuh -- the kernels of the warm-start U-Net besides the 3x3
+// tensor-core convolutions (ws_conv.cuh): weight gradients by mma.sync, the rest
+// SIMT.  Activations are NHWC BF16
 // images [n][H][W][C]; arithmetic is FP32; every reduction is two-level with
 // a fixed order (partial sums per block, then one pass over the partials), so
 // results do not depend on scheduling.

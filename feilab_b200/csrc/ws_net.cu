@@ -11,9 +11,9 @@
 //            up(d1) ++ e0: 48 -> 16, 16 -> 16                  -> d0
 //   out      1x1: 16 -> 1 (no ReLU)
 // All 3x3 layers but the first run on the tensor cores (ws_conv.cuh), their
-// input gradients too (the same convolution with flipped weights); weight
-// gradients, pooling, upsampling and the first and last layers are SIMT
-// (ws_kernels.cuh).  The image is the slice's N1 x N0 back-projection padded
+// input gradients too (the same convolution with flipped weights) and their
+// weight gradients (mma.sync); pooling, upsampling and the first and last layers
+// are SIMT (ws_kernels.cuh).  The image is the slice's N1 x N0 back-projection padded
 // to multiples of 8, divided by its RMS; the output is scaled back by the
 // same RMS times a fixed gain.
 #include <cuda_runtime.h>
