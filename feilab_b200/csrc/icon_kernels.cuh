@@ -1308,8 +1308,10 @@ __global__ void __launch_bounds__(256, 1) k_toep_kernel(const double *__restrict
         for (int j = 0; j < 8; ++j) acc[i][j] = 0.0;
     for (int j0 = j_lo; j0 < j_hi; j0 += kToepNodes) {
         __syncthreads();                             // the previous chunk's tables are consumed
-        for (int i = t; i < kToepNodes * kToepTrig; i += 256)      // nodes past the range weigh 0
-            (&nd[0][0])[i] = trig[min((size_t)j0 * kToepTrig + i, (size_t)M * kToepTrig - 1)];
+        // Nodes past the range weigh 0, those past M repeat the last node: its
+        // factors are finite, and 0 times them adds nothing.
+        for (int i = t; i < kToepNodes * kToepTrig; i += 256)
+            (&nd[0][0])[i] = trig[(size_t)min(j0 + i / kToepTrig, M - 1) * kToepTrig + i % kToepTrig];
         __syncthreads();
 #pragma unroll
         for (int i = 0; i < kToepNodes / 2; ++i) {
