@@ -536,28 +536,17 @@ icon_status build_tables(icon_plan *p, const float *xy, const float *w, int M, N
             ky2[a + i] = ky[order[i]];
         }
     }
-    // Per row, for the adjoint gather: the entries whose first non-zero tap's
-    // buffer row iy0 + tlo + n1/2 + 8 lies below each block of ph rows,
-    // relative to the row's first entry, and the block ranges of the
-    // gather's warps, cut at equal shares of entries + blocks (a block's
-    // store and bounds cost about as much as an entry).
+    // Per row, for the adjoint gather: the entries (relative to the row's first)
+    // that start below each block of ph buffer rows, and the block ranges of
+    // the gather's warps.
     const int ph = icon::ywin_ph(p->B), nblk = icon::ywin_blocks(p->n1, p->B), warps = p->thr_ya / 32;
     const int r0ofs = p->n1 / 2 + icon::kHalo;
     std::vector<unsigned short> eblk((size_t)n0 * (nblk + 1)), split((size_t)n0 * (warps + 1));
     for (int x = 0; x < n0; ++x) {
         int a = cnt[x], c = cnt[x + 1];
         if (c - a > 65535) return fail(ICON_ERR_INVALID, "more than 65535 window entries on one grid row");
-        int e = a;
-        unsigned short *off = &eblk[(size_t)x * (nblk + 1)], *cut = &split[(size_t)x * (warps + 1)];
-        for (int v = 0; v <= nblk; ++v) {
-            while (e < c && ky2[e] + r0ofs + tlo < v * ph) ++e;
-            off[v] = (unsigned short)(e - a);
-        }
-        const long long total = (long long)(c - a) + nblk;
-        for (int w = 0, v = 0; w <= warps; ++w) {
-            while (v < nblk && (long long)(off[v] + v) * warps < total * w) ++v;
-            cut[w] = (unsigned short)(w == warps ? nblk : v);
-        }
+        icon::adj_row_tables(ky2.data() + a, c - a, r0ofs + tlo, ph, nblk, warps, &eblk[(size_t)x * (nblk + 1)],
+                             &split[(size_t)x * (warps + 1)]);
         if (c > a && (ky2[a] + r0ofs < 0 || ky2[c - 1] + r0ofs + kTaps > p->n1 + 2 * icon::kHalo))
             return fail(ICON_ERR_INVALID, "window taps outside the rotated y buffer");
         // The mirrored windows of the real-image forward y-pass: buffer rows

@@ -30,12 +30,12 @@
 // (-1)^y shifts its output by n1/2, and an input rotated by n1/2 gives the
 // output times (-1)^k.
 #pragma once
+#include "adj_gather.h"
 #include "icon_device.cuh"
 #include "ws_tc.cuh"
 
 namespace icon {
 
-constexpr int kHalo = 8;      // halo rows on each side of a rotated row buffer
 constexpr int kLdPhiy = 16;   // phiy rows padded to 16 floats (four 16-byte loads)
 
 // Device view of one tilt-series geometry (all pointers are device memory).
@@ -70,16 +70,6 @@ struct Geo1 {
     const float *phi1;     // [nx][14]
     const int *i10;        // [nx] first tap, unwrapped, nondecreasing in k
 };
-
-// Layout of the adjoint gather (yadj_gather) for groups of B slices: a warp's
-// lanes are ywin_ph(B) neighbouring buffer rows times B slices (two slices a
-// lane for B = 8), and an entry's window, starting anywhere within a block of
-// ph rows, covers at most nr blocks.
-__host__ __device__ constexpr int ywin_ph(int B) { return B >= 4 ? 8 : B == 2 ? 16 : 32; }
-__host__ __device__ constexpr int ywin_nr(int B) { return B >= 4 ? 3 : 2; }
-__host__ __device__ constexpr int ywin_lp(int B) { return ywin_ph(B) * ywin_nr(B); }
-__host__ __device__ constexpr int ywin_pos(int ph, int p, int k) { return k < 2 ? 2 * p + k : 2 * ph + p; }
-__host__ __device__ constexpr int ywin_blocks(int n1, int B) { return (n1 + 2 * kHalo + ywin_ph(B) - 1) / ywin_ph(B); }
 
 #ifndef ICON_KERNELS_TEMPLATES_ONLY
 // ------------------------------------------------------------- tables ----
@@ -611,10 +601,9 @@ struct YWin {
 
 // Threads of the adjoint y-pass for rows of n1: the FFT's, at least two warps.
 __host__ __device__ constexpr int yadj_threads(int fft_threads) { return fft_threads < 64 ? 64 : fft_threads; }
-// Entries per staged chunk, and chunks in flight per warp: two CTAs per SM for
+// Chunks of kAdjChunk entries in flight per warp: two CTAs per SM for
 // the 1024-point rows of 8-slice groups, and within a block's shared memory
 // for the longest rows.
-constexpr int kAdjChunk = 8;
 __host__ __device__ constexpr int yadj_stages(int threads) { return threads <= 256 ? 3 : 2; }
 __host__ __device__ constexpr int yadj_chunk_bytes(int B)
 {
@@ -650,9 +639,10 @@ __device__ __forceinline__ void yadj_gather(const Geo &g, int x, const float2 *f
     const int es = boff[bs], ee = b1 > b0 ? boff[b1] : es;
     char *const buf = stage + warp * ST * CB;
     // Node of this lane's piece of f in the chunk from entry c0 on (entries
-    // past ee repeat the last node).
-    const int *jt = g.ent_jt + e0 + lane / C;
-    auto node_of = [&](int c0) { return __ldg(jt + min(c0, max(ee - 1 - lane / C, 0))) >> 4; };
+    // past ee repeat the last node; a warp without entries reads none).
+    const int *jt = g.ent_jt + e0;
+    const bool any = ee > es;
+    auto node_of = [&](int c0) { return any ? __ldg(jt + adj_entry(c0, lane / C, ee)) >> 4 : 0; };
     // Entries c0 .. c0+7 into buffer s, j their nodes; the windows read on past
     // ee (the table is padded by a chunk).
     const float *win = g.ent_win + (size_t)(e0 + es) * LP + 4 * lane;   // of the next chunk to issue
