@@ -46,6 +46,13 @@ inline void adj_row_tables(const int *iy, int cnt, int ofs, int ph, int nblk, in
     }
 }
 
+// First block that a warp with blocks b0..b1-1 walks: windows of the nr - 1 blocks
+// before reach into its own.  A warp without blocks walks none.
+ICON_HD inline int adj_first_block(int b0, int b1, int nr)
+{
+    return b0 == b1 ? b1 : b0 < nr - 1 ? 0 : b0 - (nr - 1);
+}
+
 // Entry of the row whose node the lane of place `at` copies for the chunk from
 // entry c0 on, in a warp whose entries end before ee: past the end the last one
 // again.  Only for warps that have entries; c0 and at are not negative.

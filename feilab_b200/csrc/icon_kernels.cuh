@@ -635,8 +635,8 @@ __device__ __forceinline__ void yadj_gather(const Geo &g, int x, const float2 *f
     const unsigned short *boff = g.ent_blk + (size_t)x * (nblk + 1);
     const int b0 = g.ent_split[x * (W + 1) + warp], b1 = g.ent_split[x * (W + 1) + warp + 1];
     const int e0 = g.row_off[x];
-    const int bs = max(b0 - (NR - 1), 0);            // windows of earlier blocks reach into the first ones
-    const int es = boff[bs], ee = b1 > b0 ? boff[b1] : es;
+    const int bs = adj_first_block(b0, b1, NR);
+    const int es = boff[bs], ee = boff[b1];
     char *const buf = stage + warp * ST * CB;
     // Node of this lane's piece of f in the chunk from entry c0 on (entries
     // past ee repeat the last node; a warp without entries reads none).

@@ -39,7 +39,9 @@ extern "C" long check(const int *ix0, const int *iy0, int M, int tlo, int thi, i
         for (int w = 0; w < warps; ++w) {
             const int b0 = cut[w], b1 = cut[w + 1];
             if (b1 < b0) ++bad;
-            const int es = off[std::max(b0 - (nr - 1), 0)], ee = b1 > b0 ? off[b1] : es;
+            const int bs = adj_first_block(b0, b1, nr), es = off[bs], ee = off[b1];
+            if (bs > b1 || (b0 == b1 && bs != b1)) ++bad;    // a warp without blocks walks none
+            if (b0 < b1 && bs != std::max(b0 - (nr - 1), 0)) ++bad;
             if (ee <= es) continue;               // a warp without entries reads no nodes
             for (int c0 = es; c0 < ee + (stages + 1) * CH; c0 += CH)
                 for (int lane = 0; lane < 32; ++lane) {
