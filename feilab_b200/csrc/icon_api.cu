@@ -237,6 +237,7 @@ struct icon_plan {
     float2 *G1 = nullptr, *P = nullptr, *f = nullptr, *rhat = nullptr, *Ahwb = nullptr, *imgc = nullptr;
     float *m = nullptr, *rows = nullptr, *outrp = nullptr, *mout = nullptr;
     float *nodes_xy = nullptr;   // [M][2] node coordinates on the device (Toeplitz kernel)
+    double *toep_part = nullptr, *toep_trig = nullptr;   // scratch of the Toeplitz kernel where P, G1 are too small
     double *part_rtr = nullptr, *part_rtar = nullptr, *alpha = nullptr;
     double *step_part = nullptr, *step = nullptr;   // relative update size (icon_solve_until)
     float *wgroup = nullptr;   // [Gcap][M] per-group weights while wgroups > 0
@@ -725,32 +726,44 @@ icon_status ensure_toeplitz(icon_plan *p, cudaStream_t st)
     if (!p->nodes_xy) ICON_TRY(p->arena.upload(&p->nodes_xy, p->xy.data(), p->xy.size()));
     xy_d = p->nodes_xy;
     const float *w = p->wgroups > 0 ? p->wuniq : p->nodes.w;
-    dim3 grid((p->n1t + icon::kToepTile - 1) / icon::kToepTile, (p->n0 + icon::kToepTile - 1) / icon::kToepTile,
-              groups_needed);
-    // Node ranges: enough CTAs for the SMs, as far as P, which like G1 no one
-    // reads before the next transform writes it, holds their sums (7 slices of 1239
-    // x 52 with 76 tilts: 32 tiles, first solve 11 ms; 34 ms in the three ranges that G1 holds).
+    dim3 grid((p->n1t + icon::kToepTile - 1) / icon::kToepTile, (p->n0 + icon::kToepTile - 1) / icon::kToepTile);
+    // Node ranges of one weight set: enough CTAs for the SMs, by the grid and nx
+    // alone (k_toep_kernel's order of summation).  Their sums go to P, which
+    // like G1 no one reads before the next transform writes it, as many
+    // weight sets at a time as it holds (7 slices of 1239 x 52 with 76 tilts: 32
+    // tiles, first solve 11 ms; 34 ms in the three ranges that G1 holds); in plans of
+    // a few slices, where it holds none, to a buffer made here once.
     const size_t plane = (size_t)p->n0 * p->n1t;
-    const size_t ctas = (size_t)grid.x * grid.y * grid.z;
-    const size_t room = (size_t)p->Gcap * p->B * std::max((size_t)p->M * kTaps, (size_t)(p->n0 / 2 + 1) * p->N1) /
-                        (plane * groups_needed);          // float2 as doubles
-    const int split = (int)std::max<size_t>(1, std::min({(size_t)16, (296 + ctas - 1) / ctas, room}));
-    // The nodes' sines and cosines in G1.
-    const size_t trig = (size_t)p->M * icon::kToepTrig, have = (size_t)p->Gcap * p->n0 * p->N1 * p->B;   // doubles
-    double *tr = (double *)p->G1, *part = (double *)p->P;
-    if (have < trig) ICON_CUDA(cudaMalloc(&tr, sizeof(double) * trig));   // more tilts than image rows
-    icon::k_toep_trig<<<(p->M + 127) / 128, 128, 0, st>>>(xy_d, p->M, p->N0, p->N1, tr);
-    grid.z = groups_needed * split;
-    icon::k_toep_kernel<<<grid, 256, 0, st>>>(tr, w, p->wgroups > 0 ? (size_t)p->M : 0, p->M, p->N0, p->N1, p->n0,
-                                              p->n1t, icon::ytoep4_fits(p->n1t) ? p->n1t / 32 : 0, split, part, p->Kt);
-    if (split > 1)
-        icon::k_toep_sum<<<dim3((unsigned)((plane + 255) / 256), groups_needed), 256, 0, st>>>(
-            part, split, plane, 1.0 / ((double)p->n0 * (double)p->n1t), p->Kt);
-    ICON_CUDA(cudaGetLastError());
-    if (have < trig) {
-        ICON_CUDA(cudaStreamSynchronize(st));
-        ICON_CUDA(cudaFree(tr));
+    const int ctas = (int)(grid.x * grid.y), split = std::max(1, std::min({16, (296 + ctas - 1) / ctas, p->nx}));
+    const size_t set = split > 1 ? plane * split : 0;     // doubles
+    size_t room = (size_t)p->Gcap * p->B * std::max((size_t)p->M * kTaps, (size_t)(p->n0 / 2 + 1) * p->N1);
+    double *part = (double *)p->P;                         // float2 as doubles
+    if (room < set) {
+        if (!p->toep_part) ICON_TRY(p->arena.alloc(&p->toep_part, set));
+        part = p->toep_part;
+        room = set;
     }
+    // The nodes' sines and cosines in G1, or (more tilts than image rows) a buffer.
+    const size_t trig = (size_t)p->M * icon::kToepTrig;
+    double *tr = (double *)p->G1;
+    if ((size_t)p->Gcap * p->n0 * p->N1 * p->B < trig) {
+        if (!p->toep_trig) ICON_TRY(p->arena.alloc(&p->toep_trig, trig));
+        tr = p->toep_trig;
+    }
+    icon::k_toep_trig<<<(p->M + 127) / 128, 128, 0, st>>>(xy_d, p->M, p->N0, p->N1, tr);
+    const int sets = (int)std::min<size_t>(65535 / split, set ? room / set : (size_t)groups_needed);   // per launch
+    for (int g0 = 0; g0 < groups_needed; g0 += sets) {
+        const int n = std::min(sets, groups_needed - g0);
+        grid.z = n * split;
+        float *K = p->Kt + (size_t)g0 * plane;
+        icon::k_toep_kernel<<<grid, 256, 0, st>>>(tr, w + (size_t)g0 * p->M, p->wgroups > 0 ? (size_t)p->M : 0, p->nx, p->nz,
+                                                  p->N0, p->N1, p->n0, p->n1t,
+                                                  icon::ytoep4_fits(p->n1t) ? p->n1t / 32 : 0, split, part, K);
+        if (split > 1)
+            icon::k_toep_sum<<<dim3((unsigned)((plane + 255) / 256), n), 256, 0, st>>>(
+                part, split, plane, 1.0 / ((double)p->n0 * (double)p->n1t), K);
+    }
+    ICON_CUDA(cudaGetLastError());
     p->kt_groups = groups_needed;
     p->kt_stale = false;
     return ICON_OK;

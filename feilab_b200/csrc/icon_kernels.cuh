@@ -1265,18 +1265,23 @@ __global__ void k_toep_trig(const float *__restrict__ xy, int M, int N0, int N1,
 // part[G][split][n0][n1] in double (k_toep_sum adds them in order): a kernel of
 // 1024 x 512 has 32 tiles for 148 SMs; its 31,232 nodes take 3.4 ms, and took 6.4
 // ms in one range by 64 x 64 tiles that evaluated the nodes' sines each.
+// Range r holds the nodes k = nx r / split .. nx (r + 1) / split - 1 of every
+// tilt, tilt by tilt (node tilt*nx + k).  So the order of K's sums depends on the
+// grid and nx alone: plans of any capacity and number of weight sets have the
+// same K, and weight 0 at a tilt's nodes gives the K of the series without it.
 __global__ void __launch_bounds__(256, 1) k_toep_kernel(const double *__restrict__ trig, const float *__restrict__ w,
-                                                     size_t wstride, int M, int N0, int N1, int n0, int n1,
+                                                     size_t wstride, int nx, int nz, int N0, int N1, int n0, int n1,
                                                      int perm_r, int split, double *__restrict__ part,
                                                      float *__restrict__ K)
 {
     __shared__ __align__(16) double F0[kToepNodes][kToepTile];   // w_j D_N0(x_j0 - k0/n0)
     __shared__ __align__(16) double F1[kToepNodes][kToepTile];   // D_N1(x_j1 - k1/n1)
     __shared__ double nd[kToepNodes][kToepTrig];     // the chunk's nodes
+    __shared__ double wn[kToepNodes];                // and weights
     const int t = threadIdx.x;
     const int k1b = blockIdx.x * kToepTile, k0b = blockIdx.y * kToepTile, grp = blockIdx.z / split;
     const int rng = blockIdx.z - grp * split;
-    const int j_lo = (int)((long long)M * rng / split), j_hi = (int)((long long)M * (rng + 1) / split);
+    const int k_lo = nx * rng / split, len = nx * (rng + 1) / split - k_lo, cnt = len * nz;
     const float *wg = w + (size_t)grp * wstride;
     const double a0 = 2.0 * N0 - 1.0, a1 = 2.0 * N1 - 1.0;
     // This thread's k for the factor tables: column c = t % 128 of both tiles,
@@ -1296,18 +1301,21 @@ __global__ void __launch_bounds__(256, 1) k_toep_kernel(const double *__restrict
     for (int i = 0; i < 8; ++i)
 #pragma unroll
         for (int j = 0; j < 8; ++j) acc[i][j] = 0.0;
-    for (int j0 = j_lo; j0 < j_hi; j0 += kToepNodes) {
+    for (int q0 = 0; q0 < cnt; q0 += kToepNodes) {
         __syncthreads();                             // the previous chunk's tables are consumed
-        // Nodes past the range weigh 0, those past M repeat the last node: its
-        // factors are finite, and 0 times them adds nothing.
-        for (int i = t; i < kToepNodes * kToepTrig; i += 256)
-            (&nd[0][0])[i] = trig[(size_t)min(j0 + i / kToepTrig, M - 1) * kToepTrig + i % kToepTrig];
+        // Node q of the range; past its end the last node again (its factors are
+        // finite) at weight 0.
+        if (t < kToepNodes * kToepTrig) {
+            const int r = t / kToepTrig, i = t - r * kToepTrig, q = min(q0 + r, cnt - 1), tilt = q / len;
+            const size_t j = (size_t)tilt * nx + k_lo + (q - tilt * len);
+            nd[r][i] = trig[j * kToepTrig + i];
+            if (i == 0) wn[r] = q0 + r < cnt ? (double)wg[j] : 0.0;
+        }
         __syncthreads();
 #pragma unroll
         for (int i = 0; i < kToepNodes / 2; ++i) {
-            const int r = r0 + 2 * i, j = j0 + r;
-            const double wj = j < j_hi ? (double)wg[j] : 0.0;
-            F0[r][c] = wj * dirichlet(nd[r][8], u0, nd[r][0], nd[r][1], nd[r][2], nd[r][3], sk0, ck0, skb0, ckb0, a0);
+            const int r = r0 + 2 * i;
+            F0[r][c] = wn[r] * dirichlet(nd[r][8], u0, nd[r][0], nd[r][1], nd[r][2], nd[r][3], sk0, ck0, skb0, ckb0, a0);
             F1[r][c] = dirichlet(nd[r][9], u1, nd[r][4], nd[r][5], nd[r][6], nd[r][7], sk1, ck1, skb1, ckb1, a1);
         }
         __syncthreads();
