@@ -486,8 +486,10 @@ void setup_xt_tma(icon_plan *p)
     p->xt_tma = ok;
 }
 
-// Builds window tables and the per-row entry lists of M nodes at xy.
-icon_status build_tables(icon_plan *p, const float *xy, const float *w, int M, NodeTables &t)
+// Builds window tables and the per-row entry lists of M nodes at xy; `adjoint`:
+// also the adjoint gather's (a reprojection line is never gathered, and its window
+// products are most of a line's tables: 256 of 328 bytes an entry in one-slice plans).
+icon_status build_tables(icon_plan *p, const float *xy, const float *w, int M, bool adjoint, NodeTables &t)
 {
     t.M = M;
     float *xy_d = nullptr;
@@ -542,12 +544,17 @@ icon_status build_tables(icon_plan *p, const float *xy, const float *w, int M, N
     // the gather's warps.
     const int ph = icon::ywin_ph(p->B), nblk = icon::ywin_blocks(p->n1, p->B), warps = p->thr_ya / 32;
     const int r0ofs = p->n1 / 2 + icon::kHalo;
-    std::vector<unsigned short> eblk((size_t)n0 * (nblk + 1)), split((size_t)n0 * (warps + 1));
+    std::vector<unsigned short> eblk, split;
+    if (adjoint) {
+        eblk.resize((size_t)n0 * (nblk + 1));
+        split.resize((size_t)n0 * (warps + 1));
+    }
     for (int x = 0; x < n0; ++x) {
         int a = cnt[x], c = cnt[x + 1];
         if (c - a > 65535) return fail(ICON_ERR_INVALID, "more than 65535 window entries on one grid row");
-        icon::adj_row_tables(ky2.data() + a, c - a, r0ofs + tlo, ph, nblk, warps, &eblk[(size_t)x * (nblk + 1)],
-                             &split[(size_t)x * (warps + 1)]);
+        if (adjoint)
+            icon::adj_row_tables(ky2.data() + a, c - a, r0ofs + tlo, ph, nblk, warps, &eblk[(size_t)x * (nblk + 1)],
+                                 &split[(size_t)x * (warps + 1)]);
         if (c > a && (ky2[a] + r0ofs < 0 || ky2[c - 1] + r0ofs + kTaps > p->n1 + 2 * icon::kHalo))
             return fail(ICON_ERR_INVALID, "window taps outside the rotated y buffer");
         // The mirrored windows of the real-image forward y-pass: buffer rows
@@ -559,10 +566,12 @@ icon_status build_tables(icon_plan *p, const float *xy, const float *w, int M, N
     ICON_TRY(p->arena.upload(&t.row_off, cnt.data(), (size_t)n0 + 1));
     ICON_TRY(p->arena.upload(&t.ent_jt, jt2.data(), E));
     ICON_TRY(p->arena.upload(&t.ent_iy0, ky2.data(), E));
-    ICON_TRY(p->arena.upload(&t.ent_blk, eblk.data(), eblk.size()));
-    ICON_TRY(p->arena.upload(&t.ent_split, split.data(), split.size()));
     ICON_TRY(p->arena.alloc(&t.ent_phiy, E * icon::kLdPhiy));
-    ICON_TRY(p->arena.alloc(&t.ent_win, (E + icon::kAdjChunk) * icon::ywin_lp(p->B)));   // staged in whole chunks
+    if (adjoint) {
+        ICON_TRY(p->arena.upload(&t.ent_blk, eblk.data(), eblk.size()));
+        ICON_TRY(p->arena.upload(&t.ent_split, split.data(), split.size()));
+        ICON_TRY(p->arena.alloc(&t.ent_win, (E + icon::kAdjChunk) * icon::ywin_lp(p->B)));   // staged in whole chunks
+    }
     icon::k_entry_tables<<<(unsigned)((E + 255) / 256), 256>>>(t.ent_jt, t.ent_iy0, (int)E, t.phiy, t.phix, tlo, thi, r0ofs,
                                                                p->B, t.ent_phiy, t.ent_win);
     ICON_CUDA(cudaGetLastError());
@@ -971,7 +980,7 @@ icon_status line_tables(icon_plan *p, float tilt_deg, NodeTables **out)
     float thn = -tilt_deg;
     std::vector<float> xy((size_t)2 * p->nx), w((size_t)p->nx, 1.0f);
     px2d(p->nx, 1, &thn, xy.data());
-    ICON_TRY(build_tables(p, xy.data(), w.data(), p->nx, *t));
+    ICON_TRY(build_tables(p, xy.data(), w.data(), p->nx, false, *t));
     *out = t.get();
     p->lines[tilt_deg] = std::move(t);
     return ICON_OK;
@@ -1130,7 +1139,7 @@ static icon_status plan_create_impl(const icon_geometry *geo, int group, icon_pl
     p->smem_y = icon::ypass_fwd_smem(p->n1, B);
     p->thr_ya = icon::yadj_threads(icon::yadj4_fits(p->n1) ? p->n1 / 32 * B : p->thr_y);
     p->smem_ya = icon::ypass_adj_smem(p->n1, B, p->thr_ya);
-    ICON_TRY(build_tables(p.get(), p->xy.data(), p->w.data(), p->M, p->nodes));
+    ICON_TRY(build_tables(p.get(), p->xy.data(), p->w.data(), p->M, true, p->nodes));
     // Toeplitz y-length: a circular convolution of the N1 rows with a kernel
     // of support 2 N1 - 1 needs 2 N1 - 1 points; the four-step kernel takes
     // 32 R for R in {4, 6, 8, 10, 12, 16, 20, 24, 32}.  ICON_TOEP_POW2=1 keeps

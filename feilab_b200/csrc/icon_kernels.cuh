@@ -108,7 +108,7 @@ __global__ void k_window(const float *__restrict__ x, int stride, int M, int n, 
 // and ewin[e], the products phix[j][t0] * phiy[j][t1] that the reference's
 // adjoint CSR stores per grid point and node (NU:44-218), placed on the
 // blocks of ph buffer rows that the entry's window covers (YWin): the value
-// of row blk*ph + p + ph*k, zero where no tap falls.
+// of row blk*ph + p + ph*k, zero where no tap falls (ewin may be null).
 __global__ void k_entry_tables(const int *__restrict__ jt, const int *__restrict__ iy0, int E,
                                const float *__restrict__ phiy, const float *__restrict__ phix, int tlo, int thi,
                                int r0ofs, int B, float *__restrict__ ephiy, float *__restrict__ ewin)
@@ -119,6 +119,7 @@ __global__ void k_entry_tables(const int *__restrict__ jt, const int *__restrict
     const float px = phix[(size_t)j * kTaps + t0];
 #pragma unroll
     for (int t = 0; t < kLdPhiy; ++t) ephiy[(size_t)e * kLdPhiy + t] = phiy[(size_t)j * kLdPhiy + t];
+    if (!ewin) return;
     const int ph = ywin_ph(B), nr = ywin_nr(B), lp = ywin_lp(B);
     const int o = (iy0[e] + r0ofs + tlo) & (ph - 1);
     for (int p = 0; p < ph; ++p)
