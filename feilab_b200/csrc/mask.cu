@@ -43,9 +43,17 @@ constexpr double kPi180 = 0.01745329252;   // MK:8
 // complex FFT, and a CTA transforms several pairs, or up to 8 neighbouring
 // columns, at once, so that every access is a run of whole sectors; the
 // columns' inverse stores the crop's rows only.  1024 x 1024, 16 slices, 300
-// rows kept: 197 us (66 + 80 + 47); one row or one 8-byte wide column per CTA
-// over the full spectrum took 642 us.
+// rows kept: 188 us the call; one row or one 8-byte wide column per CTA over the
+// full spectrum took 642 us.
 __host__ __device__ constexpr int mask_pitch(int n) { return n / 2 + 8; }
+
+// Every twiddle of the transforms is read from the table: formed by products between
+// table values, as the FFT otherwise does from global memory, they double a transform's
+// error, and with two rows in one transform the result was further from 64 bits
+// than with one (512 x 512: 5.3e-7 against 4.9e-7, now 2.5e-7; 1024 x 1024: 3.7e-7,
+// 3.1e-7, now 3.0e-7).  The columns' two transforms read a copy in shared memory
+// (16 slices of 1024: 188 us the call, 199 from global memory), the rows' one
+// transform the table itself (198 us with a copy there too).
 
 // Rows 2B*blockIdx.x .. of a slice, in pairs (a, b) as a + i b:
 // A(k) = (Z(k) + conj Z(n-k)) / 2, B(k) = (Z(k) - conj Z(n-k)) / 2i.
@@ -60,7 +68,7 @@ __global__ void __launch_bounds__(512) k_mask_rows_fwd(const float *__restrict__
     float2 *out = C + ((size_t)sl * n + y0) * P;
     auto ld = [=](int q, int b) -> float2 { return make_float2(rows[(size_t)(2 * b) * n + q], rows[(size_t)(2 * b + 1) * n + q]); };
     auto st = [=](int k, int b, float2 v) { s[k * B + b] = v; };
-    icon::fft_fused<B, B, E>(s, n, lg, tw, -1.f, ld, st);
+    icon::fft_fused<B, B, E, false, false, true>(s, n, lg, tw, -1.f, ld, st);
     __syncthreads();
     for (int i = threadIdx.x; i < (n / 2 + 1) * B; i += blockDim.x) {
         const int k = i / B, b = i - k * B;
@@ -81,18 +89,22 @@ __global__ void __launch_bounds__(512) k_mask_cols(float2 *__restrict__ C, const
     const int kx0 = B * blockIdx.x, sl = blockIdx.y, P = mask_pitch(n);
     float2 *col = C + (size_t)sl * n * P + kx0;
     const float *m = M + kx0;
+    float2 *tws = s + (size_t)n * B;
+    icon::copy_async(tws, tw, (size_t)n * sizeof(float2));
+    icon::cp_async_commit();
+    icon::cp_async_wait<0>();   // seen by all behind the barriers of the first pass, which reads none
     auto ld1 = [=](int q, int b) -> float2 { return col[(size_t)q * P + b]; };
     auto st1 = [=](int ky, int b, float2 v) {
         const float f = __ldg(&m[(size_t)ky * P + b]);
         s[ky * B + b] = make_float2(v.x * f, v.y * f);
     };
-    icon::fft_fused<B, B, E, false, B == 8>(s, n, lg, tw, -1.f, ld1, st1);
+    icon::fft_fused<B, B, E, false, B == 8, true>(s, n, lg, tws, -1.f, ld1, st1);
     __syncthreads();
     auto ld2 = [=](int q, int b) -> float2 { return s[q * B + b]; };
     auto st2 = [=](int y, int b, float2 v) {
         if ((unsigned)(y - ystart) < (unsigned)thickness) col[(size_t)y * P + b] = v;
     };
-    icon::fft_fused<B, B, E, false, B == 8>(s, n, lg, tw, +1.f, ld2, st2);
+    icon::fft_fused<B, B, E, false, B == 8, true>(s, n, lg, tws, +1.f, ld2, st2);
 }
 
 // Rows ystart + 2B*blockIdx.x .. of the crop, in pairs (a, b): the inverse FFT
@@ -120,11 +132,11 @@ __global__ void __launch_bounds__(512) k_mask_rows_inv(const float2 *__restrict_
         if (ra < thickness) o[(size_t)ra * n + x] = v.x * inv_norm;
         if (ra + 1 < thickness) o[(size_t)(ra + 1) * n + x] = v.y * inv_norm;
     };
-    icon::fft_fused<B, B, E>(s, n, lg, tw, +1.f, ld, st);
+    icon::fft_fused<B, B, E, false, false, true>(s, n, lg, tw, +1.f, ld, st);
 }
 
-// The row and column kernels' pairs and columns per CTA: 128 KB of shared
-// memory at most (sizes up to 8192).
+// The row and column kernels' transforms per CTA: 128 KB of shared memory for values
+// and 64 KB for twiddles at most (sizes up to 8192).
 template <int BR, int BC, int E>
 cudaError_t mask_limits(int bytes)
 {
@@ -137,11 +149,11 @@ template <int BR, int BC, int E>
 void mask_launch(const float *slices, float2 *C, const float *M, float *out, int n, int lg, const float2 *tw, int S,
                  int ystart, int thickness, cudaStream_t st)
 {
-    const size_t row_smem = sizeof(float2) * n * BR, col_smem = sizeof(float2) * n * BC;
+    const size_t row_smem = sizeof(float2) * n * BR, col_smem = sizeof(float2) * n * (BC + 1);
     icon::pdl(k_mask_rows_fwd<BR, E>, dim3(n / (2 * BR), S), n * BR / E, row_smem, st, slices, C, n, lg, tw);
     icon::pdl(k_mask_cols<BC, E>, dim3((n / 2 + BC) / BC, S), n * BC / E, col_smem, st, C, M, n, lg, tw, ystart, thickness);
-    icon::pdl(k_mask_rows_inv<BR, E>, dim3((thickness + 2 * BR - 1) / (2 * BR), S), n * BR / E, row_smem, st, 
-        C, out, n, lg, tw, ystart, thickness, 1.f / ((float)n * (float)n));
+    icon::pdl(k_mask_rows_inv<BR, E>, dim3((thickness + 2 * BR - 1) / (2 * BR), S), n * BR / E, row_smem, st, C, out, n,
+              lg, tw, ystart, thickness, 1.f / ((float)n * (float)n));
 }
 
 __global__ void k_crop(const float *__restrict__ slices, float *__restrict__ out, int n, int S, int ystart, int thickness)
@@ -335,7 +347,7 @@ icon_status icon_mask_create(int n, const float *tilts, int ntilt, float rate05,
     int dev = 0, optin = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    if (e == cudaSuccess && optin < 128 * 1024)
+    if (e == cudaSuccess && optin < 192 * 1024)
         return mask_fail(ICON_ERR_INVALID, "icon_mask_create: slice too large for shared memory");
     if (e == cudaSuccess) {
         if (n < 1024) e = mask_limits<4, 8, 16>(optin);
