@@ -1170,7 +1170,9 @@ static icon_status plan_create_impl(const icon_geometry *geo, int group, icon_pl
         if (e != cudaSuccess) return fail(ICON_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
         WITH_B(B, e = L::xtoep_prepare(p->n0))
         if (e != cudaSuccess) return fail(ICON_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
-        p->xt_ok = p->n0 >= 128 && p->n0 <= 8192 && (size_t)smem_max >= icon::xtoep_smem(p->n0, std::min(B, 8192 / p->n0));
+        p->xt_ok = p->n0 >= 128;
+        if (p->xt_ok && (size_t)smem_max < icon::xtoep_smem(p->n0, std::min(B, 8192 / p->n0)))
+            return fail(ICON_ERR_INVALID, "FFT buffer exceeds shared memory");
     }
     // Scratch for Gcap groups.
     size_t G = p->Gcap, Bz = B;

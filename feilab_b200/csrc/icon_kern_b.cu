@@ -14,18 +14,13 @@ template <int B>
 void Launch<B>::xpass_fwd(bool real_in, int E, dim3 grid, int threads, size_t smem, cudaStream_t st, const Geo &g,
                           const void *in, float2 *G1)
 {
-    if (real_in && g.n0 / 2 >= E) {   // half-length FFT per slice: half the threads and buffer
-        if (E == 32) pdl(k_xpass_fwd_r2c<B, 32>, grid, threads / 2, smem / 2, st, g, (const float *)in, G1);
-        else pdl(k_xpass_fwd_r2c<B, 16>, grid, threads / 2, smem / 2, st, g, (const float *)in, G1);
-        return;
-    }
-    if (E == 32) {
-        if (real_in) pdl(k_xpass_fwd<true, B, 32>, grid, threads, smem, st, g, in, G1);
-        else pdl(k_xpass_fwd<false, B, 32>, grid, threads, smem, st, g, in, G1);
-    } else {
-        if (real_in) pdl(k_xpass_fwd<true, B, 16>, grid, threads, smem, st, g, in, G1);
-        else pdl(k_xpass_fwd<false, B, 16>, grid, threads, smem, st, g, in, G1);
-    }
+    // n0 >= 128 is k_xtoep's and k_xtoep_real's (icon_api.cu: xt_ok); only the complex
+    // image of the measured Toeplitz iterations comes here with E = 32.
+    if (E == 32) pdl(k_xpass_fwd<false, B, 32>, grid, threads, smem, st, g, in, G1);
+    else if (real_in && g.n0 / 2 >= 16)   // half-length FFT per slice: half the threads and buffer
+        pdl(k_xpass_fwd_r2c<B, 16>, grid, threads / 2, smem / 2, st, g, (const float *)in, G1);
+    else if (real_in) pdl(k_xpass_fwd<true, B, 16>, grid, threads, smem, st, g, in, G1);
+    else pdl(k_xpass_fwd<false, B, 16>, grid, threads, smem, st, g, in, G1);
 }
 
 template <int B>
@@ -37,8 +32,7 @@ void Launch<B>::xpass_fwd_full(int E, dim3 grid, int threads, size_t smem, cudaS
         else pdl(k_xpass_fwd_r2c<B, 16, true>, grid, threads / 2, smem / 2, st, g, in, G1);
         return;
     }
-    if (E == 32) pdl(k_xpass_fwd<true, B, 32, true>, grid, threads, smem, st, g, in, G1);
-    else pdl(k_xpass_fwd<true, B, 16, true>, grid, threads, smem, st, g, in, G1);
+    pdl(k_xpass_fwd<true, B, 16, true>, grid, threads, smem, st, g, in, G1);   // n0 = 16
 }
 
 // The four-step register FFT (k_ytoep4) for n1 = 32 R, R in
@@ -246,8 +240,7 @@ void Launch<B>::xpass_adj(int mode, int E, dim3 grid, int threads, size_t smem, 
                           const float2 *G1, float2 *out, const float2 *Ahwb, double *part)
 {
     if (E == 32) {
-        if (mode == 0) pdl(k_xpass_adj<0, B, 32>, grid, threads, smem, st, g, G1, out, Ahwb, part);
-        else pdl(k_xpass_adj<1, B, 32>, grid, threads, smem, st, g, G1, out, Ahwb, part);
+        pdl(k_xpass_adj<1, B, 32>, grid, threads, smem, st, g, G1, out, Ahwb, part);   // mode 0: k_xtoep
     } else {
         if (mode == 0) pdl(k_xpass_adj<0, B, 16>, grid, threads, smem, st, g, G1, out, Ahwb, part);
         else pdl(k_xpass_adj<1, B, 16>, grid, threads, smem, st, g, G1, out, Ahwb, part);
@@ -355,12 +348,8 @@ cudaError_t Launch<B>::set_smem(int ex, int ey, int n1, int n1t)
         if (r != cudaSuccess && e == cudaSuccess) e = r;
     };
     if (ex == 32) {
-        set((const void *)k_xpass_fwd<true, B, 32>);
         set((const void *)k_xpass_fwd<false, B, 32>);
-        set((const void *)k_xpass_fwd_r2c<B, 32>);
         set((const void *)k_xpass_fwd_r2c<B, 32, true>);
-        set((const void *)k_xpass_fwd<true, B, 32, true>);
-        set((const void *)k_xpass_adj<0, B, 32>);
         set((const void *)k_xpass_adj<1, B, 32>);
         set((const void *)k_rows_fwd<B, 32>);
         set((const void *)k_row_adj<B, 32>);
