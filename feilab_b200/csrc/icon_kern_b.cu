@@ -182,10 +182,25 @@ cudaError_t Launch<B>::xtoep_prepare(int n0)
     }
 }
 
+// Threads of k_yfwd4, at least the FFT's R B.  What is left after the FFT are the
+// entries of a CTA, 850 or so where a real image's 61 tilts put two rows' on it,
+// and the FFT of few threads is a chain that only other CTAs on the SM cover.  So: few
+// CTAs take their entries by 256 threads (24 slices of 64 x 100 34 us the call, 51
+// with 128, 66 with 64), many by 128 (24 of 2048 x 40 422 us, 516 with 256, 488 with
+// 64); one row's entries (complex images) or a reprojection line's by 64 (lines of 8
+// slices of 4096 x 40 158 us the call, 170 and 261; 8 complex slices of 4096 x 100
+// 554, 607 and 844).
+static int yfwd_threads(int fft_threads, bool herm, dim3 grid, const Geo &g)
+{
+    const long long entries = (long long)g.M * (g.thi - g.tlo + 1) * 2;
+    const int want = !herm || entries < 64LL * g.n0 ? 64 : grid.x * grid.y <= 800 ? 256 : 128;
+    return fft_threads > want ? fft_threads : want;
+}
+
 template <int B, int R>
 static void yfwd4_go(bool herm, dim3 grid, cudaStream_t st, const Geo &g, const float2 *G1, float2 *P)
 {
-    const int threads = yfwd_threads(R * B, B);
+    const int threads = yfwd_threads(R * B, herm, grid, g);
     const size_t smem = yfwd4_smem(32 * R, B);
     if (herm) pdl(k_yfwd4<B, R, true>, grid, threads, smem, st, g, G1, P);
     else pdl(k_yfwd4<B, R, false>, grid, threads, smem, st, g, G1, P);

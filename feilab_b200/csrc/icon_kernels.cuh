@@ -1665,13 +1665,7 @@ __host__ __device__ inline bool ytoep4_fits(int n1) { return n1 % 32 == 0 && yto
 // rows a >= R/2 are zero going in and not needed coming out.
 __host__ __device__ constexpr bool yadj4_fits(int n1) { return n1 == 128 || n1 == 256 || n1 == 512 || n1 == 1024; }
 
-// Threads of the forward y-pass: the FFT's, at least four warps (entries are
-// spread over all; eight for the one- and two-slice groups of small calls).
-__host__ __device__ constexpr int yfwd_threads(int fft_threads, int B)
-{
-    const int least = B >= 4 ? 64 : 256;
-    return fft_threads < least ? least : fft_threads;
-}
+constexpr int kYfwdThreads = 256;   // of the forward y-pass at most (icon_kern_b.cu: yfwd_threads)
 __host__ __device__ constexpr size_t yfwd4_smem(int n1, int B)
 {
     return (size_t)(n1 + 2 * kHalo) * ((B == 8) ? 8 : (B == 4) ? 6 : B) * sizeof(float2) +
@@ -1679,7 +1673,7 @@ __host__ __device__ constexpr size_t yfwd4_smem(int n1, int B)
 }
 
 template <int B, int R, bool HERM>
-__global__ void __launch_bounds__(yfwd_threads(R * B, B), 512 / yfwd_threads(R * B, B))
+__global__ void __launch_bounds__(kYfwdThreads, 2)
     k_yfwd4(Geo g, const float2 *__restrict__ G1, float2 *__restrict__ P)
 {
     pdl_wait();
@@ -1688,7 +1682,8 @@ __global__ void __launch_bounds__(yfwd_threads(R * B, B), 512 / yfwd_threads(R *
     extern __shared__ float2 s[];
     const int grp = blockIdx.x, x = blockIdx.y, N1 = g.N1, h = N1 / 2;
     const int t = threadIdx.x, b = t & (B - 1), u = t >> LB;
-    const bool act = yfwd_threads(R * B, B) == R * B || t < R * B;
+    static_assert(R * B <= kYfwdThreads, "the FFT's threads");
+    const bool act = R * B == kYfwdThreads || t < R * B;
     const float2 *row = G1 + ((size_t)grp * g.n0 + x) * N1 * B;
     float2 *tws = s + (size_t)(n + 2 * kHalo) * SB;
     copy_async(tws, g.tw1, (size_t)n * sizeof(float2));
