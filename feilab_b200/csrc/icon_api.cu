@@ -643,7 +643,7 @@ icon_status launch_forward(icon_plan *p, const NodeTables &t, const void *img_in
     dim3 g3(kb, G);
     WITH_B(p->B,
         LAUNCH_B(p, K_FIN, st, (mode == 2 ? sb.fin_red : sb.fin_store) * slots,
-                 L::interp_fin(mode, g3, st, g, p->P, mode == 2 ? nullptr : f_out, mode == 2 ? p->part_rtar : nullptr)))
+                 L::interp_fin(mode, real_in, g3, st, g, p->P, mode == 2 ? nullptr : f_out, mode == 2 ? p->part_rtar : nullptr)))
     ICON_CUDA(cudaGetLastError());
     return ICON_OK;
 }

@@ -82,7 +82,17 @@ static void xt_go(int mode, cudaStream_t st, int G, const XtArgs &a)
     const dim3 grid((unsigned)(a.N1 * (B / BH)), (unsigned)G);
     const size_t smem = xtoep_smem(S::N, BH);
     if (mode == 0) pdl(k_xtoep<B, BH, LA, LNB, 0>, grid, S::T, smem, st, a);
-    else if (mode == 1) pdl(k_xtoep<B, BH, LA, LNB, 1>, grid, S::T, smem, st, a);
+    else if (mode == 1) {
+        // After a y-pass of many small blocks the early launch of fewer blocks than
+        // the SMs hold at once costs more than the gap that it saves (they seem to settle
+        // on the SMs that empty first): one slice, an iteration of 1024 x 300 57 us (80
+        // when early), 2048 x 100 54 (86), 4096 x 100 84 (103); four of 2048 x 40 51 (59). Above three fifths of what fits, and after
+        // y-passes of fewer blocks, the early launch is ahead by 1 to 3 us (8 slices of
+        // 1024 x 100 51 us, 53 without).
+        const int fit = 148 * (int)(227 * 1024 / (smem + 1024)), blocks = (int)(grid.x * grid.y);
+        const bool early = S::N * G < 2048 || 5 * blocks > 3 * fit;
+        pdl_if(early, k_xtoep<B, BH, LA, LNB, 1>, grid, S::T, smem, st, a);
+    }
     else pdl(k_xtoep<B, BH, LA, LNB, 2>, grid, S::T, smem, st, a);
 }
 template <int B, int BH, int LA, int LNB>
@@ -227,11 +237,17 @@ void Launch<B>::ypass_fwd(int E, bool herm, dim3 grid, int threads, size_t smem,
 }
 
 template <int B>
-void Launch<B>::interp_fin(int mode, dim3 grid, cudaStream_t st, const Geo &g, const float2 *P, float2 *f, double *part)
+void Launch<B>::interp_fin(int mode, bool herm, dim3 grid, cudaStream_t st, const Geo &g, const float2 *P, float2 *f,
+                           double *part)
 {
-    if (mode == 0) pdl(k_interp_fin<0, B>, grid, 256, 0, st, g, P, f, part);
-    else if (mode == 1) pdl(k_interp_fin<1, B>, grid, 256, 0, st, g, P, f, part);
-    else pdl(k_interp_fin<2, B>, grid, 256, 0, st, g, P, f, part);
+    // After the y-pass of a complex image, whose last rows are among its heaviest, the
+    // early launch costs more than the gap that it saves: 24 slices of 2048 x 40 462 us
+    // the call (526 when early), one of 1024 x 100 41 (56). Small calls keep it (64 x 40
+    // 21.4 us, 23.2 without).
+    const bool early = herm || g.n0 * (int)grid.y < 2048;
+    if (mode == 0) pdl_if(early, k_interp_fin<0, B>, grid, 256, 0, st, g, P, f, part);
+    else if (mode == 1) pdl_if(early, k_interp_fin<1, B>, grid, 256, 0, st, g, P, f, part);
+    else pdl_if(early, k_interp_fin<2, B>, grid, 256, 0, st, g, P, f, part);
 }
 
 template <int B>

@@ -27,7 +27,8 @@ struct Launch {
                                 const float2 *G1, double *part);
     static void ypass_fwd(int E, bool herm, dim3 grid, int threads, size_t smem, cudaStream_t st, const Geo &g, const float2 *G1,
                           float2 *P);
-    static void interp_fin(int mode, dim3 grid, cudaStream_t st, const Geo &g, const float2 *P, float2 *f, double *part);
+    // herm: after the y-pass of a real image.
+    static void interp_fin(int mode, bool herm, dim3 grid, cudaStream_t st, const Geo &g, const float2 *P, float2 *f, double *part);
     static void ypass_adj(int E, dim3 grid, int threads, size_t smem, cudaStream_t st, const Geo &g, const float2 *f,
                           float2 *G1);
     static void xpass_adj(int mode, int E, dim3 grid, int threads, size_t smem, cudaStream_t st, const Geo &g,

@@ -24,8 +24,9 @@ __device__ __forceinline__ void pdl_wait()
 // iterations with the NUFFT operator on 32 slices of 256 x 128 2.63 -> 2.47 ms,
 // warm-start predict of 8 slices of 1024 x 300 1.005 -> 0.978 ms, gradients of 16
 // slices of 512 x 256 3.47 -> 3.44 ms, mask of 16 slices of 1024 x 1024 202 -> 186 us.
+// early false: an ordinary launch, where measurement has the early one behind.
 template <class... P, class... A>
-inline void pdl(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A... args)
+inline void pdl_if(bool early, void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A... args)
 {
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -36,8 +37,13 @@ inline void pdl(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaS
     c.dynamicSmemBytes = smem;
     c.stream = st;
     c.attrs = &at;
-    c.numAttrs = 1;
+    c.numAttrs = early ? 1 : 0;
     cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+template <class... P, class... A>
+inline void pdl(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A... args)
+{
+    pdl_if(true, kernel, grid, threads, smem, st, args...);
 }
 
 }  // namespace icon
