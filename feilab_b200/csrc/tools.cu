@@ -33,7 +33,7 @@ struct PreFactors {
     double f[kPreMaxProjections];
 };
 
-// One cluster of kPreCluster CTAs per projection k of in[nz][ny][nx]
+// One cluster of RANKS CTAs per projection k of in[nz][ny][nx]
 // (ICONPreProcess.c:29-85):
 //   mode  = bin of the most pixels (first on ties) of a 256-bin histogram of
 //           the central region (10 % margins), bin index
@@ -51,10 +51,29 @@ struct PreFactors {
 // read L2, which holds the bands of the clusters in flight because a CTA's
 // shared memory lets one run per SM.  Extrema, bin counts and moments are
 // combined over the cluster through distributed shared memory in rank order.
-// 61 x 1024 x 1024: 398 us; with one CTA per projection, six passes and
-// divisions in double for every pixel 2374 us.  What is left is issue (about 60
-// instructions a pixel) and the last wave of clusters.
-constexpr int kPreCluster = 8;
+// The size of the clusters: one CTA runs per SM, so a call takes as many rounds as its
+// CTAs fill the SMs, and a round about 12 us plus 0.6 ns a pixel of a CTA's band
+// (one CTA: 61 x 1024 x 1024 in one round 634 us, 81 x 100 x 100 20). pre_ranks takes
+// the size of the least rounds x (20,000 + pixels of a band).  With clusters of 8
+// throughout many small projections were slower than with one CTA each: 200 of 2000 x
+// 30 129 -> 338 us, now 90; 41 of 128 x 128 28 -> 38, now 16; large ones gain from
+// fewer rounds: 61 x 1024 x 1024 398 -> 329 us (one CTA per projection, six passes and
+// divisions in double for every pixel 2374), 61 x 2048 x 2048 1590 -> 1228.
+constexpr int kPreMaxRanks = 8;
+inline int pre_ranks(long long size, int nz)
+{
+    long long best = 0;
+    int ranks = 1;
+    for (int r = 1; r <= kPreMaxRanks; r *= 2) {
+        const int places = 148 - 148 % r;                 // clusters of 8: 18
+        const long long cost = ((long long)nz * r + places - 1) / places * (20000 + size / r);
+        if (r == 1 || cost < best) {
+            best = cost;
+            ranks = r;
+        }
+    }
+    return ranks;
+}
 constexpr int kPreCache = 184 * 1024;   // shared memory for rows
 
 // Sum over the block of one double per thread (fixed order), to every thread.
@@ -72,8 +91,8 @@ __device__ double block_sum(double v, double *red)
 
 // VEC: rows are read and written as float4 (nx a multiple of 4, both stacks
 // on 16-byte boundaries).
-template <bool VEC>
-__global__ void __launch_bounds__(kPreThreads, 1) __cluster_dims__(kPreCluster, 1, 1)
+template <bool VEC, int RANKS>
+__global__ void __launch_bounds__(kPreThreads, 1) __cluster_dims__(RANKS, 1, 1)
     k_preprocess(const float *in, float *out, int nx, int ny, int normalize, int cache_rows,
                  const __grid_constant__ PreFactors factor)
 {
@@ -85,12 +104,12 @@ __global__ void __launch_bounds__(kPreThreads, 1) __cluster_dims__(kPreCluster, 
     __shared__ int hist[8][256];                     // warps w share copy w % 8
     __shared__ int bins[256];                        // this CTA's counts, read by the cluster
     __shared__ double mom[2], mode_s;                // this CTA's moments
-    const int k = blockIdx.x / kPreCluster, rank = (int)cl.block_rank();
+    const int k = blockIdx.x / RANKS, rank = (int)cl.block_rank();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, W = blockDim.x >> 5;
     const size_t size = (size_t)nx * ny;
     const float *p = in + (size_t)k * size;
     float *q = out + (size_t)k * size;
-    const int y0 = (int)((long long)ny * rank / kPreCluster), y1 = (int)((long long)ny * (rank + 1) / kPreCluster);
+    const int y0 = (int)((long long)ny * rank / RANKS), y1 = (int)((long long)ny * (rank + 1) / RANKS);
     const int xe = (int)(nx * 0.1), ye = (int)(ny * 0.1);
     const int xr = nx - xe, yr = ny - ye;            // core: xe <= x < xr, ye <= y < yr
     // Calls f(x, v) for the pixels x of row y that this lane takes.
@@ -145,7 +164,7 @@ __global__ void __launch_bounds__(kPreThreads, 1) __cluster_dims__(kPreCluster, 
     cl.sync();
     lo = cl.map_shared_rank(ext, 0)[0];
     hi = cl.map_shared_rank(ext, 0)[1];
-    for (int r = 1; r < kPreCluster; ++r) {
+    for (int r = 1; r < RANKS; ++r) {
         lo = fminf(lo, cl.map_shared_rank(ext, r)[0]);
         hi = fmaxf(hi, cl.map_shared_rank(ext, r)[1]);
     }
@@ -179,7 +198,7 @@ __global__ void __launch_bounds__(kPreThreads, 1) __cluster_dims__(kPreCluster, 
         // First bin with the largest count, over the cluster.
         if (threadIdx.x < 256) {
             int c = 0;
-            for (int r = 0; r < kPreCluster; ++r) c += cl.map_shared_rank(bins, r)[threadIdx.x];
+            for (int r = 0; r < RANKS; ++r) c += cl.map_shared_rank(bins, r)[threadIdx.x];
             hist[0][threadIdx.x] = c;
         }
         __syncthreads();
@@ -206,9 +225,12 @@ __global__ void __launch_bounds__(kPreThreads, 1) __cluster_dims__(kPreCluster, 
     const double f = normalize ? factor.f[k] : 0.0;
     double scale = 1.0;
     if (f > 0.0) {
-        // var = (sum v^2 - (sum v)^2 / size) / size in double.  (The mean of
-        // float quotients v / size that the reference subtracts is within
-        // 2^-24 of the mean, and moves the variance by the square of that.)
+        // var = (sum v^2 - (sum v)^2 / size) / size in double.  At least one pixel
+        // of the mode's bin lies within a bin of 0, so var is no less than about
+        // mean^2 / size and the difference keeps all but size 2^-53 of its digits
+        // (2e-9 for 4096 x 4096).  (The mean of float quotients v / size that the
+        // reference subtracts is within 2^-24 of the mean, and moves the variance by
+        // the square of that.)
         double s1 = 0.0, s2 = 0.0;
         for (int y = y0 + warp; y < y1; y += W)
             row(source(y), [&](int, float v0) {
@@ -224,7 +246,7 @@ __global__ void __launch_bounds__(kPreThreads, 1) __cluster_dims__(kPreCluster, 
         }
         cl.sync();
         s1 = s2 = 0.0;
-        for (int r = 0; r < kPreCluster; ++r) {
+        for (int r = 0; r < RANKS; ++r) {
             const double *m = cl.map_shared_rank(mom, r);
             s1 += m[0];
             s2 += m[1];
@@ -251,6 +273,19 @@ __global__ void __launch_bounds__(kPreThreads, 1) __cluster_dims__(kPreCluster, 
     cl.sync();   // no CTA leaves while another reads its shared memory
 }
 
+template <int RANKS>
+cudaError_t pre_launch(bool vec, const float *in, float *out, int nx, int ny, int nz, bool norm, const PreFactors &f,
+                       cudaStream_t st)
+{
+    const size_t row = sizeof(float) * (size_t)nx;
+    const int cache_rows = (int)std::min<size_t>(kPreCache / row, (size_t)(ny + RANKS - 1) / RANKS);
+    const auto kern = vec ? k_preprocess<true, RANKS> : k_preprocess<false, RANKS>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPreCache);
+    if (e != cudaSuccess) return e;
+    kern<<<nz * RANKS, kPreThreads, cache_rows * row, st>>>(in, out, nx, ny, norm ? 1 : 0, cache_rows, f);
+    return cudaGetLastError();
+}
+
 }  // namespace
 
 extern "C" {
@@ -273,13 +308,13 @@ icon_status icon_preprocess(const float *d_in, float *d_out, int nx, int ny, int
             if (!(f.f[k] > 0.0)) return tools_fail(ICON_ERR_INVALID, "icon_preprocess: tilt angle gives a non-positive variance");
         }
     }
-    const int cache_rows = (int)std::min<size_t>(kPreCache / (sizeof(float) * (size_t)nx), (size_t)ny);
     const bool vec = nx % 4 == 0 && ((uintptr_t)d_in & 15) == 0 && ((uintptr_t)d_out & 15) == 0;
-    const auto kern = vec ? k_preprocess<true> : k_preprocess<false>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPreCache);
-    if (e == cudaSuccess) {
-        kern<<<nz * kPreCluster, kPreThreads, kPreCache, st>>>(d_in, d_out, nx, ny, norm ? 1 : 0, cache_rows, f);
-        e = cudaGetLastError();
+    cudaError_t e = cudaSuccess;
+    switch (pre_ranks((long long)nx * ny, nz)) {
+    case 1: e = pre_launch<1>(vec, d_in, d_out, nx, ny, nz, norm, f, st); break;
+    case 2: e = pre_launch<2>(vec, d_in, d_out, nx, ny, nz, norm, f, st); break;
+    case 4: e = pre_launch<4>(vec, d_in, d_out, nx, ny, nz, norm, f, st); break;
+    default: e = pre_launch<8>(vec, d_in, d_out, nx, ny, nz, norm, f, st); break;
     }
     if (e != cudaSuccess) return tools_fail(ICON_ERR_CUDA, std::string("icon_preprocess: ") + cudaGetErrorString(e));
     return ICON_OK;
