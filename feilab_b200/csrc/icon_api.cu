@@ -743,7 +743,7 @@ icon_status ensure_toeplitz(icon_plan *p, cudaStream_t st)
     // tiles, first solve 11 ms; 34 ms in the three ranges that G1 holds); in plans of
     // a few slices, where it holds none, to a buffer made here once.
     const size_t plane = (size_t)p->n0 * p->n1t;
-    const int ctas = (int)(grid.x * grid.y), split = std::max(1, std::min({16, (296 + ctas - 1) / ctas, p->nx}));
+    const int ctas = (int)(grid.x * grid.y), split = std::max(1, std::min({16, (2 * icon::kSMs + ctas - 1) / ctas, p->nx}));
     const size_t set = split > 1 ? plane * split : 0;     // doubles
     size_t room = (size_t)p->Gcap * p->B * std::max((size_t)p->M * kTaps, (size_t)(p->n0 / 2 + 1) * p->N1);
     double *part = (double *)p->P;                         // float2 as doubles

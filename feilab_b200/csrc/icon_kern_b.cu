@@ -89,7 +89,7 @@ static void xt_go(int mode, cudaStream_t st, int G, const XtArgs &a)
         // when early), 2048 x 100 54 (86), 4096 x 100 84 (103); four of 2048 x 40 51 (59). Above three fifths of what fits, and after
         // y-passes of fewer blocks, the early launch is ahead by 1 to 3 us (8 slices of
         // 1024 x 100 51 us, 53 without).
-        const int fit = 148 * (int)(227 * 1024 / (smem + 1024)), blocks = (int)(grid.x * grid.y);
+        const int fit = kSMs * (int)(227 * 1024 / (smem + 1024)), blocks = (int)(grid.x * grid.y);
         const bool early = S::N * G < 2048 || 5 * blocks > 3 * fit;
         pdl_if(early, k_xtoep<B, BH, LA, LNB, 1>, grid, S::T, smem, st, a);
     }

@@ -1,9 +1,11 @@
 // pdl.cuh -- programmatic dependent launch: the launcher and the wait that belongs
-// to it.
+// to it; the number of SMs.
 #pragma once
 #include <cuda_runtime.h>
 
 namespace icon {
+
+constexpr int kSMs = 148;   // of a B200: the launch rules count in them
 
 // First statement of every kernel that is launched with programmatic dependent
 // launch: wait until the stream's previous kernel has completed and its writes

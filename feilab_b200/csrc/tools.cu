@@ -13,6 +13,7 @@
 
 #include "icon_b200.h"
 #include "icon_tools.h"
+#include "pdl.cuh"
 
 extern "C" void icon_internal_set_error(const char *msg);
 
@@ -65,7 +66,7 @@ inline int pre_ranks(long long size, int nz)
     long long best = 0;
     int ranks = 1;
     for (int r = 1; r <= kPreMaxRanks; r *= 2) {
-        const int places = 148 - 148 % r;                 // clusters of 8: 18
+        const int places = icon::kSMs / r * r;            // clusters of 8: 18
         const long long cost = ((long long)nz * r + places - 1) / places * (20000 + size / r);
         if (r == 1 || cost < best) {
             best = cost;

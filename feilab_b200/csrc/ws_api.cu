@@ -159,7 +159,7 @@ icon_status ws_conv3x3_launch(const void *in0, int cin0, const void *in1, int ci
             uint32_t cols = 32;
             while ((int)cols < th * N) cols <<= 1;
             const int per_sm = (int)std::min<size_t>(std::min<size_t>(226 * 1024 / (smem + 1024), 512 / cols), 8);
-            const unsigned grid = (unsigned)std::min<long long>(tiles, 148LL * per_sm);
+            const unsigned grid = (unsigned)std::min<long long>(tiles, (long long)icon::kSMs * per_sm);
             // No more of them on an SM than its TMEM holds at once.
             smem = std::max<size_t>(smem, 227 * 1024 / (per_sm + 1) - 896);
             const auto kern = th == 4 ? ws::k_conv3x3_halo<4> : ws::k_conv3x3_halo<2>;

@@ -606,7 +606,7 @@ __global__ void k_mse(const float *__restrict__ y, const float *__restrict__ t, 
 // warp and the block in fixed order.  (One pixel per thread, a 17-wide tree in
 // every block and 8192 partial sums: 50 + 462 us for 16 x 512 x 256 pixels;
 // 592 blocks: 25 + 5 us.)
-constexpr int kOutBlocks = 592;
+constexpr int kOutBlocks = 4 * icon::kSMs;
 
 __global__ void __launch_bounds__(256) k_conv_out_bwd(const __nv_bfloat16 *__restrict__ d, const float *__restrict__ dy,
                                                       const float *__restrict__ w, size_t npix,

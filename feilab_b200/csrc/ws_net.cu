@@ -104,7 +104,7 @@ struct WgPlan {
     int splits(int N, int Cin, long long rows) const
     {
         const int tiles = (N / co) * (Cin / ci);
-        return (int)std::max<long long>(1, std::min<long long>((444 + tiles - 1) / tiles, rows / 4));
+        return (int)std::max<long long>(1, std::min<long long>((3 * icon::kSMs + tiles - 1) / tiles, rows / 4));
     }
 };
 WgPlan wgrad_plan(int N, int cin0, int cin1)
@@ -135,7 +135,7 @@ cudaError_t wgrad_go(dim3 grid, cudaStream_t st, const __nv_bfloat16 *X0, int c0
 unsigned in_wgrad_blocks(int n, int H, int W)
 {
     const long long tiles = (long long)n * ((W + ws::kInCols - 1) / ws::kInCols) * ((H + ws::kInRows - 1) / ws::kInRows);
-    return (unsigned)std::min<long long>(tiles, 592);
+    return (unsigned)std::min<long long>(tiles, 4 * icon::kSMs);
 }
 
 struct Img {
@@ -273,7 +273,7 @@ struct icon_ws {
     {
         // Four outputs a thread where the parts stay aligned and that leaves a block
         // per SM; there the warps follow the parts, about eight a warp.
-        if (len % 4 == 0 && len >= 148 * 128) {
+        if (len % 4 == 0 && len >= icon::kSMs * 128) {
             int W = 4;
             while (W < ws::kSumWarps && W * 8 < n) W *= 2;
             icon::pdl(ws::k_sum_parts<4>, grid1(len, 128), 32 * W, 0, st, part, n, len, out);
