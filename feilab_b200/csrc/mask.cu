@@ -43,7 +43,7 @@ constexpr double kPi180 = 0.01745329252;   // MK:8
 // complex FFT, and a CTA transforms several pairs, or up to 8 neighbouring
 // columns, at once, so that every access is a run of whole sectors; the
 // columns' inverse stores the crop's rows only.  1024 x 1024, 16 slices, 300
-// rows kept: 188 us the call; one row or one 8-byte wide column per CTA over the
+// rows kept: 180 us the call; one row or one 8-byte wide column per CTA over the
 // full spectrum took 642 us.
 __host__ __device__ constexpr int mask_pitch(int n) { return n / 2 + 8; }
 
@@ -52,7 +52,7 @@ __host__ __device__ constexpr int mask_pitch(int n) { return n / 2 + 8; }
 // error, and with two rows in one transform the result was further from 64 bits
 // than with one (512 x 512: 5.3e-7 against 4.9e-7, now 2.5e-7; 1024 x 1024: 3.7e-7,
 // 3.1e-7, now 3.0e-7).  The columns' two transforms read a copy in shared memory
-// (16 slices of 1024: 188 us the call, 199 from global memory), the rows' one
+// (16 slices of 1024, 340 rows kept: 188 us the call, 199 from global memory), the rows' one
 // transform the table itself (198 us with a copy there too).
 
 // Rows 2B*blockIdx.x .. of a slice, in pairs (a, b) as a + i b:

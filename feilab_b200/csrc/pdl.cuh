@@ -22,7 +22,7 @@ __device__ __forceinline__ void pdl_wait()
 // resident while the stream's previous kernel drains, and wait (pdl_wait, first
 // thing in every kernel launched here) until that kernel has completed before
 // they touch data.  Taken where launches follow one another within microseconds to
-// tens of microseconds of work: one 64 x 40 slice forward 25.6 -> 19.9 us, 10
+// tens of microseconds of work (figures of its introduction): one 64 x 40 slice forward 25.6 -> 19.9 us, 10
 // iterations with the NUFFT operator on 32 slices of 256 x 128 2.63 -> 2.47 ms,
 // warm-start predict of 8 slices of 1024 x 300 1.005 -> 0.978 ms, gradients of 16
 // slices of 512 x 256 3.47 -> 3.44 ms, mask of 16 slices of 1024 x 1024 202 -> 186 us.

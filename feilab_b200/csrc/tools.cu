@@ -48,9 +48,8 @@ struct PreFactors {
 // The four passes over a projection (extrema, histogram, moments, result) are
 // bound by memory: 78 us for 61 projections of 1024 x 1024 read and written
 // once.  A CTA takes a band of whole rows and keeps the first of them in
-// shared memory (its only pass over DRAM fills them); the rest of the passes
-// read L2, which holds the bands of the clusters in flight because a CTA's
-// shared memory lets one run per SM.  Extrema, bin counts and moments are
+// shared memory (its first pass fills them); the rest of the passes read L2 as far
+// as it holds the bands in flight (one CTA runs per SM), and DRAM again beyond.  Extrema, bin counts and moments are
 // combined over the cluster through distributed shared memory in rank order.
 // The size of the clusters: one CTA runs per SM, so a call takes as many rounds as its
 // CTAs fill the SMs, and a round about 12 us plus 0.6 ns a pixel of a CTA's band
