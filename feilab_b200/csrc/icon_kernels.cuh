@@ -1302,17 +1302,27 @@ __global__ void __launch_bounds__(256, 1) k_toep_kernel(const double *__restrict
     for (int i = 0; i < 8; ++i)
 #pragma unroll
         for (int j = 0; j < 8; ++j) acc[i][j] = 0.0;
+    // Thread's part of the chunk from node q0 on, loaded a chunk ahead: value i of
+    // node q of the range; past its end the last node again (its factors are
+    // finite) at weight 0.
+    const int nr = t / kToepTrig, ni = t - nr * kToepTrig;
+    double nv = 0.0, nw = 0.0;
+    auto fetch = [&](int q0) {
+        if (t >= kToepNodes * kToepTrig) return;
+        const int q = min(q0 + nr, cnt - 1), tilt = q / len;
+        const size_t j = (size_t)tilt * nx + k_lo + (q - tilt * len);
+        nv = trig[j * kToepTrig + ni];
+        if (ni == 0) nw = q0 + nr < cnt ? (double)wg[j] : 0.0;
+    };
+    fetch(0);
     for (int q0 = 0; q0 < cnt; q0 += kToepNodes) {
         __syncthreads();                             // the previous chunk's tables are consumed
-        // Node q of the range; past its end the last node again (its factors are
-        // finite) at weight 0.
         if (t < kToepNodes * kToepTrig) {
-            const int r = t / kToepTrig, i = t - r * kToepTrig, q = min(q0 + r, cnt - 1), tilt = q / len;
-            const size_t j = (size_t)tilt * nx + k_lo + (q - tilt * len);
-            nd[r][i] = trig[j * kToepTrig + i];
-            if (i == 0) wn[r] = q0 + r < cnt ? (double)wg[j] : 0.0;
+            nd[nr][ni] = nv;
+            if (ni == 0) wn[nr] = nw;
         }
         __syncthreads();
+        fetch(q0 + kToepNodes);
 #pragma unroll
         for (int i = 0; i < kToepNodes / 2; ++i) {
             const int r = r0 + 2 * i;
