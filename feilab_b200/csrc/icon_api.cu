@@ -740,7 +740,7 @@ icon_status ensure_toeplitz(icon_plan *p, cudaStream_t st)
     // alone (k_toep_kernel's order of summation).  Their sums go to P, which
     // like G1 no one reads before the next transform writes it, as many
     // weight sets at a time as it holds (7 slices of 1239 x 52 with 76 tilts: 32
-    // tiles, first solve 11 ms; 34 ms in the three ranges that G1 holds); in plans of
+    // tiles, 10 ms before the first solve; 34 ms in the three ranges that G1 holds); in plans of
     // a few slices, where it holds none, to a buffer made here once.
     const size_t plane = (size_t)p->n0 * p->n1t;
     const int ctas = (int)(grid.x * grid.y), split = std::max(1, std::min({16, (2 * icon::kSMs + ctas - 1) / ctas, p->nx}));
